@@ -89,6 +89,7 @@ struct KParams {
     float* y;
     i64 ldx, ldy;
     i32 f;
+    i32 y_vec;       // rows of y are 16-byte aligned
     i32 slab_w;      // columns per slab
     i32 n_items;     // work items per slab
     i32 n_prefix;    // items that never wait (claimed `group` at a time)
@@ -219,6 +220,29 @@ struct Vec<true> {
         a.w = fmaxf(a.w, 0.f);
         return a;
     }
+    static __device__ __forceinline__ T add_xor(T a, int d) {
+        a.x += __shfl_xor_sync(0xffffffffu, a.x, d);
+        a.y += __shfl_xor_sync(0xffffffffu, a.y, d);
+        a.z += __shfl_xor_sync(0xffffffffu, a.z, d);
+        a.w += __shfl_xor_sync(0xffffffffu, a.w, d);
+        return a;
+    }
+    // Rows whose vectors are not 16-byte aligned, or a vector that reaches past the row's end: the
+    // `n` columns that exist, one by one.
+    static __device__ __forceinline__ void st_some(float* p, T v, int n) {
+        if (n > 0) p[0] = v.x;
+        if (n > 1) p[1] = v.y;
+        if (n > 2) p[2] = v.z;
+        if (n > 3) p[3] = v.w;
+    }
+    static __device__ __forceinline__ T ld_some_l2(const float* p, int n) {
+        T v = zero();
+        if (n > 0) v.x = __ldcg(p);
+        if (n > 1) v.y = __ldcg(p + 1);
+        if (n > 2) v.z = __ldcg(p + 2);
+        if (n > 3) v.w = __ldcg(p + 3);
+        return v;
+    }
 };
 template <>
 struct Vec<false> {
@@ -255,6 +279,11 @@ struct Vec<false> {
     static __device__ __forceinline__ T fma(float w, T a, T c) { return fmaf(w, a, c); }
     static __device__ __forceinline__ T mul(float w, T a) { return w * a; }
     static __device__ __forceinline__ T relu(T a) { return fmaxf(a, 0.f); }
+    static __device__ __forceinline__ T add_xor(T a, int d) { return a + __shfl_xor_sync(0xffffffffu, a, d); }
+    static __device__ __forceinline__ void st_some(float* p, T v, int n) {
+        if (n > 0) *p = v;
+    }
+    static __device__ __forceinline__ T ld_some_l2(const float* p, int n) { return n > 0 ? __ldcg(p) : 0.f; }
 };
 
 // acc[v] += sum over entries [beg,end) of val * X[col, slab columns of this lane].
@@ -318,18 +347,17 @@ __device__ __forceinline__ void gather_row(const i32* __restrict__ col,
     }
 }
 
-// The same sum for slabs of at most 64 columns (128-bit path): a row piece needs only 16 lanes, so
-// the two half-warps fetch two different delta entries at a time and their partial sums are
-// combined with one shuffle at the end.  Every lane ends up holding the total of its column group.
-template <int UNROLL>
-__device__ __forceinline__ void gather_row_half(const i32* __restrict__ col,
-                                                const float* __restrict__ val, i32 beg, i32 end,
-                                                const float* __restrict__ x_slab, i64 ldx, i32 wcols,
-                                                float4& acc, int lane) {
-    using V = Vec<true>;
-    const int li = lane & 15, half = lane >> 4;
-    const bool okh = li * 4 < wcols;
-    const float* xs = x_slab + li * 4;
+// The same sum for slabs that 2^lg < 32 lanes cover with one vector each: 32 >> lg delta entries are fetched side by
+// side, one per group of lanes, and the groups' sums are combined by shuffles at the end, so that every lane
+// holds the total of its column group.
+template <bool V4, int UNROLL>
+__device__ __forceinline__ void gather_row_narrow(const i32* __restrict__ col, const float* __restrict__ val, i32 beg,
+                                                  i32 end, const float* __restrict__ x_slab, i64 ldx, i32 wcols,
+                                                  int lg, typename Vec<V4>::T& acc, int lane) {
+    using V = Vec<V4>;
+    const int li = lane & ((1 << lg) - 1), group = lane >> lg, side = 32 >> lg;
+    const bool okh = li * V::E < wcols;
+    const float* xs = x_slab + li * V::E;
     for (i32 b = beg; b < end; b += 32) {
         const i32 n_here = min(32, end - b);
         i32 mc = 0;
@@ -338,26 +366,30 @@ __device__ __forceinline__ void gather_row_half(const i32* __restrict__ col,
             mc = __ldg(col + b + lane);
             mw = __ldg(val + b + lane);
         }
-        for (i32 j = 0; j < n_here; j += 2 * UNROLL) {
-            float4 t[UNROLL];
+        for (i32 j = 0; j < n_here; j += side * UNROLL) {
+            typename V::T t[UNROLL];
 #pragma unroll
             for (int k = 0; k < UNROLL; ++k) {
-                const i32 idx = j + 2 * k + half;
+                const i32 idx = j + k * side + group;
                 const i32 c = __shfl_sync(0xffffffffu, mc, idx & 31);
                 t[k] = V::ld_ro_if(xs + (i64)c * ldx, okh && idx < n_here);
             }
 #pragma unroll
             for (int k = 0; k < UNROLL; ++k) {
-                const i32 idx = j + 2 * k + half;
+                const i32 idx = j + k * side + group;
                 const float w = __shfl_sync(0xffffffffu, mw, idx & 31);
                 acc = V::fma(idx < n_here ? w : 0.f, t[k], acc);
             }
         }
     }
-    acc.x += __shfl_xor_sync(0xffffffffu, acc.x, 16);
-    acc.y += __shfl_xor_sync(0xffffffffu, acc.y, 16);
-    acc.z += __shfl_xor_sync(0xffffffffu, acc.z, 16);
-    acc.w += __shfl_xor_sync(0xffffffffu, acc.w, 16);
+    for (int d = 1 << lg; d < 32; d <<= 1) acc = V::add_xor(acc, d);
+}
+
+// Lanes (as a power of two) that cover `wcols` columns with one vector of E floats each.
+template <int E>
+__device__ __forceinline__ int lanes_log2(i32 wcols) {
+    const i32 lanes = (wcols + E - 1) / E;
+    return lanes <= 1 ? 0 : 32 - __clz(lanes - 1);
 }
 
 // A warp signs off; the last one out rewinds both counters for the next launch.  This holds on
@@ -392,7 +424,7 @@ __device__ __forceinline__ void decode_claim(const KParams& p, u64 t, i32& slab,
 // Everything that happens to an item once its own gather is in `acc`: park a PARTIAL share, or
 // collect the row's parked shares, add the parent's finished row, scale, store and publish.
 // Returns false when a bounded wait ran out.
-template <int NV, bool V4>
+template <int NV, bool V4, bool RAGGED = false>
 __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos, i32 out_row,
                                             i32 parent_row, i32 parent_pos, i32 info,
                                             i32 first_part, float scale, float inv_parent,
@@ -440,6 +472,10 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
         }
     }
     const i32 lane_col = c0 + lane * V::E;
+    // RAGGED: rows of y that are not 16-byte aligned, or a last vector that reaches past column f; the columns
+    // of vector v that exist are then accessed one by one
+    auto some = [&](int v) { return p.f - (lane_col + v * STEP); };
+    auto whole = [&](int v) { return !RAGGED || (p.y_vec && some(v) >= V::E); };
     if (p.mode != MODE_DELTA_ONLY) {
         if (parent_row >= 0) {
             if (!wait_ready(slab_flags + parent_pos, p.epoch, p.status, p.wait_ns)) return false;
@@ -447,7 +483,9 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
             const float ip = p.use_scale ? inv_parent : 1.0f;
 #pragma unroll
             for (int v = 0; v < NV; ++v)
-                if (ok[v]) acc[v] = V::fma(ip, V::ld_l2(prow + v * STEP), acc[v]);
+                if (ok[v])
+                    acc[v] = V::fma(ip, whole(v) ? V::ld_l2(prow + v * STEP) : V::ld_some_l2(prow + v * STEP, some(v)),
+                                    acc[v]);
         }
         if (p.use_scale) {
 #pragma unroll
@@ -458,13 +496,19 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
     if (info & ITEM_PUBLISH) {
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-            if (ok[v]) V::st(yrow + v * STEP, acc[v]);
+            if (ok[v]) {
+                if (whole(v)) V::st(yrow + v * STEP, acc[v]);
+                else V::st_some(yrow + v * STEP, acc[v], some(v));
+            }
     } else {
         // nobody reads this row again during the product: a streaming store keeps it from
         // pushing slabs of X out of L2
 #pragma unroll
         for (int v = 0; v < NV; ++v)
-            if (ok[v]) V::st_stream(yrow + v * STEP, acc[v]);
+            if (ok[v]) {
+                if (whole(v)) V::st_stream(yrow + v * STEP, acc[v]);
+                else V::st_some(yrow + v * STEP, acc[v], some(v));
+            }
     }
     if ((info & ITEM_PUBLISH) && p.mode != MODE_DELTA_ONLY) {
         __syncwarp();
@@ -480,7 +524,10 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
             float* dst = p.bcast[k] + off;
 #pragma unroll
             for (int v = 0; v < NV; ++v)
-                if (ok[v]) V::st(dst + v * STEP, acc[v]);
+                if (ok[v]) {
+                    if (whole(v)) V::st(dst + v * STEP, acc[v]);
+                    else V::st_some(dst + v * STEP, acc[v], some(v));
+                }
         }
     }
     return true;
@@ -491,7 +538,7 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
 // pointers) and the update-only mode, which gathers nothing; it is also the default form.
 // UNROLL = row fetches in flight per lane, MINB = thread blocks the register budget must allow
 // per SM.
-template <int NV, bool V4, int UNROLL, int MINB>
+template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false>
 __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
     using V = Vec<V4>;
     using T = typename V::T;
@@ -521,15 +568,16 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
             if (p.mode == MODE_UPDATE_ONLY) {
                 const float* yrow = p.y + (i64)da.x * p.ldy + c0 + lane * V::E;
 #pragma unroll
-                for (int v = 0; v < NV; ++v) acc[v] = ok[v] ? V::ld_l2(yrow + v * STEP) : V::zero();
+                for (int v = 0; v < NV; ++v) acc[v] = ok[v] ? V::ld_l2(yrow + v * STEP) : V::zero();  // (y_vec here)
             } else {
 #pragma unroll
                 for (int v = 0; v < NV; ++v) acc[v] = V::zero();
                 const i32 len = (info >> ITEM_LEN_SHIFT) & 0xff;
-                if constexpr (V4 && NV == 1) {
-                    if (wcols <= 64)
-                        gather_row_half<UNROLL>(p.col, p.val, db.x, db.x + len, p.x + c0, p.ldx, wcols, acc[0], lane);
-                    else if (wcols == 128)  // a complete slab: no per-lane predicate on the fetches
+                if constexpr (NV == 1) {
+                    if (wcols <= 16 * V::E)
+                        gather_row_narrow<V4, UNROLL>(p.col, p.val, db.x, db.x + len, p.x + c0, p.ldx, wcols,
+                                                      lanes_log2<V::E>(wcols), acc[0], lane);
+                    else if (V4 && wcols == 128)  // a complete slab: no per-lane predicate on the fetches
                         gather_row<NV, V4, UNROLL, true>(p.col, p.val, db.x, db.x + len, p.x + c0 + lane * V::E,
                                                          p.ldx, ok, acc, lane);
                     else
@@ -540,8 +588,8 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
                                                ok, acc, lane);
                 }
             }
-            if (!finish_item<NV, V4>(p, slab, pos, da.x, da.y, da.z, info, db.y, __int_as_float(db.z),
-                                     __int_as_float(db.w), acc, ok, c0, lane)) {
+            if (!finish_item<NV, V4, RAGGED>(p, slab, pos, da.x, da.y, da.z, info, db.y, __int_as_float(db.z),
+                                             __int_as_float(db.w), acc, ok, c0, lane)) {
                 leave(p, lane);
                 return;
             }
@@ -879,6 +927,8 @@ struct cbm_b200_plan {
     RowDesc* d_desc = nullptr;
     i32* d_col = nullptr;
     float* d_val = nullptr;
+    float* d_pack = nullptr;     // the operand copied to 16-byte aligned rows (when the caller's are not)
+    i64 pack_cap = 0;
     i32* d_flags = nullptr;
     i64 flags_cap = 0;
     u64* d_counter = nullptr;
@@ -931,6 +981,7 @@ extern "C" void cbm_b200_plan_destroy(cbm_b200_plan* p) {
     cudaFree(p->d_desc);
     cudaFree(p->d_col);
     cudaFree(p->d_val);
+    cudaFree(p->d_pack);
     cudaFree(p->d_flags);
     cudaFree(p->d_scratch);
     cudaFree(p->d_counter);
@@ -1350,14 +1401,23 @@ struct LaunchCfg {
     i64 n_claims = 0;
     i64 need_flags = 0;        // int32 words
     i64 need_scratch = 0;      // floats
+    bool pack = false;         // the operand is first copied to 16-byte aligned rows
+    bool ragged = false;       // 16-byte fetches, but rows of y are not aligned or end inside a vector
 };
 
 int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
-             i32 f, int mode, LaunchCfg& c) {
-    const bool can_v4 = (f % 4 == 0) && (ldy % 4 == 0) && aligned16(y) &&
-                        (mode == MODE_UPDATE_ONLY || ((ldx % 4 == 0) && aligned16(x)));
+             i32 f, int mode, bool may_pack, LaunchCfg& c) {
+    const bool y_vec = ldy % 4 == 0 && aligned16(y);
+    const bool x_vec = ldx % 4 == 0 && aligned16(x);
+    // An operand whose rows are not 16-byte aligned can only be fetched 4 bytes a lane, at less than half
+    // the rate.  Copying it to aligned rows first costs one pass over it, so it pays when every operand row
+    // is fetched several times and the product is more than a launch (2 M multiply-adds, a few us).
+    c.pack = may_pack && mode != MODE_UPDATE_ONLY && !x_vec && f > 4 && p->n_delta >= 4 * (i64)p->n_labels &&
+             p->n_delta * f >= (i64)1 << 21;
+    const bool can_v4 = mode == MODE_UPDATE_ONLY ? y_vec : x_vec || c.pack;
+    c.ragged = can_v4 && (!y_vec || f % 4 != 0);
     int tma = p->form;
-    if (!can_v4 || mode == MODE_UPDATE_ONLY) tma = 0;
+    if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY) tma = 0;
     c.tma = tma;
     if (tma) {
         const i32 slab = 256;  // 1 KB row pieces: the copy engine is bound by copies, not bytes
@@ -1403,7 +1463,7 @@ int launch_tma(KParams& kp, int sm_count, cudaStream_t s) {
     return CBM_B200_OK;
 }
 
-template <int NV, bool V4>
+template <int NV, bool V4, bool RAGGED = false>
 int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
     // Unroll depth and resident blocks per SM were chosen by measurement on B200.  For the default
     // form (one float4 per lane, 128-column slabs) 4 gathers in flight per warp at 48 resident
@@ -1411,13 +1471,30 @@ int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
     // operands and tie on narrow ones; forms that spill registers lose more than extra resident
     // warps gain.
     constexpr int kUnroll = NV == 1 ? (V4 ? 4 : 8) : 4;
-    constexpr int kResident = NV == 1 ? (V4 ? 6 : 4) : (NV == 2 ? 3 : 2);
+    constexpr int kResident = NV == 1 ? (V4 ? (RAGGED ? 5 : 6) : 4) : (NV == 2 ? 3 : 2);
     int blocks = want_blocks > 0 ? want_blocks : sm_count * (NV == 1 && V4 ? kResident : 8);
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
-    cbm_items_kernel<NV, V4, kUnroll, kResident><<<blocks, 256, 0, s>>>(kp);
+    cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED><<<blocks, 256, 0, s>>>(kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;
+}
+
+// Rows of `f` floats copied to rows of 4 * vecs floats, zero-filled: one thread per vector of the result, the
+// source read 4 bytes at a time (its rows are not aligned).  Bound by HBM.
+__global__ void __launch_bounds__(256) pack_rows_kernel(const float* __restrict__ x, i64 ldx, float* __restrict__ out,
+                                                        i32 f, i32 vecs, i64 n_vec) {
+    const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n_vec) return;
+    const i64 row = i / vecs;
+    const i32 c = (i32)(i - row * vecs) * 4;
+    const float* r = x + row * ldx + c;
+    float4 v;
+    v.x = __ldg(r);
+    v.y = c + 1 < f ? __ldg(r + 1) : 0.f;
+    v.z = c + 2 < f ? __ldg(r + 2) : 0.f;
+    v.w = c + 3 < f ? __ldg(r + 3) : 0.f;
+    reinterpret_cast<float4*>(out)[i] = v;
 }
 
 // Fills the launch parameters that do not depend on where the scratch lives, and launches.
@@ -1431,7 +1508,9 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
                 int mode, bool use_scale, u64* counter, i32* flags, float* scratch, i32 epoch,
                 cudaStream_t s, const Bcast* bc = nullptr) {
     KParams kp{};
+    kp.y_vec = ldy % 4 == 0 && aligned16(y);
     if (bc) {
+        for (int k = 0; k < bc->n; ++k) kp.y_vec = kp.y_vec && aligned16(bc->dst[k]);
         kp.n_bcast = bc->n;
         kp.bcast_relu = bc->relu;
         for (int k = 0; k < bc->n; ++k) kp.bcast[k] = bc->dst[k];
@@ -1461,6 +1540,11 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.use_scale = use_scale ? 1 : 0;
     kp.wait_ns = 2000000000ULL;
     if (c.tma) return launch_tma<256, 16, 2, 7>(kp, p->sm_count, s);
+    if (c.ragged) {
+        if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, p->n_blocks, p->sm_count, s);
+        return launch_regs<4, true, true>(kp, p->n_blocks, p->sm_count, s);
+    }
     if (c.sh.v4) {
         if (c.sh.nv == 1) return launch_regs<1, true>(kp, p->n_blocks, p->sm_count, s);
         if (c.sh.nv == 2) return launch_regs<2, true>(kp, p->n_blocks, p->sm_count, s);
@@ -1484,7 +1568,7 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (p->n_rows == 0) return CBM_B200_OK;
     DeviceGuard g(p->device);
     LaunchCfg c;
-    rc = plan_cfg(p, who, x, ldx, y, ldy, f, mode, c);
+    rc = plan_cfg(p, who, x, ldx, y, ldy, f, mode, true, c);
     if (rc) return rc;
 
     if (c.need_flags > p->flags_cap) {
@@ -1512,6 +1596,24 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (p->epoch == INT32_MAX) {  // epochs exhausted: start over on clean flags
         CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)p->flags_cap * sizeof(i32), s));
         p->epoch = 0;
+    }
+    if (c.pack) {
+        const i32 vecs = (f + 3) / 4;
+        const i64 n_vec = (i64)p->n_labels * vecs;
+        if (4 * n_vec > p->pack_cap) {
+            CBM_CUDA(cudaStreamSynchronize(s));
+            cudaFree(p->d_pack);
+            p->d_pack = nullptr;
+            p->device_bytes -= p->pack_cap * (i64)sizeof(float);
+            p->pack_cap = 0;
+            CBM_CUDA(cudaMalloc((void**)&p->d_pack, (size_t)n_vec * 16));
+            p->pack_cap = 4 * n_vec;
+            p->device_bytes += p->pack_cap * (i64)sizeof(float);
+        }
+        pack_rows_kernel<<<(unsigned)((n_vec + 255) / 256), 256, 0, s>>>(x, ldx, p->d_pack, f, vecs, n_vec);
+        CBM_CUDA(cudaGetLastError());
+        x = p->d_pack;
+        ldx = 4 * (i64)vecs;
     }
     return launch_plan(p, c, x, ldx, y, ldy, f, mode, use_scale, p->d_counter, p->d_flags, p->d_scratch,
                        ++p->epoch, s, bc);
@@ -1833,7 +1935,7 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     if (p->n_rows == 0) return CBM_B200_OK;
 
     LaunchCfg c;
-    rc = plan_cfg(p, who, x, ldx, y, ldy, f, MODE_FUSED, c);
+    rc = plan_cfg(p, who, x, ldx, y, ldy, f, MODE_FUSED, false, c);
     if (rc) return rc;
     // layout inside the fixed array: counters | ready flags | partial sums
     const i64 off_flags = 256;

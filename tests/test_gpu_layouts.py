@@ -1,0 +1,47 @@
+"""Operand layouts and widths at which the product kernels change form: row groups of 1 - 16 lanes, the last
+partial vector of a row, operands that are copied to aligned rows first, results whose rows are not aligned."""
+import numpy as np
+import pytest
+import torch
+
+from cbm4gnn_b200 import graphs
+from cbm4gnn_b200.cbm import cbm_matrix
+from helpers import sparse_product, with_self_loops
+
+pytestmark = pytest.mark.gpu
+TOL = dict(atol=1e-4, rtol=1e-4)
+
+
+@pytest.fixture(scope="module")
+def copy_graph():
+    ei = with_self_loops(graphs.copy_model(3000, 0.9, 8, 11))
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
+    assert (np.diff(c._crow) > 192).any() and c.build_info["depth"] > 2  # split rows and waiting rows
+    return ei, c
+
+
+def _buffer(rows, width, pitch):
+    return torch.full((rows, pitch), 7.0, device="cuda")[:, :width]
+
+
+@pytest.mark.parametrize("f", [1, 3, 4, 5, 8, 9, 16, 17, 31, 33, 47, 64, 65, 100, 127, 129, 131, 257])
+@pytest.mark.parametrize("aligned_x,aligned_y", [(True, True), (True, False), (False, True), (False, False)])
+def test_widths_and_pitches(copy_graph, f, aligned_x, aligned_y):
+    ei, c = copy_graph
+    x = np.random.default_rng(f).standard_normal((c.num_rows, f)).astype(np.float32)
+    up = -(-f // 4) * 4
+    xd = _buffer(c.num_rows, f, up if aligned_x else up + 1)
+    yd = _buffer(c.num_rows, f, up if aligned_y else up + 1)
+    xd.copy_(torch.from_numpy(x))
+    want = sparse_product(ei, x, True)
+    c.omp_mkl_csr_fused_spmm_update(xd, yd)
+    c.plan(0).status()
+    np.testing.assert_allclose(yd.cpu().numpy(), want, **TOL)
+    if up != f or not aligned_y:  # nothing is written beside the result's columns
+        pad = yd.as_strided((c.num_rows, yd.stride(0) - f), (yd.stride(0), 1), f)
+        assert torch.equal(pad, torch.full_like(pad, 7.0))
+    two = torch.full_like(yd, 7.0)
+    c.seq_mkl_csr_spmm(xd, two)
+    c.seq_mkl_csr_fused_update(two)
+    np.testing.assert_allclose(two.cpu().numpy(), want, **TOL)
+    torch.testing.assert_close(c.seq_torch_csr_fused_matmul(xd), yd, atol=0, rtol=1e-6)
