@@ -25,11 +25,14 @@ SOURCES = [
     os.path.join(_PKG_DIR, "csrc", "cbm_dense.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_dense_grad.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.cu"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_cluster.cu"),
 ]
 HEADERS = [
     os.path.join(_ROOT, "include", "cbm_b200.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_common.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.h"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_chunks.cuh"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_cluster.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_dense_gemm.cuh"),
 ]
 _OBJ_DIR = os.path.join(_PKG_DIR, "build")

@@ -28,6 +28,7 @@
 #include <vector>
 
 #include "cbm_b200.h"
+#include "cbm_cluster.h"
 #include "cbm_common.h"
 
 namespace cbm {
@@ -79,17 +80,33 @@ struct __align__(16) RowDesc {
 };
 enum : int { ITEM_PUBLISH = 1, ITEM_PARTIAL = 2, ITEM_LEN_SHIFT = 8, ITEM_NPART_SHIFT = 16 };
 
+// A delta entry: the column and the value to multiply it with.
+struct __align__(8) Entry {
+    i32 col;
+    float val;
+};
+
+// Clustered plans (see cbm_chunks.cuh): a run of consecutive items that a block brings into shared memory
+// together.  There every item's first entry stands at an even position.
+struct __align__(16) Chunk {
+    i32 first, count;  // items
+    i32 e0, ne;        // their entries, both even
+};
+
 enum Mode : int { MODE_FUSED = 0, MODE_DELTA_ONLY = 1, MODE_UPDATE_ONLY = 2 };
 
 struct KParams {
     const RowDesc* desc;
-    const i32* col;
-    const float* val;
+    const Entry* ent;
     const float* x;
     float* y;
     i64 ldx, ldy;
     i32 f;
     i32 y_vec;       // rows of y are 16-byte aligned
+    const Chunk* chunks;   // clustered plans: chunks, ...
+    unsigned ldx_bytes;    // ... 4 * ldx,
+    i32 run;               // ... chunks claimed `run` at a time below chunk n_run, one at a time from there on
+    i32 n_run;
     i32 slab_w;      // columns per slab
     i32 n_items;     // work items per slab
     i32 n_prefix;    // items that never wait (claimed `group` at a time)
@@ -100,7 +117,7 @@ struct KParams {
     float* scratch;  // n_slabs * n_partial * slab_w floats: partial sums of long rows
     i32 n_partial;   // PARTIAL items (positions [0, n_partial))
     u64* counter;    // [0] next claim, [1] warps that have left; both 0 between launches
-    u64 n_warps;     // warps in this launch
+    u64 n_warps;     // claimers in this launch: warps, or the blocks of a clustered plan's kernel
     i32* flags;      // n_slabs * n_items ready flags holding the epoch of the launch that set them
     i32 epoch;
     i32* status;     // 0 ok; non-zero: a wait gave up
@@ -286,13 +303,30 @@ struct Vec<false> {
     static __device__ __forceinline__ T ld_some_l2(const float* p, int n) { return n > 0 ? __ldcg(p) : 0.f; }
 };
 
+// Where the entries of a row come from: a plan's array of pairs, or a caller's two CSR arrays.
+struct PairEntries {
+    const Entry* e;
+    __device__ __forceinline__ void get(i32 i, i32& c, float& w) const {
+        const int2 q = __ldg(reinterpret_cast<const int2*>(e) + i);
+        c = q.x;
+        w = __int_as_float(q.y);
+    }
+};
+struct CsrEntries {
+    const i32* __restrict__ col;
+    const float* __restrict__ val;
+    __device__ __forceinline__ void get(i32 i, i32& c, float& w) const {
+        c = __ldg(col + i);
+        w = __ldg(val + i);
+    }
+};
+
 // acc[v] += sum over entries [beg,end) of val * X[col, slab columns of this lane].
 // The 32 lanes fetch 32 (col, val) pairs at once and pass them round by shuffle.  Row fetches are
 // issued UNROLL at a time so that several independent loads per lane are in flight; the weights
 // are picked up after the fetches have been issued.
-template <int NV, bool V4, int UNROLL, bool FULL = false>
-__device__ __forceinline__ void gather_row(const i32* __restrict__ col,
-                                           const float* __restrict__ val, i32 beg, i32 end,
+template <int NV, bool V4, int UNROLL, bool FULL = false, class Entries>
+__device__ __forceinline__ void gather_row(const Entries ent, i32 beg, i32 end,
                                            const float* __restrict__ xs, i64 ldx,
                                            const bool (&ok)[NV], typename Vec<V4>::T (&acc)[NV],
                                            int lane) {
@@ -303,10 +337,7 @@ __device__ __forceinline__ void gather_row(const i32* __restrict__ col,
         const i32 n_here = min(32, end - b);
         i32 mc = 0;
         float mw = 0.f;
-        if (lane < n_here) {
-            mc = __ldg(col + b + lane);
-            mw = __ldg(val + b + lane);
-        }
+        if (lane < n_here) ent.get(b + lane, mc, mw);
         i32 j = 0;
         for (; j + UNROLL <= n_here; j += UNROLL) {
             T t[UNROLL][NV];
@@ -350,10 +381,9 @@ __device__ __forceinline__ void gather_row(const i32* __restrict__ col,
 // The same sum for slabs that 2^lg < 32 lanes cover with one vector each: 32 >> lg delta entries are fetched side by
 // side, one per group of lanes, and the groups' sums are combined by shuffles at the end, so that every lane
 // holds the total of its column group.
-template <bool V4, int UNROLL>
-__device__ __forceinline__ void gather_row_narrow(const i32* __restrict__ col, const float* __restrict__ val, i32 beg,
-                                                  i32 end, const float* __restrict__ x_slab, i64 ldx, i32 wcols,
-                                                  int lg, typename Vec<V4>::T& acc, int lane) {
+template <bool V4, int UNROLL, class Entries>
+__device__ __forceinline__ void gather_row_narrow(const Entries ent, i32 beg, i32 end, const float* __restrict__ x_slab,
+                                                  i64 ldx, i32 wcols, int lg, typename Vec<V4>::T& acc, int lane) {
     using V = Vec<V4>;
     const int li = lane & ((1 << lg) - 1), group = lane >> lg, side = 32 >> lg;
     const bool okh = li * V::E < wcols;
@@ -362,10 +392,7 @@ __device__ __forceinline__ void gather_row_narrow(const i32* __restrict__ col, c
         const i32 n_here = min(32, end - b);
         i32 mc = 0;
         float mw = 0.f;
-        if (lane < n_here) {
-            mc = __ldg(col + b + lane);
-            mw = __ldg(val + b + lane);
-        }
+        if (lane < n_here) ent.get(b + lane, mc, mw);
         for (i32 j = 0; j < n_here; j += side * UNROLL) {
             typename V::T t[UNROLL];
 #pragma unroll
@@ -575,16 +602,16 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
                 const i32 len = (info >> ITEM_LEN_SHIFT) & 0xff;
                 if constexpr (NV == 1) {
                     if (wcols <= 16 * V::E)
-                        gather_row_narrow<V4, UNROLL>(p.col, p.val, db.x, db.x + len, p.x + c0, p.ldx, wcols,
+                        gather_row_narrow<V4, UNROLL>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0, p.ldx, wcols,
                                                       lanes_log2<V::E>(wcols), acc[0], lane);
                     else if (V4 && wcols == 128)  // a complete slab: no per-lane predicate on the fetches
-                        gather_row<NV, V4, UNROLL, true>(p.col, p.val, db.x, db.x + len, p.x + c0 + lane * V::E,
+                        gather_row<NV, V4, UNROLL, true>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0 + lane * V::E,
                                                          p.ldx, ok, acc, lane);
                     else
-                        gather_row<NV, V4, UNROLL>(p.col, p.val, db.x, db.x + len, p.x + c0 + lane * V::E,
+                        gather_row<NV, V4, UNROLL>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0 + lane * V::E,
                                                    p.ldx, ok, acc, lane);
                 } else {
-                    gather_row<NV, V4, UNROLL>(p.col, p.val, db.x, db.x + len, p.x + c0 + lane * V::E, p.ldx,
+                    gather_row<NV, V4, UNROLL>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0 + lane * V::E, p.ldx,
                                                ok, acc, lane);
                 }
             }
@@ -596,6 +623,59 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
         }
     }
 }
+
+__device__ __forceinline__ unsigned smem_addr(const void* p) {
+    return (unsigned)__cvta_generic_to_shared(p);
+}
+__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
+    unsigned done;
+    asm volatile(
+        "{\n\t.reg .pred q;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, q;\n\t}"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    return done != 0;
+}
+// Bounded: gives up after `limit_ns` (each poll itself blocks for a hardware-defined slice), or, where
+// `heed` is set, as soon as another wait of the launch has given up.
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, i32* status, u64 limit_ns = 2000000000ULL,
+                                          bool heed = false) {
+    if (mbar_try_wait(bar, parity)) return true;
+    const u64 t0 = global_ns();
+    for (unsigned spins = 0; spins < (1u << 24); ++spins) {
+        if (mbar_try_wait(bar, parity)) return true;
+        if ((spins & 63u) == 63u) {
+            if (heed && ld_relaxed(status) != 0) return false;
+            if (global_ns() - t0 > limit_ns) break;
+        }
+    }
+    atomicExch(status, CBM_B200_ERR_TIMEOUT);
+    return false;
+}
+// Global -> shared; src, dst and bytes are multiples of 16 (the host checks).
+__device__ __forceinline__ void bulk_copy_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
+    asm volatile(
+        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
+        "l"(src), "r"(bytes), "r"(bar)
+        : "memory");
+}
+__device__ __forceinline__ void fence_async_proxy() {
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+}
+
+#include "cbm_chunks.cuh"
 
 // ------------------------------------------------------------------------------------------
 // Bulk-copy form of the product kernel.
@@ -616,49 +696,6 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
 // are too small for this path; it is kept as an opt-in form (cbm_b200_plan_tune, form = 1) and the
 // register form is the default.
 // ------------------------------------------------------------------------------------------
-__device__ __forceinline__ unsigned smem_addr(const void* p) {
-    return (unsigned)__cvta_generic_to_shared(p);
-}
-__device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes)
-                 : "memory");
-}
-__device__ __forceinline__ bool mbar_try_wait(unsigned bar, unsigned parity) {
-    unsigned done;
-    asm volatile(
-        "{\n\t.reg .pred q;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 q, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, q;\n\t}"
-        : "=r"(done)
-        : "r"(bar), "r"(parity)
-        : "memory");
-    return done != 0;
-}
-// Bounded: gives up after two seconds (each poll itself blocks for a hardware-defined slice).
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, i32* status) {
-    if (mbar_try_wait(bar, parity)) return true;
-    const u64 t0 = global_ns();
-    for (unsigned spins = 0; spins < (1u << 24); ++spins) {
-        if (mbar_try_wait(bar, parity)) return true;
-        if ((spins & 63u) == 63u && global_ns() - t0 > 2000000000ULL) break;
-    }
-    atomicExch(status, CBM_B200_ERR_TIMEOUT);
-    return false;
-}
-// One row piece global -> shared; src, dst and bytes are multiples of 16 (the host checks).
-__device__ __forceinline__ void bulk_copy_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-        "l"(src), "r"(bytes), "r"(bar)
-        : "memory");
-}
-__device__ __forceinline__ void fence_async_proxy() {
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-}
-
 template <int SLABW, int NB, int STAGES>
 struct TmaLayout {
     static constexpr int SLABB = SLABW * 4;                   // bytes of one row piece
@@ -726,8 +763,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) cbm_items_tma_kernel(const KPar
             c = -1;
             w = 0.f;
             if (lane < NB && e < e_end) {
-                c = __ldg(p.col + e);
-                w = __ldg(p.val + e);
+                PairEntries{p.ent}.get(e, c, w);
             }
         };
         // start the copies of batch q into its stage
@@ -852,7 +888,7 @@ __global__ void __launch_bounds__(256, (NV >= 4 ? 2 : 3))
             ok[v] = (lane * V::E + v * STEP) < wcols;
             acc[v] = V::zero();
         }
-        gather_row<NV, V4, (NV == 1 ? 8 : 4)>(col, val, __ldg(row_b + row), __ldg(row_e + row), x + lane_col, ldx, ok,
+        gather_row<NV, V4, (NV == 1 ? 8 : 4)>(CsrEntries{col, val}, __ldg(row_b + row), __ldg(row_e + row), x + lane_col, ldx, ok,
                            acc, lane);
         float* yrow = y + (i64)row * ldy + lane_col;
 #pragma unroll
@@ -925,8 +961,9 @@ struct cbm_b200_plan {
     i32 depth = 0;
     bool normalized = false;
     RowDesc* d_desc = nullptr;
-    i32* d_col = nullptr;
-    float* d_val = nullptr;
+    Entry* d_ent = nullptr;
+    Chunk* d_chunks = nullptr;
+    i32 n_chunks = 0;            // 0: not clustered
     float* d_pack = nullptr;     // the operand copied to 16-byte aligned rows (when the caller's are not)
     i64 pack_cap = 0;
     i32* d_flags = nullptr;
@@ -979,8 +1016,8 @@ extern "C" void cbm_b200_plan_destroy(cbm_b200_plan* p) {
     if (!p) return;
     DeviceGuard g(p->device);
     cudaFree(p->d_desc);
-    cudaFree(p->d_col);
-    cudaFree(p->d_val);
+    cudaFree(p->d_ent);
+    cudaFree(p->d_chunks);
     cudaFree(p->d_pack);
     cudaFree(p->d_flags);
     cudaFree(p->d_scratch);
@@ -1000,8 +1037,10 @@ namespace {
 // The host-side schedule of one plan, before anything touches the device.
 struct Schedule {
     std::vector<RowDesc> desc;
-    std::vector<i32> pcol;
-    std::vector<float> pval;
+    std::vector<Entry> ent;
+    std::vector<Chunk> chunks;  // clustered plans
+    bool clustered = false;
+    i64 n_delta = 0;
     i32 n_prefix = 0, n_partial = 0, n_rows_owned = 0, depth = 0, n_root_children = 0, n_labels = 0;
 };
 
@@ -1021,7 +1060,7 @@ int validate_schedule(const Schedule& sch, i32 n_out) {
         const i32 n_part = (i32)((unsigned)d.info >> ITEM_NPART_SHIFT);
         const bool partial = (d.info & ITEM_PARTIAL) != 0;
         if (d.beg != cursor) return bad("entry ranges are not consecutive");
-        cursor += len;
+        cursor += sch.clustered ? (len + 1) / 2 * 2 : len;
         if (partial != (pos < sch.n_partial)) return bad("PARTIAL items must fill positions [0, n_partial)");
         if (partial) {
             if (!(d.info & ITEM_PUBLISH) || d.parent_row >= 0 || n_part != 0) return bad("malformed PARTIAL item");
@@ -1045,7 +1084,16 @@ int validate_schedule(const Schedule& sch, i32 n_out) {
             }
         }
     }
-    if (cursor != (i64)sch.pcol.size() || sch.pcol.size() != sch.pval.size()) return bad("entries not covered exactly once");
+    if (cursor != (i64)sch.ent.size()) return bad("entries not covered exactly once");
+    i32 at = 0;
+    for (const Chunk& c : sch.chunks) {
+        if (c.first != at || c.count <= 0 || c.count > MAX_CHUNK_ITEMS) return bad("chunks do not follow one another");
+        at += c.count;
+        const i64 end = at < n_items ? sch.desc[at].beg : cursor;
+        if (at > n_items || c.e0 != sch.desc[c.first].beg || c.e0 + c.ne != end || c.ne > CHUNK_ENTRIES)
+            return bad("a chunk does not hold its items' entries");
+    }
+    if (at != (sch.clustered ? n_items : 0)) return bad("items not covered by chunks");
     for (char c : collected)
         if (!c) return bad("a parked share is never collected");
     i32 rows = 0;
@@ -1054,12 +1102,66 @@ int validate_schedule(const Schedule& sch, i32 n_out) {
     return CBM_B200_OK;
 }
 
+// Cuts a clustered schedule into the chunks that blocks claim.
+void make_chunks(Schedule& sch, i32 n_prefix) {
+    const i32 n_items = (i32)sch.desc.size();
+    auto end_of = [&](i32 i) { return i + 1 < n_items ? sch.desc[i + 1].beg : (i32)sch.ent.size(); };
+    Chunk c{0, 0, 0, 0};
+    for (i32 i = 0; i < n_items; ++i) {
+        const i32 most = i < n_prefix ? MAX_CHUNK_ITEMS : MAX_CHUNK_ITEMS / 2;
+        if (c.count > 0 && (c.count >= most || i == n_prefix || end_of(i) - c.e0 > CHUNK_ENTRIES)) {
+            sch.chunks.push_back(c);
+            c.count = 0;
+        }
+        if (c.count == 0) c = Chunk{i, 0, sch.desc[i].beg, 0};
+        ++c.count;
+        c.ne = end_of(i) - c.e0;
+    }
+    if (c.count > 0) sch.chunks.push_back(c);
+}
+
+// Sorts the rows of a graph with communities by community (rank[v] = place of row v).  Returns false, and leaves
+// the rows as they are, where that would not bring row pieces into reach of an SM's L1: in a small graph (X is
+// fetched from L2 anyway and a launch is bound by latency), and where about 1 000 consecutive entries of
+// the sorted rows still name mostly different columns.  On B200, width 128: rows of 22 entries in
+// communities of 55 (ratio 0.4) gain 40 %, rows of 11 in communities of 118 (0.5) gain 15 %; copy-model graphs
+// (0.75 - 0.95), whose common columns are few hubs, gain nothing.
+bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std::vector<i32>& parent, int device,
+                   std::vector<i32>& rank) {
+    if (device < 0 || n < 16384 || crow[n] < 4 * (i64)n || crow[n] > INT32_MAX - n - 1024) return false;
+    std::vector<i32> label((size_t)n);
+    if (!cbm::cluster_rows(n, crow, col, parent.data(), device, label.data())) return false;
+    // counting sort by label, stable in v
+    std::vector<i32> start((size_t)n + 1, 0), sorted((size_t)n);
+    for (i32 v = 0; v < n; ++v) ++start[(size_t)label[v] + 1];
+    for (i32 l = 0; l < n; ++l) start[l + 1] += start[l];
+    for (i32 v = 0; v < n; ++v) sorted[start[label[v]]++] = v;
+    // distinct columns among the entries of runs of about 1 000 entries, sampled over the rows
+    i64 entries = 0, distinct = 0;
+    std::vector<i32> cols;
+    const i32 samples = 128;
+    for (i32 k = 0; k < samples; ++k) {
+        cols.clear();
+        for (i64 i = (i64)n * k / samples; i < n && cols.size() < 1024; ++i) {
+            const i32 v = sorted[i];
+            cols.insert(cols.end(), col + crow[v], col + crow[v + 1]);
+        }
+        entries += (i64)cols.size();
+        std::sort(cols.begin(), cols.end());
+        distinct += std::unique(cols.begin(), cols.end()) - cols.begin();
+    }
+    if (distinct * 10 > entries * 7) return false;
+    rank.resize((size_t)n);
+    for (i32 i = 0; i < n; ++i) rank[sorted[i]] = i;
+    return true;
+}
+
 // csr_cols > 0 schedules a plain CSR matrix with that many columns (no tree: every row hangs off
 // the virtual root, mst_row / mst_col / perm are not read); csr_cols == 0 schedules a CBM structure.
 int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,
                    const int32_t* delta_col, const float* delta_val, const float* multiplier,
                    const int32_t* perm, int32_t n_labels, int32_t own_begin, int32_t own_end, Schedule& sch,
-                   int32_t csr_cols = 0) {
+                   int32_t csr_cols = 0, int device = -1) {
     std::vector<i32> flat_row, flat_col;
     if (csr_cols > 0) {
         if (n < 0 || !delta_crow) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: NULL row pointers");
@@ -1157,18 +1259,17 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
             owned_rows.push_back(v);
         }
     std::vector<RowDesc>& desc = sch.desc;
-    std::vector<i32>& pcol = sch.pcol;
-    std::vector<float>& pval = sch.pval;
-    pcol.reserve((size_t)nd_all);
-    pval.reserve((size_t)nd_all);
+    std::vector<Entry>& ent = sch.ent;
+    std::vector<i32> rank;
+    sch.clustered = col_bound == n && cluster_order(n, delta_crow, delta_col, parent, device, rank);
+    ent.reserve((size_t)nd_all + (sch.clustered ? (size_t)n : 0));
     auto append_entries = [&](i32 v, i32 from, i32 to) {  // entries [from, to) of row v
-        const i32 beg = (i32)pcol.size();
-        for (i32 k = delta_crow[v] + from; k < delta_crow[v] + to; ++k) {
-            pcol.push_back(label(delta_col[k]));
-            pval.push_back(delta_val[k]);
-        }
+        const i32 beg = (i32)ent.size();
+        for (i32 k = delta_crow[v] + from; k < delta_crow[v] + to; ++k) ent.push_back(Entry{label(delta_col[k]), delta_val[k]});
+        if (sch.clustered && ent.size() % 2) ent.push_back(Entry{0, 0.0f});
         return beg;
     };
+    for (i32 v : owned_rows) sch.n_delta += row_len(v);
     // 1. PARTIAL items of every split row
     std::vector<i32> first_part((size_t)n, -1);
     for (i32 v : owned_rows) {
@@ -1217,13 +1318,26 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
         std::vector<i32> easy;
         for (i32 v : owned_rows)
             if (parent[v] == n && !is_split(v)) easy.push_back(v);
-        std::stable_sort(easy.begin(), easy.end(), [&](i32 a, i32 b) { return row_len(a) > row_len(b); });
+        if (sch.clustered)  // the few long rows first, then community by community
+            std::sort(easy.begin(), easy.end(), [&](i32 a, i32 b) {
+                const i32 la = row_len(a) > 64 ? row_len(a) : 0, lb = row_len(b) > 64 ? row_len(b) : 0;
+                return la != lb ? la > lb : rank[a] < rank[b];
+            });
+        else
+            std::stable_sort(easy.begin(), easy.end(), [&](i32 a, i32 b) { return row_len(a) > row_len(b); });
         for (i32 v : easy) add_row_item(v);
     }
     const i32 n_prefix = (i32)desc.size();
     // 3. everything that may wait, breadth-first: finishing items of split rows, rows with a parent
+    std::vector<i32> rest;
     for (i32 v : owned_rows)
-        if (parent[v] != n || is_split(v)) add_row_item(v);
+        if (parent[v] != n || is_split(v)) rest.push_back(v);
+    if (sch.clustered)  // level by level, so that parents stay in front of their children
+        std::sort(rest.begin(), rest.end(), [&](i32 a, i32 b) {
+            return level[a] != level[b] ? level[a] < level[b] : rank[a] < rank[b];
+        });
+    for (i32 v : rest) add_row_item(v);
+    if (sch.clustered) make_chunks(sch, n_prefix);
     sch.n_rows_owned = (i32)owned_rows.size();
     sch.n_prefix = n_prefix;
     sch.n_partial = n_partial;
@@ -1267,7 +1381,7 @@ extern "C" int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int
     *out = nullptr;
     Schedule sch;
     const int rc0 = build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm,
-                                   n_labels, own_begin, own_end, sch);
+                                   n_labels, own_begin, own_end, sch, 0, device);
     if (rc0) return rc0;
     return plan_from_schedule(sch, n, own_end - own_begin, multiplier != nullptr, device, out);
 }
@@ -1279,7 +1393,7 @@ extern "C" int cbm_b200_csr_plan_create(int32_t n_rows, int32_t n_cols, const in
     *out = nullptr;
     if (n_cols <= 0) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: n_cols must be positive");
     Schedule sch;
-    const int rc0 = build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols);
+    const int rc0 = build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols, device);
     if (rc0) return rc0;
     return plan_from_schedule(sch, n_rows, n_rows, false, device, out);
 }
@@ -1289,8 +1403,6 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
                        cbm_b200_plan** out) {
     const int32_t n_labels = sch.n_labels;
     std::vector<RowDesc>& desc = sch.desc;
-    std::vector<i32>& pcol = sch.pcol;
-    std::vector<float>& pval = sch.pval;
     const i32 n_rows_owned = sch.n_rows_owned, n_prefix = sch.n_prefix, n_partial = sch.n_partial;
     const i32 depth = sch.depth, n_root_children = sch.n_root_children;
 
@@ -1311,15 +1423,16 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
     p->n_items = (i32)desc.size();
     p->n_prefix = n_prefix;
     p->n_partial = n_partial;
-    p->n_delta = (i64)pcol.size();
+    p->n_delta = sch.n_delta;
+    p->n_chunks = (i32)sch.chunks.size();
     p->n_root_children = n_root_children;
     p->depth = depth;
     p->normalized = normalized;
     cudaDeviceProp prop{};
     if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) p->sm_count = prop.multiProcessorCount;
     int rc = upload(&p->d_desc, desc, p->device_bytes);
-    if (rc == CBM_B200_OK) rc = upload(&p->d_col, pcol, p->device_bytes);
-    if (rc == CBM_B200_OK) rc = upload(&p->d_val, pval, p->device_bytes);
+    if (rc == CBM_B200_OK) rc = upload(&p->d_ent, sch.ent, p->device_bytes);
+    if (rc == CBM_B200_OK && sch.clustered) rc = upload(&p->d_chunks, sch.chunks, p->device_bytes);
     if (rc == CBM_B200_OK) {
         cudaError_t e = cudaMalloc((void**)&p->d_counter, 2 * sizeof(u64));
         if (e == cudaSuccess) e = cudaMemset(p->d_counter, 0, 2 * sizeof(u64));
@@ -1399,6 +1512,8 @@ struct LaunchCfg {
     i32 group = 1;     // prefix items per claim
     i32 n_pclaims = 0, claims_per_slab = 0;
     i64 n_claims = 0;
+    bool chunked = false;      // the clustered plan's kernel ...
+    i32 run = 1, n_run = 0;    // ... see KParams
     i64 need_flags = 0;        // int32 words
     i64 need_scratch = 0;      // floats
     bool pack = false;         // the operand is first copied to 16-byte aligned rows
@@ -1408,18 +1523,32 @@ struct LaunchCfg {
 int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
              i32 f, int mode, bool may_pack, LaunchCfg& c) {
     const bool y_vec = ldy % 4 == 0 && aligned16(y);
-    const bool x_vec = ldx % 4 == 0 && aligned16(x);
+    const bool x_vec = ldx % 4 == 0 && aligned16(x) && ldx < (i64)1 << 30;
     // An operand whose rows are not 16-byte aligned can only be fetched 4 bytes a lane, at less than half
-    // the rate.  Copying it to aligned rows first costs one pass over it, so it pays when every operand row
-    // is fetched several times and the product is more than a launch (2 M multiply-adds, a few us).
+    // the rate (4.4 TB/s).  Copying it to aligned rows first costs a launch and one pass over it, about 5 us on a small
+    // operand, so it pays when every operand row is fetched several times and the 4-byte fetches would take
+    // some 15 us (16 M multiply-adds).
     c.pack = may_pack && mode != MODE_UPDATE_ONLY && !x_vec && f > 4 && p->n_delta >= 4 * (i64)p->n_labels &&
-             p->n_delta * f >= (i64)1 << 21;
+             p->n_delta * f >= (i64)1 << 24;
     const bool can_v4 = mode == MODE_UPDATE_ONLY ? y_vec : x_vec || c.pack;
     c.ragged = can_v4 && (!y_vec || f % 4 != 0);
     int tma = p->form;
-    if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY) tma = 0;
+    if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY || p->n_chunks > 0) tma = 0;
     c.tma = tma;
-    if (tma) {
+    // Slabs of up to 64 columns gain nothing from the clustered order (235 868 rows of 11 entries, 64 columns:
+    // 106 us against 97): several entries share a fetch there, and what a row costs is its instructions.
+    // On smaller graphs the saved round trips per row still win (20 000 rows of 12 entries, 64 columns: 26 us against 32).
+    c.chunked = p->n_chunks > 0 && can_v4 && mode != MODE_UPDATE_ONLY && (f > 64 || p->n_rows <= 65536) &&
+                (p->slab_width == 0 || p->slab_width >= 128);
+    if (c.chunked) {
+        c.sh.v4 = true;
+        c.sh.nv = 1;
+        c.sh.slab_w = 128;
+        c.sh.n_slabs = (f + c.sh.slab_w - 1) / c.sh.slab_w;
+        c.run = 4;
+        c.n_run = p->n_chunks * 3 / 4 / c.run * c.run;  // the last quarter one by one, to finish together
+        c.claims_per_slab = c.n_run / c.run + (p->n_chunks - c.n_run);
+    } else if (tma) {
         const i32 slab = 256;  // 1 KB row pieces: the copy engine is bound by copies, not bytes
         c.sh.v4 = true;
         c.sh.nv = slab / 128;
@@ -1434,8 +1563,10 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
         // only idles warps.
         c.group = ((i64)p->n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? 4 : 1;
     }
-    c.n_pclaims = (p->n_prefix + c.group - 1) / c.group;
-    c.claims_per_slab = c.n_pclaims + (p->n_items - p->n_prefix);
+    if (!c.chunked) {
+        c.n_pclaims = (p->n_prefix + c.group - 1) / c.group;
+        c.claims_per_slab = c.n_pclaims + (p->n_items - p->n_prefix);
+    }
     c.n_claims = (i64)c.claims_per_slab * c.sh.n_slabs;
     c.need_flags = (i64)c.sh.n_slabs * p->n_items;
     c.need_scratch = (i64)c.sh.n_slabs * p->n_partial * c.sh.slab_w;
@@ -1480,6 +1611,17 @@ int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
     return CBM_B200_OK;
 }
 
+template <bool RAGGED>
+int launch_chunks(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
+    constexpr int kResident = 3;  // 45 consumer warps per SM at 40 registers
+    int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
+    blocks = (int)std::max<i64>(1, std::min<i64>(blocks, kp.n_claims));
+    kp.n_warps = (u64)blocks;  // one claimer per block
+    cbm_chunks_kernel<RAGGED, 4, kResident><<<blocks, (CONSUMERS + 1) * 32, 0, s>>>(kp);
+    CBM_CUDA(cudaGetLastError());
+    return CBM_B200_OK;
+}
+
 // Rows of `f` floats copied to rows of 4 * vecs floats, zero-filled: one thread per vector of the result, the
 // source read 4 bytes at a time (its rows are not aligned).  Bound by HBM.
 __global__ void __launch_bounds__(256) pack_rows_kernel(const float* __restrict__ x, i64 ldx, float* __restrict__ out,
@@ -1516,8 +1658,11 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
         for (int k = 0; k < bc->n; ++k) kp.bcast[k] = bc->dst[k];
     }
     kp.desc = p->d_desc;
-    kp.col = p->d_col;
-    kp.val = p->d_val;
+    kp.ent = p->d_ent;
+    kp.chunks = p->d_chunks;
+    kp.run = c.run;
+    kp.n_run = c.n_run;
+    kp.ldx_bytes = (unsigned)(4 * ldx);
     kp.x = x;
     kp.y = y;
     kp.ldx = ldx;
@@ -1540,6 +1685,9 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.use_scale = use_scale ? 1 : 0;
     kp.wait_ns = 2000000000ULL;
     if (c.tma) return launch_tma<256, 16, 2, 7>(kp, p->sm_count, s);
+    if (c.chunked)
+        return c.ragged ? launch_chunks<true>(kp, p->n_blocks, p->sm_count, s)
+                        : launch_chunks<false>(kp, p->n_blocks, p->sm_count, s);
     if (c.ragged) {
         if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, p->n_blocks, p->sm_count, s);
         if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, p->n_blocks, p->sm_count, s);

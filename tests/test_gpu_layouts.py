@@ -45,3 +45,34 @@ def test_widths_and_pitches(copy_graph, f, aligned_x, aligned_y):
     c.seq_mkl_csr_fused_update(two)
     np.testing.assert_allclose(two.cpu().numpy(), want, **TOL)
     torch.testing.assert_close(c.seq_torch_csr_fused_matmul(xd), yd, atol=0, rtol=1e-6)
+
+
+@pytest.fixture(scope="module", params=[2, 40])
+def community_graph(request):
+    """Enough rows with common columns that the plan works on them community by community (16 384 and more); with 40
+    expected links per node rows also share a parent, so that some of them wait."""
+    n = 16384 + 5
+    ei = with_self_loops(graphs.stochastic_block_model(n, 400, 3.5, 0.8, 8.0 if request.param == 2 else 40.0, 1.0, 5))
+    ei = np.concatenate([ei, [[7] * 700, list(range(1000, 1700))]], axis=1)  # one row that is split
+    key = np.unique(ei[0] * n + ei[1])
+    ei = np.stack([key // n, key % n])
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
+    return ei, c
+
+
+@pytest.mark.parametrize("f", [5, 16, 61, 64, 65, 100, 128, 129, 200])
+@pytest.mark.parametrize("pad", [0, 1, 3])
+def test_rows_in_community_order(community_graph, f, pad):
+    ei, c = community_graph
+    x = np.random.default_rng(f).standard_normal((c.num_rows, f)).astype(np.float32)
+    xd, yd = _buffer(c.num_rows, f, f + pad), _buffer(c.num_rows, f, f + pad)
+    xd.copy_(torch.from_numpy(x))
+    want = sparse_product(ei, x, True)
+    for _ in range(2):
+        c.omp_mkl_csr_fused_spmm_update(xd, yd)
+    c.plan(0).status()
+    np.testing.assert_allclose(yd.cpu().numpy(), want, **TOL)
+    two = torch.full_like(yd, 7.0)
+    c.seq_mkl_csr_spmm(xd, two)
+    c.seq_mkl_csr_fused_update(two)
+    np.testing.assert_allclose(two.cpu().numpy(), want, **TOL)
