@@ -103,6 +103,7 @@ struct KParams {
     i64 ldx, ldy;
     i32 f;
     i32 y_vec;       // rows of y are 16-byte aligned
+    i32 in_turn;     // entries are added strictly one after the other, also in narrow slabs
     const Chunk* chunks;   // clustered plans: chunks, ...
     unsigned ldx_bytes;    // ... 4 * ldx,
     i32 run;               // ... chunks claimed `run` at a time below chunk n_run, one at a time from there on
@@ -601,7 +602,7 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
                 for (int v = 0; v < NV; ++v) acc[v] = V::zero();
                 const i32 len = (info >> ITEM_LEN_SHIFT) & 0xff;
                 if constexpr (NV == 1) {
-                    if (wcols <= 16 * V::E)
+                    if (wcols <= 16 * V::E && !p.in_turn)
                         gather_row_narrow<V4, UNROLL>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0, p.ldx, wcols,
                                                       lanes_log2<V::E>(wcols), acc[0], lane);
                     else if (V4 && wcols == 128)  // a complete slab: no per-lane predicate on the fetches
@@ -1516,12 +1517,13 @@ struct LaunchCfg {
     i32 run = 1, n_run = 0;    // ... see KParams
     i64 need_flags = 0;        // int32 words
     i64 need_scratch = 0;      // floats
+    bool in_turn = false;      // see KParams
     bool pack = false;         // the operand is first copied to 16-byte aligned rows
     bool ragged = false;       // 16-byte fetches, but rows of y are not aligned or end inside a vector
 };
 
 int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
-             i32 f, int mode, bool may_pack, LaunchCfg& c) {
+             i32 f, int mode, bool may_pack, bool in_turn, LaunchCfg& c) {
     const bool y_vec = ldy % 4 == 0 && aligned16(y);
     const bool x_vec = ldx % 4 == 0 && aligned16(x) && ldx < (i64)1 << 30;
     // An operand whose rows are not 16-byte aligned can only be fetched 4 bytes a lane, at less than half
@@ -1530,7 +1532,8 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
     // some 15 us (16 M multiply-adds).
     c.pack = may_pack && mode != MODE_UPDATE_ONLY && !x_vec && f > 4 && p->n_delta >= 4 * (i64)p->n_labels &&
              p->n_delta * f >= (i64)1 << 24;
-    const bool can_v4 = mode == MODE_UPDATE_ONLY ? y_vec : x_vec || c.pack;
+    c.in_turn = in_turn;
+    const bool can_v4 = !in_turn && (mode == MODE_UPDATE_ONLY ? y_vec : x_vec || c.pack);
     c.ragged = can_v4 && (!y_vec || f % 4 != 0);
     int tma = p->form;
     if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY || p->n_chunks > 0) tma = 0;
@@ -1651,6 +1654,7 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
                 cudaStream_t s, const Bcast* bc = nullptr) {
     KParams kp{};
     kp.y_vec = ldy % 4 == 0 && aligned16(y);
+    kp.in_turn = c.in_turn;
     if (bc) {
         for (int k = 0; k < bc->n; ++k) kp.y_vec = kp.y_vec && aligned16(bc->dst[k]);
         kp.n_bcast = bc->n;
@@ -1704,7 +1708,7 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
 }
 
 int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
-             int mode, bool use_scale, cudaStream_t s, const Bcast* bc = nullptr) {
+             int mode, bool use_scale, cudaStream_t s, const Bcast* bc = nullptr, bool in_turn = false) {
     if (!p) return cbm::fail(CBM_B200_ERR_ARG, std::string(who) + ": NULL plan");
     int rc = check_dense(who, x, ldx, y, ldy, f);
     if (rc) return rc;
@@ -1716,7 +1720,7 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (p->n_rows == 0) return CBM_B200_OK;
     DeviceGuard g(p->device);
     LaunchCfg c;
-    rc = plan_cfg(p, who, x, ldx, y, ldy, f, mode, true, c);
+    rc = plan_cfg(p, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
     if (rc) return rc;
 
     if (c.need_flags > p->flags_cap) {
@@ -1905,8 +1909,9 @@ extern "C" int cbm_b200_spmm_update_host(cbm_b200_plan* p, const float* x, float
                                        (size_t)p->n_labels, cudaMemcpyHostToDevice, p->copy_in));
         CBM_CUDA(cudaEventRecord(p->events[2 * k], p->copy_in));
         CBM_CUDA(cudaStreamWaitEvent(s, p->events[2 * k], 0));
+        // the short tail is summed as the device-operand product of this width sums its last columns
         int rc = run_plan(p, "spmm_update_host", p->stage_x + c0, ld, p->stage_y + c0, ld, w, MODE_FUSED,
-                          normalized != 0, s);
+                          normalized != 0, s, nullptr, w % 4 != 0 && c0 > 0);
         if (rc) return rc;
         CBM_CUDA(cudaEventRecord(p->events[2 * k + 1], s));
         CBM_CUDA(cudaStreamWaitEvent(p->copy_out, p->events[2 * k + 1], 0));
@@ -2083,7 +2088,7 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     if (p->n_rows == 0) return CBM_B200_OK;
 
     LaunchCfg c;
-    rc = plan_cfg(p, who, x, ldx, y, ldy, f, MODE_FUSED, false, c);
+    rc = plan_cfg(p, who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
     if (rc) return rc;
     // layout inside the fixed array: counters | ready flags | partial sums
     const i64 off_flags = 256;
