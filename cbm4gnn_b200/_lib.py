@@ -22,7 +22,7 @@ LIB_PATH = os.path.join(_PKG_DIR, "libcbm_b200.so")
 SOURCES = [
     os.path.join(_PKG_DIR, "csrc", "cbm_engine.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_builder.cpp"),
-    os.path.join(_PKG_DIR, "csrc", "cbm_dense.cu"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_map.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_dense_grad.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.cu"),
@@ -34,6 +34,7 @@ HEADERS = [
     os.path.join(_PKG_DIR, "csrc", "cbm_chunks.cuh"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_dense_gemm.cuh"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_map.cuh"),
 ]
 _OBJ_DIR = os.path.join(_PKG_DIR, "build")
 
@@ -52,7 +53,7 @@ def _cutlass_includes() -> list[str]:
     for r in roots:
         if r and os.path.exists(os.path.join(r, "include", "cutlass", "cutlass.h")):
             return [os.path.join(r, "include"), os.path.join(r, "tools", "util", "include")]
-    raise RuntimeError("CUTLASS headers not found: set CUTLASS_HOME (needed to compile csrc/cbm_dense.cu)")
+    raise RuntimeError("CUTLASS headers not found: set CUTLASS_HOME (needed to compile csrc/cbm_dense_grad.cu)")
 
 # Every symbol include/cbm_b200.h declares; the CPU test-suite checks the library exports all of them.
 EXPORTED = [

@@ -1,0 +1,498 @@
+// Dense maps of the GCN layers on the 5th-generation tensor cores (sm_100a): forward Y = X W^T and input
+// gradient dX = dY W, fp32-accurate (see cbm_map.cuh).
+//
+// A GCN layer of the reference is `lin` followed by `propagate`
+// (gnns/graph_convolutional_network/cbm_gcn.py:21-24): a bias-free [N,in] x [in,out] map in fp32.
+// N is the number of nodes and the weights are small, so a map reads X once, writes Y once, and should be bound by
+// HBM; what stood in the way was the split of both operands into bf16 terms, repeated for every tile.
+//   * W is split once per block into shared memory (swizzled K-major rows, 3 terms, up to 192 KB) and stays
+//     there: blocks are persistent and walk over row tiles of X.
+//   * X goes from global memory to registers (16-byte loads, whole 32-byte sectors), is split there and stored
+//     straight into tensor memory as the A operand: it never passes through shared memory, whose bandwidth
+//     is left to the tensor cores for W.
+//   * 8 warps load and split (two groups, alternate 32-deep chunks, the next chunk's loads in flight), one warp issues
+//     the MMAs, 8 warps add up the accumulators and store Y with the ReLU or the mask applied (32 x 64 sums each).
+//   * Y leaves (and the mask arrives) in whole 128-byte lines, 32 x 32 sums turned round through 4 KB of shared memory
+//     per warp.
+// 235 868 rows, against three-term GEMMs that split both operands for every 128 x 128 x 16 tile: 128 -> 256 96 us
+// (200), 256 -> 64 79 (100), 256 -> 256 175 (349), gradient 256 -> 128 101 (189).
+#include "cbm_map.cuh"
+
+#include <atomic>
+#include <mutex>
+#include <type_traits>
+
+namespace cbm_map {
+
+int sm_count() {
+    static std::atomic<int> cached[64];
+    int dev = 0, n = 148;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return n;
+    n = cached[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 148;
+        cached[dev].store(n, std::memory_order_relaxed);
+    }
+    return n;
+}
+
+int* timeout_word() {
+    static std::once_flag once;
+    static int* word = nullptr;
+    std::call_once(once, [] {
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
+            word = static_cast<int*>(p);
+            *word = 0;
+        }
+    });
+    return word;
+}
+
+int check_timeout(const char* who) {
+    int* w = timeout_word();
+    if (!w) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": no usable CUDA device on this thread");
+    if (*(volatile int*)w) {
+        *(volatile int*)w = 0;
+        return cbm::fail(CBM_B200_ERR_TIMEOUT, std::string(who) + ": a bounded wait of an earlier dense map ran out; its result is invalid");
+    }
+    return CBM_B200_OK;
+}
+
+namespace {
+
+// Two warps of each kind per scheduler: a warp alone on one issues an instruction every 4 - 5 cycles, and with 4
+// epilogue warps (or 4 producers) their work, not memory or the MMAs, was the bound.
+constexpr int PRODUCER_WARPS = 8, EPILOGUE_WARPS = 8;
+constexpr int MMA_WARP = PRODUCER_WARPS + EPILOGUE_WARPS;
+constexpr int THREADS = 20 * 32;  // five warpgroups (of the last only one warp works), 96 registers a thread at launch ...
+constexpr int LAUNCH_REGS = 96, PRODUCER_REGS = 104, EPILOGUE_REGS = 112, MMA_REGS = 40;  // ... and after the split
+static_assert(PRODUCER_REGS > LAUNCH_REGS && EPILOGUE_REGS > LAUNCH_REGS && MMA_REGS < LAUNCH_REGS &&
+                  256 * PRODUCER_REGS + 256 * EPILOGUE_REGS + 128 * MMA_REGS <= THREADS * LAUNCH_REGS,
+              "setmaxnreg.inc and .dec only go up and down, within the registers of the launch");
+constexpr int SMEM_MAX = 192 * 1024;     // for the split weights
+constexpr int TURN_BYTES = 32 * 32 * 4;  // per epilogue warp
+
+struct MapParams {
+    const float* a;    // [m, k]
+    const float* b;    // [n, k], or [k, n] when B_TRANS
+    float* d;          // [m, n]
+    const float* aux;  // [m, n]: the result is zeroed where aux is not positive
+    int64_t lda, ldb, ldd, ldaux;
+    int m, n, k;
+    int bn;            // columns of a tile, a multiple of 16, at most 128
+    int row_tiles;
+    int steps;         // ceil(k / 16)
+    int a_vec, d_vec, aux_vec;  // rows are 16-byte aligned
+    int relu_in, relu_out, add; // max(a, 0) first; max(d, 0) last; d += instead of d =
+    int* timeout;
+};
+
+// EXTRA: 0 plain, 1 with a mask, 2 with any of a mask and earlier passes' results to add to.
+template <bool B_TRANS, int EXTRA>
+__global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__ MapParams p) {
+    extern __shared__ unsigned char smem_raw[];
+    __shared__ u64 s_bar[2 * A_SLOTS + 5];  // A full x4, A empty x4, accumulator full x2, accumulator empty x2, drained
+    __shared__ u32 s_tmem;
+    __shared__ int s_gave_up;
+    unsigned char* smem = smem_raw + ((1024 - (smem_u32(smem_raw) & 1023)) & 1023);
+    const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
+    const u32 bars = smem_u32(s_bar);
+    const u32 a_full = bars, a_empty = bars + 8 * A_SLOTS, d_full = bars + 16 * A_SLOTS, d_empty = d_full + 16, drained = d_full + 32;
+    const int n0 = blockIdx.x * p.bn;
+    const int chunks = (p.steps + 1) / 2;                // 32-deep chunks of a row tile
+    const int kblocks = (chunks + 1) / 2;                // 64-deep blocks
+    const u32 block = (u32)p.bn * 128;                   // one 64-deep block of one term of W
+    const u32 term = block * (u32)kblocks;
+    unsigned char* turn = smem + 3 * term;
+
+    if (warp == MMA_WARP) tmem_alloc(smem_u32(&s_tmem));
+    if (threadIdx.x == 0) {
+        for (int s = 0; s < A_SLOTS; ++s) {
+            bar_init(a_full + 8 * s, 4);
+            bar_init(a_empty + 8 * s, 1);
+        }
+        for (int s = 0; s < 2; ++s) {
+            bar_init(d_full + 8 * s, 1);
+            bar_init(d_empty + 8 * s, EPILOGUE_WARPS);
+        }
+        bar_init(drained, 1);
+        s_gave_up = 0;
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    // the weights, split, into shared memory
+    const int k8s = 2 * p.steps;
+    for (int i = threadIdx.x; i < p.bn * k8s; i += THREADS) {
+        const int n = B_TRANS ? i % p.bn : i / k8s;
+        const int k8 = B_TRANS ? i / p.bn : i % k8s;
+        float x[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+            const int k = k8 * 8 + j;
+            x[j] = n0 + n < p.n && k < p.k ? __ldg(B_TRANS ? p.b + (int64_t)k * p.ldb + n0 + n : p.b + (int64_t)(n0 + n) * p.ldb + k) : 0.f;
+        }
+        store_split8(smem + (u32)(k8 >> 3) * block + swizzled((u32)n, (u32)(k8 & 7)), term, x);
+    }
+    fence_async();
+    fence_before();
+    __syncthreads();
+    fence_after();
+    const u32 tmem = __shfl_sync(0xffffffffu, s_tmem, 0);
+    volatile int* gave_up = &s_gave_up;
+
+    if (warp < PRODUCER_WARPS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PRODUCER_REGS));
+        const int quarter = warp & 3, group = warp >> 2;
+        const int row_in = quarter * 32 + (lane >> 2), k_in = 4 * (lane & 3);
+        float4 v[2][4][2];  // [buffer][8-row group][16-deep step]
+        // fetches only; what lies past column k is zeroed when the values are used
+        auto load = [&](int buf, int tile, int c) {
+            const float* s0 = p.a + (int64_t)(tile * 128 + row_in) * p.lda + c * CHUNK_K + k_in;
+            const int left = p.m - (tile * 128 + row_in), k = c * CHUNK_K + k_in;
+            if (p.a_vec) {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) v[buf][i][s] = fetch4(s0 + 8 * i * p.lda + 16 * s, 8 * i < left && k + 16 * s < p.k);
+            } else {
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                    for (int s = 0; s < 2; ++s) {
+                        const float* at = s0 + 8 * i * p.lda + 16 * s;
+                        const bool row = 8 * i < left;
+                        v[buf][i][s].x = fetch1(at, row && k + 16 * s < p.k);
+                        v[buf][i][s].y = fetch1(at + 1, row && k + 16 * s + 1 < p.k);
+                        v[buf][i][s].z = fetch1(at + 2, row && k + 16 * s + 2 < p.k);
+                        v[buf][i][s].w = fetch1(at + 3, row && k + 16 * s + 3 < p.k);
+                    }
+            }
+        };
+        // this group's chunks: those whose running number has the group's parity
+        int tile = blockIdx.y, c = group;
+        while (c >= chunks) {
+            c -= chunks;
+            tile += gridDim.y;
+        }
+        if (tile < p.row_tiles) load(0, tile, c);
+        for (u32 run = group; tile < p.row_tiles; run += 4) {
+#pragma unroll
+            for (int buf = 0; buf < 2; ++buf) {
+                if (tile >= p.row_tiles) break;
+                int next_tile = tile, next_c = c + 2;
+                while (next_c >= chunks) {
+                    next_c -= chunks;
+                    next_tile += gridDim.y;
+                }
+                if (next_tile < p.row_tiles) load(buf ^ 1, next_tile, next_c);
+                const u32 r = run + 2 * buf, slot = r % A_SLOTS;
+                if (r >= A_SLOTS && !warp_wait(a_empty + 8 * slot, ((r / A_SLOTS) + 1) & 1, gave_up, p.timeout)) goto done;
+                const u32 at = tmem + A_COL + slot * A_SLOT_COLS + ((u32)(quarter * 32) << 16);
+                const bool ragged_k = p.a_vec && c * CHUNK_K + CHUNK_K > p.k;
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                    u32 t[3][8];
+#pragma unroll
+                    for (int i = 2 * h; i < 2 * h + 2; ++i)
+#pragma unroll
+                        for (int s = 0; s < 2; ++s) {
+                            float4 x = v[buf][i][s];
+                            if (ragged_k) {  // an aligned row's last vector may reach past column k
+                                const int k = c * CHUNK_K + 16 * s + k_in;
+                                x.y = k + 1 < p.k ? x.y : 0.f;
+                                x.z = k + 2 < p.k ? x.z : 0.f;
+                                x.w = k + 3 < p.k ? x.w : 0.f;
+                            }
+                            if (p.relu_in) x = make_float4(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f), fmaxf(x.z, 0.f), fmaxf(x.w, 0.f));
+                            const int o = 4 * s + 2 * (i & 1);
+                            split2(x.x, x.y, t[0][o], t[1][o], t[2][o]);
+                            split2(x.z, x.w, t[0][o + 1], t[1][o + 1], t[2][o + 1]);
+                        }
+#pragma unroll
+                    for (int q = 0; q < 3; ++q)
+                        asm volatile(
+                            "tcgen05.st.sync.aligned.16x256b.x2.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(
+                                at + 16 * q + ((u32)(16 * h) << 16)),
+                            "r"(t[q][0]), "r"(t[q][1]), "r"(t[q][2]), "r"(t[q][3]), "r"(t[q][4]), "r"(t[q][5]), "r"(t[q][6]),
+                            "r"(t[q][7])
+                            : "memory");
+                }
+                wait_st();
+                fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(a_full + 8 * slot);
+                tile = next_tile;
+                c = next_c;
+            }
+        }
+    } else if (warp >= MMA_WARP) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(MMA_REGS));
+        if (warp > MMA_WARP) goto done;
+        const u32 idesc = idesc_of((u32)p.bn);
+        const u32 b0 = smem_u32(smem);
+        u32 run = 0, it = 0;
+        bool ok = true;
+        for (int tile = blockIdx.y; tile < p.row_tiles && ok; tile += gridDim.y)
+            for (int kb = 0; kb < kblocks; ++kb, ++it) {
+                const u32 ds = it & 1, use = it >> 1;
+                if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
+                fence_after();
+                const u32 d = tmem + ds * D_COLS;
+                const int here = min(2, chunks - 2 * kb);
+                for (int c = 0; c < here && ok; ++c) {
+                    const u32 slot = (run + c) % A_SLOTS;
+                    if (!(ok = warp_wait(a_full + 8 * slot, ((run + c) / A_SLOTS) & 1, gave_up, p.timeout))) break;
+                    fence_after();
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        if (4 * kb + 2 * c + s < p.steps)
+                            mma_small(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, b0 + (u32)kb * block + 32 * (2 * c + s), term, idesc,
+                                      c + s > 0);
+                }
+                if (!ok) break;
+                for (int c = 0; c < here; ++c) {
+                    const u32 slot = (run + c) % A_SLOTS;
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        if (4 * kb + 2 * c + s < p.steps)
+                            mma(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, desc_of(b0 + (u32)kb * block + 32 * (2 * c + s)), idesc, true);
+                    commit(a_empty + 8 * slot);
+                }
+                commit(d_full + 8 * ds);
+                run += here;
+            }
+        if (!ok) {  // the MMAs under way end before the block frees its tensor memory
+            commit(drained);
+            for (u32 spins = 0; spins < (1u << 20) && !bar_poll(drained, 0); ++spins) {
+            }
+            __syncwarp();
+        }
+    } else {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(EPILOGUE_REGS));
+        // This warp: 32 rows by up to two blocks of 32 columns from column c_lo on; lane = row while the sums are
+        // collected, then, block by block, lane = 4 columns from 4 * (lane % 8) on of the rows lane / 8 + 4 i.
+        const int quarter = warp & 3, half = (warp - PRODUCER_WARPS) >> 2;
+        const int first_width = min(p.bn, (p.bn + 63) / 64 * 32);
+        const int c_lo = half * first_width, width = half ? p.bn - first_width : first_width;
+        const int row_in = quarter * 32 + (lane >> 3), col_in = c_lo + 4 * (lane & 7);
+        float4* mine = reinterpret_cast<float4*>(turn + (warp - PRODUCER_WARPS) * TURN_BYTES);
+        u32 it = 0;
+        for (int tile = blockIdx.y; tile < p.row_tiles; tile += gridDim.y) {
+            const int row0 = tile * 128 + row_in;
+            // Of the mask only one bit per value is kept, fetched while the products of this tile are under way.
+            u32 keep[2] = {0xffffffffu, 0xffffffffu};
+            if (EXTRA && p.aux) {
+                float4 x[2][8];
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    const int col = 32 * b + col_in, left = col < c_lo + width ? p.n - n0 - col : 0;
+                    const float* s0 = p.aux + (int64_t)row0 * p.ldaux + n0 + col;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const float* s = s0 + 4 * i * p.ldaux;
+                        const bool in = row0 + 4 * i < p.m;
+                        if (p.aux_vec) {
+                            x[b][i] = fetch4(s, in && left > 0);  // what lies past column n is not stored
+                        } else {
+                            x[b][i].x = fetch1(s, in && left > 0);
+                            x[b][i].y = fetch1(s + 1, in && left > 1);
+                            x[b][i].z = fetch1(s + 2, in && left > 2);
+                            x[b][i].w = fetch1(s + 3, in && left > 3);
+                        }
+                    }
+                }
+#pragma unroll
+                for (int b = 0; b < 2; ++b) {
+                    u32 bits = 0;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i)
+                        bits |= ((x[b][i].x > 0.f ? 1u : 0u) | (x[b][i].y > 0.f ? 2u : 0u) | (x[b][i].z > 0.f ? 4u : 0u) |
+                                 (x[b][i].w > 0.f ? 8u : 0u))
+                                << (4 * i);
+                    keep[b] = bits;
+                }
+            }
+            // The first block sets the sums, the others add to them (told apart at compile time: the sums must not
+            // be live while the mask is fetched).
+            float acc[2][32];
+            auto collect = [&](auto first) -> bool {
+                const u32 ds = it & 1, use = it >> 1;
+                if (!warp_wait(d_full + 8 * ds, use & 1, gave_up, p.timeout)) return false;
+                fence_after();
+                const u32 at = tmem + ds * D_COLS + c_lo + ((u32)(quarter * 32) << 16);
+#pragma unroll
+                for (int q = 0; q < 4; ++q) {
+                    float r[16];
+                    if (16 * q < width)
+                        asm volatile(
+                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+                            "%14, %15}, [%16];"
+                            : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
+                              "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
+                            : "r"(at + 16 * q));
+                    wait_ld();
+#pragma unroll
+                    for (int i = 0; i < 16; ++i) {
+                        asm volatile("" : "+f"(r[i]));  // not before the wait
+                        float& s = acc[q >> 1][16 * (q & 1) + i];
+                        if constexpr (decltype(first)::value) s = r[i];
+                        else s += r[i];
+                    }
+                }
+                fence_before();
+                __syncwarp();
+                if (lane == 0) bar_arrive(d_empty + 8 * ds);
+                ++it;
+                return true;
+            };
+            if (!collect(std::true_type{})) goto done;
+            for (int kb = 1; kb < kblocks; ++kb)
+                if (!collect(std::false_type{})) goto done;
+#pragma unroll
+            for (int b = 0; b < 2; ++b) {
+                if (32 * b >= width) break;
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    mine[lane * 8 + (j ^ (lane & 7))] = make_float4(acc[b][4 * j], acc[b][4 * j + 1], acc[b][4 * j + 2], acc[b][4 * j + 3]);
+                __syncwarp();
+                const int col = 32 * b + col_in, left = col < c_lo + width ? p.n - n0 - col : 0;
+                float* d0 = p.d + (int64_t)row0 * p.ldd + n0 + col;
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    const int r = (lane >> 3) + 4 * i;
+                    float4 y = mine[r * 8 + ((lane & 7) ^ (r & 7))];
+                    float* d = d0 + 4 * i * p.ldd;
+                    const int here = row0 + 4 * i < p.m ? left : 0;
+                    if constexpr (EXTRA) {
+                        if (EXTRA == 2 && p.add) {
+                            if (here > 0) y.x += d[0];
+                            if (here > 1) y.y += d[1];
+                            if (here > 2) y.z += d[2];
+                            if (here > 3) y.w += d[3];
+                        }
+                        const u32 bits = keep[b] >> (4 * i);
+                        y = make_float4(bits & 1 ? y.x : 0.f, bits & 2 ? y.y : 0.f, bits & 4 ? y.z : 0.f, bits & 8 ? y.w : 0.f);
+                    }
+                    if (p.relu_out) y = make_float4(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f), fmaxf(y.z, 0.f), fmaxf(y.w, 0.f));
+                    if (p.d_vec && here >= 4) {
+                        *reinterpret_cast<float4*>(d) = y;
+                    } else {
+                        if (here > 0) d[0] = y.x;
+                        if (here > 1) d[1] = y.y;
+                        if (here > 2) d[2] = y.z;
+                        if (here > 3) d[3] = y.w;
+                    }
+                }
+                __syncwarp();
+            }
+        }
+    }
+done:
+    __syncwarp();
+    fence_before();
+    __syncthreads();
+    if (warp == MMA_WARP) tmem_free(tmem);
+}
+
+bool aligned_rows(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; }
+
+int round_up(int v, int to) { return (v + to - 1) / to * to; }
+
+// d [m, n] = a [m, k] b^T, b [n, k] (b_trans: [k, n]).
+int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_t ldb, bool b_trans, float* d, int64_t ldd,
+            const float* aux, int64_t ldaux, int m, int n, int k, bool relu_in, bool relu_out, cudaStream_t stream) {
+    if (const int rc = check_timeout(who)) return rc;
+    const int sms = sm_count();
+    const int row_tiles = (m + 127) / 128;
+    // Tile width: up to 128 columns (an epilogue warp keeps 32 x 64 sums in registers), less where their split
+    // weights, up to 512 of the contraction, would not fit into shared memory (a longer contraction is cut into
+    // passes that add to d).  Few row tiles: narrower, so that every SM has a tile, down to 32 columns.
+    const int n16 = round_up(n, 16);
+    const auto depth = [](int bn) { return SMEM_MAX / (384 * bn) * 64; };  // contraction that fits beside bn columns
+    int bn = std::min(n16, 128);
+    while (bn > 16 && depth(bn) < std::min(k, 512)) bn -= 16;
+    const int want = std::max((n16 + bn - 1) / bn, std::min(sms / row_tiles, (n16 + 31) / 32));
+    bn = round_up((n16 + want - 1) / want, 16);
+    const int n_tiles = (n16 + bn - 1) / bn;
+    const int most = std::min(round_up(k, 16), depth(bn));
+    const int passes = (k + most - 1) / most;
+    const int seg = round_up((k + passes - 1) / passes, 16);
+    for (int k0 = 0; k0 < k; k0 += seg) {
+        MapParams p{};
+        const bool last = k0 + seg >= k;
+        p.a = a + k0;
+        p.b = b_trans ? b + (int64_t)k0 * ldb : b + k0;
+        p.d = d;
+        p.lda = lda;
+        p.ldb = ldb;
+        p.ldd = ldd;
+        p.m = m;
+        p.n = n;
+        p.k = std::min(seg, k - k0);
+        p.bn = bn;
+        p.row_tiles = row_tiles;
+        p.steps = (p.k + 15) / 16;
+        p.a_vec = aligned_rows(p.a, lda);
+        p.d_vec = aligned_rows(d, ldd);
+        p.relu_in = relu_in;
+        p.relu_out = relu_out && last;
+        p.add = k0 > 0;
+        if (aux) {
+            p.aux = aux;
+            p.ldaux = ldaux;
+            p.aux_vec = aligned_rows(aux, ldaux);
+        }
+        p.timeout = timeout_word();
+        auto kern = b_trans ? (p.add ? map_kernel<true, 2> : p.aux ? map_kernel<true, 1> : map_kernel<true, 0>)
+                            : (p.add ? map_kernel<false, 2> : map_kernel<false, 0>);
+        const size_t smem = (size_t)3 * ((p.steps + 3) / 4) * bn * 128 + EPILOGUE_WARPS * TURN_BYTES + 1024;
+        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 SMEM_MAX + EPILOGUE_WARPS * TURN_BYTES + 1024) != cudaSuccess)
+            return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": shared memory size refused");
+        const dim3 grid(n_tiles, std::max(1, std::min(row_tiles, sms / n_tiles)));
+        // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
+        kern<<<grid, THREADS, std::max<size_t>(smem, 120 * 1024), stream>>>(p);
+        if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
+    }
+    return CBM_B200_OK;
+}
+
+}  // namespace
+}  // namespace cbm_map
+
+using namespace cbm_map;
+
+extern "C" int cbm_b200_dense_forward(const float* x, int64_t ldx, const float* w, int64_t ldw, float* y, int64_t ldy,
+                                      int32_t n_rows, int32_t n_in, int32_t n_out, void* stream) {
+    if (!x || !w || !y || n_rows < 0 || n_in <= 0 || n_out <= 0)
+        return cbm::fail(CBM_B200_ERR_ARG, "dense_forward: bad arguments");
+    if (n_rows == 0) return CBM_B200_OK;
+    return run_map("dense_forward", x, ldx, w, ldw, false, y, ldy, nullptr, 0, n_rows, n_out, n_in, false, false, (cudaStream_t)stream);
+}
+
+extern "C" int cbm_b200_dense_forward_relu(const float* x, int64_t ldx, const float* w, int64_t ldw, float* y,
+                                           int64_t ldy, int32_t n_rows, int32_t n_in, int32_t n_out, void* stream) {
+    if (!x || !w || !y || n_rows < 0 || n_in <= 0 || n_out <= 0)
+        return cbm::fail(CBM_B200_ERR_ARG, "dense_forward_relu: bad arguments");
+    if (n_rows == 0) return CBM_B200_OK;
+    return run_map("dense_forward_relu", x, ldx, w, ldw, false, y, ldy, nullptr, 0, n_rows, n_out, n_in, false, true, (cudaStream_t)stream);
+}
+
+extern "C" int cbm_b200_dense_grad_input(const float* dy, int64_t lddy, const float* w, int64_t ldw, float* dx,
+                                         int64_t lddx, int32_t n_rows, int32_t n_in, int32_t n_out, void* stream) {
+    if (!dy || !w || !dx || n_rows < 0 || n_in <= 0 || n_out <= 0)
+        return cbm::fail(CBM_B200_ERR_ARG, "dense_grad_input: bad arguments");
+    if (n_rows == 0) return CBM_B200_OK;
+    return run_map("dense_grad_input", dy, lddy, w, ldw, true, dx, lddx, nullptr, 0, n_rows, n_in, n_out, false, false, (cudaStream_t)stream);
+}
+
+extern "C" int cbm_b200_dense_grad_input_relu(const float* dy, int64_t lddy, const float* w, int64_t ldw, const float* h,
+                                              int64_t ldh, float* dx, int64_t lddx, int32_t n_rows, int32_t n_in,
+                                              int32_t n_out, void* stream) {
+    if (!dy || !w || !h || !dx || n_rows < 0 || n_in <= 0 || n_out <= 0)
+        return cbm::fail(CBM_B200_ERR_ARG, "dense_grad_input_relu: bad arguments");
+    if (ldh < n_in) return cbm::fail(CBM_B200_ERR_ARG, "dense_grad_input_relu: rows of h must hold n_in floats");
+    if (n_rows == 0) return CBM_B200_OK;
+    return run_map("dense_grad_input_relu", dy, lddy, w, ldw, true, dx, lddx, h, ldh, n_rows, n_in, n_out, false, false,
+                   (cudaStream_t)stream);
+}
