@@ -23,7 +23,7 @@ SOURCES = [
     os.path.join(_PKG_DIR, "csrc", "cbm_engine.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_builder.cpp"),
     os.path.join(_PKG_DIR, "csrc", "cbm_map.cu"),
-    os.path.join(_PKG_DIR, "csrc", "cbm_dense_grad.cu"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_map_grad.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.cu"),
 ]
@@ -33,27 +33,10 @@ HEADERS = [
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_chunks.cuh"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.h"),
-    os.path.join(_PKG_DIR, "csrc", "cbm_dense_gemm.cuh"),
     os.path.join(_PKG_DIR, "csrc", "cbm_map.cuh"),
 ]
 _OBJ_DIR = os.path.join(_PKG_DIR, "build")
 
-
-def _cutlass_includes() -> list[str]:
-    """Header trees of CUTLASS / CuTe (the dense maps instantiate their sm100 templates): the
-    environment variable CUTLASS_HOME, else the copy vendored inside the flashinfer package."""
-    roots = [os.environ.get("CUTLASS_HOME")]
-    try:
-        import importlib.util
-        spec = importlib.util.find_spec("flashinfer")
-        if spec and spec.submodule_search_locations:
-            roots.append(os.path.join(list(spec.submodule_search_locations)[0], "data", "cutlass"))
-    except Exception:
-        pass
-    for r in roots:
-        if r and os.path.exists(os.path.join(r, "include", "cutlass", "cutlass.h")):
-            return [os.path.join(r, "include"), os.path.join(r, "tools", "util", "include")]
-    raise RuntimeError("CUTLASS headers not found: set CUTLASS_HOME (needed to compile csrc/cbm_dense_grad.cu)")
 
 # Every symbol include/cbm_b200.h declares; the CPU test-suite checks the library exports all of them.
 EXPORTED = [
@@ -110,8 +93,7 @@ def needs_build() -> bool:
 
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile the library for sm_100a next to this file and return its path.  Every source is
-    compiled to its own object (kept under ``build/``, so that touching the engine does not
-    recompile the CUTLASS instantiations, which take over a minute) and the objects are linked."""
+    compiled to its own object (kept under ``build/``, so that touching one does not recompile the others) and the objects are linked."""
     if not force and not needs_build():
         return LIB_PATH
     os.makedirs(_OBJ_DIR, exist_ok=True)
@@ -129,10 +111,6 @@ def build(force: bool = False, verbose: bool = False) -> str:
             "-I", os.path.join(_ROOT, "include"),
             "-I", os.path.join(_PKG_DIR, "csrc"),
         ]
-        if os.path.basename(src).startswith("cbm_dense"):
-            cmd += ["--expt-relaxed-constexpr", "-diag-suppress", "20012"]
-            for inc in _cutlass_includes():
-                cmd += ["-I", inc]
         if verbose:
             cmd[1:1] = ["-Xptxas", "-v"]
         cmd += ["-c", src, "-o", obj]
@@ -144,7 +122,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             raise RuntimeError("nvcc failed:\n" + " ".join(cmd) + "\n" + res.stdout + res.stderr)
         return res.stderr
 
-    # the sources are compiled side by side: the CUTLASS instantiations alone take minutes
+    # the sources are compiled side by side
     from concurrent.futures import ThreadPoolExecutor
     with ThreadPoolExecutor(max_workers=max(1, len(jobs))) as pool:
         log = list(pool.map(compile_one, jobs))
