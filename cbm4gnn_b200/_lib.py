@@ -66,9 +66,11 @@ EXPORTED = [
     "cbm_b200_probe_l2_read_gbps",
     "cbm_b200_dense_forward",
     "cbm_b200_dense_forward_relu",
+    "cbm_b200_dense_forward_of_relu",
     "cbm_b200_dense_grad_input",
     "cbm_b200_dense_grad_input_relu",
     "cbm_b200_dense_grad_weight",
+    "cbm_b200_dense_grad_weight_of_relu",
     "cbm_b200_dense_grad_weight_workspace",
     "cbm_b200_spmm_update_host",
     "cbm_b200_copy2d_async",
@@ -190,8 +192,11 @@ def lib() -> ctypes.CDLL:
         sig(name, c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_int32, c_void_p)
     sig("cbm_b200_dense_grad_input_relu", c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
         c_int32, c_int32, c_int32, c_void_p)
-    sig("cbm_b200_dense_grad_weight", c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int32,
-        c_int32, c_int32, c_void_p, c_int64, c_void_p)
+    sig("cbm_b200_dense_forward_of_relu", c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32,
+        c_int32, c_int32, c_void_p)
+    for name in ("cbm_b200_dense_grad_weight", "cbm_b200_dense_grad_weight_of_relu"):
+        sig(name, c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_int32, c_void_p,
+            c_int64, c_void_p)
     sig("cbm_b200_dense_grad_weight_workspace", c_int64, c_int32, c_int32, c_int32)
     sig("cbm_b200_copy2d_async", c_int32, c_void_p, c_int64, c_void_p, c_int64, c_int64, c_int64, c_int32, c_void_p)
     sig("cbm_b200_spmm_update_host", c_int32, c_void_p, c_void_p, c_void_p, c_int32, c_int32)

@@ -461,21 +461,22 @@ class cbm_matrix:
 
 
 def _product(cbm: "cbm_matrix", x: torch.Tensor) -> torch.Tensor:
-    """``A @ x`` / normalized product into a fresh tensor.  A CUDA operand whose width is not a
-    multiple of 4 floats is first copied into a zero-padded buffer: the 128-bit kernel path on
-    the padded width is faster than the scalar path on the exact width, copy included."""
-    x = x.contiguous()
+    """``A @ x`` / normalized product into a fresh tensor.  On a GPU any row-major operand is taken as it
+    is, and the rows of the result are 16-byte aligned whatever its width."""
     f = x.size(1)
-    run = cbm.seq_mkl_csr_fused_spmm_update if cbm.normalized else cbm.seq_mkl_csr_spmm_update
-    if x.is_cuda and f % 4 != 0 and f > 4:
-        fp = -(-f // 4) * 4
-        xp = torch.zeros((x.size(0), fp), dtype=x.dtype, device=x.device)
-        xp[:, :f] = x
-        yp = torch.empty((cbm.num_rows, fp), dtype=x.dtype, device=x.device)
-        run(xp, yp)
-        return yp[:, :f]
-    y = torch.empty((cbm.num_rows, f), dtype=x.dtype, device=x.device)
-    run(x, y)
+    if not x.is_cuda:
+        x = x.contiguous()
+        y = x.new_empty((cbm.num_rows, f))
+    else:
+        if x.stride(1) != 1 or x.stride(0) < f:
+            x = x.contiguous()
+        y = x.new_empty((cbm.num_rows, -(-f // 4) * 4))
+        if f % 4:
+            y = y[:, :f]
+    if cbm.col_multiplier is not None:
+        cbm._run("cbm_b200_fused_spmm_update", x, y, host_normalized=True)
+    else:
+        cbm._run("cbm_b200_spmm_update", x, y, host_normalized=False)
     return y
 
 

@@ -18,7 +18,6 @@
 // (200), 256 -> 64 79 (100), 256 -> 256 175 (349), gradient 256 -> 128 101 (189).
 #include "cbm_map.cuh"
 
-#include <atomic>
 #include <mutex>
 #include <type_traits>
 
@@ -398,9 +397,24 @@ bool aligned_rows(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_
 
 int round_up(int v, int to) { return (v + to - 1) / to * to; }
 
+template <bool B_TRANS, int EXTRA>
+int launch(const char* who, const MapParams& p, int sms, cudaStream_t stream) {
+    if (!allow_smem<map_kernel<B_TRANS, EXTRA>>(SMEM_MAX + EPILOGUE_WARPS * TURN_BYTES + 1024))
+        return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": shared memory size refused");
+    const int n_tiles = (p.n + p.bn - 1) / p.bn;
+    const dim3 grid(n_tiles, std::max(1, std::min(p.row_tiles, sms / n_tiles)));
+    // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
+    const int smem = std::max(3 * ((p.steps + 3) / 4) * p.bn * 128 + EPILOGUE_WARPS * TURN_BYTES + 1024, 120 * 1024);
+    map_kernel<B_TRANS, EXTRA><<<grid, THREADS, smem, stream>>>(p);
+    if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
+    return CBM_B200_OK;
+}
+
 // d [m, n] = a [m, k] b^T, b [n, k] (b_trans: [k, n]).
 int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_t ldb, bool b_trans, float* d, int64_t ldd,
             const float* aux, int64_t ldaux, int m, int n, int k, bool relu_in, bool relu_out, cudaStream_t stream) {
+    if (lda < k || ldb < (b_trans ? n : k) || ldd < n)
+        return cbm::fail(CBM_B200_ERR_ARG, std::string(who) + ": a leading dimension is smaller than its row");
     if (const int rc = check_timeout(who)) return rc;
     const int sms = sm_count();
     const int row_tiles = (m + 127) / 128;
@@ -413,7 +427,6 @@ int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_
     while (bn > 16 && depth(bn) < std::min(k, 512)) bn -= 16;
     const int want = std::max((n16 + bn - 1) / bn, std::min(sms / row_tiles, (n16 + 31) / 32));
     bn = round_up((n16 + want - 1) / want, 16);
-    const int n_tiles = (n16 + bn - 1) / bn;
     const int most = std::min(round_up(k, 16), depth(bn));
     const int passes = (k + most - 1) / most;
     const int seg = round_up((k + passes - 1) / passes, 16);
@@ -443,16 +456,10 @@ int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_
             p.aux_vec = aligned_rows(aux, ldaux);
         }
         p.timeout = timeout_word();
-        auto kern = b_trans ? (p.add ? map_kernel<true, 2> : p.aux ? map_kernel<true, 1> : map_kernel<true, 0>)
-                            : (p.add ? map_kernel<false, 2> : map_kernel<false, 0>);
-        const size_t smem = (size_t)3 * ((p.steps + 3) / 4) * bn * 128 + EPILOGUE_WARPS * TURN_BYTES + 1024;
-        if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 SMEM_MAX + EPILOGUE_WARPS * TURN_BYTES + 1024) != cudaSuccess)
-            return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": shared memory size refused");
-        const dim3 grid(n_tiles, std::max(1, std::min(row_tiles, sms / n_tiles)));
-        // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
-        kern<<<grid, THREADS, std::max<size_t>(smem, 120 * 1024), stream>>>(p);
-        if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
+        const int rc = b_trans ? (p.add ? launch<true, 2>(who, p, sms, stream)
+                                        : p.aux ? launch<true, 1>(who, p, sms, stream) : launch<true, 0>(who, p, sms, stream))
+                               : (p.add ? launch<false, 2>(who, p, sms, stream) : launch<false, 0>(who, p, sms, stream));
+        if (rc) return rc;
     }
     return CBM_B200_OK;
 }
@@ -476,6 +483,15 @@ extern "C" int cbm_b200_dense_forward_relu(const float* x, int64_t ldx, const fl
         return cbm::fail(CBM_B200_ERR_ARG, "dense_forward_relu: bad arguments");
     if (n_rows == 0) return CBM_B200_OK;
     return run_map("dense_forward_relu", x, ldx, w, ldw, false, y, ldy, nullptr, 0, n_rows, n_out, n_in, false, true, (cudaStream_t)stream);
+}
+
+extern "C" int cbm_b200_dense_forward_of_relu(const float* x, int64_t ldx, const float* w, int64_t ldw, float* y, int64_t ldy,
+                                              int32_t n_rows, int32_t n_in, int32_t n_out, int32_t relu, void* stream) {
+    if (!x || !w || !y || n_rows < 0 || n_in <= 0 || n_out <= 0)
+        return cbm::fail(CBM_B200_ERR_ARG, "dense_forward_of_relu: bad arguments");
+    if (n_rows == 0) return CBM_B200_OK;
+    return run_map("dense_forward_of_relu", x, ldx, w, ldw, false, y, ldy, nullptr, 0, n_rows, n_out, n_in, true, relu != 0,
+                   (cudaStream_t)stream);
 }
 
 extern "C" int cbm_b200_dense_grad_input(const float* dy, int64_t lddy, const float* w, int64_t ldw, float* dx,

@@ -15,6 +15,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cstdint>
 #include <string>
 
@@ -41,6 +42,18 @@ int* timeout_word();
 int check_timeout(const char* who);
 // SMs of the current device.
 int sm_count();
+// Lets a kernel use that much shared memory; asked for once per device, not on every call.
+template <auto Kernel>
+bool allow_smem(int bytes) {
+    static std::atomic<u64> done{0};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return false;
+    const u64 bit = dev < 64 ? 1ull << dev : 0;
+    if (done.load(std::memory_order_acquire) & bit) return true;
+    if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess) return false;
+    done.fetch_or(bit, std::memory_order_release);
+    return true;
+}
 
 #ifdef __CUDACC__
 __device__ __forceinline__ u32 smem_u32(const void* p) { return (u32)__cvta_generic_to_shared(p); }

@@ -29,6 +29,7 @@ struct GradParams {
     int bn;          // columns of b in a tile, 64 or 128
     int n_tiles;     // tiles along n
     int chunks_per;  // 32-row chunks per block, even
+    int relu_a, relu_b;  // max(., 0) first
     int b_vec;       // pairs of columns of b are 8-byte aligned
     int* timeout;
 };
@@ -103,7 +104,14 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
             const u32 slot = (u32)c % A_SLOTS;
             u32 t[3][CHUNK_K / 2];
 #pragma unroll
-            for (int i = 0; i < CHUNK_K / 2; ++i) split2(v[2 * i], v[2 * i + 1], t[0][i], t[1][i], t[2][i]);
+            for (int i = 0; i < CHUNK_K / 2; ++i) {
+                float x = v[2 * i], y = v[2 * i + 1];
+                if (p.relu_a) {
+                    x = fmaxf(x, 0.f);
+                    y = fmaxf(y, 0.f);
+                }
+                split2(x, y, t[0][i], t[1][i], t[2][i]);
+            }
             if (c + 2 < chunks) load(c + 2);
             if (c >= A_SLOTS && !warp_wait(empty + 8 * slot, ((u32)c / A_SLOTS + 1) & 1, gave_up, p.timeout)) goto done;
             const u32 at = tmem + A_COL + slot * A_SLOT_COLS + ((u32)(quarter * 32) << 16);
@@ -158,10 +166,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
                 const u32 row = (u32)((task >> 2) * 64 + lane), k8 = (slot & 1) * 4 + (u32)(task & 3);
                 float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = v[i][j].x;
+                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? fmaxf(v[i][j].x, 0.f) : v[i][j].x;
                 store_split8(at + swizzled(row, k8), term, x);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = v[i][j].y;
+                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? fmaxf(v[i][j].y, 0.f) : v[i][j].y;
                 store_split8(at + swizzled(row + 32, k8), term, x);
             }
             if (c + 1 < chunks) load(c + 1);
@@ -333,11 +341,13 @@ extern "C" int64_t cbm_b200_dense_grad_weight_workspace(int32_t n_rows, int32_t 
     return (int64_t)split_of(n_rows, n_in, n_out).ranges * n_in * n_out * (int64_t)sizeof(float);
 }
 
-extern "C" int cbm_b200_dense_grad_weight(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw,
-                                          int64_t lddw, int32_t n_rows, int32_t n_in, int32_t n_out, void* workspace,
-                                          int64_t workspace_bytes, void* stream) {
+namespace {
+int run_grad(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw, int64_t lddw, int32_t n_rows, int32_t n_in,
+             int32_t n_out, bool relu_x, void* workspace, int64_t workspace_bytes, void* stream) {
     if (!dy || !x || !dw || n_rows < 0 || n_in <= 0 || n_out <= 0)
         return cbm::fail(CBM_B200_ERR_ARG, "dense_grad_weight: bad arguments");
+    if (lddy < n_out || ldx < n_in || lddw < n_in)
+        return cbm::fail(CBM_B200_ERR_ARG, "dense_grad_weight: a leading dimension is smaller than its row");
     if (const int rc = check_timeout("dense_grad_weight")) return rc;
     cudaStream_t s = (cudaStream_t)stream;
     const Split t = split_of(n_rows, n_in, n_out);
@@ -355,17 +365,32 @@ extern "C" int cbm_b200_dense_grad_weight(const float* dy, int64_t lddy, const f
     p.bn = t.bn;
     p.n_tiles = t.n_tiles;
     p.chunks_per = t.chunks_per;
+    p.relu_a = t.turn && relu_x;
+    p.relu_b = !t.turn && relu_x;
     p.b_vec = (reinterpret_cast<uintptr_t>(p.b) & 7) == 0 && p.ldb % 2 == 0;
     p.part = static_cast<float*>(workspace);
     p.timeout = timeout_word();
     // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
     const int smem = 120 * 1024;
     static_assert(2 * 3 * D_COLS * 128 + 1024 <= 120 * 1024, "two stages of B");
-    if (cudaFuncSetAttribute(grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem) != cudaSuccess)
+    if (!allow_smem<grad_kernel>(smem))
         return cbm::fail(CBM_B200_ERR_CUDA, "dense_grad_weight: shared memory size refused");
     grad_kernel<<<dim3(t.m_tiles * t.n_tiles, t.ranges), GRAD_THREADS, smem, s>>>(p);
     const int64_t size = (int64_t)n_in * n_out;
     reduce_parts_kernel<<<(unsigned)((size + 31) / 32), 256, 0, s>>>(p.part, t.ranges, p.m, p.n, dw, lddw, t.turn ? 1 : 0);
     if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, "dense_grad_weight: launch failed");
     return CBM_B200_OK;
+}
+}  // namespace
+
+extern "C" int cbm_b200_dense_grad_weight(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw,
+                                          int64_t lddw, int32_t n_rows, int32_t n_in, int32_t n_out, void* workspace,
+                                          int64_t workspace_bytes, void* stream) {
+    return run_grad(dy, lddy, x, ldx, dw, lddw, n_rows, n_in, n_out, false, workspace, workspace_bytes, stream);
+}
+
+extern "C" int cbm_b200_dense_grad_weight_of_relu(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw,
+                                                  int64_t lddw, int32_t n_rows, int32_t n_in, int32_t n_out,
+                                                  void* workspace, int64_t workspace_bytes, void* stream) {
+    return run_grad(dy, lddy, x, ldx, dw, lddw, n_rows, n_in, n_out, true, workspace, workspace_bytes, stream);
 }

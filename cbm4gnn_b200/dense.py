@@ -10,113 +10,90 @@ through ``torch.nn.functional.linear``.
 """
 from __future__ import annotations
 
-import ctypes
-
 import torch
 
 from . import _lib
+from .cbm import _raw_stream
 
 
-def _pad4(v: int) -> int:
-    return -(-v // 4) * 4
+_current_device = torch._C._cuda_getDevice
 
 
-def _aligned(t: torch.Tensor) -> torch.Tensor:
-    """Row-major, 16-byte aligned rows (row stride a multiple of 4 floats): as is, or a copy."""
-    if t.stride(1) == 1 and t.stride(0) % 4 == 0 and t.data_ptr() % 16 == 0 and t.stride(0) >= t.size(1):
-        return t
-    out = torch.empty((t.size(0), _pad4(t.size(1))), dtype=t.dtype, device=t.device)
-    out[:, :t.size(1)].copy_(t)
-    if out.size(1) != t.size(1):
-        out[:, t.size(1):].zero_()
-    return out[:, :t.size(1)]
+def _rows(t: torch.Tensor) -> torch.Tensor:
+    """Row-major with unit column stride: as is, or a copy.  The maps take rows of any width at any
+    pitch; 16-byte aligned ones are read four values at a time."""
+    s = t.stride()
+    return t if s[1] == 1 and s[0] >= t.size(1) else t.contiguous()
 
 
-def _widen(t: torch.Tensor, cols: int) -> torch.Tensor:
-    """``t`` with zero columns appended up to ``cols`` (a copy only when needed)."""
-    t = _aligned(t)
-    if t.size(1) == cols:
-        return t
-    out = torch.zeros((t.size(0), cols), dtype=t.dtype, device=t.device)
-    out[:, :t.size(1)].copy_(t)
-    return out
+def _new_rows(n: int, width: int, like: torch.Tensor) -> torch.Tensor:
+    """An uninitialised [n, width] tensor whose rows are 16-byte aligned."""
+    if width % 4 == 0:
+        return like.new_empty((n, width))
+    return like.new_empty((n, -(-width // 4) * 4))[:, :width]
 
 
-def _stream(t: torch.Tensor) -> ctypes.c_void_p:
-    return ctypes.c_void_p(torch.cuda.current_stream(t.device).cuda_stream)
+def _ld(t: torch.Tensor) -> int:
+    return max(t.stride(0), t.size(1))
 
 
-def dense_forward(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, relu: bool = False) -> torch.Tensor:
-    """``x @ w.T`` (``relu``: followed by ``max(., 0)`` in the GEMM's epilogue) for CUDA fp32 ``x``
-    [N, in] and ``w`` [out, in]; ``out`` (optional) is an [N, out] view with 16-byte aligned rows
-    that receives the result."""
+def _call(name: str, dev: int, *args) -> None:
+    """One library call on device ``dev``'s current stream."""
+    fn = getattr(_lib.lib(), name)
+    if _current_device() == dev:
+        rc = fn(*args, _raw_stream(dev))
+    else:
+        with torch.cuda.device(dev):
+            rc = fn(*args, _raw_stream(dev))
+    if rc:
+        _lib.check(rc)
+
+
+def dense_forward(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = None, relu: bool = False,
+                  relu_in: bool = False) -> torch.Tensor:
+    """``x @ w.T`` (``relu``: followed by ``max(., 0)`` in the GEMM's epilogue; ``relu_in``: of
+    ``max(x, 0)``, taken as the operand is read) for CUDA fp32 ``x`` [N, in] and ``w`` [out, in];
+    ``out`` (optional) is an [N, out] tensor that receives the result."""
     n, n_in, n_out = x.size(0), x.size(1), w.size(0)
-    ip, op = _pad4(n_in), _pad4(n_out)
-    xa, wa = _widen(x, ip), _widen(w, ip)
-    if op != n_out:
-        wp = torch.zeros((op, ip), dtype=w.dtype, device=w.device)
-        wp[:n_out].copy_(wa)
-        wa = wp
-    direct = out is not None and op == n_out and out.stride(1) == 1 and out.stride(0) % 4 == 0 and out.data_ptr() % 16 == 0
-    y = out if direct else torch.empty((n, op), dtype=x.dtype, device=x.device)
-    with torch.cuda.device(x.device):
-        fn = _lib.lib().cbm_b200_dense_forward_relu if relu else _lib.lib().cbm_b200_dense_forward
-        _lib.check(fn(xa.data_ptr(), xa.stride(0), wa.data_ptr(), wa.stride(0), y.data_ptr(), y.stride(0), n, ip, op, _stream(x)))
-    if direct:
-        return out
-    y = y[:, :n_out]
-    if out is not None:
-        out.copy_(y)
-        return out
-    return y
+    x, w = _rows(x), _rows(w)
+    direct = out is not None and out.stride(1) == 1 and out.stride(0) >= n_out
+    y = out if direct else _new_rows(n, n_out, x)
+    args = (x.data_ptr(), _ld(x), w.data_ptr(), _ld(w), y.data_ptr(), _ld(y), n, n_in, n_out)
+    if relu_in:
+        _call("cbm_b200_dense_forward_of_relu", x.get_device(), *args, 1 if relu else 0)
+    else:
+        _call("cbm_b200_dense_forward_relu" if relu else "cbm_b200_dense_forward", x.get_device(), *args)
+    return y if out is None or direct else out.copy_(y)
 
 
 def dense_grad_input(gy: torch.Tensor, w: torch.Tensor, relu_output: torch.Tensor | None = None) -> torch.Tensor:
-    """``gy @ w`` for ``gy`` [N, out], ``w`` [out, in].  With ``relu_output`` [N, in] (the output of
-    the ReLU this gradient flows back through) the result is zeroed where that output is zero, in
-    the GEMM's epilogue."""
+    """``gy @ w`` for ``gy`` [N, out], ``w`` [out, in].  With ``relu_output`` [N, in] (the output, or
+    the input, of the ReLU this gradient flows back through) the result is zeroed where that is not
+    positive, in the GEMM's epilogue."""
     n, n_out, n_in = gy.size(0), gy.size(1), w.size(1)
-    ip, op = _pad4(n_in), _pad4(n_out)
-    ga = _widen(gy, op)
-    wa = _widen(w, ip)
-    if op != n_out:
-        wp = torch.zeros((op, ip), dtype=w.dtype, device=w.device)
-        wp[:n_out].copy_(wa)
-        wa = wp
-    gx = torch.empty((n, ip), dtype=gy.dtype, device=gy.device)
-    with torch.cuda.device(gy.device):
-        if relu_output is None:
-            _lib.check(_lib.lib().cbm_b200_dense_grad_input(ga.data_ptr(), ga.stride(0), wa.data_ptr(), wa.stride(0),
-                                                            gx.data_ptr(), gx.stride(0), n, ip, op, _stream(gy)))
-        else:
-            ha = _widen(relu_output, ip)
-            _lib.check(_lib.lib().cbm_b200_dense_grad_input_relu(ga.data_ptr(), ga.stride(0), wa.data_ptr(), wa.stride(0),
-                                                                 ha.data_ptr(), ha.stride(0), gx.data_ptr(), gx.stride(0),
-                                                                 n, ip, op, _stream(gy)))
-    return gx[:, :n_in]
+    gy, w = _rows(gy), _rows(w)
+    gx = _new_rows(n, n_in, gy)
+    args = (gy.data_ptr(), _ld(gy), w.data_ptr(), _ld(w))
+    to = (gx.data_ptr(), _ld(gx), n, n_in, n_out)
+    if relu_output is None:
+        _call("cbm_b200_dense_grad_input", gy.get_device(), *args, *to)
+    else:
+        h = _rows(relu_output)
+        _call("cbm_b200_dense_grad_input_relu", gy.get_device(), *args, h.data_ptr(), _ld(h), *to)
+    return gx
 
 
-_workspaces: dict = {}
-
-
-def dense_grad_weight(gy: torch.Tensor, x: torch.Tensor) -> torch.Tensor:
-    """``gy.T @ x`` for ``gy`` [N, out], ``x`` [N, in]: the weight gradient [out, in].  The partial
-    results of the row chunks go through one workspace per device, so calls on one device must not
-    overlap (autograd issues them on one stream)."""
+def dense_grad_weight(gy: torch.Tensor, x: torch.Tensor, relu_x: bool = False) -> torch.Tensor:
+    """``gy.T @ x`` for ``gy`` [N, out], ``x`` [N, in]: the weight gradient [out, in] (``relu_x``: of
+    ``max(x, 0)``).  The partial results of the row ranges go through a workspace from torch's
+    allocator, which is stream-ordered: calls on different streams and threads do not share one."""
     n, n_out, n_in = gy.size(0), gy.size(1), x.size(1)
-    ip, op = _pad4(n_in), _pad4(n_out)
-    ga, xa = _widen(gy, op), _widen(x, ip)
-    L = _lib.lib()
-    need = int(L.cbm_b200_dense_grad_weight_workspace(n, ip, op))
-    ws = _workspaces.get(gy.device)
-    if ws is None or ws.numel() < need:
-        ws = torch.empty(need, dtype=torch.uint8, device=gy.device)
-        _workspaces[gy.device] = ws
-    gw = torch.empty((op, ip), dtype=gy.dtype, device=gy.device)
-    with torch.cuda.device(gy.device):
-        _lib.check(L.cbm_b200_dense_grad_weight(ga.data_ptr(), ga.stride(0), xa.data_ptr(), xa.stride(0), gw.data_ptr(),
-                                                gw.stride(0), n, ip, op, ws.data_ptr(), ws.numel(), _stream(gy)))
-    return gw[:n_out, :n_in]
+    gy, x = _rows(gy), _rows(x)
+    gw = gy.new_empty((n_out, n_in))
+    ws = gy.new_empty(_lib.lib().cbm_b200_dense_grad_weight_workspace(n, n_in, n_out) // 4)
+    _call("cbm_b200_dense_grad_weight_of_relu" if relu_x else "cbm_b200_dense_grad_weight", gy.get_device(), gy.data_ptr(),
+          _ld(gy), x.data_ptr(), _ld(x), gw.data_ptr(), n_in, n, n_in, n_out, ws.data_ptr(), 4 * ws.numel())
+    return gw
 
 
 class _DenseMap(torch.autograd.Function):
@@ -149,6 +126,33 @@ class _DenseMapRelu(torch.autograd.Function):
         gx = dense_grad_input(gy, weight) if ctx.needs_input_grad[0] else None
         gw = dense_grad_weight(gy, x) if ctx.needs_input_grad[1] else None
         return gx, gw
+
+
+class _ReluThenMap(torch.autograd.Function):
+    """``relu(a) @ w.T`` for the ReLU in front of a map that opens its layer: taken as the map reads
+    ``a``, masked in the epilogue of the input gradient, taken again as the weight gradient reads ``a``,
+    so that no elementwise kernel passes over the activations in either direction."""
+
+    @staticmethod
+    def forward(ctx, a, weight):
+        ctx.save_for_backward(a, weight)
+        return dense_forward(a, weight, relu_in=True)
+
+    @staticmethod
+    def backward(ctx, gy):
+        a, weight = ctx.saved_tensors
+        ga = dense_grad_input(gy, weight, relu_output=a) if ctx.needs_input_grad[0] else None
+        gw = dense_grad_weight(gy, a, relu_x=True) if ctx.needs_input_grad[1] else None
+        return ga, gw
+
+
+def relu_linear(a: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``relu(a) @ weight.T`` in fp32 accuracy, differentiable in both arguments."""
+    if not a.is_cuda:
+        return torch.nn.functional.linear(a.relu(), weight)
+    if a.dtype != torch.float32 or weight.dtype != torch.float32:
+        raise RuntimeError("dense map: fp32 operands expected")
+    return _ReluThenMap.apply(a, weight)
 
 
 def linear_relu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:

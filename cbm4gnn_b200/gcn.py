@@ -15,7 +15,7 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from .dense import linear, linear_relu, relu_linear_linear
+from .dense import linear, linear_relu, relu_linear, relu_linear_linear
 from .message_passing import CBMCudaMessagePassing
 
 
@@ -102,18 +102,26 @@ class GCNModel(nn.Module):
     def forward(self, x, edge_index):
         """Where a layer that propagates first is followed by one that propagates last, the two dense
         maps and the ReLU between them are adjacent — ``A (relu((A x) W1^T) W2^T)`` — and run as one
-        differentiable step (``relu_linear_linear``)."""
+        differentiable step (``relu_linear_linear``).  Where a layer that propagates last is followed by one
+        that does too, the ReLU between the product and the map is taken as the map reads its operand
+        (``relu_linear``)."""
         last = len(self.layers) - 1
         i = 0
+        pending = False  # x still lacks the ReLU of the layer before
         while i <= last:
             layer = self.layers[i]
             nxt = self.layers[i + 1] if i < last else None
+            if x.is_cuda and not layer.propagate_first():
+                u = relu_linear(x, layer.lin.weight) if pending else _fp32_linear(layer.lin, x)
+                x, pending = layer.propagate_only(u, edge_index), i < last
+                i += 1
+                continue
+            if pending:
+                x, pending = x.relu(), False
             if nxt is not None and x.is_cuda and layer.propagate_first() and not nxt.propagate_first():
                 p = layer.propagate_only(x, edge_index)
                 u = relu_linear_linear(p, layer.lin.weight, nxt.lin.weight)
-                x = nxt.propagate_only(u, edge_index)
-                if i + 1 < last:
-                    x = x.relu()
+                x, pending = nxt.propagate_only(u, edge_index), i + 1 < last
                 i += 2
                 continue
             x = layer(x, edge_index, relu=i < last)

@@ -223,18 +223,22 @@ int cbm_b200_selftest_wait(int32_t device, int32_t wait_ms, void* stream);
  * Dense maps of the GCN layers: `lin` of gnns/graph_convolutional_network/cbm_gcn.py:21-24 (a
  * bias-free [N,in] x [in,out] fp32 map, there torch_geometric's Linear on the CPU) and its two
  * gradients, as fp32-accurate GEMMs on the tensor cores (every operand split into three bf16
- * terms, fp32 accumulation in tensor memory).  All pointers [dev], row-major, 16-byte aligned;
- * n_in, n_out and every leading dimension must be multiples of 4 floats.
+ * terms, fp32 accumulation in tensor memory).  All pointers [dev], row-major, any width and leading
+ * dimension; rows that are 16-byte aligned are read and written four values at a time.
  *   cbm_b200_dense_forward      y [n_rows,n_out] = x [n_rows,n_in] * w^T,  w [n_out,n_in]
  *   cbm_b200_dense_forward_relu y = max(x * w^T, 0): the map followed by the ReLU that sits between two
  *                               layers (benchmark/parallel/benchmark_gcn_cpu.py:70-89), in the epilogue
  *   cbm_b200_dense_grad_input   dx [n_rows,n_in] = dy [n_rows,n_out] * w
- *   cbm_b200_dense_grad_input_relu  the same, set to 0 wherever h [n_rows,n_in] is 0: the gradient that
- *                               flows back through the ReLU whose output h was (the mask in the epilogue)
+ *   cbm_b200_dense_grad_input_relu  the same, set to 0 wherever h [n_rows,n_in] is not positive: the
+ *                               gradient that flows back through the ReLU whose output (or input) h was
  *   cbm_b200_dense_grad_weight  dw [n_out,n_in]  = dy^T * x; contracts over the rows in up to
  *                               CBM_B200_DENSE_MAX_CHUNKS independent chunks whose partial results
  *                               are summed in a fixed order; `workspace` [dev] must hold
  *                               cbm_b200_dense_grad_weight_workspace(...) bytes.
+ *   cbm_b200_dense_forward_of_relu      y = max(x, 0) * w^T (`relu`: max of that and 0): the ReLU in front
+ *                               of a map that opens its layer, taken as x is read
+ *   cbm_b200_dense_grad_weight_of_relu  dw = dy^T * max(x, 0), the same map's weight gradient; its input
+ *                               gradient is cbm_b200_dense_grad_input_relu with h = x
  * ------------------------------------------------------------------------------------------ */
 #define CBM_B200_DENSE_MAX_CHUNKS 296
 int cbm_b200_dense_forward(const float* x, int64_t ldx, const float* w, int64_t ldw, float* y,
@@ -246,6 +250,11 @@ int cbm_b200_dense_grad_input(const float* dy, int64_t lddy, const float* w, int
 int cbm_b200_dense_grad_input_relu(const float* dy, int64_t lddy, const float* w, int64_t ldw, const float* h,
                                    int64_t ldh, float* dx, int64_t lddx, int32_t n_rows, int32_t n_in,
                                    int32_t n_out, void* stream);
+int cbm_b200_dense_forward_of_relu(const float* x, int64_t ldx, const float* w, int64_t ldw, float* y, int64_t ldy,
+                                   int32_t n_rows, int32_t n_in, int32_t n_out, int32_t relu, void* stream);
+int cbm_b200_dense_grad_weight_of_relu(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw, int64_t lddw,
+                                       int32_t n_rows, int32_t n_in, int32_t n_out, void* workspace,
+                                       int64_t workspace_bytes, void* stream);
 int64_t cbm_b200_dense_grad_weight_workspace(int32_t n_rows, int32_t n_in, int32_t n_out);
 int cbm_b200_dense_grad_weight(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw,
                                int64_t lddw, int32_t n_rows, int32_t n_in, int32_t n_out,

@@ -1,0 +1,57 @@
+"""The dense-map kernels at the edges of their tiles, blocks and passes, against float64."""
+import pytest
+import torch
+
+from cbm4gnn_b200 import dense
+
+pytestmark = pytest.mark.gpu
+
+
+def _operand(rows, cols, pad, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return torch.randn((rows, cols + pad), generator=g, device="cuda")[:, :cols]
+
+
+def _close(got, a, b):
+    """Within 3e-7 of sum |a||b|, what fp32 accuracy of every product and sum allows."""
+    want, scale = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    assert got.shape == want.shape
+    assert float(((got.double() - want).abs() / scale.clamp(min=1e-30)).max()) < 3e-7
+
+
+# rows: one, a tile's edge, more tiles than blocks; widths: one value, edges of the 16-, 32- and 64-deep steps, of the
+# 16-, 64- and 128-wide tiles, a contraction of several passes (1433 columns beside 128 results)
+@pytest.mark.parametrize("n,n_in,n_out", [(1, 1, 1), (127, 16, 15), (128, 17, 16), (129, 31, 17), (130, 33, 47), (257, 63, 64),
+                                          (200, 65, 65), (100, 127, 128), (333, 129, 130), (150, 300, 256), (70, 1433, 128),
+                                          (20000, 100, 257)])
+@pytest.mark.parametrize("pad", [0, 1, 4])
+def test_forward_and_gradients_at_tile_edges(n, n_in, n_out, pad):
+    x, w, gy = _operand(n, n_in, pad, 1), _operand(n_out, n_in, pad, 2), _operand(n, n_out, pad, 3)
+    xr = x.relu()
+    _close(dense.dense_forward(x, w), x, w.t())
+    _close(dense.dense_forward(x, w, relu_in=True), xr, w.t())
+    assert torch.equal(dense.dense_forward(x, w, relu=True), dense.dense_forward(x, w).relu())
+    gx = dense.dense_grad_input(gy, w)
+    _close(gx, gy, w)
+    masked = dense.dense_grad_input(gy, w, relu_output=x)  # the ReLU's input serves as well as its output
+    assert torch.equal(masked, torch.where(x > 0, gx, torch.zeros_like(gx)))
+    _close(dense.dense_grad_weight(gy, x), gy.t(), x)
+    _close(dense.dense_grad_weight(gy, x, relu_x=True), gy.t(), xr)
+
+
+def test_long_contraction_keeps_its_accuracy():
+    """Sums over many rows and columns are carried rounded, not cut off: the result drifts by no more than a few
+    units of fp32's last place."""
+    x, gy, w = _operand(60000, 256, 0, 4), _operand(60000, 64, 0, 5), _operand(64, 256, 0, 9)
+    for got, want in ((dense.dense_grad_weight(gy, x), gy.double().t() @ x.double()),
+                      (dense.dense_forward(x, w), x.double() @ w.double().t())):
+        assert float((got.double() - want).norm() / want.norm()) < 3e-7
+
+
+def test_relu_in_front_of_a_map_and_its_gradients():
+    a, w = _operand(500, 70, 0, 6).requires_grad_(True), _operand(20, 70, 0, 7).requires_grad_(True)
+    g = _operand(500, 20, 0, 8)
+    got = torch.autograd.grad(dense.relu_linear(a, w), (a, w), g)
+    want = torch.autograd.grad(a.double().relu() @ w.double().t(), (a, w), g.double())
+    for p, q in zip(got, want):
+        torch.testing.assert_close(p, q, atol=1e-5, rtol=1e-5)
