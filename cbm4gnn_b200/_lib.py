@@ -45,6 +45,7 @@ EXPORTED = [
     "cbm_b200_build",
     "cbm_b200_build_gpu",
     "cbm_b200_built_candidates_on_gpu",
+    "cbm_b200_edge_degrees",
     "cbm_b200_built_info",
     "cbm_b200_built_export_csr",
     "cbm_b200_built_export_coo",
@@ -162,6 +163,7 @@ def lib() -> ctypes.CDLL:
     sig("cbm_b200_build_gpu", c_int32, c_void_p, c_void_p, c_int64, c_int32, c_int32, c_void_p, c_int32, c_int32,
         POINTER(c_void_p))
     sig("cbm_b200_built_candidates_on_gpu", c_int32, c_void_p)
+    sig("cbm_b200_edge_degrees", c_int32, c_void_p, c_void_p, c_int64, i32p, c_void_p)
     sig("cbm_b200_built_info", c_int32, c_void_p, POINTER(c_int64), POINTER(c_int64), i32p, i32p,
         POINTER(c_double))
     sig("cbm_b200_built_export_csr", c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,

@@ -135,7 +135,9 @@ class cbm_matrix:
         row = _as_i32(ei[0])
         col = _as_i32(ei[1])
         # square matrix sized by the largest index present (cbm/cbm.py:15)
-        n = int(max(row.max(initial=-1), col.max(initial=-1))) + 1
+        n32 = ctypes.c_int32(0)
+        _lib.check(_lib.lib().cbm_b200_edge_degrees(_ptr(row), _ptr(col), row.shape[0], ctypes.byref(n32), None))
+        n = n32.value
         self.alpha = int(alpha)
         self.normalized = bool(normalized)
         self.num_rows = n
@@ -147,7 +149,8 @@ class cbm_matrix:
         else:
             # D^-1/2 from the row degrees of a binary matrix (cbm/cbm.py:34-41); a row without
             # entries gets inf exactly as there.
-            deg = torch.from_numpy(np.bincount(row, minlength=n).astype(np.float32))
+            deg = torch.empty(n)
+            _lib.check(_lib.lib().cbm_b200_edge_degrees(_ptr(row), _ptr(col), row.shape[0], ctypes.byref(n32), _ptr(deg)))
             self.col_multiplier = deg.pow(-0.5)
             mul = _as_f32(self.col_multiplier)
 
@@ -157,8 +160,8 @@ class cbm_matrix:
         self._plans: dict[int, _Plan] = {}
         self._transposed: "cbm_matrix | None" = None
 
-        crow64 = torch.from_numpy(self._crow.astype(np.int64))
-        col64 = torch.from_numpy(self._dcol.astype(np.int64))
+        crow64 = torch.from_numpy(self._crow).to(torch.int64)  # (torch converts on several threads)
+        col64 = torch.from_numpy(self._dcol).to(torch.int64)
         val = torch.from_numpy(self._dval)
         csr = torch.sparse_csr_tensor(crow64, col64, val, size=(n, n), check_invariants=False)
         if deltas_format == "coo":

@@ -39,27 +39,95 @@ double now_s() {
     return std::chrono::duration<double>(clk::now().time_since_epoch()).count();
 }
 
+// Memory that is not cleared first: the threads that fill it touch its pages, not one thread for all.
+template <class T>
+struct Raw {
+    std::unique_ptr<T[]> p;
+    size_t n = 0;
+    void alloc(size_t count) {
+        p.reset(count ? new T[count] : nullptr);
+        n = count;
+    }
+    T* data() { return p.get(); }
+    const T* data() const { return p.get(); }
+    size_t size() const { return n; }
+    bool empty() const { return n == 0; }
+    T& operator[](size_t i) { return p[i]; }
+    const T& operator[](size_t i) const { return p[i]; }
+};
+
 // ------------------------------------------------------------------------------------------
 // Pattern CSR with sorted, de-duplicated columns.
 // ------------------------------------------------------------------------------------------
 struct Pattern {
     i32 n = 0;
     std::vector<i64> ptr;  // n+1
-    std::vector<i32> idx;  // nnz
+    Raw<i32> idx;          // nnz
     i32 len(i32 r) const { return (i32)(ptr[r + 1] - ptr[r]); }
 };
+
+// Stable counting sort of `nnz` values by key in [0, n), several threads: each counts the keys of its own stretch of the
+// input, the counts are turned into places bucket by bucket, and each thread writes its stretch there.
+// key(i) and value(i) give the i-th element; ptr (n + 1) and out receive the buckets.
+template <class Key, class Value>
+void bucket_sort(i64 nnz, i32 n, Key key, Value value, std::vector<i64>& ptr, i32* out) {
+    // a stretch is worth a thread from some 100 000 elements on, and no more threads than the counters' memory bears out
+    const int T = (int)std::max<i64>(1, std::min<i64>({(i64)omp_get_max_threads(), nnz / 100000, nnz / std::max(n, 1) + 1}));
+    ptr.assign((size_t)n + 1, 0);
+    std::vector<std::vector<i32>> place((size_t)T);
+#pragma omp parallel num_threads(T)
+    {
+        const int t = omp_get_thread_num(), threads = omp_get_num_threads();
+        for (int q = t; q < T; q += threads) {
+            std::vector<i32>& mine = place[(size_t)q];
+            mine.assign((size_t)n, 0);
+            for (i64 i = nnz * q / T, e = nnz * (q + 1) / T; i < e; ++i) ++mine[(size_t)key(i)];
+        }
+#pragma omp barrier
+#pragma omp for schedule(static)
+        for (i32 k = 0; k < n; ++k) {  // places inside the bucket, and the bucket's size
+            i32 at = 0;
+            for (int q = 0; q < T; ++q) {
+                const i32 c = place[(size_t)q][k];
+                place[(size_t)q][k] = at;
+                at += c;
+            }
+            ptr[(size_t)k + 1] = at;
+        }
+#pragma omp single
+        for (i32 k = 0; k < n; ++k) ptr[(size_t)k + 1] += ptr[k];
+        for (int q = t; q < T; q += threads) {
+            std::vector<i32>& mine = place[(size_t)q];
+            for (i64 i = nnz * q / T, e = nnz * (q + 1) / T; i < e; ++i) {
+                const i32 k = key(i);
+                out[ptr[k] + mine[(size_t)k]++] = value(i);
+            }
+        }
+    }
+}
 
 Pattern make_csr(const i32* row, const i32* col, i64 nnz, i32 n) {
     Pattern p;
     p.n = n;
     p.ptr.assign((size_t)n + 1, 0);
-    for (i64 i = 0; i < nnz; ++i) p.ptr[(size_t)row[i] + 1]++;
-    for (i32 r = 0; r < n; ++r) p.ptr[r + 1] += p.ptr[r];
-    std::vector<i32> tmp((size_t)nnz);
-    {
-        std::vector<i64> cur(p.ptr.begin(), p.ptr.end() - 1);
-        for (i64 i = 0; i < nnz; ++i) tmp[(size_t)cur[row[i]]++] = col[i];
+    // The usual input is sorted by row and column without duplicates (a coalesced edge list): then it is the pattern.
+    bool sorted = true;
+#pragma omp parallel for schedule(static) reduction(&& : sorted)
+    for (i64 i = 1; i < nnz; ++i) sorted = sorted && (row[i - 1] < row[i] || (row[i - 1] == row[i] && col[i - 1] < col[i]));
+    if (sorted) {
+        p.idx.alloc((size_t)nnz);
+#pragma omp parallel for schedule(static)
+        for (i64 i = 0; i < nnz; ++i) {
+            p.idx[(size_t)i] = col[i];
+            if (i == 0 || row[i - 1] != row[i])  // the rows up to this one begin no later than here
+                for (i32 r = i == 0 ? 0 : row[i - 1] + 1; r <= row[i]; ++r) p.ptr[r] = i;
+        }
+        for (i32 r = nnz ? row[nnz - 1] + 1 : 0; r <= n; ++r) p.ptr[r] = nnz;
+        return p;
     }
+    Raw<i32> tmp;
+    tmp.alloc((size_t)nnz);
+    bucket_sort(nnz, n, [&](i64 i) { return row[i]; }, [&](i64 i) { return col[i]; }, p.ptr, tmp.data());
     // sort + dedupe each row, then compact
     std::vector<i32> newlen((size_t)n);
 #pragma omp parallel for schedule(dynamic, 256)
@@ -71,7 +139,7 @@ Pattern make_csr(const i32* row, const i32* col, i64 nnz, i32 n) {
     }
     std::vector<i64> nptr((size_t)n + 1, 0);
     for (i32 r = 0; r < n; ++r) nptr[r + 1] = nptr[r] + newlen[r];
-    p.idx.resize((size_t)nptr[n]);
+    p.idx.alloc((size_t)nptr[n]);
 #pragma omp parallel for schedule(static)
     for (i32 r = 0; r < n; ++r)
         std::copy(tmp.data() + p.ptr[r], tmp.data() + p.ptr[r] + newlen[r], p.idx.data() + nptr[r]);
@@ -82,14 +150,15 @@ Pattern make_csr(const i32* row, const i32* col, i64 nnz, i32 n) {
 Pattern transpose(const Pattern& a) {
     Pattern t;
     t.n = a.n;
-    t.ptr.assign((size_t)a.n + 1, 0);
-    for (i32 c : a.idx) t.ptr[(size_t)c + 1]++;
-    for (i32 r = 0; r < a.n; ++r) t.ptr[r + 1] += t.ptr[r];
-    t.idx.resize(a.idx.size());
-    std::vector<i64> cur(t.ptr.begin(), t.ptr.end() - 1);
-    for (i32 r = 0; r < a.n; ++r)
-        for (i64 k = a.ptr[r]; k < a.ptr[r + 1]; ++k) t.idx[(size_t)cur[a.idx[k]]++] = r;
-    return t;  // rows inside each column list come out ascending
+    const i64 nnz = (i64)a.idx.size();
+    t.idx.alloc((size_t)nnz);
+    Raw<i32> row_of;
+    row_of.alloc((size_t)nnz);
+#pragma omp parallel for schedule(static)
+    for (i32 r = 0; r < a.n; ++r) std::fill(row_of.data() + a.ptr[r], row_of.data() + a.ptr[r + 1], r);
+    // stable, so rows inside each column list come out ascending
+    bucket_sort(nnz, a.n, [&](i64 i) { return a.idx[(size_t)i]; }, [&](i64 i) { return row_of[(size_t)i]; }, t.ptr, t.idx.data());
+    return t;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -126,11 +195,12 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
     };
     // rank of every column in the rare-to-frequent order (ties by id)
     std::vector<i32> by_freq((size_t)n);
-    for (i32 c = 0; c < n; ++c) by_freq[c] = c;
-    std::sort(by_freq.begin(), by_freq.end(), [&](i32 x, i32 y) {
-        const i32 fx = at.len(x), fy = at.len(y);
-        return fx != fy ? fx < fy : x < y;
-    });
+    {
+        i32 most = 0;
+        for (i32 c = 0; c < n; ++c) most = std::max(most, at.len(c));
+        std::vector<i64> at_freq;
+        bucket_sort(n, most + 1, [&](i64 c) { return at.len((i32)c); }, [](i64 c) { return (i32)c; }, at_freq, by_freq.data());
+    }
     std::vector<i32> rank((size_t)n);
     for (i32 i = 0; i < n; ++i) rank[by_freq[i]] = i;
 
@@ -144,7 +214,8 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
         const double t_a = now_s();
         // rows with their columns replaced by ranks, rarest first: a prefix of such a row is the
         // set of its rarest columns
-        std::vector<i32> row_rank(a.idx.size());
+        Raw<i32> row_rank;
+        row_rank.alloc(a.idx.size());
 #pragma omp parallel for schedule(dynamic, 256)
         for (i32 r = 0; r < n; ++r) {
             i32* b = row_rank.data() + a.ptr[r];
@@ -173,7 +244,10 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
     }
     std::vector<i32>().swap(by_freq);
     const bool host_all = on_host.empty();
+    bool any_host = host_all;
+    for (char h : on_host) any_host = any_host || h;
 
+    if (any_host) {
 #pragma omp parallel
     {
         std::vector<uint64_t> in_u(((size_t)n + 63) / 64, 0);  // bit per column: is it in row u?
@@ -260,7 +334,8 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
         }
     }
 
-    if (!host_all) {  // parents finished on the host were appended behind the GPU's: restore (parent, child) order
+    }
+    if (!host_all && any_host) {  // parents finished on the host were appended behind the GPU's: restore (parent, child) order
 #pragma omp parallel for schedule(dynamic, 16)
         for (i32 b = 0; b < n_blocks; ++b)
             std::sort(found[b].begin(), found[b].end(),
@@ -355,6 +430,14 @@ bool solve_arborescence(const Candidates& g, i32 n, Arborescence& out, std::stri
     const i32 SETTLED = -1;
     std::vector<i32> mark((size_t)V, 0);  // 0 fresh, >0 id of the path it is on, SETTLED
     mark[n] = SETTLED;
+    out.parent.assign((size_t)n, -1);
+    // A vertex whose only in-edge is the virtual one hangs off the root whatever the others choose (most vertices of a
+    // graph that compresses little): it takes no part in the search.
+    for (i32 v = 0; v < n; ++v)
+        if (g.off[v + 1] - g.off[v] == 1) {
+            out.parent[v] = n;
+            mark[v] = SETTLED;
+        }
     std::vector<i32> path;
 
     for (i32 s = 0; s < n; ++s) {
@@ -468,7 +551,6 @@ bool solve_arborescence(const Candidates& g, i32 n, Arborescence& out, std::stri
     std::vector<i32> roots;
     for (i32 x = F - 1; x >= 0; --x)
         if (f_parent[x] < 0) roots.push_back(x);
-    out.parent.assign((size_t)n, -1);
     while (!roots.empty()) {
         const i32 top = roots.back();
         roots.pop_back();
@@ -513,8 +595,8 @@ struct cbm_b200_built {
     std::vector<i32> mst_col;    // n
     std::vector<i32> bfs;        // n, visiting order
     std::vector<i32> d_crow;     // n+1
-    std::vector<i32> d_col;
-    std::vector<float> d_val;
+    Raw<i32> d_col;
+    Raw<float> d_val;
     i64 n_candidates = 0;
     i32 n_root_children = 0;
     i32 depth = 0;
@@ -548,12 +630,16 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
     if (n < 0 || nnz < 0 || (nnz > 0 && (!row || !col)))
         return cbm::fail(CBM_B200_ERR_ARG, "build: bad sizes or NULL index arrays");
     if (n >= INT32_MAX - 2) return cbm::fail(CBM_B200_ERR_ARG, "build: n too large for int32");
-    for (i64 i = 0; i < nnz; ++i)
-        if (row[i] < 0 || row[i] >= n || col[i] < 0 || col[i] >= n)
-            return cbm::fail(CBM_B200_ERR_ARG, "build: index out of range at entry " +
-                                                   std::to_string(i));
     const int prev_threads = omp_get_max_threads();
     if (n_threads > 0) omp_set_num_threads(n_threads);
+    i64 outside = nnz;  // first entry out of range
+#pragma omp parallel for schedule(static) reduction(min : outside)
+    for (i64 i = 0; i < nnz; ++i)
+        if (row[i] < 0 || row[i] >= n || col[i] < 0 || col[i] >= n) outside = std::min(outside, i);
+    if (outside < nnz) {
+        if (n_threads > 0) omp_set_num_threads(prev_threads);
+        return cbm::fail(CBM_B200_ERR_ARG, "build: index out of range at entry " + std::to_string(outside));
+    }
     int status = CBM_B200_OK;
     try {
         // owned until it is handed to the caller: an exception on the way frees it
@@ -561,13 +647,14 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
         b->n = n;
         const double t0 = now_s();
         Pattern a = make_csr(row, col, nnz, n);
+        b->seconds[3] = now_s() - t0;
         Arborescence arb;
         {
             Pattern at = transpose(a);
             bool on_gpu = false;
             Candidates g = make_candidates(a, at, alpha, device, &on_gpu);
             b->candidates_on_gpu = on_gpu ? 1 : 0;
-            std::vector<i32>().swap(at.idx);
+            at.idx.alloc(0);
             b->n_candidates = g.total;
             const double t1 = now_s();
             b->seconds[0] = t1 - t0;
@@ -651,8 +738,8 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
             }
             b->d_crow[v + 1] = (i32)total;
         }
-        b->d_col.resize((size_t)total);
-        b->d_val.resize((size_t)total);
+        b->d_col.alloc((size_t)total);
+        b->d_val.alloc((size_t)total);
 #pragma omp parallel for schedule(dynamic, 512)
         for (i32 v = 0; v < n; ++v) {
             const i32 u = arb.parent[v];
@@ -684,6 +771,9 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
             for (; pu < eu; ++pu) emit(*pu, false);
             for (; pv < ev; ++pv) emit(*pv, true);
         }
+        if (std::getenv("CBM_B200_BUILD_TRACE"))
+            std::fprintf(stderr, "[cbm build] csr %.4f, transpose + candidates %.4f, arborescence %.4f, tree + deltas %.4f s\n", b->seconds[3],
+                         b->seconds[0] - b->seconds[3], b->seconds[1], now_s() - t2);
         b->seconds[2] = now_s() - t2;
         b->seconds[3] = now_s() - t0;
         *out = b.release();
@@ -719,8 +809,12 @@ extern "C" int cbm_b200_built_export_csr(const cbm_b200_built* b, int32_t* mst_r
     std::copy(b->mst_row.begin(), b->mst_row.end(), mst_row);
     std::copy(b->mst_col.begin(), b->mst_col.end(), mst_col);
     std::copy(b->d_crow.begin(), b->d_crow.end(), delta_crow);
-    std::copy(b->d_col.begin(), b->d_col.end(), delta_col);
-    std::copy(b->d_val.begin(), b->d_val.end(), delta_val);
+    const i64 total = (i64)b->d_col.size();
+#pragma omp parallel for schedule(static)
+    for (i64 i = 0; i < total; ++i) {
+        delta_col[i] = b->d_col[(size_t)i];
+        delta_val[i] = b->d_val[(size_t)i];
+    }
     if (parent) std::copy(b->parent.begin(), b->parent.end(), parent);
     return CBM_B200_OK;
 }
@@ -741,3 +835,43 @@ extern "C" int cbm_b200_built_export_coo(const cbm_b200_built* b, int32_t* delta
 }
 
 extern "C" void cbm_b200_built_free(cbm_b200_built* b) { delete b; }
+
+extern "C" int cbm_b200_edge_degrees(const int32_t* row, const int32_t* col, int64_t nnz, int32_t* n, float* degree) {
+    if (!n || nnz < 0 || (nnz > 0 && (!row || !col))) return cbm::fail(CBM_B200_ERR_ARG, "edge_degrees: bad arguments");
+    if (!degree) {
+        i32 most = -1;
+        bool negative = false;
+#pragma omp parallel for schedule(static) reduction(max : most) reduction(|| : negative)
+        for (i64 i = 0; i < nnz; ++i) {
+            most = std::max(most, std::max(row[i], col[i]));
+            negative = negative || row[i] < 0;
+        }
+        if (negative) return cbm::fail(CBM_B200_ERR_ARG, "edge_degrees: negative row index");
+        *n = most + 1;
+        return CBM_B200_OK;
+    }
+    const i32 rows = *n;
+    std::vector<i32> count;
+    try {
+        count.assign((size_t)std::max(rows, 0), 0);
+    } catch (const std::bad_alloc&) {
+        return cbm::fail(CBM_B200_ERR_ALLOC, "edge_degrees: out of host memory");
+    }
+    // runs of equal rows (the edges are usually sorted by row) cost one addition each
+#pragma omp parallel for schedule(static)
+    for (i64 b = 0; b < nnz; b += 4096) {
+        const i64 e = std::min<i64>(nnz, b + 4096);
+        for (i64 i = b; i < e;) {
+            i64 j = i + 1;
+            while (j < e && row[j] == row[i]) ++j;
+            if (row[i] >= 0 && row[i] < rows) {
+#pragma omp atomic
+                count[(size_t)row[i]] += (i32)(j - i);
+            }
+            i = j;
+        }
+    }
+#pragma omp parallel for schedule(static)
+    for (i32 r = 0; r < rows; ++r) degree[r] = (float)count[(size_t)r];
+    return CBM_B200_OK;
+}

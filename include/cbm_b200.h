@@ -69,6 +69,11 @@ int cbm_b200_build_gpu(const int32_t* row, const int32_t* col, int64_t nnz, int3
                        const float* col_mul, int32_t n_threads, int32_t device, cbm_b200_built** out);
 int cbm_b200_built_candidates_on_gpu(const cbm_b200_built* b);
 
+/* Size and row degrees of an edge list [host]: with degree == NULL, *n = 1 + the largest index present
+ * (0 for an empty list); else degree[0 .. *n) = the number of entries of each row, as floats (the
+ * multiplier of the normalized form is their -1/2 power, cbm/cbm.py:34-41). */
+int cbm_b200_edge_degrees(const int32_t* row, const int32_t* col, int64_t nnz, int32_t* n, float* degree);
+
 /* Sizes and statistics of a built structure.  Any out-pointer may be NULL.
  *   n_delta       number of delta entries (= total weight of the arborescence)
  *   n_candidates  number of candidate edges offered to the solver, virtual edges included
