@@ -123,7 +123,8 @@ void cbm_b200_plan_destroy(cbm_b200_plan* p);
 /* Host-only twin of cbm_b200_plan_create (same arguments minus the device): builds the schedule,
  * runs the pre-launch checks (every item waits only for earlier items, whoever is waited for
  * publishes, every row produced and every parked partial sum collected exactly once) and reports
- * its sizes.  Needs no GPU; plan_create runs the same checks. */
+ * its sizes.  Needs no GPU; plan_create runs the same checks (on a graph whose mean row is short it cuts long
+ * rows finer than reported here, and a graph with communities it orders by them). */
 int cbm_b200_schedule_info(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
                            const int32_t* delta_crow, const int32_t* delta_col,
                            const float* delta_val, const float* multiplier, const int32_t* perm,
