@@ -567,7 +567,8 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
 // pointers) and the update-only mode, which gathers nothing; it is also the default form.
 // UNROLL = row fetches in flight per lane, MINB = thread blocks the register budget must allow
 // per SM.
-template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false>
+// NARROW: every slab is at most 64 columns wide.
+template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false, bool NARROW = false>
 __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
     using V = Vec<V4>;
     using T = typename V::T;
@@ -602,7 +603,10 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
 #pragma unroll
                 for (int v = 0; v < NV; ++v) acc[v] = V::zero();
                 const i32 len = (info >> ITEM_LEN_SHIFT) & 0xff;
-                if constexpr (NV == 1) {
+                if constexpr (NARROW) {
+                    gather_row_narrow<V4, UNROLL>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0, p.ldx, wcols,
+                                                  lanes_log2<V::E>(wcols), acc[0], lane);
+                } else if constexpr (NV == 1) {
                     if (wcols <= 16 * V::E && !p.in_turn)
                         gather_row_narrow<V4, UNROLL>(PairEntries{p.ent}, db.x, db.x + len, p.x + c0, p.ldx, wcols,
                                                       lanes_log2<V::E>(wcols), acc[0], lane);
@@ -1623,6 +1627,20 @@ int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
     return CBM_B200_OK;
 }
 
+// Operands of at most 64 columns: a kernel of their own, whose smaller register need keeps 48 warps resident also where
+// rows of y are not aligned.  Fetches in flight x resident blocks, 235 868 rows of 11 entries, 64 columns / 400 000 of
+// 22, 47 columns: 4 x 6 97 / 279 us, 6 x 5 100 / 288, 8 x 5 104 / 298, 8 x 4 110 / 310.
+template <bool RAGGED>
+int launch_narrow(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
+    constexpr int kResident = 6;
+    int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
+    blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
+    kp.n_warps = (u64)blocks * 8;
+    cbm_items_kernel<1, true, 4, kResident, RAGGED, true><<<blocks, 256, 0, s>>>(kp);
+    CBM_CUDA(cudaGetLastError());
+    return CBM_B200_OK;
+}
+
 template <bool RAGGED>
 int launch_chunks(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
     constexpr int kResident = 3;  // 45 consumer warps per SM at 40 registers
@@ -1701,6 +1719,8 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     if (c.chunked)
         return c.ragged ? launch_chunks<true>(kp, p->n_blocks, p->sm_count, s)
                         : launch_chunks<false>(kp, p->n_blocks, p->sm_count, s);
+    if (c.sh.v4 && c.sh.nv == 1 && f <= 64 && mode != MODE_UPDATE_ONLY)
+        return c.ragged ? launch_narrow<true>(kp, p->n_blocks, p->sm_count, s) : launch_narrow<false>(kp, p->n_blocks, p->sm_count, s);
     if (c.ragged) {
         if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, p->n_blocks, p->sm_count, s);
         if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, p->n_blocks, p->sm_count, s);
