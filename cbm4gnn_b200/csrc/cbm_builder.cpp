@@ -34,6 +34,10 @@ namespace {
 using i32 = int32_t;
 using i64 = int64_t;
 
+// Work (in elements) from which a loop is shared between threads: below it, waking them takes longer than the loop, and
+// they go on spinning beside whatever the caller does next.
+constexpr i64 SHARED_WORK = 200000;
+
 double now_s() {
     using clk = std::chrono::steady_clock;
     return std::chrono::duration<double>(clk::now().time_since_epoch()).count();
@@ -112,11 +116,11 @@ Pattern make_csr(const i32* row, const i32* col, i64 nnz, i32 n) {
     p.ptr.assign((size_t)n + 1, 0);
     // The usual input is sorted by row and column without duplicates (a coalesced edge list): then it is the pattern.
     bool sorted = true;
-#pragma omp parallel for schedule(static) reduction(&& : sorted)
+#pragma omp parallel for schedule(static) reduction(&& : sorted) if (nnz > SHARED_WORK)
     for (i64 i = 1; i < nnz; ++i) sorted = sorted && (row[i - 1] < row[i] || (row[i - 1] == row[i] && col[i - 1] < col[i]));
     if (sorted) {
         p.idx.alloc((size_t)nnz);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nnz > SHARED_WORK)
         for (i64 i = 0; i < nnz; ++i) {
             p.idx[(size_t)i] = col[i];
             if (i == 0 || row[i - 1] != row[i])  // the rows up to this one begin no later than here
@@ -130,7 +134,7 @@ Pattern make_csr(const i32* row, const i32* col, i64 nnz, i32 n) {
     bucket_sort(nnz, n, [&](i64 i) { return row[i]; }, [&](i64 i) { return col[i]; }, p.ptr, tmp.data());
     // sort + dedupe each row, then compact
     std::vector<i32> newlen((size_t)n);
-#pragma omp parallel for schedule(dynamic, 256)
+#pragma omp parallel for schedule(dynamic, 256) if (nnz > SHARED_WORK)
     for (i32 r = 0; r < n; ++r) {
         i32* b = tmp.data() + p.ptr[r];
         i32* e = tmp.data() + p.ptr[r + 1];
@@ -140,7 +144,7 @@ Pattern make_csr(const i32* row, const i32* col, i64 nnz, i32 n) {
     std::vector<i64> nptr((size_t)n + 1, 0);
     for (i32 r = 0; r < n; ++r) nptr[r + 1] = nptr[r] + newlen[r];
     p.idx.alloc((size_t)nptr[n]);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nnz > SHARED_WORK)
     for (i32 r = 0; r < n; ++r)
         std::copy(tmp.data() + p.ptr[r], tmp.data() + p.ptr[r] + newlen[r], p.idx.data() + nptr[r]);
     p.ptr.swap(nptr);
@@ -154,7 +158,7 @@ Pattern transpose(const Pattern& a) {
     t.idx.alloc((size_t)nnz);
     Raw<i32> row_of;
     row_of.alloc((size_t)nnz);
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nnz > SHARED_WORK)
     for (i32 r = 0; r < a.n; ++r) std::fill(row_of.data() + a.ptr[r], row_of.data() + a.ptr[r + 1], r);
     // stable, so rows inside each column list come out ascending
     bucket_sort(nnz, a.n, [&](i64 i) { return a.idx[(size_t)i]; }, [&](i64 i) { return row_of[(size_t)i]; }, t.ptr, t.idx.data());
@@ -216,7 +220,7 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
         // set of its rarest columns
         Raw<i32> row_rank;
         row_rank.alloc(a.idx.size());
-#pragma omp parallel for schedule(dynamic, 256)
+#pragma omp parallel for schedule(dynamic, 256) if ((i64)a.idx.size() > SHARED_WORK)
         for (i32 r = 0; r < n; ++r) {
             i32* b = row_rank.data() + a.ptr[r];
             for (i64 k = a.ptr[r]; k < a.ptr[r + 1]; ++k) row_rank[(size_t)k] = rank[a.idx[(size_t)k]];
@@ -236,7 +240,7 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
             for (i32 u : left) on_host[u] = 1;
             // in the order the host search emits: by parent block, inside a block by (parent, child)
             for (const cbm::CandTriple& t : triples) found[(size_t)(t.src / block)].push_back({t.src, t.dst, t.w});
-#pragma omp parallel for schedule(dynamic, 16)
+#pragma omp parallel for schedule(dynamic, 16) if ((i64)triples.size() > SHARED_WORK)
             for (i32 b = 0; b < n_blocks; ++b)
                 std::sort(found[b].begin(), found[b].end(),
                           [](const Tri& x, const Tri& y) { return x.src != y.src ? x.src < y.src : x.dst < y.dst; });
@@ -633,7 +637,7 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
     const int prev_threads = omp_get_max_threads();
     if (n_threads > 0) omp_set_num_threads(n_threads);
     i64 outside = nnz;  // first entry out of range
-#pragma omp parallel for schedule(static) reduction(min : outside)
+#pragma omp parallel for schedule(static) reduction(min : outside) if (nnz > SHARED_WORK)
     for (i64 i = 0; i < nnz; ++i)
         if (row[i] < 0 || row[i] >= n || col[i] < 0 || col[i] >= n) outside = std::min(outside, i);
     if (outside < nnz) {
@@ -705,7 +709,7 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
         // deltas by sorted merge (cbm/cbm_extensions.cpp:186-261; values :504-584 when col_mul)
         b->d_crow.assign((size_t)n + 1, 0);
         std::vector<i32> dlen((size_t)n, 0);
-#pragma omp parallel for schedule(dynamic, 512)
+#pragma omp parallel for schedule(dynamic, 512) if ((i64)a.idx.size() > SHARED_WORK)
         for (i32 v = 0; v < n; ++v) {
             const i32 u = arb.parent[v];
             if (u == n) {
@@ -740,7 +744,7 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
         }
         b->d_col.alloc((size_t)total);
         b->d_val.alloc((size_t)total);
-#pragma omp parallel for schedule(dynamic, 512)
+#pragma omp parallel for schedule(dynamic, 512) if ((i64)a.idx.size() > SHARED_WORK)
         for (i32 v = 0; v < n; ++v) {
             const i32 u = arb.parent[v];
             i32* oc = b->d_col.data() + b->d_crow[v];
@@ -810,7 +814,7 @@ extern "C" int cbm_b200_built_export_csr(const cbm_b200_built* b, int32_t* mst_r
     std::copy(b->mst_col.begin(), b->mst_col.end(), mst_col);
     std::copy(b->d_crow.begin(), b->d_crow.end(), delta_crow);
     const i64 total = (i64)b->d_col.size();
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (total > SHARED_WORK)
     for (i64 i = 0; i < total; ++i) {
         delta_col[i] = b->d_col[(size_t)i];
         delta_val[i] = b->d_val[(size_t)i];
@@ -841,7 +845,7 @@ extern "C" int cbm_b200_edge_degrees(const int32_t* row, const int32_t* col, int
     if (!degree) {
         i32 most = -1;
         bool negative = false;
-#pragma omp parallel for schedule(static) reduction(max : most) reduction(|| : negative)
+#pragma omp parallel for schedule(static) reduction(max : most) reduction(|| : negative) if (nnz > SHARED_WORK)
         for (i64 i = 0; i < nnz; ++i) {
             most = std::max(most, std::max(row[i], col[i]));
             negative = negative || row[i] < 0;
@@ -858,7 +862,7 @@ extern "C" int cbm_b200_edge_degrees(const int32_t* row, const int32_t* col, int
         return cbm::fail(CBM_B200_ERR_ALLOC, "edge_degrees: out of host memory");
     }
     // runs of equal rows (the edges are usually sorted by row) cost one addition each
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (nnz > SHARED_WORK)
     for (i64 b = 0; b < nnz; b += 4096) {
         const i64 e = std::min<i64>(nnz, b + 4096);
         for (i64 i = b; i < e;) {
@@ -871,7 +875,7 @@ extern "C" int cbm_b200_edge_degrees(const int32_t* row, const int32_t* col, int
             i = j;
         }
     }
-#pragma omp parallel for schedule(static)
+#pragma omp parallel for schedule(static) if (rows > SHARED_WORK)
     for (i32 r = 0; r < rows; ++r) degree[r] = (float)count[(size_t)r];
     return CBM_B200_OK;
 }

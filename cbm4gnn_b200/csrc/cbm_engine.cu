@@ -23,6 +23,7 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <new>
 #include <string>
 #include <utility>
@@ -562,6 +563,63 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
     return true;
 }
 
+#ifndef RN
+#define RN 4
+#define NR 6
+#define NG 4
+#endif
+// Several whole rows that wait for nobody (prefix items, positions [first, end), none of them PARTIAL) by one warp, 2^lg
+// lanes for each: for slabs of at most 16 vectors, where a row's fixed costs - descriptor, entries, store, each a trip to
+// memory - outweigh its fetches.  Neighbours in the prefix are of about equal length.
+template <bool V4, bool RAGGED, int UNROLL>
+__device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 first, i32 end, i32 c0, i32 wcols, int lg, int lane) {
+    using V = Vec<V4>;
+    using T = typename V::T;
+    const int width = 1 << lg, li = lane & (width - 1);
+    const bool has = li * V::E < wcols;
+    const float* xs = p.x + c0 + li * V::E;
+    for (i32 base = first; base < end; base += 32 >> lg) {
+        const i32 pos = base + (lane >> lg);
+        const bool on = pos < end;
+        const int4 da = __ldg((const int4*)(p.desc + min(pos, end - 1)));
+        const int4 db = __ldg((const int4*)(p.desc + min(pos, end - 1)) + 1);
+        const i32 len = on ? (da.w >> ITEM_LEN_SHIFT) & 0xff : 0;
+        const i32 most = (i32)__reduce_max_sync(0xffffffffu, (unsigned)len);
+        T acc = V::zero();
+        for (i32 b = 0; b < most; b += width) {
+            i32 mc = 0;
+            float mw = 0.f;
+            if (b + li < len) PairEntries{p.ent}.get(db.x + b + li, mc, mw);
+            const i32 here = min(width, most - b);
+            for (i32 j = 0; j < here; j += UNROLL) {
+                T t[UNROLL];
+#pragma unroll
+                for (int k = 0; k < UNROLL; ++k) {
+                    const i32 c = __shfl_sync(0xffffffffu, mc, j + k, width);
+                    t[k] = V::ld_ro_if(xs + (i64)c * p.ldx, has && j + k < here && b + j + k < len);
+                }
+#pragma unroll
+                for (int k = 0; k < UNROLL; ++k) {
+                    const float w = __shfl_sync(0xffffffffu, mw, j + k, width);
+                    acc = V::fma(j + k < here && b + j + k < len ? w : 0.f, t[k], acc);
+                }
+            }
+        }
+        if (p.use_scale && p.mode != MODE_DELTA_ONLY) acc = V::mul(__int_as_float(db.z), acc);
+        if (on && has) {
+            const i32 col = c0 + li * V::E, some = p.f - col;
+            float* y = p.y + (i64)da.x * p.ldy + col;
+            if (RAGGED && !(p.y_vec && some >= V::E)) V::st_some(y, acc, some);
+            else if (da.w & ITEM_PUBLISH) V::st(y, acc);
+            else V::st_stream(y, acc);
+        }
+        if (p.mode != MODE_DELTA_ONLY) {
+            __syncwarp();
+            if (on && li == 0 && (da.w & ITEM_PUBLISH)) st_release(p.flags + (i64)slab * p.n_items + pos, p.epoch);
+        }
+    }
+}
+
 // Product kernel, register form: one warp per (item, column slab), the gather held in registers.
 // Serves operands the bulk-copy form cannot take (width not a multiple of 4 floats, unaligned
 // pointers) and the update-only mode, which gathers nothing; it is also the default form.
@@ -589,6 +647,13 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
         bool ok[NV];
 #pragma unroll
         for (int v = 0; v < NV; ++v) ok[v] = (lane * V::E + v * STEP) < wcols;
+        if constexpr (NARROW) {
+            const int lg = lanes_log2<V::E>(wcols);
+            if (lg >= 3 && count > 1 && first >= p.n_partial && first + count <= p.n_prefix && p.n_bcast == 0) {
+                rows_narrow<V4, RAGGED, RN>(p, slab, first, first + count, c0, wcols, lg, lane);
+                continue;
+            }
+        }
         for (i32 pos = first; pos < first + count; ++pos) {
             const int4 da = __ldg((const int4*)(p.desc + pos));
             const int4 db = __ldg((const int4*)(p.desc + pos) + 1);
@@ -921,13 +986,13 @@ struct Shape {
 // 0.55 / 0.71 ms against 0.63 / 0.77 ms for 256 columns; 236 000 rows, width 256: 0.307 against
 // 0.324 ms): the one-vector form holds eight row fetches per lane in 56 registers and keeps 32 warps
 // per SM, the two-vector form four fetches in 72 registers and 24 warps.
-i32 default_slab_v4(i64 /*n_labels*/) { return 128; }
+constexpr i32 DEFAULT_SLAB = 128;
 
-Shape pick_shape(i32 f, i32 want_slab, bool can_v4, i64 n_labels) {
+Shape pick_shape(i32 f, i32 want_slab, bool can_v4) {
     Shape s{};
     s.v4 = can_v4;
     const i32 lane_w = s.v4 ? 128 : 32;  // columns covered by one vector per lane
-    i32 slab = want_slab > 0 ? want_slab : (s.v4 ? default_slab_v4(n_labels) : 64);
+    i32 slab = want_slab > 0 ? want_slab : (s.v4 ? DEFAULT_SLAB : 64);
     if (s.v4 && (want_slab == 64 || want_slab == 32)) {  // narrow slabs on request: half-warp gather
         s.nv = 1;
         s.slab_w = want_slab;
@@ -1007,13 +1072,12 @@ struct DeviceGuard {
 };
 
 template <class T>
-int upload(T** dst, const std::vector<T>& src, i64& bytes) {
+int upload(T** dst, const T* src, size_t count, i64& bytes) {
     *dst = nullptr;
-    const size_t sz = std::max<size_t>(src.size(), 1) * sizeof(T);
+    const size_t sz = std::max<size_t>(count, 1) * sizeof(T);
     CBM_CUDA(cudaMalloc((void**)dst, sz));
     bytes += (i64)sz;
-    if (!src.empty())
-        CBM_CUDA(cudaMemcpy(*dst, src.data(), src.size() * sizeof(T), cudaMemcpyHostToDevice));
+    if (count) CBM_CUDA(cudaMemcpy(*dst, src, count * sizeof(T), cudaMemcpyHostToDevice));
     return CBM_B200_OK;
 }
 
@@ -1045,7 +1109,8 @@ namespace {
 // The host-side schedule of one plan, before anything touches the device.
 struct Schedule {
     std::vector<RowDesc> desc;
-    std::vector<Entry> ent;
+    std::unique_ptr<Entry[]> ent;  // not cleared first: the threads that fill it touch its pages
+    i64 n_ent = 0;
     std::vector<Chunk> chunks;  // clustered plans
     bool clustered = false;
     i64 n_delta = 0;
@@ -1092,7 +1157,7 @@ int validate_schedule(const Schedule& sch, i32 n_out) {
             }
         }
     }
-    if (cursor != (i64)sch.ent.size()) return bad("entries not covered exactly once");
+    if (cursor != sch.n_ent) return bad("entries not covered exactly once");
     i32 at = 0;
     for (const Chunk& c : sch.chunks) {
         if (c.first != at || c.count <= 0 || c.count > MAX_CHUNK_ITEMS) return bad("chunks do not follow one another");
@@ -1113,7 +1178,7 @@ int validate_schedule(const Schedule& sch, i32 n_out) {
 // Cuts a clustered schedule into the chunks that blocks claim.
 void make_chunks(Schedule& sch, i32 n_prefix) {
     const i32 n_items = (i32)sch.desc.size();
-    auto end_of = [&](i32 i) { return i + 1 < n_items ? sch.desc[i + 1].beg : (i32)sch.ent.size(); };
+    auto end_of = [&](i32 i) { return i + 1 < n_items ? sch.desc[i + 1].beg : (i32)sch.n_ent; };
     Chunk c{0, 0, 0, 0};
     for (i32 i = 0; i < n_items; ++i) {
         const i32 most = i < n_prefix ? MAX_CHUNK_ITEMS : MAX_CHUNK_ITEMS / 2;
@@ -1273,14 +1338,16 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
             owned_rows.push_back(v);
         }
     std::vector<RowDesc>& desc = sch.desc;
-    std::vector<Entry>& ent = sch.ent;
     std::vector<i32> rank;
     sch.clustered = col_bound == n && cluster_order(n, delta_crow, delta_col, parent, device, rank);
-    ent.reserve((size_t)nd_all + (sch.clustered ? (size_t)n : 0));
+    // items get their entry ranges now; the entries are filled in at the end, on several threads
+    std::vector<i64> source;  // per item: its first entry in the delta arrays
+    source.reserve((size_t)n);
     auto append_entries = [&](i32 v, i32 from, i32 to) {  // entries [from, to) of row v
-        const i32 beg = (i32)ent.size();
-        for (i32 k = delta_crow[v] + from; k < delta_crow[v] + to; ++k) ent.push_back(Entry{label(delta_col[k]), delta_val[k]});
-        if (sch.clustered && ent.size() % 2) ent.push_back(Entry{0, 0.0f});
+        const i32 beg = (i32)sch.n_ent;
+        source.push_back((i64)delta_crow[v] + from);
+        sch.n_ent += to - from;
+        if (sch.clustered) sch.n_ent += sch.n_ent % 2;
         return beg;
     };
     for (i32 v : owned_rows) sch.n_delta += row_len(v);
@@ -1338,7 +1405,13 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
                 return la != lb ? la > lb : rank[a] < rank[b];
             });
         else
-            std::stable_sort(easy.begin(), easy.end(), [&](i32 a, i32 b) { return row_len(a) > row_len(b); });
+            {   // counting sort, stable
+                std::vector<i32> place((size_t)SPLIT_OVER + 2, 0), sorted(easy.size());
+                for (i32 v : easy) ++place[(size_t)(SPLIT_OVER - row_len(v)) + 1];
+                for (i32 l = 0; l <= SPLIT_OVER; ++l) place[l + 1] += place[l];
+                for (i32 v : easy) sorted[(size_t)place[(size_t)(SPLIT_OVER - row_len(v))]++] = v;
+                easy.swap(sorted);
+            }
         for (i32 v : easy) add_row_item(v);
     }
     const i32 n_prefix = (i32)desc.size();
@@ -1351,6 +1424,17 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
             return level[a] != level[b] ? level[a] < level[b] : rank[a] < rank[b];
         });
     for (i32 v : rest) add_row_item(v);
+    sch.ent.reset(new Entry[(size_t)std::max<i64>(sch.n_ent, 1)]);
+    const i32 n_items = (i32)desc.size();
+    // (half of the threads: those that have finished spin for a while, beside the caller's first product)
+    const int threads = (int)std::max<i64>(1, std::min<i64>(omp_get_max_threads() / 2, sch.n_ent / 100000));
+#pragma omp parallel for schedule(static) num_threads(threads)
+    for (i32 i = 0; i < n_items; ++i) {
+        const i32 len = (desc[i].info >> ITEM_LEN_SHIFT) & 0xff;
+        Entry* e = sch.ent.get() + desc[i].beg;
+        for (i32 k = 0; k < len; ++k) e[k] = Entry{label(delta_col[source[i] + k]), delta_val[source[i] + k]};
+        if (sch.clustered && len % 2) e[len] = Entry{0, 0.0f};
+    }
     if (sch.clustered) make_chunks(sch, n_prefix);
     sch.n_rows_owned = (i32)owned_rows.size();
     sch.n_prefix = n_prefix;
@@ -1442,11 +1526,11 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
     p->n_root_children = n_root_children;
     p->depth = depth;
     p->normalized = normalized;
-    cudaDeviceProp prop{};
-    if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) p->sm_count = prop.multiProcessorCount;
-    int rc = upload(&p->d_desc, desc, p->device_bytes);
-    if (rc == CBM_B200_OK) rc = upload(&p->d_ent, sch.ent, p->device_bytes);
-    if (rc == CBM_B200_OK && sch.clustered) rc = upload(&p->d_chunks, sch.chunks, p->device_bytes);
+    int sms = 0;  // (the one attribute: all properties together take milliseconds)
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) p->sm_count = sms;
+    int rc = upload(&p->d_desc, desc.data(), desc.size(), p->device_bytes);
+    if (rc == CBM_B200_OK) rc = upload(&p->d_ent, sch.ent.get(), (size_t)sch.n_ent, p->device_bytes);
+    if (rc == CBM_B200_OK && sch.clustered) rc = upload(&p->d_chunks, sch.chunks.data(), sch.chunks.size(), p->device_bytes);
     if (rc == CBM_B200_OK) {
         cudaError_t e = cudaMalloc((void**)&p->d_counter, 2 * sizeof(u64));
         if (e == cudaSuccess) e = cudaMemset(p->d_counter, 0, 2 * sizeof(u64));
@@ -1456,6 +1540,20 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
         if (e != cudaSuccess)
             rc = cbm::fail(CBM_B200_ERR_CUDA, std::string("plan_create: ") + cudaGetErrorString(e));
         p->device_bytes += 16;
+    }
+    if (rc == CBM_B200_OK) {
+        // ready flags for operands of up to 512 columns and parked sums for one slab: most products then allocate nothing
+        const i64 flags = 4 * (i64)p->n_items, slots = (i64)p->n_partial * DEFAULT_SLAB;
+        cudaError_t e = flags ? cudaMalloc((void**)&p->d_flags, (size_t)flags * sizeof(i32)) : cudaSuccess;
+        if (e == cudaSuccess && flags) e = cudaMemset(p->d_flags, 0, (size_t)flags * sizeof(i32));
+        if (e == cudaSuccess && slots) e = cudaMalloc((void**)&p->d_scratch, (size_t)slots * sizeof(float));
+        if (e != cudaSuccess) {
+            rc = cbm::fail(CBM_B200_ERR_CUDA, std::string("plan_create: ") + cudaGetErrorString(e));
+        } else {
+            p->flags_cap = flags;
+            p->scratch_cap = slots;
+            p->device_bytes += flags * (i64)sizeof(i32) + slots * (i64)sizeof(float);
+        }
     }
     if (rc != CBM_B200_OK) {
         const std::string keep = cbm::last_error_slot();
@@ -1572,12 +1670,12 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
         c.sh.n_slabs = (f + slab - 1) / slab;
         c.group = 16;
     } else {
-        c.sh = pick_shape(f, p->slab_width, can_v4, p->n_labels);
+        c.sh = pick_shape(f, p->slab_width, can_v4);
         // never-waiting items are claimed 4 at a time: measured best on B200 (fewer trips to the
         // claim counter, which bounds short-row workloads; larger groups unbalance the long rows).
         // A small product keeps single claims: with fewer claims than resident warps, grouping
         // only idles warps.
-        c.group = ((i64)p->n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? 4 : 1;
+        c.group = ((i64)p->n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 ? NG : 4) : 1;
     }
     if (!c.chunked) {
         c.n_pclaims = (p->n_prefix + c.group - 1) / c.group;
@@ -1632,7 +1730,7 @@ int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
 // 22, 47 columns: 4 x 6 97 / 279 us, 6 x 5 100 / 288, 8 x 5 104 / 298, 8 x 4 110 / 310.
 template <bool RAGGED>
 int launch_narrow(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
-    constexpr int kResident = 6;
+    constexpr int kResident = NR;
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
@@ -1857,7 +1955,7 @@ extern "C" int cbm_b200_csr_spmm(int32_t n_rows, const int32_t* row_b, const int
     if (!x) return cbm::fail(CBM_B200_ERR_ARG, "csr_spmm: x is NULL");
     if (n_rows == 0) return CBM_B200_OK;
     const bool can_v4 = (f % 4 == 0) && (ldy % 4 == 0) && (ldx % 4 == 0) && aligned16(y) && aligned16(x);
-    const Shape sh = pick_shape(f, 256, can_v4, 0);
+    const Shape sh = pick_shape(f, 256, can_v4);
     const i64 n_units = (i64)sh.n_slabs * n_rows;
     int dev = 0, sms = 148;
     if (cudaGetDevice(&dev) == cudaSuccess)
