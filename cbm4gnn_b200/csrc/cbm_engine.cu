@@ -563,14 +563,10 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
     return true;
 }
 
-#ifndef RN
-#define RN 4
-#define NR 6
-#define NG 4
-#endif
 // Several whole rows that wait for nobody (prefix items, positions [first, end), none of them PARTIAL) by one warp, 2^lg
 // lanes for each: for slabs of at most 16 vectors, where a row's fixed costs - descriptor, entries, store, each a trip to
-// memory - outweigh its fetches.  Neighbours in the prefix are of about equal length.
+// memory - outweigh its fetches.  Neighbours in the prefix are of about equal length.  235 868 rows of 11 entries, 64
+// columns: 97 us one by one, 84 side by side with 2 fetches per row in flight, 85 with 4, 93 with 8.
 template <bool V4, bool RAGGED, int UNROLL>
 __device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 first, i32 end, i32 c0, i32 wcols, int lg, int lane) {
     using V = Vec<V4>;
@@ -650,7 +646,7 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
         if constexpr (NARROW) {
             const int lg = lanes_log2<V::E>(wcols);
             if (lg >= 3 && count > 1 && first >= p.n_partial && first + count <= p.n_prefix && p.n_bcast == 0) {
-                rows_narrow<V4, RAGGED, RN>(p, slab, first, first + count, c0, wcols, lg, lane);
+                rows_narrow<V4, RAGGED, 2>(p, slab, first, first + count, c0, wcols, lg, lane);
                 continue;
             }
         }
@@ -1673,9 +1669,11 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
         c.sh = pick_shape(f, p->slab_width, can_v4);
         // never-waiting items are claimed 4 at a time: measured best on B200 (fewer trips to the
         // claim counter, which bounds short-row workloads; larger groups unbalance the long rows).
+        // Rows in community order are of mixed, mostly short length: 8 at a time where they are narrow (400 000 rows of
+        // 47 columns 275 -> 269 us; 50 000 rows in order of length 46 -> 65).
         // A small product keeps single claims: with fewer claims than resident warps, grouping
         // only idles warps.
-        c.group = ((i64)p->n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 ? NG : 4) : 1;
+        c.group = ((i64)p->n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && p->n_chunks > 0 ? 8 : 4) : 1;
     }
     if (!c.chunked) {
         c.n_pclaims = (p->n_prefix + c.group - 1) / c.group;
@@ -1730,7 +1728,7 @@ int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
 // 22, 47 columns: 4 x 6 97 / 279 us, 6 x 5 100 / 288, 8 x 5 104 / 298, 8 x 4 110 / 310.
 template <bool RAGGED>
 int launch_narrow(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
-    constexpr int kResident = NR;
+    constexpr int kResident = 6;
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
