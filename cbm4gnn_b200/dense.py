@@ -128,33 +128,6 @@ class _DenseMapRelu(torch.autograd.Function):
         return gx, gw
 
 
-class _ReluThenMap(torch.autograd.Function):
-    """``relu(a) @ w.T`` for the ReLU in front of a map that opens its layer: taken as the map reads
-    ``a``, masked in the epilogue of the input gradient, taken again as the weight gradient reads ``a``,
-    so that no elementwise kernel passes over the activations in either direction."""
-
-    @staticmethod
-    def forward(ctx, a, weight):
-        ctx.save_for_backward(a, weight)
-        return dense_forward(a, weight, relu_in=True)
-
-    @staticmethod
-    def backward(ctx, gy):
-        a, weight = ctx.saved_tensors
-        ga = dense_grad_input(gy, weight, relu_output=a) if ctx.needs_input_grad[0] else None
-        gw = dense_grad_weight(gy, a, relu_x=True) if ctx.needs_input_grad[1] else None
-        return ga, gw
-
-
-def relu_linear(a: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """``relu(a) @ weight.T`` in fp32 accuracy, differentiable in both arguments."""
-    if not a.is_cuda:
-        return torch.nn.functional.linear(a.relu(), weight)
-    if a.dtype != torch.float32 or weight.dtype != torch.float32:
-        raise RuntimeError("dense map: fp32 operands expected")
-    return _ReluThenMap.apply(a, weight)
-
-
 def linear_relu(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``relu(x @ weight.T)`` in fp32 accuracy, differentiable in both arguments."""
     if not x.is_cuda:

@@ -15,7 +15,8 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from .dense import linear, linear_relu, relu_linear, relu_linear_linear
+from .cbm import _product
+from .dense import dense_forward, dense_grad_input, dense_grad_weight, linear, linear_relu
 from .message_passing import CBMCudaMessagePassing
 
 
@@ -80,6 +81,65 @@ class CBMParallelTorchCSRSparseMatrixGCN(CBMCudaGCN):
     two_step = True
 
 
+def _stack_forward(x, steps, weights, kept=None):
+    """A stack of layers as one list of ``steps``, two to a layer: a structure stands for its product, ``None``
+    for the dense map by the next of ``weights``.  The ReLU in front of every layer but the first is taken by the
+    map before it as it stores, else by the map after it as it reads, and is a pass of its own only between two
+    products.  ``kept`` receives the operand of every step."""
+    last, j = len(steps) - 1, 0
+    for k, step in enumerate(steps):
+        relu = k > 0 and k % 2 == 0  # a ReLU in front of this step
+        if step is not None:
+            if relu and steps[k - 1] is not None:
+                x = x.relu()
+            if kept is not None:
+                kept.append(x)
+            x = _product(step, x)
+        else:
+            if kept is not None:
+                kept.append(x)
+            x = dense_forward(x, weights[j], relu=k % 2 == 1 and k < last, relu_in=relu and steps[k - 1] is not None)
+            j += 1
+    return x
+
+
+class _Stack(torch.autograd.Function):
+    """``_stack_forward`` as one differentiable step.  On a graph of a few thousand nodes the kernels of a training
+    step take 110 us and everything else is the host's: a function to a layer, or to a map and a product, costs
+    more in the two passes than the launches in it (4096 rows, 500-64-7: 285 us a step with four of them, 245 with one)."""
+
+    @staticmethod
+    def forward(ctx, x, steps, *weights):
+        kept = []
+        y = _stack_forward(x, steps, weights, kept)
+        ctx.steps = steps
+        ctx.save_for_backward(*weights, *kept)
+        return y
+
+    @staticmethod
+    def backward(ctx, g):
+        steps, needs = ctx.steps, ctx.needs_input_grad
+        n = len(needs) - 2
+        weights, kept = ctx.saved_tensors[:n], ctx.saved_tensors[n:]
+        maps = [k for k, step in enumerate(steps) if step is None]
+        # the gradient flows down to the features, or to the lowest map that wants one for its weight
+        lowest = -1 if needs[0] else next(k for k, need in zip(maps, needs[2:]) if need)
+        grads, j = [None] * n, n
+        for k in range(len(steps) - 1, max(lowest, 0) - 1, -1):
+            step, operand, relu = steps[k], kept[k], k > 0 and k % 2 == 0
+            if step is not None:
+                g = _product(step.transposed(), g)
+                if relu:
+                    g = torch.ops.aten.threshold_backward(g, operand, 0.0)
+                continue
+            j -= 1
+            if needs[2 + j]:
+                grads[j] = dense_grad_weight(g, operand, relu_x=relu and steps[k - 1] is not None)
+            if k > lowest:
+                g = dense_grad_input(g, weights[j], relu_output=operand if relu else None)
+        return (g if needs[0] else None, None, *grads)
+
+
 class GCNModel(nn.Module):
     """``len(widths) - 1`` GCN layers with ReLU between them, sharing one CBM structure."""
 
@@ -100,30 +160,27 @@ class GCNModel(nn.Module):
             layer.cached_a_t = structure
 
     def forward(self, x, edge_index):
-        """Where a layer that propagates first is followed by one that propagates last, the two dense
-        maps and the ReLU between them are adjacent — ``A (relu((A x) W1^T) W2^T)`` — and run as one
-        differentiable step (``relu_linear_linear``).  Where a layer that propagates last is followed by one
-        that does too, the ReLU between the product and the map is taken as the map reads its operand
-        (``relu_linear``)."""
-        last = len(self.layers) - 1
-        i = 0
-        pending = False  # x still lacks the ReLU of the layer before
-        while i <= last:
-            layer = self.layers[i]
-            nxt = self.layers[i + 1] if i < last else None
-            if x.is_cuda and not layer.propagate_first():
-                u = relu_linear(x, layer.lin.weight) if pending else _fp32_linear(layer.lin, x)
-                x, pending = layer.propagate_only(u, edge_index), i < last
-                i += 1
-                continue
-            if pending:
-                x, pending = x.relu(), False
-            if nxt is not None and x.is_cuda and layer.propagate_first() and not nxt.propagate_first():
-                p = layer.propagate_only(x, edge_index)
-                u = relu_linear_linear(p, layer.lin.weight, nxt.lin.weight)
-                x, pending = nxt.propagate_only(u, edge_index), i + 1 < last
-                i += 2
-                continue
+        """Layers of this library's own class run as one step (``_Stack``); where one was replaced, derived from,
+        given hooks or told to go by two steps, or off the GPU, layer by layer."""
+        layers = list(self.layers)
+        if x.is_cuda and x.dtype == torch.float32 and all(map(_plain, layers)):
+            steps, weights = [], []
+            for layer in layers:
+                structure = layer._structure(edge_index, x.dtype, x.device)
+                steps += (structure, None) if layer.propagate_first() else (None, structure)
+                weights.append(layer.lin.weight)
+            if torch.is_grad_enabled() and (x.requires_grad or any(w.requires_grad for w in weights)):
+                return _Stack.apply(x, steps, *weights)
+            return _stack_forward(x, steps, weights)
+        last = len(layers) - 1
+        for i, layer in enumerate(layers):
             x = layer(x, edge_index, relu=i < last)
-            i += 1
         return x
+
+
+def _plain(layer) -> bool:
+    if type(layer) is not CBMCudaGCN or layer.two_step:
+        return False
+    w = layer.lin.weight
+    return w.is_cuda and w.dtype == torch.float32 and not (
+        layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks)

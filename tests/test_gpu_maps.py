@@ -3,6 +3,7 @@ import pytest
 import torch
 
 from cbm4gnn_b200 import dense
+from cbm4gnn_b200.gcn import GCNModel
 
 pytestmark = pytest.mark.gpu
 
@@ -48,10 +49,31 @@ def test_long_contraction_keeps_its_accuracy():
         assert float((got.double() - want).norm() / want.norm()) < 3e-7
 
 
-def test_relu_in_front_of_a_map_and_its_gradients():
-    a, w = _operand(500, 70, 0, 6).requires_grad_(True), _operand(20, 70, 0, 7).requires_grad_(True)
-    g = _operand(500, 20, 0, 8)
-    got = torch.autograd.grad(dense.relu_linear(a, w), (a, w), g)
-    want = torch.autograd.grad(a.double().relu() @ w.double().t(), (a, w), g.double())
-    for p, q in zip(got, want):
-        torch.testing.assert_close(p, q, atol=1e-5, rtol=1e-5)
+@pytest.mark.parametrize("widths", [(6, 9, 20, 5), (20, 9, 6, 3), (20, 6, 9, 5), (6, 20, 5, 9), (6, 20, 7)])
+@pytest.mark.parametrize("x_grad,frozen", [(True, ()), (False, ()), (False, (0,)), (True, (0, 1))])
+def test_stack_of_layers_and_its_gradients(widths, x_grad, frozen):
+    """Every order of products and maps next to one another, and gradients that stop at any of the layers,
+    against float64 autograd over the dense adjacency."""
+    n = 300
+    gen = torch.Generator().manual_seed(sum(widths))
+    a = torch.rand((n, n), generator=gen) < 0.03
+    a = (a | a.t()).fill_diagonal_(True)
+    edges = a.nonzero().t().contiguous()
+    model = GCNModel(list(widths), alpha=2).cuda()
+    for i in frozen:
+        model.layers[i].lin.weight.requires_grad_(False)
+    x = torch.randn((n, widths[0]), generator=gen).cuda().requires_grad_(x_grad)
+    d = a.sum(1).double().rsqrt()
+    adjacency = (d[:, None] * a.double() * d).cuda()
+    h = x.double()
+    for i, layer in enumerate(model.layers):
+        h = adjacency @ h @ layer.lin.weight.double().t()
+        h = h.relu() if i < len(model.layers) - 1 else h
+    got = model(x, edges.cuda())
+    g = torch.randn(got.shape, generator=gen).cuda()
+    wrt = [w for w in model.parameters() if w.requires_grad] + ([x] if x_grad else [])
+    torch.testing.assert_close(got, h.float(), atol=1e-5, rtol=1e-5)
+    with torch.no_grad():
+        assert torch.equal(model(x, edges.cuda()), got)
+    for p, q in zip(torch.autograd.grad(got, wrt, g), torch.autograd.grad(h, wrt, g.double())):
+        torch.testing.assert_close(p, q, atol=1e-4, rtol=1e-4)
