@@ -26,6 +26,7 @@ SOURCES = [
     os.path.join(_PKG_DIR, "csrc", "cbm_map_grad.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.cu"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_sequence.cpp"),
 ]
 HEADERS = [
     os.path.join(_ROOT, "include", "cbm_b200.h"),
@@ -65,6 +66,7 @@ EXPORTED = [
     "cbm_b200_csr_plan_create",
     "cbm_b200_spmm_update_bcast",
     "cbm_b200_probe_l2_read_gbps",
+    "cbm_b200_sequence",
     "cbm_b200_dense_forward",
     "cbm_b200_dense_forward_relu",
     "cbm_b200_dense_forward_of_relu",
@@ -196,6 +198,7 @@ def lib() -> ctypes.CDLL:
         c_int32, c_int32, c_int32, c_void_p)
     sig("cbm_b200_dense_forward_of_relu", c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32,
         c_int32, c_int32, c_void_p)
+    sig("cbm_b200_sequence", c_int32, c_void_p, c_int32, c_void_p, c_int32, c_void_p)
     for name in ("cbm_b200_dense_grad_weight", "cbm_b200_dense_grad_weight_of_relu"):
         sig(name, c_int32, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_int32, c_int32, c_int32, c_void_p,
             c_int64, c_void_p)

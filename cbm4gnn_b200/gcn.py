@@ -15,9 +15,9 @@ from __future__ import annotations
 import torch
 from torch import nn
 
-from .cbm import _product
-from .dense import dense_forward, dense_grad_input, dense_grad_weight, linear, linear_relu
+from .dense import linear, linear_relu
 from .message_passing import CBMCudaMessagePassing
+from .stack import run_stack
 
 
 def _fp32_linear(lin: nn.Linear, x: torch.Tensor) -> torch.Tensor:
@@ -81,65 +81,6 @@ class CBMParallelTorchCSRSparseMatrixGCN(CBMCudaGCN):
     two_step = True
 
 
-def _stack_forward(x, steps, weights, kept=None):
-    """A stack of layers as one list of ``steps``, two to a layer: a structure stands for its product, ``None``
-    for the dense map by the next of ``weights``.  The ReLU in front of every layer but the first is taken by the
-    map before it as it stores, else by the map after it as it reads, and is a pass of its own only between two
-    products.  ``kept`` receives the operand of every step."""
-    last, j = len(steps) - 1, 0
-    for k, step in enumerate(steps):
-        relu = k > 0 and k % 2 == 0  # a ReLU in front of this step
-        if step is not None:
-            if relu and steps[k - 1] is not None:
-                x = x.relu()
-            if kept is not None:
-                kept.append(x)
-            x = _product(step, x)
-        else:
-            if kept is not None:
-                kept.append(x)
-            x = dense_forward(x, weights[j], relu=k % 2 == 1 and k < last, relu_in=relu and steps[k - 1] is not None)
-            j += 1
-    return x
-
-
-class _Stack(torch.autograd.Function):
-    """``_stack_forward`` as one differentiable step.  On a graph of a few thousand nodes the kernels of a training
-    step take 110 us and everything else is the host's: a function to a layer, or to a map and a product, costs
-    more in the two passes than the launches in it (4096 rows, 500-64-7: 285 us a step with four of them, 245 with one)."""
-
-    @staticmethod
-    def forward(ctx, x, steps, *weights):
-        kept = []
-        y = _stack_forward(x, steps, weights, kept)
-        ctx.steps = steps
-        ctx.save_for_backward(*weights, *kept)
-        return y
-
-    @staticmethod
-    def backward(ctx, g):
-        steps, needs = ctx.steps, ctx.needs_input_grad
-        n = len(needs) - 2
-        weights, kept = ctx.saved_tensors[:n], ctx.saved_tensors[n:]
-        maps = [k for k, step in enumerate(steps) if step is None]
-        # the gradient flows down to the features, or to the lowest map that wants one for its weight
-        lowest = -1 if needs[0] else next(k for k, need in zip(maps, needs[2:]) if need)
-        grads, j = [None] * n, n
-        for k in range(len(steps) - 1, max(lowest, 0) - 1, -1):
-            step, operand, relu = steps[k], kept[k], k > 0 and k % 2 == 0
-            if step is not None:
-                g = _product(step.transposed(), g)
-                if relu:
-                    g = torch.ops.aten.threshold_backward(g, operand, 0.0)
-                continue
-            j -= 1
-            if needs[2 + j]:
-                grads[j] = dense_grad_weight(g, operand, relu_x=relu and steps[k - 1] is not None)
-            if k > lowest:
-                g = dense_grad_input(g, weights[j], relu_output=operand if relu else None)
-        return (g if needs[0] else None, None, *grads)
-
-
 class GCNModel(nn.Module):
     """``len(widths) - 1`` GCN layers with ReLU between them, sharing one CBM structure."""
 
@@ -160,7 +101,7 @@ class GCNModel(nn.Module):
             layer.cached_a_t = structure
 
     def forward(self, x, edge_index):
-        """Layers of this library's own class run as one step (``_Stack``); where one was replaced, derived from,
+        """Layers of this library's own class run as one step (stack.py); where one was replaced, derived from,
         given hooks or told to go by two steps, or off the GPU, layer by layer."""
         layers = list(self.layers)
         if x.is_cuda and x.dtype == torch.float32 and all(map(_plain, layers)):
@@ -169,9 +110,7 @@ class GCNModel(nn.Module):
                 structure = layer._structure(edge_index, x.dtype, x.device)
                 steps += (structure, None) if layer.propagate_first() else (None, structure)
                 weights.append(layer.lin.weight)
-            if torch.is_grad_enabled() and (x.requires_grad or any(w.requires_grad for w in weights)):
-                return _Stack.apply(x, steps, *weights)
-            return _stack_forward(x, steps, weights)
+            return run_stack(x, steps, weights)
         last = len(layers) - 1
         for i, layer in enumerate(layers):
             x = layer(x, edge_index, relu=i < last)

@@ -261,6 +261,22 @@ int cbm_b200_dense_forward_of_relu(const float* x, int64_t ldx, const float* w, 
 int cbm_b200_dense_grad_weight_of_relu(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw, int64_t lddw,
                                        int32_t n_rows, int32_t n_in, int32_t n_out, void* workspace,
                                        int64_t workspace_bytes, void* stream);
+
+/* --------------------------------------------------------------------------------------------
+ * A list of the calls above, issued one after another on `stream`; stops at the first that fails and
+ * returns its status.  A call is CBM_B200_CALL_WORDS words, the first its kind, the rest the arguments:
+ *   PRODUCT      plan, x, ldx, y, ldy, f, normalized
+ *   MAP          x, ldx, w, ldw, y, ldy, n_rows, n_in, n_out, max(x, 0) first, max(., 0) last
+ *   GRAD_INPUT   dy, lddy, w, ldw, h (or -1), ldh, dx, lddx, n_rows, n_in, n_out
+ *   GRAD_WEIGHT  dy, lddy, x, ldx, dw, lddw, n_rows, n_in, n_out, max(x, 0) first, workspace, its bytes
+ * An array is named by (number of its base) + 256 * (offset in bytes); bases [host] holds the addresses.
+ * ------------------------------------------------------------------------------------------ */
+#define CBM_B200_CALL_WORDS 13
+#define CBM_B200_CALL_PRODUCT 0
+#define CBM_B200_CALL_MAP 1
+#define CBM_B200_CALL_GRAD_INPUT 2
+#define CBM_B200_CALL_GRAD_WEIGHT 3
+int cbm_b200_sequence(const int64_t* calls, int32_t n_calls, const int64_t* bases, int32_t n_bases, void* stream);
 int64_t cbm_b200_dense_grad_weight_workspace(int32_t n_rows, int32_t n_in, int32_t n_out);
 int cbm_b200_dense_grad_weight(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* dw,
                                int64_t lddw, int32_t n_rows, int32_t n_in, int32_t n_out,

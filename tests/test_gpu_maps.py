@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from cbm4gnn_b200 import dense
+from cbm4gnn_b200 import dense, stack
 from cbm4gnn_b200.gcn import GCNModel
 
 pytestmark = pytest.mark.gpu
@@ -50,10 +50,12 @@ def test_long_contraction_keeps_its_accuracy():
 
 
 @pytest.mark.parametrize("widths", [(6, 9, 20, 5), (20, 9, 6, 3), (20, 6, 9, 5), (6, 20, 5, 9), (6, 20, 7)])
+@pytest.mark.parametrize("listed_bytes", [stack.LISTED_BYTES, 0])
 @pytest.mark.parametrize("x_grad,frozen", [(True, ()), (False, ()), (False, (0,)), (True, (0, 1))])
-def test_stack_of_layers_and_its_gradients(widths, x_grad, frozen):
+def test_stack_of_layers_and_its_gradients(widths, x_grad, frozen, listed_bytes, monkeypatch):
     """Every order of products and maps next to one another, and gradients that stop at any of the layers,
-    against float64 autograd over the dense adjacency."""
+    against float64 autograd over the dense adjacency; calls issued from a list and one by one."""
+    monkeypatch.setattr(stack, "LISTED_BYTES", listed_bytes)
     n = 300
     gen = torch.Generator().manual_seed(sum(widths))
     a = torch.rand((n, n), generator=gen) < 0.03
