@@ -51,7 +51,7 @@ constexpr int kThreads = 512;
 constexpr int kMaxPrefix = 65000;
 
 __global__ void __launch_bounds__(kThreads) candidate_kernel(const SearchParams p) {
-    __shared__ i32 s_u, s_touched;
+    __shared__ i32 s_u, s_touched, s_passed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = kThreads / 32;
     u32* hits = p.hits + (i64)blockIdx.x * p.hits_stride;
     i32* touched = p.touched + (i64)blockIdx.x * p.touched_stride;
@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(kThreads) candidate_kernel(const SearchParams 
     for (;;) {
         if (tid == 0) {
             s_u = (i32)atomicAdd(p.out_count + 1, 1ULL);
-            s_touched = 0;
+            s_touched = s_passed = 0;
         }
         __syncthreads();
         const i32 u = s_u;
@@ -102,39 +102,46 @@ __global__ void __launch_bounds__(kThreads) candidate_kernel(const SearchParams 
         // 2. rows with enough hits in the prefix: exact intersection, then the rule
         const i32 n_touched = s_touched;
         // Every lane looks at one touched row: nearly all fall at the number of hits, and a warp that took them one by
-        // one spent its time waiting for that counter (100 000 rows: 7.8 ms the whole search).
-        for (i32 t0 = 32 * warp; t0 < n_touched; t0 += 32 * n_warps) {
-            i32 v = -1, nv = 0, in_prefix = 0;
-            i64 vb = 0;
-            if (t0 + lane < n_touched) {
-                v = touched[t0 + lane];
-                const u32 w = atomicAnd(hits + (v >> 1), (v & 1) ? 0x0000ffffu : 0xffff0000u);  // read and clear
-                in_prefix = (i32)(((v & 1) ? (w >> 16) : w) & 0xffffu);
-                if (v != u && in_prefix >= j_hits) {
-                    vb = p.row_ptr[v];
-                    nv = (i32)(p.row_ptr[v + 1] - vb);
-                }
+        // one spent its time waiting for that counter (100 000 rows: 7.8 ms the whole search, 2.5 so).  Those that
+        // pass are gathered at the front of the list and dealt out to the warps one at a time: where many pass, a
+        // warp that dealt with its own 32 kept the block waiting (132 534 rows of 265 entries: 2.6 s, 0.93 so).
+        for (i32 t0 = 0; t0 < n_touched; t0 += kThreads) {
+            i32 v = u;
+            bool pass = false;
+            if (t0 + tid < n_touched) {
+                v = touched[t0 + tid];
+                const u32 mine = (v & 1) ? 0xffff0000u : 0x0000ffffu;
+                const i32 in_prefix = (i32)((__ldcg(hits + (v >> 1)) & mine) >> ((v & 1) * 16));
+                pass = v != u && in_prefix >= j_hits && p.row_ptr[v + 1] - p.row_ptr[v] >= need;
+                if (!pass) atomicAnd(hits + (v >> 1), ~mine);
             }
-            unsigned left = __ballot_sync(0xffffffffu, nv >= need);  // (need is at least 1)
-            while (left) {
-                const int from = __ffs(left) - 1;
-                left &= left - 1;
-                const i32 v1 = __shfl_sync(0xffffffffu, v, from), nv1 = __shfl_sync(0xffffffffu, nv, from);
-                i32 both = __shfl_sync(0xffffffffu, in_prefix, from);
-                if (has_tail) {
-                    const i64 vb1 = __shfl_sync(0xffffffffu, vb, from);
-                    i32 cnt = 0;
-                    for (i32 k = lane; k < nv1; k += 32) {
-                        const i32 r = p.row_rank[vb1 + k];
-                        cnt += (i32)((bitmap[r >> 5] >> (r & 31)) & 1u);
-                    }
-                    both = (i32)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+            __syncthreads();  // all of this stretch is read: the list may grow into it
+            if (pass) touched[atomicAdd(&s_passed, 1)] = v;
+        }
+        __syncthreads();
+        const i32 n_passed = s_passed;
+        for (i32 t = warp; t < n_passed; t += n_warps) {
+            const i32 v = touched[t];
+            i32 both = 0;
+            if (lane == 0) {
+                const u32 w = atomicAnd(hits + (v >> 1), (v & 1) ? 0x0000ffffu : 0xffff0000u);  // read and clear
+                both = (i32)(((v & 1) ? (w >> 16) : w) & 0xffffu);
+            }
+            both = __shfl_sync(0xffffffffu, both, 0);
+            const i64 vb = p.row_ptr[v];
+            const i32 nv = (i32)(p.row_ptr[v + 1] - vb);
+            if (has_tail) {
+                i32 cnt = 0;
+                for (i32 k = lane; k < nv; k += 32) {
+                    const i32 r = p.row_rank[vb + k];
+                    cnt += (i32)((bitmap[r >> 5] >> (r & 31)) & 1u);
                 }
-                const i32 h = nu + nv1 - 2 * both;
-                if (h < nv1 - p.alpha && lane == 0) {  // cbm/cbm_extensions.cpp:93-101
-                    const u64 pos = atomicAdd(p.out_count, 1ULL);
-                    if ((i64)pos < p.out_cap) p.out[pos] = cbm::CandTriple{u, v1, h};
-                }
+                both = (i32)__reduce_add_sync(0xffffffffu, (unsigned)cnt);
+            }
+            const i32 h = nu + nv - 2 * both;
+            if (h < nv - p.alpha && lane == 0) {  // cbm/cbm_extensions.cpp:93-101
+                const u64 pos = atomicAdd(p.out_count, 1ULL);
+                if ((i64)pos < p.out_cap) p.out[pos] = cbm::CandTriple{u, v, h};
             }
         }
         __syncthreads();
@@ -188,7 +195,10 @@ int gpu_candidates(int device, int32_t n, int32_t alpha, const int64_t* row_ptr,
     p.hits_stride = ((int64_t)n + 1) / 2 + 1;
     p.touched_stride = n;
     p.bitmap_stride = ((int64_t)n + 31) / 32 + 1;
-    p.out_cap = std::max<int64_t>(1ll << 20, 16ll * n);
+    // Room for the candidates: a list that turns out too short costs a second search, a needlessly long one its
+    // allocation.  Rows that resemble one another closely have the more candidates the more entries they have (132 534
+    // rows of 265 entries, 16 a row were too few: 4.7 s instead of 1.9).
+    p.out_cap = std::max<int64_t>({1ll << 20, 16ll * n, nnz / 2});
     Arena mem;
     const size_t o_row_ptr = mem.plan<i64>((size_t)n + 1), o_col_ptr = mem.plan<i64>((size_t)n + 1);
     const size_t o_row_rank = mem.plan<i32>((size_t)nnz), o_col_of_rank = mem.plan<i32>((size_t)n);
