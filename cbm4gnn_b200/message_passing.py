@@ -5,8 +5,8 @@ Mirrors gnns/message_passing/cbm_message_passing.py:7-107 of the reference: the 
 (assignable from outside, as benchmark/parallel/benchmark_gcn_cpu.py:62-66 does to share one
 structure between layers), and dispatches to the normalized or plain product.  The four reference
 class names are kept; there the ``MKL`` classes call the one-step product and the ``Torch`` classes
-the two-step path (``deltas @ x`` then the in-place update, cbm_message_passing.py:80-107), and the
-same distinction is kept here on the CUDA kernels (``two_step``).  Unlike the reference, the output is a fresh tensor on
+the two-step path (``deltas @ x`` then the in-place update, cbm_message_passing.py:80-107); here
+``two_step`` calls the methods of that name, which run the one-step kernel for the same result.  Unlike the reference, the output is a fresh tensor on
 every call (the reference caches and aliases one output buffer, cbm_message_passing.py:26-29), and
 the product is differentiable with respect to ``x``.
 """
@@ -31,7 +31,7 @@ class CBMCudaMessagePassing(nn.Module):
         self.alpha = alpha
         self.cached_a_t = None
 
-    two_step = False  # True: delta product, then the update-only kernel
+    two_step = False  # True: through the methods named after the reference's two-step products
 
     def _structure(self, edge_index: torch.Tensor, dtype, device=None) -> cbm_matrix:
         if self.cached and self.cached_a_t is not None:
