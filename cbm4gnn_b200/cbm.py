@@ -149,7 +149,7 @@ class cbm_matrix:
         else:
             # D^-1/2 from the row degrees of a binary matrix (cbm/cbm.py:34-41); a row without
             # entries gets inf exactly as there.
-            deg = torch.empty(n)
+            deg = torch.empty(n, dtype=torch.float32, device="cpu")  # whatever torch's defaults are: the call writes n host floats
             _lib.check(_lib.lib().cbm_b200_edge_degrees(_ptr(row), _ptr(col), row.shape[0], ctypes.byref(n32), _ptr(deg)))
             self.col_multiplier = deg.pow(-0.5)
             mul = _as_f32(self.col_multiplier)

@@ -283,3 +283,20 @@ def test_check_format_rejects_corrupted_structures():
         c.check_format(e)
     c._dval[:] = keep
     c.check_format(e)
+
+
+@pytest.mark.parametrize("dtype,device", [(torch.float64, None), (torch.bfloat16, None), (torch.float32, "meta")])
+def test_multiplier_and_deltas_whatever_the_defaults_of_torch(dtype, device):
+    """The row degrees are 32-bit floats in host memory also where new tensors are by default something else."""
+    ei = torch.from_numpy(with_self_loops(graphs.copy_model(300, 0.8, 3, 1))).to(torch.int32)
+    values = torch.ones(ei.shape[1])
+    want = cbm_matrix(ei, values, alpha=2, normalized=True)
+    torch.set_default_dtype(dtype)
+    torch.set_default_device(device)
+    try:
+        got = cbm_matrix(ei, values, alpha=2, normalized=True)
+    finally:
+        torch.set_default_dtype(torch.float32)
+        torch.set_default_device(None)
+    assert got.col_multiplier.dtype == torch.float32 and torch.equal(got.col_multiplier, want.col_multiplier)
+    assert np.array_equal(got._dcol, want._dcol) and np.array_equal(got._dval, want._dval)
