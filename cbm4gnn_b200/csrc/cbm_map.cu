@@ -76,7 +76,7 @@ struct MapParams {
     const float* a;    // [m, k]
     const float* b;    // [n, k], or [k, n] when B_TRANS
     float* d;          // [m, n]
-    const float* aux;  // [m, n]: the result is zeroed where aux is not positive
+    const float* aux;  // [m, n]: the result is zeroed where aux <= 0
     int64_t lda, ldb, ldd, ldaux;
     int m, n, k;
     int bn;            // columns of a tile, a multiple of 16, at most 128
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                                 x.z = k + 2 < p.k ? x.z : 0.f;
                                 x.w = k + 3 < p.k ? x.w : 0.f;
                             }
-                            if (p.relu_in) x = make_float4(fmaxf(x.x, 0.f), fmaxf(x.y, 0.f), fmaxf(x.z, 0.f), fmaxf(x.w, 0.f));
+                            if (p.relu_in) x = relu(x);
                             const int o = 4 * s + 2 * (i & 1);
                             split2(x.x, x.y, t[0][o], t[1][o], t[2][o]);
                             split2(x.z, x.w, t[0][o + 1], t[1][o + 1], t[2][o + 1]);
@@ -305,8 +305,9 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                     u32 bits = 0;
 #pragma unroll
                     for (int i = 0; i < 8; ++i)
-                        bits |= ((x[b][i].x > 0.f ? 1u : 0u) | (x[b][i].y > 0.f ? 2u : 0u) | (x[b][i].z > 0.f ? 4u : 0u) |
-                                 (x[b][i].w > 0.f ? 8u : 0u))
+                        // (a NaN lets the gradient through, as the backward of torch.relu does)
+                        bits |= ((x[b][i].x <= 0.f ? 0u : 1u) | (x[b][i].y <= 0.f ? 0u : 2u) | (x[b][i].z <= 0.f ? 0u : 4u) |
+                                 (x[b][i].w <= 0.f ? 0u : 8u))
                                 << (4 * i);
                     keep[b] = bits;
                 }
@@ -372,7 +373,7 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                         const u32 bits = keep[b] >> (4 * i);
                         y = make_float4(bits & 1 ? y.x : 0.f, bits & 2 ? y.y : 0.f, bits & 4 ? y.z : 0.f, bits & 8 ? y.w : 0.f);
                     }
-                    if (p.relu_out) y = make_float4(fmaxf(y.x, 0.f), fmaxf(y.y, 0.f), fmaxf(y.z, 0.f), fmaxf(y.w, 0.f));
+                    if (p.relu_out) y = relu(y);
                     if (p.d_vec && here >= 4) {
                         *reinterpret_cast<float4*>(d) = y;
                     } else {

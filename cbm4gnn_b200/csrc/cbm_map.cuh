@@ -171,6 +171,14 @@ __device__ __forceinline__ float4 fetch4(const float* p, bool on) {
     return v;
 }
 
+// max(x, 0) that passes NaN on, as torch.relu does (fmaxf would make it 0).
+__device__ __forceinline__ float relu(float x) {
+    float y;
+    asm("max.NaN.f32 %0, %1, 0f00000000;" : "=f"(y) : "f"(x));
+    return y;
+}
+__device__ __forceinline__ float4 relu(float4 x) { return make_float4(relu(x.x), relu(x.y), relu(x.z), relu(x.w)); }
+
 // Two neighbours of the contraction (x at the lower address) -> their three bf16 pairs.
 __device__ __forceinline__ void split2(float x, float y, u32& b0, u32& b1, u32& b2) {
     asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(b0) : "f"(y), "f"(x));

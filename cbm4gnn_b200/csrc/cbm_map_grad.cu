@@ -126,8 +126,8 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
             for (int i = 0; i < CHUNK_K / 2; ++i) {
                 float x = v[2 * i], y = v[2 * i + 1];
                 if (p.relu_a) {
-                    x = fmaxf(x, 0.f);
-                    y = fmaxf(y, 0.f);
+                    x = relu(x);
+                    y = relu(y);
                 }
                 split2(x, y, t[0][i], t[1][i], t[2][i]);
             }
@@ -185,10 +185,10 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
                 const u32 row = (u32)((task >> 2) * 64 + lane), k8 = (slot & 1) * 4 + (u32)(task & 3);
                 float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? fmaxf(v[i][j].x, 0.f) : v[i][j].x;
+                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? relu(v[i][j].x) : v[i][j].x;
                 store_split8(at + swizzled(row, k8), term, x);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? fmaxf(v[i][j].y, 0.f) : v[i][j].y;
+                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? relu(v[i][j].y) : v[i][j].y;
                 store_split8(at + swizzled(row + 32, k8), term, x);
                 if (c + 1 < chunks) load(c + 1, i);  // as soon as its registers are free, ahead of the other tasks
             }

@@ -68,8 +68,8 @@ def dense_forward(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = N
 
 def dense_grad_input(gy: torch.Tensor, w: torch.Tensor, relu_output: torch.Tensor | None = None) -> torch.Tensor:
     """``gy @ w`` for ``gy`` [N, out], ``w`` [out, in].  With ``relu_output`` [N, in] (the output, or
-    the input, of the ReLU this gradient flows back through) the result is zeroed where that is not
-    positive, in the GEMM's epilogue."""
+    the input, of the ReLU this gradient flows back through) the result is zeroed where that is <= 0,
+    in the GEMM's epilogue."""
     n, n_out, n_in = gy.size(0), gy.size(1), w.size(1)
     gy, w = _rows(gy), _rows(w)
     gx = _new_rows(n, n_in, gy)

@@ -235,7 +235,7 @@ int cbm_b200_selftest_wait(int32_t device, int32_t wait_ms, void* stream);
  *   cbm_b200_dense_forward_relu y = max(x * w^T, 0): the map followed by the ReLU that sits between two
  *                               layers (benchmark/parallel/benchmark_gcn_cpu.py:70-89), in the epilogue
  *   cbm_b200_dense_grad_input   dx [n_rows,n_in] = dy [n_rows,n_out] * w
- *   cbm_b200_dense_grad_input_relu  the same, set to 0 wherever h [n_rows,n_in] is not positive: the
+ *   cbm_b200_dense_grad_input_relu  the same, set to 0 wherever h [n_rows,n_in] <= 0: the
  *                               gradient that flows back through the ReLU whose output (or input) h was
  *   cbm_b200_dense_grad_weight  dw [n_out,n_in]  = dy^T * x; contracts over the rows in up to
  *                               CBM_B200_DENSE_MAX_CHUNKS independent chunks whose partial results
@@ -245,6 +245,7 @@ int cbm_b200_selftest_wait(int32_t device, int32_t wait_ms, void* stream);
  *                               of a map that opens its layer, taken as x is read
  *   cbm_b200_dense_grad_weight_of_relu  dw = dy^T * max(x, 0), the same map's weight gradient; its input
  *                               gradient is cbm_b200_dense_grad_input_relu with h = x
+ * NaN passes through every ReLU and is not masked, as in torch.
  * ------------------------------------------------------------------------------------------ */
 #define CBM_B200_DENSE_MAX_CHUNKS 296
 int cbm_b200_dense_forward(const float* x, int64_t ldx, const float* w, int64_t ldw, float* y,

@@ -79,3 +79,43 @@ def test_stack_of_layers_and_its_gradients(widths, x_grad, frozen, listed_bytes,
         assert torch.equal(model(x, edges.cuda()), got)
     for p, q in zip(torch.autograd.grad(got, wrt, g), torch.autograd.grad(h, wrt, g.double())):
         torch.testing.assert_close(p, q, atol=1e-4, rtol=1e-4)
+
+
+def test_nan_passes_through_every_relu():
+    """As through torch.relu and its backward: a NaN stays a NaN and lets the gradient through."""
+    nan = float("nan")
+    x, w, gy = _operand(140, 40, 0, 1), _operand(24, 40, 0, 2), _operand(140, 24, 0, 3)
+    x[3, 5] = x[130, 39] = nan
+    rows = x.isnan().any(1)
+    for got in (dense.dense_forward(x, w, relu=True), dense.dense_forward(x, w, relu_in=True)):
+        assert torch.equal(got.isnan(), rows[:, None].expand_as(got))
+    gx = dense.dense_grad_input(gy, w)
+    assert torch.equal(dense.dense_grad_input(gy, w, relu_output=x), torch.where(x <= 0, torch.zeros_like(gx), gx))
+    for a, b in ((gy, x), (x, gy)):  # both orientations of the weight gradient
+        assert torch.equal(dense.dense_grad_weight(a, b, relu_x=True).isnan(), (a.t() @ b.relu()).isnan())
+
+
+@pytest.mark.parametrize("widths", [(6, 9, 20, 5), (20, 9, 6, 3), (20, 6, 9, 5), (6, 20, 5, 9)])
+@pytest.mark.parametrize("listed_bytes", [stack.LISTED_BYTES, 0])
+def test_nan_in_a_stack_of_layers(widths, listed_bytes, monkeypatch):
+    """One NaN feature: outputs and gradients have their NaN where the layers called one by one have them."""
+    monkeypatch.setattr(stack, "LISTED_BYTES", listed_bytes)
+    n = 60
+    gen = torch.Generator().manual_seed(3)
+    a = torch.rand((n, n), generator=gen) < 0.02
+    edges = (a | a.t()).fill_diagonal_(True).nonzero().t().contiguous().cuda()
+    model = GCNModel(list(widths), alpha=2).cuda()
+    x = torch.randn((n, widths[0]), generator=gen)
+    x[7, 2] = float("nan")
+    x = x.cuda().requires_grad_(True)
+    wrt = [x, *model.parameters()]
+    got = model(x, edges)
+    want = x
+    for i, layer in enumerate(model.layers):
+        want = layer(want, edges)
+        want = want.relu() if i < len(model.layers) - 1 else want
+    assert 0 < int(want.isnan().any(1).sum()) < n
+    torch.testing.assert_close(got, want, atol=1e-5, rtol=1e-5, equal_nan=True)
+    g = torch.randn(got.shape, generator=gen).cuda()
+    for p, q in zip(torch.autograd.grad(got, wrt, g), torch.autograd.grad(want, wrt, g)):
+        torch.testing.assert_close(p, q, atol=1e-4, rtol=1e-4, equal_nan=True)
