@@ -235,13 +235,11 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
             for (int kb = 0; kb < kblocks; ++kb, ++it) {
                 const u32 ds = it & 1, use = it >> 1;
                 if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
-                fence_after();
                 const u32 d = tmem + ds * D_COLS;
                 const int here = min(2, chunks - 2 * kb);
                 for (int c = 0; c < here && ok; ++c) {
                     const u32 slot = (run + c) % A_SLOTS;
                     if (!(ok = warp_wait(a_full + 8 * slot, ((run + c) / A_SLOTS) & 1, gave_up, p.timeout))) break;
-                    fence_after();
 #pragma unroll
                     for (int s = 0; s < 2; ++s)
                         if (4 * kb + 2 * c + s < p.steps)
@@ -318,7 +316,6 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
             auto collect = [&](auto first) -> bool {
                 const u32 ds = it & 1, use = it >> 1;
                 if (!warp_wait(d_full + 8 * ds, use & 1, gave_up, p.timeout)) return false;
-                fence_after();
                 const u32 at = tmem + ds * D_COLS + c_lo + ((u32)(quarter * 32) << 16);
 #pragma unroll
                 for (int q = 0; q < 4; ++q) {

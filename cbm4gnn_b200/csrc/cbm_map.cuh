@@ -77,8 +77,11 @@ __device__ __forceinline__ bool bar_poll(u32 bar, u32 parity) {
         : "memory");
     return done != 0;
 }
-// Bounded wait of a whole warp; `gave_up` (shared memory) lets every role of the block stop once one wait has
-// run out.
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+// Bounded wait of a whole warp, and the fence without which what it then does in tensor memory (loads, stores, MMAs)
+// would not be ordered behind what the barrier reports.  `gave_up` (shared memory) lets every role of the block stop
+// once one wait has run out.
 __device__ __forceinline__ bool warp_wait(u32 bar, u32 parity, volatile int* gave_up, int* timeout) {
     u64 t0 = 0;
     bool ok = true;
@@ -95,7 +98,9 @@ __device__ __forceinline__ bool warp_wait(u32 bar, u32 parity, volatile int* gav
             }
         }
     }
-    return __all_sync(0xffffffffu, ok);
+    ok = __all_sync(0xffffffffu, ok);
+    fence_after();
+    return ok;
 }
 
 // ---- tensor memory and tcgen05 ------------------------------------------------------------------
@@ -106,8 +111,6 @@ __device__ __forceinline__ void tmem_alloc(u32 where) {
 __device__ __forceinline__ void tmem_free(u32 base) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "n"(TMEM_COLS));
 }
-__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

@@ -202,13 +202,11 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
         for (int kb = 0; kb < kblocks; ++kb) {
             const u32 ds = kb & 1, use = kb >> 1;
             if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
-            fence_after();
             const u32 d = tmem + ds * D_COLS;
             const int here = min(2, chunks - 2 * kb);
             for (int c = 0; c < here && ok; ++c) {
                 const u32 r = 2 * kb + c, slot = r % A_SLOTS;
                 if (!(ok = warp_wait(full + 8 * slot, (r / A_SLOTS) & 1, gave_up, p.timeout))) break;
-                fence_after();
 #pragma unroll
                 for (int s = 0; s < 2; ++s)
                     mma_small(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, b0 + (slot >> 1) * stage + (slot & 1) * 64 + 32 * s, term,
@@ -242,7 +240,6 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
             const u32 ds = kb & 1, use = kb >> 1;
             if (!warp_wait(d_full + 8 * ds, use & 1, gave_up, p.timeout)) goto done;
             if (c_lo < p.bn) {
-                fence_after();
                 const u32 at = tmem + ds * D_COLS + c_lo + ((u32)(quarter * 32) << 16);
 #pragma unroll
                 for (int g = 0; g < 4; ++g) {  // 16 columns at a time
