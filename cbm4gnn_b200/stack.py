@@ -195,6 +195,8 @@ class _ListedStack(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         x, kept, *weights = ctx.saved_tensors
+        # (a saved-tensor hook may hand them back in another layout)
+        x, kept, weights = _rows_of(x), kept.contiguous(), [w.contiguous() for w in weights]
         shapes, needs = ctx.shapes, ctx.needs_input_grad
         dev, n, width, g = x.get_device(), x.size(0), x.size(1), _rows_of(g)
         calls = _backward_list(_plans([None if s is None else s.transposed() for s in ctx.steps], dev), shapes, n, max(x.stride(0), width),

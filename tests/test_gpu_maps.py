@@ -119,3 +119,25 @@ def test_nan_in_a_stack_of_layers(widths, listed_bytes, monkeypatch):
     g = torch.randn(got.shape, generator=gen).cuda()
     for p, q in zip(torch.autograd.grad(got, wrt, g), torch.autograd.grad(want, wrt, g)):
         torch.testing.assert_close(p, q, atol=1e-4, rtol=1e-4, equal_nan=True)
+
+
+@pytest.mark.parametrize("listed_bytes", [stack.LISTED_BYTES, 0])
+def test_saved_tensor_hooks_that_change_the_layout(listed_bytes, monkeypatch):
+    monkeypatch.setattr(stack, "LISTED_BYTES", listed_bytes)
+    edges = torch.arange(50).repeat(2, 1).cuda()
+    model = GCNModel([20, 9, 6, 3], alpha=2).cuda()
+    x = torch.randn(50, 20, device="cuda", requires_grad=True)
+    g = torch.randn(50, 3, device="cuda")
+    wrt = [x, *model.parameters()]
+    want = torch.autograd.grad(model(x, edges), wrt, g)
+
+    def turn(t):
+        return t.t().contiguous() if t.dim() == 2 else torch.stack([t, t], 1)
+
+    def turn_back(t):
+        return t.t() if t.size(1) != 2 else t[:, 0]
+
+    with torch.autograd.graph.saved_tensors_hooks(turn, turn_back):
+        y = model(x, edges)
+    for p, q in zip(torch.autograd.grad(y, wrt, g), want):
+        assert torch.equal(p, q)
