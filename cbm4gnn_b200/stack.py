@@ -43,7 +43,10 @@ class _Stack(torch.autograd.Function):
     them, 245 with one)."""
 
     @staticmethod
-    def forward(ctx, x, steps, *weights):
+    def forward(ctx, x, steps, keep, *weights):
+        """``keep``: a backward pass may follow; the operands of the steps are let go as they are used up otherwise."""
+        if not keep:
+            return _stack_forward(x, steps, weights)
         kept = []
         y = _stack_forward(x, steps, weights, kept)
         ctx.steps = steps
@@ -53,11 +56,11 @@ class _Stack(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         steps, needs = ctx.steps, ctx.needs_input_grad
-        n, saved = len(needs) - 2, ctx.saved_tensors
+        n, saved = len(needs) - 3, ctx.saved_tensors
         weights, kept = saved[:n], saved[n:]
         maps = [k for k, step in enumerate(steps) if step is None]
         # the gradient flows down to the features, or to the lowest map that wants one for its weight
-        lowest = -1 if needs[0] else next(k for k, need in zip(maps, needs[2:]) if need)
+        lowest = -1 if needs[0] else next(k for k, need in zip(maps, needs[3:]) if need)
         grads, j = [None] * n, n
         for k in range(len(steps) - 1, max(lowest, 0) - 1, -1):
             step, operand, relu = steps[k], kept[k], k > 0 and k % 2 == 0
@@ -67,11 +70,11 @@ class _Stack(torch.autograd.Function):
                     g = torch.ops.aten.threshold_backward(g, operand, 0.0)
                 continue
             j -= 1
-            if needs[2 + j]:
+            if needs[3 + j]:
                 grads[j] = dense_grad_weight(g, operand, relu_x=relu and steps[k - 1] is not None)
             if k > lowest:
                 g = dense_grad_input(g, weights[j], relu_output=operand if relu else None)
-        return (g if needs[0] else None, None, *grads)
+        return (g if needs[0] else None, None, None, *grads)
 
 
 # ------------------------------------------------------------------------------- small graphs: listed calls
@@ -224,9 +227,11 @@ def _listable(x, steps, shapes, weights):
 
 
 def run_stack(x, steps, weights):
-    """The result of the stack for CUDA fp32 ``x`` and ``weights``, differentiable in both."""
+    """The result of the stack for CUDA fp32 ``x`` and ``weights``, differentiable in both.  The functions are never
+    gone round, also where no backward pass can follow: forward-mode differentiation has to meet (and be refused by)
+    them."""
     shapes = tuple(tuple(w.shape) for w in weights)
-    listed = _listable(x, steps, shapes, weights)
-    if torch.is_grad_enabled() and (x.requires_grad or any(w.requires_grad for w in weights)):
-        return _ListedStack.apply(x, steps, shapes, *weights) if listed else _Stack.apply(x, steps, *weights)
-    return _listed_forward(x, steps, shapes, weights)[0] if listed else _stack_forward(x, steps, weights)
+    if _listable(x, steps, shapes, weights):
+        return _ListedStack.apply(x, steps, shapes, *weights)
+    keep = torch.is_grad_enabled() and (x.requires_grad or any(w.requires_grad for w in weights))
+    return _Stack.apply(x, steps, keep, *weights)

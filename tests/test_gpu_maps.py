@@ -141,3 +141,18 @@ def test_saved_tensor_hooks_that_change_the_layout(listed_bytes, monkeypatch):
         y = model(x, edges)
     for p, q in zip(torch.autograd.grad(y, wrt, g), want):
         assert torch.equal(p, q)
+
+
+@pytest.mark.parametrize("listed_bytes", [stack.LISTED_BYTES, 0])
+def test_forward_mode_is_refused(listed_bytes, monkeypatch):
+    """No silent loss of a tangent, whether or not anything asks for a gradient."""
+    import torch.autograd.forward_ad as forward_ad
+    monkeypatch.setattr(stack, "LISTED_BYTES", listed_bytes)
+    edges = torch.arange(50).repeat(2, 1).cuda()
+    model = GCNModel([20, 9, 6, 3], alpha=2).cuda().requires_grad_(False)
+    x = torch.randn(50, 20, device="cuda")
+    want = model(x, edges)
+    with forward_ad.dual_level(), pytest.raises(RuntimeError, match="jvp"):
+        model(forward_ad.make_dual(x, torch.ones_like(x)), edges)
+    with torch.no_grad():
+        assert torch.equal(model(x, edges), want) and not want.requires_grad
