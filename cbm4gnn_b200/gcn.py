@@ -14,6 +14,7 @@ from __future__ import annotations
 
 import torch
 from torch import nn
+from torch.nn.modules.module import _has_any_global_hook
 
 from .dense import linear, linear_relu
 from .message_passing import CBMCudaMessagePassing
@@ -102,9 +103,9 @@ class GCNModel(nn.Module):
 
     def forward(self, x, edge_index):
         """Layers of this library's own class run as one step (stack.py); where one was replaced, derived from,
-        given hooks or told to go by two steps, or off the GPU, layer by layer."""
+        given hooks (of its own or for all modules) or told to go by two steps, or off the GPU, layer by layer."""
         layers = list(self.layers)
-        if x.is_cuda and x.dtype == torch.float32 and all(map(_plain, layers)):
+        if x.is_cuda and x.dtype == torch.float32 and not _has_any_global_hook() and all(map(_plain, layers)):
             steps, weights = [], []
             for layer in layers:
                 structure = layer._structure(edge_index, x.dtype, x.device)
@@ -118,7 +119,7 @@ class GCNModel(nn.Module):
 
 
 def _plain(layer) -> bool:
-    if type(layer) is not CBMCudaGCN or layer.two_step:
+    if type(layer) is not CBMCudaGCN or layer.two_step or "forward" in vars(layer):
         return False
     w = layer.lin.weight
     return w.is_cuda and w.dtype == torch.float32 and not (

@@ -156,3 +156,20 @@ def test_forward_mode_is_refused(listed_bytes, monkeypatch):
         model(forward_ad.make_dual(x, torch.ones_like(x)), edges)
     with torch.no_grad():
         assert torch.equal(model(x, edges), want) and not want.requires_grad
+
+
+def test_layers_are_called_where_someone_looks_at_them():
+    """Hooks for all modules and a forward replaced on one layer see every call."""
+    edges = torch.arange(50).repeat(2, 1).cuda()
+    model = GCNModel([20, 9, 6, 3], alpha=2).cuda()
+    x = torch.randn(50, 20, device="cuda")
+    want, seen = model(x, edges), []
+    hook = torch.nn.modules.module.register_module_forward_hook(lambda module, args, out: seen.append(type(module)))
+    try:
+        torch.testing.assert_close(model(x, edges), want)
+    finally:
+        hook.remove()
+    assert seen == [type(model.layers[0])] * 3 + [GCNModel]
+    layer = model.layers[1]
+    layer.forward = lambda h, edge_index, relu=False: type(layer).forward(layer, h, edge_index, relu) * 0
+    assert not model(x, edges).any()
