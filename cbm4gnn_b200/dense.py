@@ -37,6 +37,14 @@ def _ld(t: torch.Tensor) -> int:
     return max(t.stride(0), t.size(1))
 
 
+def _check(t: torch.Tensor, u: torch.Tensor, match: bool, what: str) -> None:
+    """The kernels read as far as the sizes they are given say: operands that do not fit together are refused here."""
+    if not match:
+        raise RuntimeError(f"dense map: shape mismatch, {what} of {tuple(t.shape)} and {tuple(u.shape)}")
+    if t.device != u.device:
+        raise RuntimeError(f"dense map: operands on {t.device} and {u.device}")
+
+
 def _call(name: str, dev: int, *args) -> None:
     """One library call on device ``dev``'s current stream."""
     fn = getattr(_lib.lib(), name)
@@ -54,6 +62,7 @@ def dense_forward(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = N
     """``x @ w.T`` (``relu``: followed by ``max(., 0)`` in the GEMM's epilogue; ``relu_in``: of
     ``max(x, 0)``, taken as the operand is read) for CUDA fp32 ``x`` [N, in] and ``w`` [out, in];
     ``out`` (optional) is an [N, out] tensor that receives the result."""
+    _check(x, w, x.dim() == 2 and w.dim() == 2 and x.size(1) == w.size(1), "x @ w.T")
     n, n_in, n_out = x.size(0), x.size(1), w.size(0)
     x, w = _rows(x), _rows(w)
     direct = out is not None and out.stride(1) == 1 and out.stride(0) >= n_out
@@ -70,7 +79,10 @@ def dense_grad_input(gy: torch.Tensor, w: torch.Tensor, relu_output: torch.Tenso
     """``gy @ w`` for ``gy`` [N, out], ``w`` [out, in].  With ``relu_output`` [N, in] (the output, or
     the input, of the ReLU this gradient flows back through) the result is zeroed where that is <= 0,
     in the GEMM's epilogue."""
+    _check(gy, w, gy.dim() == 2 and w.dim() == 2 and gy.size(1) == w.size(0), "gy @ w")
     n, n_out, n_in = gy.size(0), gy.size(1), w.size(1)
+    if relu_output is not None:
+        _check(gy, relu_output, relu_output.shape == (n, n_in), "gy @ w and its mask")
     gy, w = _rows(gy), _rows(w)
     gx = _new_rows(n, n_in, gy)
     args = (gy.data_ptr(), _ld(gy), w.data_ptr(), _ld(w))
@@ -87,6 +99,7 @@ def dense_grad_weight(gy: torch.Tensor, x: torch.Tensor, relu_x: bool = False) -
     """``gy.T @ x`` for ``gy`` [N, out], ``x`` [N, in]: the weight gradient [out, in] (``relu_x``: of
     ``max(x, 0)``).  The partial results of the row ranges go through a workspace from torch's
     allocator, which is stream-ordered: calls on different streams and threads do not share one."""
+    _check(gy, x, gy.dim() == 2 and x.dim() == 2 and gy.size(0) == x.size(0), "gy.T @ x")
     n, n_out, n_in = gy.size(0), gy.size(1), x.size(1)
     gy, x = _rows(gy), _rows(x)
     gw = gy.new_empty((n_out, n_in))

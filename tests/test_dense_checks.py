@@ -1,0 +1,25 @@
+"""Operands of the dense maps that do not fit together are refused before anything reaches the library."""
+import pytest
+import torch
+
+from cbm4gnn_b200 import dense
+
+
+@pytest.mark.parametrize("call", [
+    lambda: dense.dense_forward(torch.ones(8, 5), torch.ones(3, 6)),
+    lambda: dense.dense_forward(torch.ones(8, 6), torch.ones(3, 5)),
+    lambda: dense.dense_forward(torch.ones(2, 8, 5), torch.ones(3, 5)),
+    lambda: dense.dense_forward(torch.ones(8, 5), torch.ones(5)),
+    lambda: dense.dense_grad_input(torch.ones(8, 4), torch.ones(3, 6)),
+    lambda: dense.dense_grad_input(torch.ones(8, 3), torch.ones(3, 6), relu_output=torch.ones(7, 6)),
+    lambda: dense.dense_grad_input(torch.ones(8, 3), torch.ones(3, 6), relu_output=torch.ones(8, 5)),
+    lambda: dense.dense_grad_weight(torch.ones(8, 3), torch.ones(7, 6)),
+])
+def test_operands_that_do_not_fit_together(call):
+    with pytest.raises(RuntimeError, match="shape mismatch"):
+        call()
+
+
+def test_operands_on_two_devices():
+    with pytest.raises(RuntimeError, match="operands on cpu and meta"):
+        dense.dense_forward(torch.ones(8, 5), torch.ones((3, 5), device="meta"))
