@@ -65,7 +65,8 @@ def dense_forward(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor | None = N
     _check(x, w, x.dim() == 2 and w.dim() == 2 and x.size(1) == w.size(1), "x @ w.T")
     n, n_in, n_out = x.size(0), x.size(1), w.size(0)
     x, w = _rows(x), _rows(w)
-    direct = out is not None and out.stride(1) == 1 and out.stride(0) >= n_out
+    direct = (out is not None and out.shape == (n, n_out) and out.dtype == x.dtype and out.device == x.device
+              and out.stride(1) == 1 and out.stride(0) >= n_out)  # anything else is copied to, or refused, by torch
     y = out if direct else _new_rows(n, n_out, x)
     args = (x.data_ptr(), _ld(x), w.data_ptr(), _ld(w), y.data_ptr(), _ld(y), n, n_in, n_out)
     if relu_in:
