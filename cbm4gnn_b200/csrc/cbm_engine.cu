@@ -566,49 +566,61 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
 
 // Several whole rows that wait for nobody (prefix items, positions [first, end), none of them PARTIAL) by one warp, 2^lg
 // lanes for each: for slabs of at most 16 vectors, where a row's fixed costs - descriptor, entries, store, each a trip to
-// memory - outweigh its fetches.  Neighbours in the prefix are of about equal length.  235 868 rows of 11 entries, 64
-// columns: 97 us one by one, 84 side by side with 2 fetches per row in flight, 85 with 4, 93 with 8.
-template <bool V4, bool RAGGED, int UNROLL>
-__device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 first, i32 end, i32 c0, i32 wcols, int lg, int lane) {
+// memory - outweigh its fetches.  Neighbours in the prefix are of about equal length.  A row's entries are summed as
+// gather_row_narrow sums them, in 32 >> lg interleaved shares: which of the two a row gets depends on where its claim
+// falls, its bits do not.
+template <bool V4, bool RAGGED, int LG>
+__device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 first, i32 end, i32 c0, i32 wcols, int lane) {
     using V = Vec<V4>;
     using T = typename V::T;
-    const int width = 1 << lg, li = lane & (width - 1);
+    constexpr int width = 1 << LG, SHARES = 32 >> LG, UNROLL = 2;
+    const int li = lane & (width - 1);
     const bool has = li * V::E < wcols;
     const float* xs = p.x + c0 + li * V::E;
-    for (i32 base = first; base < end; base += 32 >> lg) {
-        const i32 pos = base + (lane >> lg);
+    for (i32 base = first; base < end; base += SHARES) {
+        const i32 pos = base + (lane >> LG);
         const bool on = pos < end;
         const int4 da = __ldg((const int4*)(p.desc + min(pos, end - 1)));
         const int4 db = __ldg((const int4*)(p.desc + min(pos, end - 1)) + 1);
         const i32 len = on ? (da.w >> ITEM_LEN_SHIFT) & 0xff : 0;
         const i32 most = (i32)__reduce_max_sync(0xffffffffu, (unsigned)len);
-        T acc = V::zero();
+        T acc[SHARES];
+#pragma unroll
+        for (int s = 0; s < SHARES; ++s) acc[s] = V::zero();
         for (i32 b = 0; b < most; b += width) {
             i32 mc = 0;
             float mw = 0.f;
             if (b + li < len) PairEntries{p.ent}.get(db.x + b + li, mc, mw);
             const i32 here = min(width, most - b);
-            for (i32 j = 0; j < here; j += UNROLL) {
-                T t[UNROLL];
+            for (i32 j0 = 0; j0 < here; j0 += SHARES) {
 #pragma unroll
-                for (int k = 0; k < UNROLL; ++k) {
-                    const i32 c = __shfl_sync(0xffffffffu, mc, j + k, width);
-                    t[k] = V::ld_ro_if(xs + (i64)c * p.ldx, has && j + k < here && b + j + k < len);
-                }
+                for (int h = 0; h < SHARES; h += UNROLL) {
+                    const i32 j = j0 + h;
+                    T t[UNROLL];
 #pragma unroll
-                for (int k = 0; k < UNROLL; ++k) {
-                    const float w = __shfl_sync(0xffffffffu, mw, j + k, width);
-                    acc = V::fma(j + k < here && b + j + k < len ? w : 0.f, t[k], acc);
+                    for (int k = 0; k < UNROLL; ++k) {
+                        const i32 c = __shfl_sync(0xffffffffu, mc, j + k, width);
+                        t[k] = V::ld_ro_if(xs + (i64)c * p.ldx, has && b + j + k < len);
+                    }
+#pragma unroll
+                    for (int k = 0; k < UNROLL; ++k) {
+                        const float w = __shfl_sync(0xffffffffu, mw, j + k, width);
+                        acc[h + k] = V::fma(b + j + k < len ? w : 0.f, t[k], acc[h + k]);
+                    }
                 }
             }
         }
-        if (p.use_scale && p.mode != MODE_DELTA_ONLY) acc = V::mul(__int_as_float(db.z), acc);
+#pragma unroll
+        for (int d = 1; d < SHARES; d <<= 1)
+#pragma unroll
+            for (int s = 0; s < SHARES; s += 2 * d) acc[s] = V::fma(1.0f, acc[s + d], acc[s]);
+        if (p.use_scale && p.mode != MODE_DELTA_ONLY) acc[0] = V::mul(__int_as_float(db.z), acc[0]);
         if (on && has) {
             const i32 col = c0 + li * V::E, some = p.f - col;
             float* y = p.y + (i64)da.x * p.ldy + col;
-            if (RAGGED && !(p.y_vec && some >= V::E)) V::st_some(y, acc, some);
-            else if (da.w & ITEM_PUBLISH) V::st(y, acc);
-            else V::st_stream(y, acc);
+            if (RAGGED && !(p.y_vec && some >= V::E)) V::st_some(y, acc[0], some);
+            else if (da.w & ITEM_PUBLISH) V::st(y, acc[0]);
+            else V::st_stream(y, acc[0]);
         }
         if (p.mode != MODE_DELTA_ONLY) {
             __syncwarp();
@@ -647,7 +659,8 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
         if constexpr (NARROW) {
             const int lg = lanes_log2<V::E>(wcols);
             if (lg >= 3 && count > 1 && first >= p.n_partial && first + count <= p.n_prefix && p.n_bcast == 0) {
-                rows_narrow<V4, RAGGED, 2>(p, slab, first, first + count, c0, wcols, lg, lane);
+                if (lg == 4) rows_narrow<V4, RAGGED, 4>(p, slab, first, first + count, c0, wcols, lane);
+                else rows_narrow<V4, RAGGED, 3>(p, slab, first, first + count, c0, wcols, lane);
                 continue;
             }
         }

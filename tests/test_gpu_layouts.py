@@ -1,10 +1,12 @@
 """Operand layouts and widths at which the product kernels change form: row groups of 1 - 16 lanes, the last
 partial vector of a row, operands that are copied to aligned rows first, results whose rows are not aligned."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
-from cbm4gnn_b200 import graphs
+from cbm4gnn_b200 import _lib, graphs
 from cbm4gnn_b200.cbm import cbm_matrix
 from helpers import sparse_product, with_self_loops
 
@@ -76,3 +78,35 @@ def test_rows_in_community_order(community_graph, f, pad):
     c.seq_mkl_csr_spmm(xd, two)
     c.seq_mkl_csr_fused_update(two)
     np.testing.assert_allclose(two.cpu().numpy(), want, **TOL)
+
+
+@pytest.fixture(scope="module")
+def many_rows():
+    """So many rows that wait for nobody that a warp claims several (256 for each SM and more): narrow ones are then
+    worked on side by side."""
+    ei = with_self_loops(graphs.copy_model(45000, 0.6, 4, 3))
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=8, normalized=True, build_device=0)
+    length = np.diff(c._crow)
+    assert ((c._parent == c.num_rows) & (length <= 96)).sum() > 37888 and (length > 192).any()
+    return ei, c
+
+
+@pytest.mark.parametrize("f", [3, 13, 17, 29, 32, 33, 47, 61, 64])
+@pytest.mark.parametrize("pad", [0, 1, 4])
+def test_rows_side_by_side(many_rows, f, pad):
+    """Narrow rows: right, and with the same bits whether several share a warp (the product) or each has its own
+    (delivery to further buffers)."""
+    ei, c = many_rows
+    n, pitch = c.num_rows, -(-f // 4) * 4 + pad
+    x = np.random.default_rng(f).standard_normal((n, f)).astype(np.float32)
+    xd, yd, own, sent = (_buffer(n, f, pitch) for _ in range(4))
+    xd.copy_(torch.from_numpy(x))
+    c.omp_mkl_csr_fused_spmm_update(xd, yd)
+    to = (ctypes.c_void_p * 1)(sent.data_ptr())
+    _lib.check(_lib.lib().cbm_b200_spmm_update_bcast(c.plan(0).handle, xd.data_ptr(), pitch, own.data_ptr(), pitch, f, 1, 0, 1,
+                                                     to, torch.cuda.current_stream().cuda_stream))
+    c.plan(0).status()
+    np.testing.assert_allclose(yd.cpu().numpy(), sparse_product(ei, x, True), **TOL)
+    assert torch.equal(own, yd) and torch.equal(sent, yd)
+    pad_of = yd.as_strided((n, pitch - f), (pitch, 1), f)
+    assert torch.equal(pad_of, torch.full_like(pad_of, 7.0))
