@@ -14,8 +14,9 @@
 //     the MMAs, 8 warps add up the accumulators and store Y with the ReLU or the mask applied (32 x 64 sums each).
 //   * Y leaves (and the mask arrives) in whole 128-byte lines, 32 x 32 sums turned round through 4 KB of shared memory
 //     per warp.
-// 235 868 rows, against three-term GEMMs that split both operands for every 128 x 128 x 16 tile: 128 -> 256 96 us
-// (200), 256 -> 64 79 (100), 256 -> 256 175 (349), gradient 256 -> 128 101 (189).
+// Every 16-deep step has an accumulator of its own (see cbm_map.cuh), so the sums are added up every 16 columns; with
+// accumulators of 64 columns 128 -> 256 took 96 us.  235 868 rows, against three-term GEMMs that split both operands
+// for every 128 x 128 x 16 tile: 128 -> 256 128 us (201), 256 -> 64 93 (101), 100 000 rows 256 -> 256 100 (153).
 #include "cbm_map.cuh"
 
 #include <mutex>
@@ -232,31 +233,21 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
         u32 run = 0, it = 0;
         bool ok = true;
         for (int tile = blockIdx.y; tile < p.row_tiles && ok; tile += gridDim.y)
-            for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                const u32 ds = it & 1, use = it >> 1;
-                if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
-                const u32 d = tmem + ds * D_COLS;
-                const int here = min(2, chunks - 2 * kb);
-                for (int c = 0; c < here && ok; ++c) {
-                    const u32 slot = (run + c) % A_SLOTS;
-                    if (!(ok = warp_wait(a_full + 8 * slot, ((run + c) / A_SLOTS) & 1, gave_up, p.timeout))) break;
+            for (int c = 0; c < chunks && ok; ++c, ++run) {
+                const u32 slot = run % A_SLOTS, a = tmem + A_COL + slot * A_SLOT_COLS;
+                const u32 b = b0 + (u32)(c >> 1) * block + 64 * (c & 1);
+                if (!(ok = warp_wait(a_full + 8 * slot, (run / A_SLOTS) & 1, gave_up, p.timeout))) break;
 #pragma unroll
-                    for (int s = 0; s < 2; ++s)
-                        if (4 * kb + 2 * c + s < p.steps)
-                            mma_small(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, b0 + (u32)kb * block + 32 * (2 * c + s), term, idesc,
-                                      c + s > 0);
+                for (int s = 0; s < 2; ++s) {
+                    if (2 * c + s >= p.steps) break;
+                    const u32 ds = it & 1, use = it >> 1, d = tmem + ds * D_COLS;
+                    if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
+                    mma_small(d, a + 8 * s, b + 32 * s, term, idesc, false);
+                    mma(d, a + 8 * s, desc_of(b + 32 * s), idesc, true);
+                    commit(d_full + 8 * ds);
+                    ++it;
                 }
-                if (!ok) break;
-                for (int c = 0; c < here; ++c) {
-                    const u32 slot = (run + c) % A_SLOTS;
-#pragma unroll
-                    for (int s = 0; s < 2; ++s)
-                        if (4 * kb + 2 * c + s < p.steps)
-                            mma(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, desc_of(b0 + (u32)kb * block + 32 * (2 * c + s)), idesc, true);
-                    commit(a_empty + 8 * slot);
-                }
-                commit(d_full + 8 * ds);
-                run += here;
+                if (ok) commit(a_empty + 8 * slot);
             }
         if (!ok) {  // the MMAs under way end before the block frees its tensor memory
             commit(drained);
@@ -310,7 +301,7 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                     keep[b] = bits;
                 }
             }
-            // The first block sets the sums, the others add to them (told apart at compile time: the sums must not
+            // The first step sets the sums, the others add to them (told apart at compile time: the sums must not
             // be live while the mask is fetched).
             float acc[2][32];
             auto collect = [&](auto first) -> bool {
@@ -329,11 +320,15 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                             : "r"(at + 16 * q));
                     wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        asm volatile("" : "+f"(r[i]));  // not before the wait
-                        float& s = acc[q >> 1][16 * (q & 1) + i];
-                        if constexpr (decltype(first)::value) s = r[i];
-                        else s += r[i];
+                    for (int i = 0; i < 16; i += 2) {
+                        asm volatile("" : "+f"(r[i]), "+f"(r[i + 1]));  // not before the wait
+                        float &s = acc[q >> 1][16 * (q & 1) + i], &t = acc[q >> 1][16 * (q & 1) + i + 1];
+                        if constexpr (decltype(first)::value) {
+                            s = r[i];
+                            t = r[i + 1];
+                        } else {
+                            add2(s, t, r[i], r[i + 1]);
+                        }
                     }
                 }
                 fence_before();
@@ -343,7 +338,7 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                 return true;
             };
             if (!collect(std::true_type{})) goto done;
-            for (int kb = 1; kb < kblocks; ++kb)
+            for (int s = 1; s < p.steps; ++s)
                 if (!collect(std::false_type{})) goto done;
 #pragma unroll
             for (int b = 0; b < 2; ++b) {

@@ -6,11 +6,15 @@
 // below 2^-24 of |a||b|.
 //
 // The tensor cores cut the accumulator off at every step instead of rounding it, always towards zero, so a long
-// contraction in one accumulator drifts: 1.7e-6 of the result for 256 columns, 1e-5 for the rows of a graph.
-// Hence the contraction is done in blocks of 64.  Within a block the five small products of every step come
-// first, while the accumulator is 2^-8 of what it will be, then the four large ones; and every block starts
-// a fresh accumulator, which the epilogue warps add to sums in registers, rounded.  Measured against float64:
-// 8e-8 - 1e-7 of the result for 64 - 600 columns, 1.7e-7 for 235 868 rows (cuBLAS fp32: 1.4e-7 - 4e-7, 1.5e-6).
+// contraction in one accumulator drifts: 1.7e-6 of the result for 256 columns, 1e-5 for the rows of a graph.  Hence
+// an accumulator holds a short stretch of the contraction only: first the small products, while it is 2^-8 of what
+// it will be, then the large ones; the epilogue warps add it to sums in registers, rounded.
+//   * Forward and input gradient: 16 columns, one step.  With 64 columns the maps took three quarters of the time, but
+//     the drift (6e-8 of the result instead of 4e-8) is the same for all rows and does not average out in the product that
+//     follows: 128 -> 256 -> 64 with its products 1.36e-7 against 1.17e-7 of the result; 64 columns 7.9e-8 against 6.3e-8.
+//   * Weight gradient: 64 rows, 1.7e-7 for 235 868 rows (256 to 64 columns).
+// Measured against float64: 6e-8 - 1.2e-7 of the result for 64 - 512 columns (cuBLAS fp32: 1.4e-7 - 4e-7; 1.5e-6 over
+// 235 868 rows).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -142,6 +146,13 @@ __device__ __forceinline__ u64 desc_of(u32 addr) {
 }
 // 16-byte piece `k8` (8 bf16) of row `row` in that layout, from the start of the 64-wide block of rows.
 __device__ __forceinline__ u32 swizzled(u32 row, u32 k8) { return row * 128 + ((k8 ^ (row & 7)) << 4); }
+
+// (s, t) += (x, y), both with one instruction.
+__device__ __forceinline__ void add2(float& s, float& t, float x, float y) {
+    asm("{\n\t.reg .b64 a, b;\n\tmov.b64 a, {%0, %1};\n\tmov.b64 b, {%2, %3};\n\tadd.rn.f32x2 a, a, b;\n\tmov.b64 {%0, %1}, a;\n\t}"
+        : "+f"(s), "+f"(t)
+        : "f"(x), "f"(y));
+}
 
 // The five small products of one 16-deep step, smallest first; `b_term` bytes lie between B's terms.
 __device__ __forceinline__ void mma_small(u32 d, u32 a, u32 b, u32 b_term, u32 idesc, bool add) {
