@@ -14,7 +14,7 @@ import ctypes
 import os
 import shutil
 import subprocess
-from ctypes import POINTER, c_char_p, c_double, c_float, c_int32, c_int64, c_void_p
+from ctypes import POINTER, c_char_p, c_double, c_float, c_int32, c_int64, c_uint64, c_void_p
 
 _PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 _ROOT = os.path.dirname(_PKG_DIR)
@@ -54,6 +54,8 @@ EXPORTED = [
     "cbm_b200_plan_create",
     "cbm_b200_plan_destroy",
     "cbm_b200_schedule_info",
+    "cbm_b200_schedule_as_planned",
+    "cbm_b200_plan_schedule",
     "cbm_b200_plan_info",
     "cbm_b200_plan_tune",
     "cbm_b200_plan_status",
@@ -177,6 +179,9 @@ def lib() -> ctypes.CDLL:
     sig("cbm_b200_plan_destroy", None, c_void_p)
     sig("cbm_b200_schedule_info", c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
         c_void_p, c_void_p, c_int32, c_int32, c_int32, i32p, i32p, i32p, i32p)
+    sig("cbm_b200_schedule_as_planned", c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+        c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
+    sig("cbm_b200_plan_schedule", c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
     sig("cbm_b200_plan_info", c_int32, c_void_p, i32p, POINTER(c_int64), i32p, i32p,
         POINTER(c_int64))
     sig("cbm_b200_plan_tune", c_int32, c_void_p, c_int32, c_int32, c_int32, c_int32)

@@ -1035,6 +1035,7 @@ struct cbm_b200_plan {
     i32 n_items = 0;   // work items per slab (rows + extra segments of long rows)
     i32 n_prefix = 0;  // items that never wait
     i32 n_partial = 0; // PARTIAL items = scratch slots per slab
+    i32 segment = 0;   // delta entries of a PARTIAL item
     float* d_scratch = nullptr;
     i64 scratch_cap = 0;
     i64 n_delta = 0;
@@ -1192,6 +1193,7 @@ struct Schedule {
     i64 n_ent = 0;
     std::vector<Chunk> chunks;  // clustered plans
     bool clustered = false;
+    i32 segment = 0;  // delta entries of a PARTIAL item
     i64 n_delta = 0;
     i32 n_prefix = 0, n_partial = 0, n_rows_owned = 0, depth = 0, n_root_children = 0, n_labels = 0;
 };
@@ -1272,17 +1274,30 @@ void make_chunks(Schedule& sch, i32 n_prefix) {
     if (c.count > 0) sch.chunks.push_back(c);
 }
 
+// How a schedule is cut and ordered.  As a plan on a GPU is: long rows cut finer where the mean row is short, communities
+// looked for on `device` or, for a check without a GPU, given as `labels` (row v belongs to community labels[v]).
+struct Rules {
+    bool as_plan = false;
+    int device = -1;
+    const i32* labels = nullptr;
+};
+
 // Sorts the rows of a graph with communities by community (rank[v] = place of row v).  Returns false, and leaves
 // the rows as they are, where that would not bring row pieces into reach of an SM's L1: in a small graph (X is
 // fetched from L2 anyway and a launch is bound by latency), and where about 1 000 consecutive entries of
 // the sorted rows still name mostly different columns.  On B200, width 128: rows of 22 entries in
 // communities of 55 (ratio 0.4) gain 40 %, rows of 11 in communities of 118 (0.5) gain 15 %; copy-model graphs
 // (0.75 - 0.95), whose common columns are few hubs, gain nothing.
-bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std::vector<i32>& parent, int device,
+bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std::vector<i32>& parent, const Rules& rules,
                    std::vector<i32>& rank) {
-    if (device < 0 || n < 16384 || crow[n] < 4 * (i64)n || crow[n] > INT32_MAX - n - 1024) return false;
-    std::vector<i32> label((size_t)n);
-    if (!cbm::cluster_rows(n, crow, col, parent.data(), device, label.data())) return false;
+    std::vector<i32> label;
+    if (rules.labels) {
+        label.assign(rules.labels, rules.labels + n);
+    } else {
+        if (rules.device < 0 || n < 16384 || crow[n] < 4 * (i64)n || crow[n] > INT32_MAX - n - 1024) return false;
+        label.resize((size_t)n);
+        if (!cbm::cluster_rows(n, crow, col, parent.data(), rules.device, label.data())) return false;
+    }
     // counting sort by label, stable in v
     std::vector<i32> start((size_t)n + 1, 0), sorted((size_t)n);
     for (i32 v = 0; v < n; ++v) ++start[(size_t)label[v] + 1];
@@ -1302,7 +1317,7 @@ bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std
         std::sort(cols.begin(), cols.end());
         distinct += std::unique(cols.begin(), cols.end()) - cols.begin();
     }
-    if (distinct * 10 > entries * 7) return false;
+    if (!rules.labels && distinct * 10 > entries * 7) return false;
     rank.resize((size_t)n);
     for (i32 i = 0; i < n; ++i) rank[sorted[i]] = i;
     return true;
@@ -1313,7 +1328,7 @@ bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std
 int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,
                    const int32_t* delta_col, const float* delta_val, const float* multiplier,
                    const int32_t* perm, int32_t n_labels, int32_t own_begin, int32_t own_end, Schedule& sch,
-                   int32_t csr_cols = 0, int device = -1) {
+                   int32_t csr_cols = 0, const Rules& rules = Rules()) {
     std::vector<i32> flat_row, flat_col;
     if (csr_cols > 0) {
         if (n < 0 || !delta_crow) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: NULL row pointers");
@@ -1401,7 +1416,7 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
     // segments only add parked sums (40 000 rows of 152 entries: 194 us, 201, 234).
     i32 longest = 0;
     for (i32 v = 0; v < n; ++v) longest = std::max(longest, delta_crow[v + 1] - delta_crow[v]);
-    const bool fine = device >= 0 && nd_all <= 64 * (i64)n && longest <= 64 * 0xffff;
+    const bool fine = rules.as_plan && nd_all <= 64 * (i64)n && longest <= 64 * 0xffff;
     const i32 SEG = fine ? 64 : 128, SPLIT_OVER = fine ? 96 : 192;
     auto row_len = [&](i32 v) { return delta_crow[v + 1] - delta_crow[v]; };
     auto is_split = [&](i32 v) { return row_len(v) > SPLIT_OVER; };
@@ -1418,7 +1433,8 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
         }
     std::vector<RowDesc>& desc = sch.desc;
     std::vector<i32> rank;
-    sch.clustered = col_bound == n && cluster_order(n, delta_crow, delta_col, parent, device, rank);
+    sch.clustered = col_bound == n && cluster_order(n, delta_crow, delta_col, parent, rules, rank);
+    sch.segment = SEG;
     // items get their entry ranges now; the entries are filled in at the end, on several threads
     std::vector<i64> source;  // per item: its first entry in the delta arrays
     source.reserve((size_t)n);
@@ -1545,6 +1561,41 @@ extern "C" int cbm_b200_schedule_info(int32_t n, const int32_t* mst_row, const i
 }
 
 namespace {
+// FNV-1a over the items in their order, 8 bytes at a time.
+uint64_t fingerprint_of(const RowDesc* desc, size_t n) {
+    static_assert(sizeof(RowDesc) == 32, "four words an item");
+    uint64_t h = 0xcbf29ce484222325ull;
+    for (size_t i = 0; i < n; ++i) {
+        uint64_t w[4];
+        std::memcpy(w, desc + i, sizeof(w));
+        for (uint64_t v : w) h = (h ^ v) * 0x100000001b3ull;
+    }
+    return h;
+}
+}  // namespace
+
+extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
+                                            const int32_t* delta_crow, const int32_t* delta_col,
+                                            const float* delta_val, const float* multiplier,
+                                            const int32_t* labels, int32_t* n_items, int32_t* n_prefix,
+                                            int32_t* n_partial, int32_t* n_chunks, int32_t* segment,
+                                            uint64_t* fingerprint) {
+    for (i32 v = 0; labels && v < n; ++v)
+        if (labels[v] < 0 || labels[v] >= n) return cbm::fail(CBM_B200_ERR_ARG, "schedule_as_planned: label out of range");
+    Schedule sch;
+    const int rc = build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, sch, 0,
+                                  Rules{true, -1, labels});
+    if (rc) return rc;
+    if (n_items) *n_items = (i32)sch.desc.size();
+    if (n_prefix) *n_prefix = sch.n_prefix;
+    if (n_partial) *n_partial = sch.n_partial;
+    if (n_chunks) *n_chunks = (i32)sch.chunks.size();
+    if (segment) *segment = sch.segment;
+    if (fingerprint) *fingerprint = fingerprint_of(sch.desc.data(), sch.desc.size());
+    return CBM_B200_OK;
+}
+
+namespace {
 int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized, int32_t device,
                        cbm_b200_plan** out);
 }
@@ -1558,7 +1609,7 @@ extern "C" int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int
     *out = nullptr;
     Schedule sch;
     const int rc0 = build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm,
-                                   n_labels, own_begin, own_end, sch, 0, device);
+                                   n_labels, own_begin, own_end, sch, 0, Rules{true, device, nullptr});
     if (rc0) return rc0;
     return plan_from_schedule(sch, n, own_end - own_begin, multiplier != nullptr, device, out);
 }
@@ -1570,7 +1621,8 @@ extern "C" int cbm_b200_csr_plan_create(int32_t n_rows, int32_t n_cols, const in
     *out = nullptr;
     if (n_cols <= 0) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: n_cols must be positive");
     Schedule sch;
-    const int rc0 = build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols, device);
+    const int rc0 = build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols,
+                                   Rules{true, device, nullptr});
     if (rc0) return rc0;
     return plan_from_schedule(sch, n_rows, n_rows, false, device, out);
 }
@@ -1600,6 +1652,7 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
     p->n_items = (i32)desc.size();
     p->n_prefix = n_prefix;
     p->n_partial = n_partial;
+    p->segment = sch.segment;
     p->n_delta = sch.n_delta;
     p->n_chunks = (i32)sch.chunks.size();
     p->n_root_children = n_root_children;
@@ -1647,6 +1700,23 @@ extern "C" int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64
     if (n_root_children) *n_root_children = p->n_root_children;
     if (depth) *depth = p->depth;
     if (device_bytes) *device_bytes = p->device_bytes;
+    return CBM_B200_OK;
+}
+
+extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+                                      int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
+    if (!p) return cbm::fail(CBM_B200_ERR_ARG, "plan_schedule: NULL plan");
+    if (n_items) *n_items = p->n_items;
+    if (n_prefix) *n_prefix = p->n_prefix;
+    if (n_partial) *n_partial = p->n_partial;
+    if (n_chunks) *n_chunks = p->n_chunks;
+    if (segment) *segment = p->segment;
+    if (fingerprint) {
+        DeviceGuard g(p->device);
+        std::vector<RowDesc> desc((size_t)p->n_items);
+        if (p->n_items) CBM_CUDA(cudaMemcpy(desc.data(), p->d_desc, desc.size() * sizeof(RowDesc), cudaMemcpyDeviceToHost));
+        *fingerprint = fingerprint_of(desc.data(), desc.size());
+    }
     return CBM_B200_OK;
 }
 

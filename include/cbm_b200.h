@@ -120,21 +120,35 @@ int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int32_t* mst_c
 
 void cbm_b200_plan_destroy(cbm_b200_plan* p);
 
-/* Host-only twin of cbm_b200_plan_create (same arguments minus the device): builds the schedule,
- * runs the pre-launch checks (every item waits only for earlier items, whoever is waited for
+/* Host-only twin of cbm_b200_plan_create (same arguments minus the device): builds a schedule with rows cut at
+ * 192 entries, runs the pre-launch checks (every item waits only for earlier items, whoever is waited for
  * publishes, every row produced and every parked partial sum collected exactly once) and reports
- * its sizes.  Needs no GPU; plan_create runs the same checks (on a graph whose mean row is short it cuts long
- * rows finer than reported here, and a graph with communities it orders by them). */
+ * its sizes.  Needs no GPU; plan_create runs the same construction and checks by its own rules, see below. */
 int cbm_b200_schedule_info(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
                            const int32_t* delta_crow, const int32_t* delta_col,
                            const float* delta_val, const float* multiplier, const int32_t* perm,
                            int32_t n_labels, int32_t own_begin, int32_t own_end, int32_t* n_items,
                            int32_t* n_prefix, int32_t* n_partial, int32_t* n_rows);
 
+/* The same by the rules of cbm_b200_plan_create, for a whole matrix in its own order: rows cut finer where the mean row
+ * is short, and, with labels != NULL (labels[v] in [0, n): the community of row v), community by community in chunks, as
+ * plan_create orders a graph whose communities it finds on the GPU.  The fingerprint is a hash of the items in their order. */
+int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
+                                 const int32_t* delta_crow, const int32_t* delta_col,
+                                 const float* delta_val, const float* multiplier, const int32_t* labels,
+                                 int32_t* n_items, int32_t* n_prefix, int32_t* n_partial, int32_t* n_chunks,
+                                 int32_t* segment, uint64_t* fingerprint);
+
 /* Figures used by the byte model: rows computed by this plan, delta entries of those rows, rows
  * whose parent is the virtual root, tree depth, and device bytes held by the plan. */
 int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64_t* n_delta,
                        int32_t* n_root_children, int32_t* depth, int64_t* device_bytes);
+
+/* The schedule a plan holds: work items per column slab, those that never wait, parked partial sums, chunks (0: not in
+ * community order), delta entries of a partial sum, and the fingerprint of cbm_b200_schedule_as_planned (its items are
+ * fetched from the GPU when it is asked for).  Any out-pointer may be NULL. */
+int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+                           int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
 
 /* Tuning knobs (0 keeps the default): column-slab width in floats, thread blocks per launch, the
  * column-chunk width (a multiple of 4) of the host-buffer pipeline below, and the kernel form

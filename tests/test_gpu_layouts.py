@@ -59,6 +59,9 @@ def community_graph(request):
     key = np.unique(ei[0] * n + ei[1])
     ei = np.stack([key // n, key % n])
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
+    made = c.plan(0).schedule()
+    assert made["n_chunks"] > 0 and made["n_partial"] > 0 and made["n_items"] > made["n_prefix"]
+    assert request.param == 2 or c.build_info["depth"] > 1
     return ei, c
 
 
@@ -78,6 +81,16 @@ def test_rows_in_community_order(community_graph, f, pad):
     c.seq_mkl_csr_spmm(xd, two)
     c.seq_mkl_csr_fused_update(two)
     np.testing.assert_allclose(two.cpu().numpy(), want, **TOL)
+    own, sent = _buffer(c.num_rows, f, f + pad), _buffer(c.num_rows, f, f + pad)
+    _deliver(c, xd, own, sent, relu=True)
+    assert torch.equal(own, yd) and torch.equal(sent, yd.relu())
+
+
+def _deliver(c, x, y, to, relu=False):
+    """The product with its rows also stored to a further buffer."""
+    _lib.check(_lib.lib().cbm_b200_spmm_update_bcast(
+        c.plan(0).handle, x.data_ptr(), x.stride(0), y.data_ptr(), y.stride(0), x.size(1), 1, int(relu), 1,
+        (ctypes.c_void_p * 1)(to.data_ptr()), torch.cuda.current_stream().cuda_stream))
 
 
 @pytest.fixture(scope="module")
@@ -87,7 +100,8 @@ def many_rows():
     ei = with_self_loops(graphs.copy_model(45000, 0.6, 4, 3))
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=8, normalized=True, build_device=0)
     length = np.diff(c._crow)
-    assert ((c._parent == c.num_rows) & (length <= 96)).sum() > 37888 and (length > 192).any()
+    made = c.plan(0).schedule()
+    assert made["n_chunks"] == 0 and made["n_prefix"] - made["n_partial"] > 37888 and (length > 192).any()
     return ei, c
 
 
@@ -102,9 +116,7 @@ def test_rows_side_by_side(many_rows, f, pad):
     xd, yd, own, sent = (_buffer(n, f, pitch) for _ in range(4))
     xd.copy_(torch.from_numpy(x))
     c.omp_mkl_csr_fused_spmm_update(xd, yd)
-    to = (ctypes.c_void_p * 1)(sent.data_ptr())
-    _lib.check(_lib.lib().cbm_b200_spmm_update_bcast(c.plan(0).handle, xd.data_ptr(), pitch, own.data_ptr(), pitch, f, 1, 0, 1,
-                                                     to, torch.cuda.current_stream().cuda_stream))
+    _deliver(c, xd, own, sent)
     c.plan(0).status()
     np.testing.assert_allclose(yd.cpu().numpy(), sparse_product(ei, x, True), **TOL)
     assert torch.equal(own, yd) and torch.equal(sent, yd)

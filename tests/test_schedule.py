@@ -90,3 +90,50 @@ def test_schedule_of_shards_and_refusals():
     perm[1] = 0
     rc, _ = _schedule(c, perm=perm, n_labels=n)
     assert rc == 1
+
+
+def _as_planned(c, labels=None):
+    n = c.num_rows
+    p = lambda a: None if a is None else ctypes.c_void_p(a.ctypes.data)
+    out, mark = [ctypes.c_int32() for _ in range(5)], ctypes.c_uint64()
+    mult = None if c.col_multiplier is None else c.col_multiplier.numpy()
+    labels = None if labels is None else np.ascontiguousarray(labels, dtype=np.int32)
+    rc = _lib.lib().cbm_b200_schedule_as_planned(n, p(c.mst_row.numpy()), p(c.mst_col.numpy()), p(c._crow), p(c._dcol), p(c._dval),
+                                                 p(mult), p(labels), *[ctypes.byref(o) for o in out], ctypes.byref(mark))
+    return rc, [o.value for o in out], mark.value
+
+
+def _hub_graph():
+    """A tree some levels deep, a row of 700 entries and rows of odd length."""
+    ei = with_self_loops(graphs.copy_model(1500, 0.9, 8, 11))
+    n = int(ei.max()) + 1
+    key = np.unique(np.concatenate([ei[0] * n + ei[1], 7 * n + np.arange(700, 1400)]))
+    return np.stack([key // n, key % n])
+
+
+@pytest.mark.parametrize("make,segment", [(lambda: _cbm(_hub_graph(), 2, normalized=True), 64),
+                                          (lambda: _cbm(with_self_loops(graphs.copy_model(1000, 0.95, 40, 3)), 1000), 128)])
+@pytest.mark.parametrize("communities", [None, 1, 7, 300])
+def test_schedule_by_the_rules_of_a_plan(make, segment, communities):
+    """Rows cut by the length of the mean row; with communities also the order, the chunks and the paired entries pass the
+    checks (every item behind those it waits for, chunks that hold their items' entries)."""
+    c = make()
+    n, length = c.num_rows, np.diff(c._crow)
+    assert (length.mean() <= 64) == (segment == 64) and (length % 2).any()
+    labels = None if communities is None else np.random.default_rng(1).integers(0, communities, n)
+    rc, got, mark = _as_planned(c, labels)
+    assert rc == 0, _lib.lib().cbm_b200_last_error()
+    split = length > 3 * segment // 2
+    n_partial = int((-(-length[split] // segment) - 1).sum())
+    easy = int(((c._parent == n) & ~split).sum())
+    assert got[:3] == [n + n_partial, n_partial + easy, n_partial] and got[4] == segment and n_partial > 0
+    assert (got[3] > 0) == (labels is not None) and got[3] * 32 >= (got[0] if labels is not None else 0)
+    assert _as_planned(c, labels)[2] == mark
+    if labels is not None and communities > 1:
+        assert mark != _as_planned(c)[2]
+
+
+def test_labels_out_of_range_are_refused():
+    c = _cbm(graphs.erdos_renyi(25, 0.5, 1), 2)
+    for label in (-1, c.num_rows):
+        assert _as_planned(c, np.full(c.num_rows, label))[0] == 1
