@@ -122,3 +122,14 @@ def test_rows_side_by_side(many_rows, f, pad):
     assert torch.equal(own, yd) and torch.equal(sent, yd)
     pad_of = yd.as_strided((n, pitch - f), (pitch, 1), f)
     assert torch.equal(pad_of, torch.full_like(pad_of, 7.0))
+
+
+@pytest.mark.parametrize("n,mu,deg_in", [(60_000, 3.5, 12.0), (200_000, 4.0, 8.0)])
+def test_plans_of_one_graph_are_the_same(n, mu, deg_in):
+    ei = with_self_loops(graphs.stochastic_block_model(n, n // 50, mu, 0.8, deg_in, 3.0, 5))
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True, build_device=0)
+    first = c.plan(0).schedule()
+    assert first["n_chunks"] > 0  # rows in the order of communities found on the GPU
+    for _ in range(4):
+        c._plans.clear()
+        assert c.plan(0).schedule() == first
