@@ -705,6 +705,68 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
     }
 }
 
+// The register form for products that may park only the partial sums of the longest rows (the fixed scratch array, see
+// cbm_b200_spmm_update_static): the PARTIAL items from position `kept` on are left out, and the finishing items they
+// belong to gather those segments themselves, one after the other and in the same order, so that the results are the
+// same bits.  Positions, flags and slots are numbered without the `out` items left out; p holds the counts so numbered.
+template <int NV, bool V4>
+__global__ void __launch_bounds__(256, NV == 1 ? 4 : 2) cbm_items_frugal_kernel(const KParams p, i32 out, i32 segment) {
+    using V = Vec<V4>;
+    using T = typename V::T;
+    constexpr int STEP = 32 * V::E, UNROLL = 4;
+    const int lane = threadIdx.x & 31;
+    const i32 kept = p.n_partial;
+    for (;;) {
+        u64 t = 0;
+        if (lane == 0) t = atomicAdd(p.counter, 1ULL);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        if (t >= (u64)p.n_claims) {
+            leave(p, lane);
+            return;
+        }
+        i32 slab, first, count;
+        decode_claim(p, t, slab, first, count);
+        const i32 c0 = slab * p.slab_w;
+        const i32 wcols = min(p.slab_w, p.f - c0);
+        bool ok[NV];
+#pragma unroll
+        for (int v = 0; v < NV; ++v) ok[v] = (lane * V::E + v * STEP) < wcols;
+        auto gather = [&](i32 beg, i32 len, T(&acc)[NV]) {
+#pragma unroll
+            for (int v = 0; v < NV; ++v) acc[v] = V::zero();
+            if (NV == 1 && wcols <= 16 * V::E)
+                gather_row_narrow<V4, UNROLL>(PairEntries{p.ent}, beg, beg + len, p.x + c0, p.ldx, wcols, lanes_log2<V::E>(wcols),
+                                              acc[0], lane);
+            else
+                gather_row<NV, V4, UNROLL>(PairEntries{p.ent}, beg, beg + len, p.x + c0 + lane * V::E, p.ldx, ok, acc, lane);
+        };
+        for (i32 pos = first; pos < first + count; ++pos) {
+            const i32 item = pos < kept ? pos : pos + out;
+            const int4 da = __ldg((const int4*)(p.desc + item));
+            const int4 db = __ldg((const int4*)(p.desc + item) + 1);
+            i32 info = da.w;
+            T acc[NV];
+            gather(db.x, (info >> ITEM_LEN_SHIFT) & 0xff, acc);
+            const i32 n_part = (i32)((unsigned)info >> ITEM_NPART_SHIFT);
+            if (n_part > 0 && db.y >= kept) {
+                const i32 beg = __ldg(&p.desc[db.y].beg);
+                for (i32 k = 0; k < n_part; ++k) {
+                    T part[NV];
+                    gather(beg + k * segment, segment, part);
+#pragma unroll
+                    for (int v = 0; v < NV; ++v) acc[v] = V::fma(1.0f, part[v], acc[v]);
+                }
+                info &= (1 << ITEM_NPART_SHIFT) - 1;
+            }
+            if (!finish_item<NV, V4, V4>(p, slab, pos, da.x, da.y, da.z - out, info, db.y, __int_as_float(db.z),
+                                         __int_as_float(db.w), acc, ok, c0, lane)) {
+                leave(p, lane);
+                return;
+            }
+        }
+    }
+}
+
 __device__ __forceinline__ unsigned smem_addr(const void* p) {
     return (unsigned)__cvta_generic_to_shared(p);
 }
@@ -1036,6 +1098,8 @@ struct cbm_b200_plan {
     i32 n_prefix = 0;  // items that never wait
     i32 n_partial = 0; // PARTIAL items = scratch slots per slab
     i32 segment = 0;   // delta entries of a PARTIAL item
+    std::vector<i32> part_ends;  // see Schedule
+    i32 n_partial_coarse = 0;
     float* d_scratch = nullptr;
     i64 scratch_cap = 0;
     i64 n_delta = 0;
@@ -1194,6 +1258,8 @@ struct Schedule {
     std::vector<Chunk> chunks;  // clustered plans
     bool clustered = false;
     i32 segment = 0;  // delta entries of a PARTIAL item
+    std::vector<i32> part_ends;  // where each split row's PARTIAL items end
+    i32 n_partial_coarse = 0;    // how many there would be with rows of more than 192 entries cut at 128
     i64 n_delta = 0;
     i32 n_prefix = 0, n_partial = 0, n_rows_owned = 0, depth = 0, n_root_children = 0, n_labels = 0;
 };
@@ -1446,10 +1512,14 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
         return beg;
     };
     for (i32 v : owned_rows) sch.n_delta += row_len(v);
-    // 1. PARTIAL items of every split row
-    std::vector<i32> first_part((size_t)n, -1);
-    for (i32 v : owned_rows) {
-        if (!is_split(v)) continue;
+    // 1. PARTIAL items of every split row, the rows with most of them first (a product that cannot park all of them parks
+    // those of the longest rows)
+    std::vector<i32> first_part((size_t)n, -1), split_rows;
+    for (i32 v : owned_rows)
+        if (is_split(v)) split_rows.push_back(v);
+    std::stable_sort(split_rows.begin(), split_rows.end(), [&](i32 a, i32 b) { return (row_len(a) - 1) / SEG > (row_len(b) - 1) / SEG; });
+    for (i32 v : split_rows) {
+        if (row_len(v) > 192) sch.n_partial_coarse += (row_len(v) - 1) / 128;
         const i32 n_part = (row_len(v) + SEG - 1) / SEG - 1;
         if (n_part > 0xffff)
             return cbm::fail(CBM_B200_ERR_ARG, "plan_create: a row has more than 8388480 delta entries");
@@ -1466,6 +1536,7 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
             q.inv_parent = 1.0f;
             desc.push_back(q);
         }
+        sch.part_ends.push_back((i32)desc.size());
     }
     const i32 n_partial = (i32)desc.size();
     // 2. unsplit children of the virtual root, longest first
@@ -1653,6 +1724,8 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
     p->n_prefix = n_prefix;
     p->n_partial = n_partial;
     p->segment = sch.segment;
+    p->part_ends.swap(sch.part_ends);
+    p->n_partial_coarse = sch.n_partial_coarse;
     p->n_delta = sch.n_delta;
     p->n_chunks = (i32)sch.chunks.size();
     p->n_root_children = n_root_children;
@@ -1773,6 +1846,7 @@ struct LaunchCfg {
     bool in_turn = false;      // see KParams
     bool pack = false;         // the operand is first copied to 16-byte aligned rows
     bool ragged = false;       // 16-byte fetches, but rows of y are not aligned or end inside a vector
+    i32 left_out = 0;          // PARTIAL items, the last ones, that the finishing items do themselves
 };
 
 int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
@@ -1918,6 +1992,15 @@ struct Bcast {
     float* dst[CBM_B200_MAX_BCAST] = {nullptr};
 };
 
+template <int NV, bool V4>
+int launch_frugal(KParams& kp, i32 out, i32 segment, int sm_count, cudaStream_t s) {
+    const int blocks = (int)std::max<i64>(1, std::min<i64>(sm_count * (NV == 1 ? 4 : 2), (kp.n_claims + 7) / 8));
+    kp.n_warps = (u64)blocks * 8;
+    cbm_items_frugal_kernel<NV, V4><<<blocks, 256, 0, s>>>(kp, out, segment);
+    CBM_CUDA(cudaGetLastError());
+    return CBM_B200_OK;
+}
+
 int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
                 int mode, bool use_scale, u64* counter, i32* flags, float* scratch, i32 epoch,
                 cudaStream_t s, const Bcast* bc = nullptr) {
@@ -1942,14 +2025,14 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.ldy = ldy;
     kp.f = f;
     kp.slab_w = c.sh.slab_w;
-    kp.n_items = p->n_items;
-    kp.n_prefix = p->n_prefix;
+    kp.n_items = p->n_items - c.left_out;
+    kp.n_prefix = p->n_prefix - c.left_out;
     kp.group = c.group;
     kp.n_pclaims = c.n_pclaims;
     kp.claims_per_slab = c.claims_per_slab;
     kp.n_claims = c.n_claims;
     kp.scratch = scratch;
-    kp.n_partial = p->n_partial;
+    kp.n_partial = p->n_partial - c.left_out;
     kp.counter = counter;
     kp.flags = flags;
     kp.epoch = epoch;
@@ -1957,6 +2040,17 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.mode = mode;
     kp.use_scale = use_scale ? 1 : 0;
     kp.wait_ns = 2000000000ULL;
+    if (c.left_out > 0) {
+        const i32 out = c.left_out, seg = p->segment;
+        if (c.sh.v4) {
+            if (c.sh.nv == 1) return launch_frugal<1, true>(kp, out, seg, p->sm_count, s);
+            if (c.sh.nv == 2) return launch_frugal<2, true>(kp, out, seg, p->sm_count, s);
+            return launch_frugal<4, true>(kp, out, seg, p->sm_count, s);
+        }
+        if (c.sh.nv == 1) return launch_frugal<1, false>(kp, out, seg, p->sm_count, s);
+        if (c.sh.nv == 2) return launch_frugal<2, false>(kp, out, seg, p->sm_count, s);
+        return launch_frugal<4, false>(kp, out, seg, p->sm_count, s);
+    }
     if (c.tma) return launch_tma<256, 16, 2, 7>(kp, p->sm_count, s);
     if (c.chunked)
         return c.ragged ? launch_chunks<true>(kp, p->n_blocks, p->sm_count, s)
@@ -2395,6 +2489,42 @@ int static_scratch_address(int device, unsigned char** out) {
 
 i64 round_up_256(i64 v) { return (v + 255) / 256 * 256; }
 
+// layout inside the fixed array: counters | ready flags | partial sums
+i64 static_need(i64 n_flags, i64 n_scratch) { return 256 + round_up_256(n_flags * (i64)sizeof(i32)) + n_scratch * (i64)sizeof(float); }
+
+// A product that does not fit the fixed array with all partial sums parked: what it takes is decided by a schedule whose
+// rows are cut only beyond 192 entries, at 128, and by operands that are fetched 16 bytes a lane only where all rows are
+// aligned, so that finer cuts and wider fetches, which need more, refuse no product.  One that would fit so parks the
+// sums of as many of its longest rows as there is room for.  50 000 rows of the second benchmark configuration's kind,
+// 500 columns: 10.1 MiB with 5 076 sums, 4.2 MiB with the 1 719 of coarser cuts; 238 us here with the sums that there is
+// room for, 215 with all of them on the ordinary path, 244 with the coarser cuts.
+bool fit_static(const cbm_b200_plan* p, const float* x, i64 ldx, const float* y, i64 ldy, i32 f, LaunchCfg& c) {
+    const bool x_vec = ldx % 4 == 0 && aligned16(x), all_vec = f % 4 == 0 && x_vec && ldy % 4 == 0 && aligned16(y);
+    const i32 want = p->form && all_vec ? 256 : p->slab_width;
+    const Shape coarse = pick_shape(f, want, all_vec);
+    const i64 rows = (i64)p->n_items - p->n_partial;
+    if (static_need(coarse.n_slabs * (rows + p->n_partial_coarse), (i64)coarse.n_slabs * p->n_partial_coarse * coarse.slab_w) >
+        (i64)CBM_B200_STATIC_SCRATCH_BYTES)
+        return false;
+    c = LaunchCfg{};
+    c.sh = pick_shape(f, want, x_vec && ldx < (i64)1 << 30);
+    c.ragged = c.sh.v4 && !all_vec;
+    const i64 per_sum = (i64)c.sh.n_slabs * (c.sh.slab_w + 1) * (i64)sizeof(i32);
+    const i64 room = (i64)CBM_B200_STATIC_SCRATCH_BYTES - static_need(c.sh.n_slabs * rows, 0) - 256;
+    const auto& ends = p->part_ends;
+    const auto past = std::upper_bound(ends.begin(), ends.end(), std::max<i64>(0, room / per_sum));
+    const i32 kept = past == ends.begin() ? 0 : past[-1];
+    c.left_out = p->n_partial - kept;
+    const i32 n_prefix = p->n_prefix - c.left_out;
+    c.group = (i64)n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256 ? 4 : 1;
+    c.n_pclaims = (n_prefix + c.group - 1) / c.group;
+    c.claims_per_slab = c.n_pclaims + (p->n_items - p->n_prefix);
+    c.n_claims = (i64)c.claims_per_slab * c.sh.n_slabs;
+    c.need_flags = (i64)c.sh.n_slabs * (rows + kept);
+    c.need_scratch = (i64)c.sh.n_slabs * kept * c.sh.slab_w;
+    return static_need(c.need_flags, c.need_scratch) <= (i64)CBM_B200_STATIC_SCRATCH_BYTES;
+}
+
 }  // namespace
 
 extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int64_t ldx, float* y,
@@ -2412,11 +2542,8 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     LaunchCfg c;
     rc = plan_cfg(p, who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
     if (rc) return rc;
-    // layout inside the fixed array: counters | ready flags | partial sums
-    const i64 off_flags = 256;
-    const i64 off_slots = off_flags + round_up_256(c.need_flags * (i64)sizeof(i32));
-    const i64 need = off_slots + c.need_scratch * (i64)sizeof(float);
-    if (need > (i64)CBM_B200_STATIC_SCRATCH_BYTES)
+    const i64 need = static_need(c.need_flags, c.need_scratch);
+    if (need > (i64)CBM_B200_STATIC_SCRATCH_BYTES && !fit_static(p, x, ldx, y, ldy, f, c))
         return cbm::fail(CBM_B200_ERR_ARG,
                          std::string(who) + ": this product needs " + std::to_string(need) +
                              " bytes of scratch, the fixed array holds " +
@@ -2429,6 +2556,7 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     rc = static_scratch_address(p->device, &base);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
+    const i64 off_flags = 256, off_slots = off_flags + round_up_256(c.need_flags * (i64)sizeof(i32));
     // counters and flags must start at zero; the partial sums are written before they are read
     CBM_CUDA(cudaMemsetAsync(base, 0, (size_t)(off_flags + c.need_flags * (i64)sizeof(i32)), s));
     // flags were just cleared, so any non-zero mark will do as this launch's epoch

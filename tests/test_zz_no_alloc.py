@@ -74,3 +74,44 @@ def test_static_scratch_rejects_oversized_products():
     assert rc == 1
     msg = L.cbm_b200_last_error().decode()
     assert "bytes of scratch" in msg and str(8 << 20) in msg
+
+
+def _hubs_on_blocks():
+    """470 000 short rows, which leave little of the fixed array, and 20 of 2 000 entries."""
+    n = 470_000
+    rng = np.random.default_rng(3)
+    ei = graphs.stochastic_block_model(n, n // 50, 3.5, 0.8, 3.0, 1.0, 5)
+    hub = np.repeat(np.arange(20) * 1000, 2000)
+    key = np.unique(np.concatenate([ei[0] * n + ei[1], hub * n + rng.integers(0, n, hub.size), np.arange(n) * (n + 1)]))
+    return np.stack([key // n, key % n])
+
+
+@pytest.mark.parametrize("make,alpha", [(lambda: add_self_loops(torch.from_numpy(graphs.copy_model(50_000, 0.7, 5, 3))).numpy(), 8),
+                                        (_hubs_on_blocks, 2)])
+def test_what_is_refused_does_not_depend_on_how_finely_rows_are_cut(make, alpha):
+    """Parked sums that do not all fit the fixed array are those of the longest rows; as long as a schedule with rows cut at
+    192 entries would fit, the product runs, with the ordinary entry point's bits."""
+    L = _lib.lib()
+    ei = torch.from_numpy(make())
+    c = cbm_matrix(ei.to(torch.int32), torch.ones(ei.shape[1]), alpha=alpha, normalized=True, build_device=0)
+    plan, n = c.plan(0), c.num_rows
+    made, length = plan.schedule(), np.diff(c._crow)
+    coarse = int((-(-length[length > 192] // 128) - 1).sum())
+    assert made["segment"] == 64 and 0 < coarse < made["n_partial"]
+    gen = torch.Generator(device="cuda").manual_seed(7)
+    for f, pad in ((500, 0), (500, 4), (497, 3), (499, 0), (480, 0), (401, 0)):
+        slabs, unaligned, odd = -(-f // 128), (f + pad) % 4 != 0, f % 4 != 0 or (f + pad) % 4 != 0
+        assert 4 * slabs * (n + coarse + 128 * coarse) < 8 << 20 < 4 * slabs * (n + made["n_partial"] * 129)
+        x = torch.randn((n, f + pad), device="cuda", generator=gen)[:, :f]
+        want, got = (torch.full((n, f + pad), float("nan"), device="cuda")[:, :f] for _ in range(2))
+        rc = L.cbm_b200_spmm_update_static(plan.handle, x.data_ptr(), f + pad, got.data_ptr(), f + pad, f, 1,
+                                           torch.cuda.current_stream().cuda_stream)
+        if odd and n > 400_000:  # counted in slabs of 64 columns: more flags than room
+            assert rc == 1 and b"bytes of scratch" in L.cbm_b200_last_error()
+            continue
+        _lib.check(rc)
+        _call(L.cbm_b200_fused_spmm_update, plan, x, want, f)
+        plan.status()
+        # an unaligned operand of this size is copied to aligned rows by the ordinary entry point, and its sums are added
+        # in another order where the last slab is narrow: within fp32 rounding of the longest row
+        torch.testing.assert_close(got, want, atol=0 if not unaligned else 1e-5, rtol=0 if not unaligned else 1e-5)
