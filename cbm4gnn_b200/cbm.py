@@ -470,9 +470,15 @@ class cbm_matrix:
         return _CBMMatmul.apply(x, self, two_step)
 
 
+def result_pitch(width: int) -> int:
+    """Row pitch of a product's result on a GPU."""
+    return width if width < 4 else -(-width // 4) * 4
+
+
 def _product(cbm: "cbm_matrix", x: torch.Tensor) -> torch.Tensor:
     """``A @ x`` / normalized product into a fresh tensor.  On a GPU any row-major operand is taken as it
-    is, and the rows of the result are 16-byte aligned whatever its width."""
+    is, and the rows of the result are 16-byte aligned unless it is narrower than one 16-byte vector: such a
+    result is contiguous."""
     f = x.size(1)
     if not x.is_cuda:
         x = x.contiguous()
@@ -480,8 +486,8 @@ def _product(cbm: "cbm_matrix", x: torch.Tensor) -> torch.Tensor:
     else:
         if x.stride(1) != 1 or x.stride(0) < f:
             x = x.contiguous()
-        y = x.new_empty((cbm.num_rows, -(-f // 4) * 4))
-        if f % 4:
+        y = x.new_empty((cbm.num_rows, result_pitch(f)))
+        if f > 4 and f % 4:
             y = y[:, :f]
     if cbm.col_multiplier is not None:
         cbm._run("cbm_b200_fused_spmm_update", x, y, host_normalized=True)

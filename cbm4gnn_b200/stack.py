@@ -11,7 +11,7 @@ from array import array
 import torch
 
 from . import _lib
-from .cbm import _product, _raw_stream
+from .cbm import _product, _raw_stream, result_pitch
 from .dense import dense_forward, dense_grad_input, dense_grad_weight
 
 
@@ -116,6 +116,11 @@ def _pitch(width):
     return -(-width // 4) * 4
 
 
+def _pitch_out(width, step):
+    """Row pitch of what ``step`` leaves for the caller: as the product or the map called by itself."""
+    return _pitch(width) if step is None else result_pitch(width)
+
+
 @functools.lru_cache(maxsize=128)
 def _forward_list(steps, shapes, n, ldx):
     """``steps``: (plan, normalized) or None; ``shapes``: of the weights.  Bases: x, the allocation, the result, the
@@ -125,7 +130,7 @@ def _forward_list(steps, shapes, n, ldx):
     for k, step in enumerate(steps):
         operands.append((*at, width))
         after = width if step else shapes[j][0]
-        to = (out.room(n * _pitch(after)) if k < last else 2, _pitch(after))
+        to = (out.room(n * _pitch(after)), _pitch(after)) if k < last else (2, _pitch_out(after, step))
         if step:
             out.add(_PRODUCT, step[0], *at, *to, width, step[1])
         else:
@@ -149,7 +154,7 @@ def _backward_list(steps, shapes, n, ldx, ldg, needs):
         step, (place, ld, width), relu = steps[k], operands[k], k > 0 and k % 2 == 0
         to = None
         if k > lowest:
-            to = (out.room(n * _pitch(width)) if k else 4, _pitch(width))
+            to = (out.room(n * _pitch(width)), _pitch(width)) if k else (4, _pitch_out(width, step))
         if step:
             out.add(_PRODUCT, step[0], *at, *to, width, step[1])
         else:
@@ -180,9 +185,10 @@ def _listed_forward(x, steps, shapes, weights):
     calls, _ = _forward_list(_plans(steps, dev), shapes, n, max(x.stride(0), x.size(1)))
     # a stack ends in a map to this width, or in a product of it
     width = shapes[-1][0]
-    y, space = x.new_empty((n, _pitch(width))), x.new_empty(calls.floats)
+    pitch = _pitch_out(width, steps[-1])
+    y, space = x.new_empty((n, pitch)), x.new_empty(calls.floats)
     calls.issue(dev, [x.data_ptr(), space.data_ptr(), y.data_ptr(), *(w.data_ptr() for w in weights)])
-    return (y if width % 4 == 0 else y[:, :width]), x, space
+    return (y if width == pitch else y[:, :width]), x, space
 
 
 class _ListedStack(torch.autograd.Function):
@@ -205,11 +211,12 @@ class _ListedStack(torch.autograd.Function):
         calls = _backward_list(_plans([None if s is None else s.transposed() for s in ctx.steps], dev), shapes, n, max(x.stride(0), width),
                                max(g.stride(0), g.size(1)), (needs[0], *needs[3:]))
         space = x.new_empty(calls.floats)
-        gx = x.new_empty((n, _pitch(width))) if needs[0] else None
+        pitch = _pitch_out(width, ctx.steps[0])
+        gx = x.new_empty((n, pitch)) if needs[0] else None
         gws = [x.new_empty(shape) if need else None for shape, need in zip(shapes, needs[3:])]
         calls.issue(dev, [x.data_ptr(), kept.data_ptr(), g.data_ptr(), space.data_ptr(), gx.data_ptr() if needs[0] else 0,
                           *(w.data_ptr() for w in weights), *(0 if gw is None else gw.data_ptr() for gw in gws)])
-        if needs[0] and width % 4:
+        if needs[0] and width != pitch:
             gx = gx[:, :width]
         return (gx, None, None, *gws)
 

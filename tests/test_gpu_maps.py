@@ -187,3 +187,22 @@ def test_error_of_the_maps_and_its_drift(n, n_in, n_out, bound):
         off = got.double() - want
         assert float(off.norm() / want.norm()) < bound
         assert float((off * want.sign()).mean() / want.abs().mean()) > -4.6e-8
+
+
+@pytest.mark.parametrize("listed_bytes", [stack.LISTED_BYTES, 0])
+@pytest.mark.parametrize("width", [1, 2, 3, 4])
+def test_narrow_products_are_contiguous(width, listed_bytes, monkeypatch):
+    """A few classes at the end, or a few features in front, of a stack; views of them as of any contiguous tensor."""
+    monkeypatch.setattr(stack, "LISTED_BYTES", listed_bytes)
+    edges = torch.arange(50).repeat(2, 1).cuda()
+    out = GCNModel([8, 6, width], alpha=2).cuda()(torch.randn(50, 8, device="cuda"), edges)
+    assert out.is_contiguous() and out.view(-1).shape == (50 * width,)
+    x = torch.randn(50, width, device="cuda", requires_grad=True)
+    model = GCNModel([width, 8, 5], alpha=2).cuda()
+    y = model(x, edges)
+    gx, = torch.autograd.grad(y, x, torch.ones_like(y))
+    assert gx.is_contiguous() and y.stride() == (8, 1)
+    h = (x.double() @ model.layers[0].lin.weight.double().t()).relu()  # (the graph is the identity)
+    want, = torch.autograd.grad(h @ model.layers[1].lin.weight.double().t(), x, torch.ones(50, 5, device="cuda").double())
+    torch.testing.assert_close(gx, want, atol=1e-5, rtol=1e-5)
+    assert model.layers[0].cached_a_t.matmul(x).is_contiguous()
