@@ -37,16 +37,24 @@ int sm_count() {
 }
 
 int* timeout_word() {
-    static std::once_flag once;
-    static int* word = nullptr;
-    std::call_once(once, [] {
-        void* p = nullptr;
-        if (cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped) == cudaSuccess) {
-            word = static_cast<int*>(p);
-            *word = 0;
-        }
-    });
-    return word;
+    static std::mutex making;
+    static std::atomic<int*> made{nullptr};
+    if (int* word = made.load(std::memory_order_acquire)) return word;
+    std::lock_guard<std::mutex> hold(making);
+    if (int* word = made.load(std::memory_order_acquire)) return word;
+    // The first map of a process may be one that is captured into a graph: the allocation is no part of it.
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    if (cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) return nullptr;
+    void* p = nullptr;
+    const cudaError_t e = cudaHostAlloc(&p, sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped);
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) {  // the next call tries again
+        cudaGetLastError();
+        return nullptr;
+    }
+    *static_cast<int*>(p) = 0;
+    made.store(static_cast<int*>(p), std::memory_order_release);
+    return static_cast<int*>(p);
 }
 
 int check_timeout(const char* who) {

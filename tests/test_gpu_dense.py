@@ -121,3 +121,27 @@ def test_two_maps_around_a_relu_as_one_step():
     # CPU operands take the torch path
     pc, c1, c2 = p[:100].cpu(), w1.cpu(), w2.cpu()
     assert torch.allclose(dense.relu_linear_linear(pc, c1, c2), (pc @ c1.t()).relu() @ c2.t())
+
+
+def test_first_map_of_a_process_may_be_a_captured_one():
+    """What the maps set up once per process does not end a stream capture."""
+    import os
+    import subprocess
+    import sys
+    code = """
+import torch
+from cbm4gnn_b200 import dense
+x, w = torch.randn(300, 40, device="cuda"), torch.randn(24, 40, device="cuda")
+g = torch.cuda.CUDAGraph()
+with torch.cuda.graph(g):
+    y = dense.dense_forward(x, w)
+    gw = dense.dense_grad_weight(y, x)
+for _ in range(2):
+    x.normal_()
+    g.replay()
+    assert torch.allclose(y, x @ w.t(), atol=1e-4) and torch.allclose(gw, y.t() @ x, atol=1e-2, rtol=1e-4)
+print("captured")
+"""
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    done = subprocess.run([sys.executable, "-c", code], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.stdout.strip() == "captured", done.stderr
