@@ -78,13 +78,15 @@ void bucket_sort(i64 nnz, i32 n, Key key, Value value, std::vector<i64>& ptr, i3
     // a stretch is worth a thread from some 100 000 elements on, and no more threads than the counters' memory bears out
     const int T = (int)std::max<i64>(1, std::min<i64>({(i64)omp_get_max_threads(), nnz / 100000, nnz / std::max(n, 1) + 1}));
     ptr.assign((size_t)n + 1, 0);
-    std::vector<std::vector<i32>> place((size_t)T);
+    Raw<i32> counters;  // allocated out here: an exception must not leave the parallel region
+    counters.alloc((size_t)T * (size_t)n);
+    const auto place = [&](int q) { return counters.data() + (size_t)q * (size_t)n; };
 #pragma omp parallel num_threads(T)
     {
         const int t = omp_get_thread_num(), threads = omp_get_num_threads();
         for (int q = t; q < T; q += threads) {
-            std::vector<i32>& mine = place[(size_t)q];
-            mine.assign((size_t)n, 0);
+            i32* mine = place(q);
+            std::fill(mine, mine + n, 0);
             for (i64 i = nnz * q / T, e = nnz * (q + 1) / T; i < e; ++i) ++mine[(size_t)key(i)];
         }
 #pragma omp barrier
@@ -92,8 +94,8 @@ void bucket_sort(i64 nnz, i32 n, Key key, Value value, std::vector<i64>& ptr, i3
         for (i32 k = 0; k < n; ++k) {  // places inside the bucket, and the bucket's size
             i32 at = 0;
             for (int q = 0; q < T; ++q) {
-                const i32 c = place[(size_t)q][k];
-                place[(size_t)q][k] = at;
+                const i32 c = place(q)[k];
+                place(q)[k] = at;
                 at += c;
             }
             ptr[(size_t)k + 1] = at;
@@ -101,7 +103,7 @@ void bucket_sort(i64 nnz, i32 n, Key key, Value value, std::vector<i64>& ptr, i3
 #pragma omp single
         for (i32 k = 0; k < n; ++k) ptr[(size_t)k + 1] += ptr[k];
         for (int q = t; q < T; q += threads) {
-            std::vector<i32>& mine = place[(size_t)q];
+            i32* mine = place(q);
             for (i64 i = nnz * q / T, e = nnz * (q + 1) / T; i < e; ++i) {
                 const i32 k = key(i);
                 out[ptr[k] + mine[(size_t)k]++] = value(i);

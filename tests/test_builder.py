@@ -300,3 +300,34 @@ def test_multiplier_and_deltas_whatever_the_defaults_of_torch(dtype, device):
         torch.set_default_device(None)
     assert got.col_multiplier.dtype == torch.float32 and torch.equal(got.col_multiplier, want.col_multiplier)
     assert np.array_equal(got._dcol, want._dcol) and np.array_equal(got._dval, want._dval)
+
+
+@pytest.mark.parametrize("room", [12, 13, 14, 14.5, 15, 15.5])
+def test_memory_that_runs_out_is_an_error_not_an_abort(room):
+    """The counting sort of an unsorted edge list allocates before its threads start: a process whose memory is limited so
+    that the row pointers and the sorted columns (12 bytes a row here) fit and the threads' counters do not gets a
+    status back."""
+    import os
+    import subprocess
+    import sys
+    code = f"""
+import ctypes, resource
+import numpy as np
+L = ctypes.CDLL({_lib.LIB_PATH!r})
+L.cbm_b200_last_error.restype = ctypes.c_char_p
+def build(n):
+    row = np.arange(n, dtype=np.int32)[::-1].copy()
+    out, p = ctypes.c_void_p(), ctypes.c_void_p(row.ctypes.data)
+    return row, lambda: L.cbm_b200_build(p, p, ctypes.c_int64(n), n, 0, None, 0, ctypes.byref(out))
+row, run = build(300_000)
+assert run() == 0  # the threads are there now
+n = 8_000_000
+row, run = build(n)
+used = int(next(s for s in open("/proc/self/status") if s.startswith("VmSize")).split()[1]) * 1024
+resource.setrlimit(resource.RLIMIT_AS, (used + int({room} * n), resource.getrlimit(resource.RLIMIT_AS)[1]))
+print(run(), L.cbm_b200_last_error().decode())
+"""
+    _lib.lib()  # (built)
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                          env=dict(os.environ, OMP_NUM_THREADS="4"))
+    assert done.returncode == 0 and "memory" in done.stdout, (done.returncode, done.stdout, done.stderr[-300:])
