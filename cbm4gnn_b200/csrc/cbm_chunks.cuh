@@ -108,21 +108,13 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, MINB) cbm_chunks_kernel(
 
     if (threadIdx.x >= CONSUMERS * 32) {  // producer
         if (lane != 0) return;
-        i32 slab = 0, chunk = 0, left = 0;
         for (unsigned seq = 0;; ++seq) {
             const unsigned st = seq % STAGES;
-            if (left == 0) {
-                const u64 t = atomicAdd(p.counter, 1ULL);
-                if (t < (u64)p.n_claims) {
-                    slab = (i32)((unsigned)t / (unsigned)p.claims_per_slab);
-                    const i32 r = (i32)t - slab * p.claims_per_slab;
-                    const i32 n_runs = p.n_run / p.run;
-                    left = r < n_runs ? p.run : 1;
-                    chunk = r < n_runs ? r * p.run : p.n_run + (r - n_runs);
-                }
-            }
+            const u64 t = atomicAdd(p.counter, 1ULL);
+            const bool last = t >= (u64)p.n_claims;
+            const i32 slab = last ? 0 : (i32)((unsigned)t / (unsigned)p.claims_per_slab);
             Chunk c{0, 0, 0, 0};
-            if (left > 0) *reinterpret_cast<int4*>(&c) = __ldg(reinterpret_cast<const int4*>(p.chunks + chunk));
+            if (!last) *reinterpret_cast<int4*>(&c) = __ldg(reinterpret_cast<const int4*>(p.chunks + ((i32)t - slab * p.claims_per_slab)));
             if (seq >= STAGES &&
                 !mbar_wait(bars + 8 * (STAGES + st), ((seq / STAGES) + 1) & 1, p.status, 2 * p.wait_ns, true)) {
                 // Nothing may still be on its way into this block's shared memory when it retires: the
@@ -133,7 +125,7 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, MINB) cbm_chunks_kernel(
             }
             s_info[st] = make_int4(slab, c.first, c.count, c.e0);
             s_ticket[st] = 0;
-            if (left == 0) {  // tells the consumers to leave; they have waited for every copy before this
+            if (last) {  // tells the consumers to leave; they have waited for every copy before this
                 mbar_arrive(bars + 8 * st);
                 break;
             }
@@ -143,8 +135,6 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, MINB) cbm_chunks_kernel(
             mbar_expect_tx(bars + 8 * st, n_desc + n_ent);
             bulk_copy_g2s(smem_addr(at), p.desc + c.first, n_desc, bars + 8 * st);
             if (n_ent) bulk_copy_g2s(smem_addr(at + DESC_BYTES), p.ent + c.e0, n_ent, bars + 8 * st);
-            ++chunk;
-            --left;
         }
         leave(p, 0);
         return;

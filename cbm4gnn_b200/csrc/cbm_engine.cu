@@ -107,10 +107,8 @@ struct KParams {
     i32 f;
     i32 y_vec;       // rows of y are 16-byte aligned
     i32 in_turn;     // entries are added strictly one after the other, also in narrow slabs
-    const Chunk* chunks;   // clustered plans: chunks, ...
-    unsigned ldx_bytes;    // ... 4 * ldx,
-    i32 run;               // ... chunks claimed `run` at a time below chunk n_run, one at a time from there on
-    i32 n_run;
+    const Chunk* chunks;   // clustered plans: chunks ...
+    unsigned ldx_bytes;    // ... and 4 * ldx
     i32 slab_w;      // columns per slab
     i32 n_items;     // work items per slab
     i32 n_prefix;    // items that never wait (claimed `group` at a time)
@@ -1839,8 +1837,7 @@ struct LaunchCfg {
     i32 group = 1;     // prefix items per claim
     i32 n_pclaims = 0, claims_per_slab = 0;
     i64 n_claims = 0;
-    bool chunked = false;      // the clustered plan's kernel ...
-    i32 run = 1, n_run = 0;    // ... see KParams
+    bool chunked = false;      // the clustered plan's kernel
     i64 need_flags = 0;        // int32 words
     i64 need_scratch = 0;      // floats
     bool in_turn = false;      // see KParams
@@ -1865,9 +1862,11 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
     int tma = p->form;
     if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY || p->n_chunks > 0) tma = 0;
     c.tma = tma;
-    // Slabs of up to 64 columns gain nothing from the clustered order (235 868 rows of 11 entries, 64 columns:
-    // 106 us against 97): several entries share a fetch there, and what a row costs is its instructions.
-    // On smaller graphs the saved round trips per row still win (20 000 rows of 12 entries, 64 columns: 26 us against 32).
+    // Slabs of up to 64 columns gain nothing from the clustered order on large graphs (235 868 rows of 11 entries, 64
+    // columns: 106 us against 97): several entries share a fetch there, and what a row costs is its instructions.
+    // On smaller graphs the saved round trips per row still win, the more rows wait: 64 columns, few waiting rows, 17 000
+    // rows 22 us against 32, 45 000 34 against 34, 60 000 41 against 39; three quarters waiting, 17 000 39 against 45,
+    // 50 000 60 against 68.
     c.chunked = p->n_chunks > 0 && can_v4 && mode != MODE_UPDATE_ONLY && (f > 64 || p->n_rows <= 65536) &&
                 (p->slab_width == 0 || p->slab_width >= 128);
     if (c.chunked) {
@@ -1875,9 +1874,10 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
         c.sh.nv = 1;
         c.sh.slab_w = 128;
         c.sh.n_slabs = (f + c.sh.slab_w - 1) / c.sh.slab_w;
-        c.run = 4;
-        c.n_run = p->n_chunks * 3 / 4 / c.run * c.run;  // the last quarter one by one, to finish together
-        c.claims_per_slab = c.n_run / c.run + (p->n_chunks - c.n_run);
+        // One chunk to a claim.  Four of them, up to the last quarter, kept waiting rows from being handed out and small
+        // products from using all blocks: 17 000 rows, three quarters of them waiting, 256 columns 70 us against 47 (54
+        // by the items kernel in breadth-first order), 30 000 with few waiting 54 against 41, the same from 60 000 on.
+        c.claims_per_slab = p->n_chunks;
     } else if (tma) {
         const i32 slab = 256;  // 1 KB row pieces: the copy engine is bound by copies, not bytes
         c.sh.v4 = true;
@@ -2016,8 +2016,6 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.desc = p->d_desc;
     kp.ent = p->d_ent;
     kp.chunks = p->d_chunks;
-    kp.run = c.run;
-    kp.n_run = c.n_run;
     kp.ldx_bytes = (unsigned)(4 * ldx);
     kp.x = x;
     kp.y = y;
