@@ -26,6 +26,7 @@
 #include <memory>
 #include <mutex>
 #include <new>
+#include <stdexcept>
 #include <string>
 #include <utility>
 #include <vector>
@@ -1612,6 +1613,20 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
 
 }  // namespace
 
+namespace {
+// Runs what may allocate host memory: no exception leaves the library.
+template <class F>
+int guarded(const char* who, F run) {
+    try {
+        return run();
+    } catch (const std::bad_alloc&) {
+        return cbm::fail(CBM_B200_ERR_ALLOC, std::string(who) + ": out of host memory");
+    } catch (const std::length_error&) {
+        return cbm::fail(CBM_B200_ERR_ALLOC, std::string(who) + ": out of host memory");
+    }
+}
+}  // namespace
+
 extern "C" int cbm_b200_schedule_info(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
                                       const int32_t* delta_crow, const int32_t* delta_col,
                                       const float* delta_val, const float* multiplier,
@@ -1619,8 +1634,9 @@ extern "C" int cbm_b200_schedule_info(int32_t n, const int32_t* mst_row, const i
                                       int32_t own_end, int32_t* n_items, int32_t* n_prefix,
                                       int32_t* n_partial, int32_t* n_rows) {
     Schedule sch;
-    const int rc = build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm,
-                                  n_labels, own_begin, own_end, sch);
+    const int rc = guarded("schedule_info", [&] {
+        return build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm, n_labels, own_begin, own_end, sch);
+    });
     if (rc) return rc;
     if (n_items) *n_items = (i32)sch.desc.size();
     if (n_prefix) *n_prefix = sch.n_prefix;
@@ -1652,8 +1668,10 @@ extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, c
     for (i32 v = 0; labels && v < n; ++v)
         if (labels[v] < 0 || labels[v] >= n) return cbm::fail(CBM_B200_ERR_ARG, "schedule_as_planned: label out of range");
     Schedule sch;
-    const int rc = build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, sch, 0,
-                                  Rules{true, -1, labels});
+    const int rc = guarded("schedule_as_planned", [&] {
+        return build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, sch, 0,
+                              Rules{true, -1, labels});
+    });
     if (rc) return rc;
     if (n_items) *n_items = (i32)sch.desc.size();
     if (n_prefix) *n_prefix = sch.n_prefix;
@@ -1677,8 +1695,10 @@ extern "C" int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int
     if (!out) return cbm::fail(CBM_B200_ERR_ARG, "plan_create: out is NULL");
     *out = nullptr;
     Schedule sch;
-    const int rc0 = build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm,
-                                   n_labels, own_begin, own_end, sch, 0, Rules{true, device, nullptr});
+    const int rc0 = guarded("plan_create", [&] {
+        return build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm, n_labels, own_begin, own_end,
+                              sch, 0, Rules{true, device, nullptr});
+    });
     if (rc0) return rc0;
     return plan_from_schedule(sch, n, own_end - own_begin, multiplier != nullptr, device, out);
 }
@@ -1690,8 +1710,10 @@ extern "C" int cbm_b200_csr_plan_create(int32_t n_rows, int32_t n_cols, const in
     *out = nullptr;
     if (n_cols <= 0) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: n_cols must be positive");
     Schedule sch;
-    const int rc0 = build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols,
-                                   Rules{true, device, nullptr});
+    const int rc0 = guarded("csr_plan_create", [&] {
+        return build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols,
+                              Rules{true, device, nullptr});
+    });
     if (rc0) return rc0;
     return plan_from_schedule(sch, n_rows, n_rows, false, device, out);
 }
@@ -1784,9 +1806,10 @@ extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, 
     if (segment) *segment = p->segment;
     if (fingerprint) {
         DeviceGuard g(p->device);
-        std::vector<RowDesc> desc((size_t)p->n_items);
-        if (p->n_items) CBM_CUDA(cudaMemcpy(desc.data(), p->d_desc, desc.size() * sizeof(RowDesc), cudaMemcpyDeviceToHost));
-        *fingerprint = fingerprint_of(desc.data(), desc.size());
+        std::unique_ptr<RowDesc[]> desc(new (std::nothrow) RowDesc[(size_t)p->n_items]);
+        if (!desc) return cbm::fail(CBM_B200_ERR_ALLOC, "plan_schedule: out of host memory");
+        if (p->n_items) CBM_CUDA(cudaMemcpy(desc.get(), p->d_desc, (size_t)p->n_items * sizeof(RowDesc), cudaMemcpyDeviceToHost));
+        *fingerprint = fingerprint_of(desc.get(), (size_t)p->n_items);
     }
     return CBM_B200_OK;
 }

@@ -137,3 +137,31 @@ def test_labels_out_of_range_are_refused():
     c = _cbm(graphs.erdos_renyi(25, 0.5, 1), 2)
     for label in (-1, c.num_rows):
         assert _as_planned(c, np.full(c.num_rows, label))[0] == 1
+
+
+@pytest.mark.parametrize("room", [2, 6, 12, 30, 60])
+@pytest.mark.parametrize("entry", ["schedule_info", "schedule_as_planned"])
+def test_memory_that_runs_out_is_an_error_not_an_abort(entry, room):
+    """A schedule of 8 000 000 rows takes over 100 bytes a row; with less (``room`` bytes) the call returns."""
+    import os
+    import subprocess
+    import sys
+    code = f"""
+import ctypes, resource
+import numpy as np
+L = ctypes.CDLL({_lib.LIB_PATH!r})
+L.cbm_b200_last_error.restype = ctypes.c_char_p
+n = 8_000_000
+col, val, crow = np.arange(n, dtype=np.int32), np.ones(n, np.float32), np.arange(n + 1, dtype=np.int32)
+row = np.zeros(n + 2, np.int32)
+row[n + 1] = n  # every row a child of the virtual root
+p = lambda a: ctypes.c_void_p(a.ctypes.data)
+rest = [None, 0, 0, n, None, None, None, None] if {entry!r} == "schedule_info" else [None] * 7
+used = int(next(s for s in open("/proc/self/status") if s.startswith("VmSize")).split()[1]) * 1024
+resource.setrlimit(resource.RLIMIT_AS, (used + {room} * n, resource.getrlimit(resource.RLIMIT_AS)[1]))
+print(L.cbm_b200_{entry}(n, p(row), p(col), p(crow), p(col), p(val), None, *rest), L.cbm_b200_last_error().decode())
+"""
+    _lib.lib()  # (built)
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                          env=dict(os.environ, OMP_NUM_THREADS="2"))
+    assert done.returncode == 0 and "memory" in done.stdout, (done.returncode, done.stdout, done.stderr[-300:])
