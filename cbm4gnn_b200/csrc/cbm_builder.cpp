@@ -853,6 +853,7 @@ extern "C" int cbm_b200_edge_degrees(const int32_t* row, const int32_t* col, int
             negative = negative || row[i] < 0;
         }
         if (negative) return cbm::fail(CBM_B200_ERR_ARG, "edge_degrees: negative row index");
+        if (most >= INT32_MAX - 2) return cbm::fail(CBM_B200_ERR_ARG, "edge_degrees: index too large for int32 sizes");
         *n = most + 1;
         return CBM_B200_OK;
     }

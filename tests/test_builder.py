@@ -331,3 +331,10 @@ print(run(), L.cbm_b200_last_error().decode())
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                           env=dict(os.environ, OMP_NUM_THREADS="4"))
     assert done.returncode == 0 and "memory" in done.stdout, (done.returncode, done.stdout, done.stderr[-300:])
+
+
+@pytest.mark.parametrize("normalized", [False, True])
+@pytest.mark.parametrize("edge,message", [([-1, 0], "negative row"), ([0, -1], "out of range"), ([2**31 - 1, 0], "too large")])
+def test_indices_out_of_range_are_refused(edge, message, normalized):
+    with pytest.raises(RuntimeError, match=message):
+        cbm_matrix(torch.tensor([[0, 1, edge[0]], [0, 1, edge[1]]]), torch.ones(3), normalized=normalized)
