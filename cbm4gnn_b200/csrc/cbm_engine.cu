@@ -1204,9 +1204,10 @@ void pool_leave(int device) {
 template <class T>
 int grow(cbm_b200_plan* p, T*& at, i64& cap, i64 need, bool zeroed, cudaStream_t s) {
     if (need <= cap) return CBM_B200_OK;
-    // a launch in flight may still read the old one, on whatever stream
-    CBM_CUDA(at ? cudaDeviceSynchronize() : cudaStreamSynchronize(s));
-    if (at) CBM_CUDA(cudaFreeAsync(at, s));
+    if (at) {  // a launch in flight may still read the old one, on whatever stream
+        CBM_CUDA(cudaDeviceSynchronize());
+        CBM_CUDA(cudaFreeAsync(at, s));
+    }
     p->device_bytes -= cap * (i64)sizeof(T);
     at = nullptr;
     cap = 0;
