@@ -2347,7 +2347,9 @@ extern "C" int cbm_b200_spmm_update_host(cbm_b200_plan* p, const float* x, float
                                        (size_t)p->n_labels, cudaMemcpyHostToDevice, p->copy_in));
         CBM_CUDA(cudaEventRecord(p->events[2 * k], p->copy_in));
         CBM_CUDA(cudaStreamWaitEvent(s, p->events[2 * k], 0));
-        // the short tail is summed as the device-operand product of this width sums its last columns
+        // The short tail is summed entry by entry, as a device operand of this width with unaligned rows is where it is not
+        // copied to aligned ones.  Where it is, or where the last slab is at most 64 columns wide, some of its
+        // columns are summed in another order there: host and device operands agree to fp32 rounding, not to the bit.
         int rc = run_plan(p, "spmm_update_host", p->stage_x + c0, ld, p->stage_y + c0, ld, w, MODE_FUSED,
                           normalized != 0, s, nullptr, w % 4 != 0 && c0 > 0);
         if (rc) return rc;
@@ -2471,11 +2473,11 @@ extern "C" double cbm_b200_probe_l2_read_gbps(int32_t device) {
 // ------------------------------------------------------------------------------------------
 // Product without any allocation in the call path.
 //
-// The ordinary product entry points grow the plan's ready-flag and partial-sum buffers with
-// cudaMalloc the first time a wider operand arrives.  Some callers must never reach an allocator
+// The ordinary product entry points grow the plan's ready-flag and partial-sum buffers, and the room for a packed
+// operand, from the device's workspace pool the first time a wider operand arrives.  Some callers must never reach an allocator
 // once they are running: a serving loop that has handed all device memory to its own pool, code
 // that runs while a stream is being captured, a real-time path that cannot absorb the implicit
-// device synchronisation of cudaMalloc/cudaFree.  For them the same kernel is offered with its
+// device synchronisation of an allocation.  For them the same kernel is offered with its
 // per-call scratch (claim counters, ready flags, partial sums of long rows) carved out of one
 // fixed array that lives in the library image: every GPU that loads the library holds
 // CBM_B200_STATIC_SCRATCH_BYTES of it until the process exits.

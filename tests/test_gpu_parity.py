@@ -326,8 +326,9 @@ def test_bulk_copy_form_matches_register_form(c1):
 
 
 def test_host_operands_pinned_and_pageable_agree(c1):
-    """Page-locked host operands travel through copy kernels, pageable ones through the runtime's
-    copies; both must give the device-resident result exactly."""
+    """Page-locked host operands travel in column chunks, pageable ones whole, through page-locked
+    slots: both run the same chunks' products.  At these sizes the device-resident operand's columns
+    are summed in the same order as well, so all three give the same bits."""
     ei, c = c1
     n = c.num_rows
     for f in (500, 130, 64):
