@@ -9,6 +9,7 @@ import functools
 from array import array
 
 import torch
+from torch.autograd import forward_ad
 
 from . import _lib
 from .cbm import _product, _raw_stream, result_pitch
@@ -234,11 +235,12 @@ def _listable(x, steps, shapes, weights):
 
 
 def run_stack(x, steps, weights):
-    """The result of the stack for CUDA fp32 ``x`` and ``weights``, differentiable in both.  The functions are never
-    gone round, also where no backward pass can follow: forward-mode differentiation has to meet (and be refused by)
-    them."""
+    """The result of the stack for CUDA fp32 ``x`` and ``weights``, differentiable in both.  Its function is gone round
+    only where neither a backward pass can follow nor forward-mode differentiation is going on, which has to meet (and
+    be refused by) it: applying a function to three layers takes the host 10 us of 55."""
     shapes = tuple(tuple(w.shape) for w in weights)
-    if _listable(x, steps, shapes, weights):
-        return _ListedStack.apply(x, steps, shapes, *weights)
     keep = torch.is_grad_enabled() and (x.requires_grad or any(w.requires_grad for w in weights))
-    return _Stack.apply(x, steps, keep, *weights)
+    listed = _listable(x, steps, shapes, weights)
+    if keep or forward_ad._current_level >= 0:
+        return _ListedStack.apply(x, steps, shapes, *weights) if listed else _Stack.apply(x, steps, keep, *weights)
+    return _listed_forward(x, steps, shapes, weights)[0] if listed else _stack_forward(x, steps, weights)

@@ -152,8 +152,14 @@ def test_forward_mode_is_refused(listed_bytes, monkeypatch):
     model = GCNModel([20, 9, 6, 3], alpha=2).cuda().requires_grad_(False)
     x = torch.randn(50, 20, device="cuda")
     want = model(x, edges)
-    with forward_ad.dual_level(), pytest.raises(RuntimeError, match="jvp"):
-        model(forward_ad.make_dual(x, torch.ones_like(x)), edges)
+    with forward_ad.dual_level():
+        with pytest.raises(RuntimeError, match="jvp"):
+            model(forward_ad.make_dual(x, torch.ones_like(x)), edges)
+        with torch.no_grad(), pytest.raises(RuntimeError, match="jvp"):
+            model(forward_ad.make_dual(x, torch.ones_like(x)), edges)
+    for call in (lambda: torch.func.jvp(lambda t: model(t, edges), (x,), (x,)), lambda: torch.func.vmap(lambda t: model(t, edges))(x[None])):
+        with pytest.raises(RuntimeError):
+            call()
     with torch.no_grad():
         assert torch.equal(model(x, edges), want) and not want.requires_grad
 
