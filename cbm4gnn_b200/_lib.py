@@ -26,6 +26,7 @@ SOURCES = [
     os.path.join(_PKG_DIR, "csrc", "cbm_map_grad.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.cu"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.cu"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_lift.cpp"),
     os.path.join(_PKG_DIR, "csrc", "cbm_sequence.cpp"),
 ]
 HEADERS = [
@@ -34,6 +35,7 @@ HEADERS = [
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_chunks.cuh"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.h"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_lift.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_map.cuh"),
 ]
 _OBJ_DIR = os.path.join(_PKG_DIR, "build")
@@ -55,6 +57,7 @@ EXPORTED = [
     "cbm_b200_plan_destroy",
     "cbm_b200_schedule_info",
     "cbm_b200_schedule_as_planned",
+    "cbm_b200_schedule_lifted",
     "cbm_b200_plan_schedule",
     "cbm_b200_plan_info",
     "cbm_b200_plan_tune",
@@ -181,6 +184,7 @@ def lib() -> ctypes.CDLL:
         c_void_p, c_void_p, c_int32, c_int32, c_int32, i32p, i32p, i32p, i32p)
     sig("cbm_b200_schedule_as_planned", c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
         c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
+    sig("cbm_b200_schedule_lifted", c_int32, c_int32, *[c_void_p] * 7, i32p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p)
     sig("cbm_b200_plan_schedule", c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
     sig("cbm_b200_plan_info", c_int32, c_void_p, i32p, POINTER(c_int64), i32p, i32p,
         POINTER(c_int64))

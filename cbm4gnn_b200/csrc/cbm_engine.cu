@@ -23,17 +23,21 @@
 #include <algorithm>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <new>
 #include <stdexcept>
 #include <string>
+#include <system_error>
+#include <thread>
 #include <utility>
 #include <vector>
 
 #include "cbm_b200.h"
 #include "cbm_cluster.h"
 #include "cbm_common.h"
+#include "cbm_lift.h"
 
 namespace cbm {
 std::string& last_error_slot() {
@@ -1087,28 +1091,37 @@ Shape pick_shape(i32 f, i32 want_slab, bool can_v4) {
 }  // namespace
 
 // ------------------------------------------------------------------------------------------
+// A schedule on the device.
+struct DeviceSchedule {
+    i32 n_items = 0;   // work items per slab (rows + extra segments of long rows); 0: there is none
+    i32 n_prefix = 0;  // items that never wait
+    i32 n_partial = 0; // PARTIAL items = scratch slots per slab
+    i32 segment = 0;   // entries of a PARTIAL item
+    i32 n_chunks = 0;  // 0: not clustered
+    i64 n_entries = 0;
+    std::vector<i32> part_ends;  // see Schedule
+    i32 n_partial_coarse = 0;
+    RowDesc* d_desc = nullptr;
+    Entry* d_ent = nullptr;
+    Chunk* d_chunks = nullptr;
+};
+
 struct cbm_b200_plan {
     int device = 0;
     i32 n = 0;
     i32 n_labels = 0;  // rows of the dense right-hand side
     i32 n_out = 0;     // rows of the output shard (owned label range)
     i32 n_rows = 0;    // rows actually computed
-    i32 n_items = 0;   // work items per slab (rows + extra segments of long rows)
-    i32 n_prefix = 0;  // items that never wait
-    i32 n_partial = 0; // PARTIAL items = scratch slots per slab
-    i32 segment = 0;   // delta entries of a PARTIAL item
-    std::vector<i32> part_ends;  // see Schedule
-    i32 n_partial_coarse = 0;
+    // The structure's own schedule, and the one with rows lifted out of the tree (cbm_lift.cpp), which the product in
+    // one pass goes by where there is one.  The halves of the product (delta product, update) need the tree itself.
+    DeviceSchedule tree, lifted;
+    const DeviceSchedule& schedule_for(i32 mode) const { return mode == MODE_FUSED && lifted.n_items > 0 ? lifted : tree; }
     float* d_scratch = nullptr;
     i64 scratch_cap = 0;
     i64 n_delta = 0;
     i32 n_root_children = 0;
     i32 depth = 0;
     bool normalized = false;
-    RowDesc* d_desc = nullptr;
-    Entry* d_ent = nullptr;
-    Chunk* d_chunks = nullptr;
-    i32 n_chunks = 0;            // 0: not clustered
     float* d_pack = nullptr;     // the operand copied to 16-byte aligned rows (when the caller's are not)
     i64 pack_cap = 0;
     i32* d_flags = nullptr;
@@ -1233,9 +1246,11 @@ extern "C" void cbm_b200_plan_destroy(cbm_b200_plan* p) {
         cudaStreamSynchronize(p->own_stream);
         pool_leave(p->device);
     }
-    cudaFree(p->d_desc);
-    cudaFree(p->d_ent);
-    cudaFree(p->d_chunks);
+    for (const DeviceSchedule* d : {&p->tree, &p->lifted}) {
+        cudaFree(d->d_desc);
+        cudaFree(d->d_ent);
+        cudaFree(d->d_chunks);
+    }
     cudaFree(p->d_counter);
     cudaFree(p->d_status);
     cudaFreeHost(p->bounce);
@@ -1340,6 +1355,17 @@ void make_chunks(Schedule& sch, i32 n_prefix) {
     if (c.count > 0) sch.chunks.push_back(c);
 }
 
+// What a plan is made from, checked: the arrays as the caller has them, and the tree they describe.
+struct Structure {
+    i32 n = 0, n_labels = 0, own_begin = 0, own_end = 0;
+    bool csr = false, square = false;
+    const i32 *crow = nullptr, *col = nullptr, *perm = nullptr;
+    const float *val = nullptr, *multiplier = nullptr;
+    std::vector<i32> parent, level;  // of every row; parent n: the virtual root
+    std::vector<i32> rows;           // those the plan computes, breadth-first
+    i32 label(i32 v) const { return perm ? perm[v] : v; }
+};
+
 // How a schedule is cut and ordered.  As a plan on a GPU is: long rows cut finer where the mean row is short, communities
 // looked for on `device` or, for a check without a GPU, given as `labels` (row v belongs to community labels[v]).
 struct Rules {
@@ -1354,15 +1380,16 @@ struct Rules {
 // the sorted rows still name mostly different columns.  On B200, width 128: rows of 22 entries in
 // communities of 55 (ratio 0.4) gain 40 %, rows of 11 in communities of 118 (0.5) gain 15 %; copy-model graphs
 // (0.75 - 0.95), whose common columns are few hubs, gain nothing.
-bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std::vector<i32>& parent, const Rules& rules,
-                   std::vector<i32>& rank) {
+bool cluster_order(const Structure& st, const Rules& rules, std::vector<i32>& rank) {
+    const i32 n = st.n;
+    const i32 *crow = st.crow, *col = st.col;
     std::vector<i32> label;
     if (rules.labels) {
         label.assign(rules.labels, rules.labels + n);
     } else {
         if (rules.device < 0 || n < 16384 || crow[n] < 4 * (i64)n || crow[n] > INT32_MAX - n - 1024) return false;
         label.resize((size_t)n);
-        if (!cbm::cluster_rows(n, crow, col, parent.data(), rules.device, label.data())) return false;
+        if (!cbm::cluster_rows(n, crow, col, st.parent.data(), rules.device, label.data())) return false;
     }
     // counting sort by label, stable in v
     std::vector<i32> start((size_t)n + 1, 0), sorted((size_t)n);
@@ -1389,12 +1416,11 @@ bool cluster_order(int32_t n, const int32_t* crow, const int32_t* col, const std
     return true;
 }
 
-// csr_cols > 0 schedules a plain CSR matrix with that many columns (no tree: every row hangs off
-// the virtual root, mst_row / mst_col / perm are not read); csr_cols == 0 schedules a CBM structure.
-int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,
+// csr_cols > 0: a plain CSR matrix with that many columns (no tree: every row hangs off
+// the virtual root, mst_row / mst_col / perm are not read); csr_cols == 0: a CBM structure.
+int read_structure(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,
                    const int32_t* delta_col, const float* delta_val, const float* multiplier,
-                   const int32_t* perm, int32_t n_labels, int32_t own_begin, int32_t own_end, Schedule& sch,
-                   int32_t csr_cols = 0, const Rules& rules = Rules()) {
+                   const int32_t* perm, int32_t n_labels, int32_t own_begin, int32_t own_end, int32_t csr_cols, Structure& st) {
     std::vector<i32> flat_row, flat_col;
     if (csr_cols > 0) {
         if (n < 0 || !delta_crow) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: NULL row pointers");
@@ -1424,7 +1450,8 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
     // ---- validate the tree: every row exactly once, reachable from the virtual root ----
     if (mst_row[0] != 0 || mst_row[n + 1] != n)
         return cbm::fail(CBM_B200_ERR_FORMAT, "plan_create: mst_row must run from 0 to n");
-    std::vector<i32> parent((size_t)n, -1);
+    std::vector<i32>& parent = st.parent;
+    parent.assign((size_t)n, -1);
     for (i32 u = 0; u <= n; ++u) {
         if (mst_row[u] > mst_row[u + 1])
             return cbm::fail(CBM_B200_ERR_FORMAT, "plan_create: mst_row not monotone");
@@ -1438,7 +1465,8 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
     }
     std::vector<i32> order;  // breadth-first from the virtual root
     order.reserve((size_t)n);
-    std::vector<i32> level((size_t)n + 1, 0);
+    std::vector<i32>& level = st.level;
+    level.assign((size_t)n + 1, 0);
     {
         std::vector<i32> q;
         q.reserve((size_t)n + 1);
@@ -1474,20 +1502,7 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
         const i32 l = label(v);
         return l >= own_begin && l < own_end;
     };
-
-    // ---- schedule (layout described at RowDesc) ----
-    // Delta entries per item of a split row, and the length from which rows are split.  Rows of a plan are cut finer where
-    // the mean row is short: a long row is then what a product ends on (100 000 rows of 31 entries, 500 columns: 397 us with
-    // segments of 128, 390 with 64, 429 with 32; 50 000 rows, 64 columns: 56, 48, 50); where long rows are the rule, finer
-    // segments only add parked sums (40 000 rows of 152 entries: 194 us, 201, 234).
-    i32 longest = 0;
-    for (i32 v = 0; v < n; ++v) longest = std::max(longest, delta_crow[v + 1] - delta_crow[v]);
-    const bool fine = rules.as_plan && nd_all <= 64 * (i64)n && longest <= 64 * 0xffff;
-    const i32 SEG = fine ? 64 : 128, SPLIT_OVER = fine ? 96 : 192;
-    auto row_len = [&](i32 v) { return delta_crow[v + 1] - delta_crow[v]; };
-    auto is_split = [&](i32 v) { return row_len(v) > SPLIT_OVER; };
-    std::vector<i32> owned_rows;  // breadth-first
-    owned_rows.reserve((size_t)(own_end - own_begin));
+    st.rows.reserve((size_t)std::min<i64>(n, own_end - own_begin));
     for (i32 v : order)
         if (owned(v)) {
             const i32 u = parent[v];
@@ -1495,18 +1510,51 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
                 return cbm::fail(CBM_B200_ERR_ARG,
                                  "plan_create: owned range cuts a subtree (parent of an owned row "
                                  "is not owned)");
-            owned_rows.push_back(v);
+            st.rows.push_back(v);
         }
+    st.n = n;
+    st.n_labels = csr_cols > 0 ? csr_cols : n_labels;
+    st.own_begin = own_begin;
+    st.own_end = own_end;
+    st.square = col_bound == n;
+    st.csr = csr_cols > 0;
+    st.crow = delta_crow;
+    st.col = delta_col;
+    st.val = delta_val;
+    st.multiplier = multiplier;
+    st.perm = perm;
+    return CBM_B200_OK;
+}
+
+// The schedule (layout described at RowDesc) of the structure's rows, or with `lift` of the tree with some of them
+// lifted; `rank`: their order by community, empty where the graph has none.
+int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vector<i32>& rank, const Rules& rules, Schedule& sch) {
+    const i32 n = st.n, own_begin = st.own_begin, own_end = st.own_end;
+    const std::vector<i32>&parent = lift ? lift->parent : st.parent, &level = lift ? lift->level : st.level;
+    const std::vector<i32>& owned_rows = st.rows;
+    const float* multiplier = st.multiplier;
+    auto label = [&](i32 v) { return st.label(v); };
+    auto row_len = [&](i32 v) { return lift ? lift->len[v] : st.crow[v + 1] - st.crow[v]; };
+    const i64 nd_all = lift ? lift->n_entries : st.crow[n], nd_rows = lift ? (i64)owned_rows.size() : n;
+    // Delta entries per item of a split row, and the length from which rows are split.  Rows of a plan are cut finer where
+    // the mean row is short: a long row is then what a product ends on (100 000 rows of 31 entries, 500 columns: 397 us with
+    // segments of 128, 390 with 64, 429 with 32; 50 000 rows, 64 columns: 56, 48, 50); where long rows are the rule, finer
+    // segments only add parked sums (40 000 rows of 152 entries: 194 us, 201, 234).
+    i32 longest = 0;
+    for (i32 v = 0; v < n; ++v) longest = std::max(longest, row_len(v));
+    const bool fine = rules.as_plan && nd_all <= 64 * nd_rows && longest <= 64 * 0xffff;
+    const i32 SEG = fine ? 64 : 128, SPLIT_OVER = fine ? 96 : 192;
+    auto is_split = [&](i32 v) { return row_len(v) > SPLIT_OVER; };
     std::vector<RowDesc>& desc = sch.desc;
-    std::vector<i32> rank;
-    sch.clustered = col_bound == n && cluster_order(n, delta_crow, delta_col, parent, rules, rank);
+    sch.clustered = !rank.empty();
     sch.segment = SEG;
     // items get their entry ranges now; the entries are filled in at the end, on several threads
-    std::vector<i64> source;  // per item: its first entry in the delta arrays
+    std::vector<i64> source;  // per item: its first entry in the delta arrays, or ~ its first in those of the lifted rows
     source.reserve((size_t)n);
     auto append_entries = [&](i32 v, i32 from, i32 to) {  // entries [from, to) of row v
         const i32 beg = (i32)sch.n_ent;
-        source.push_back((i64)delta_crow[v] + from);
+        const i64 at = (lift ? lift->at[v] : st.crow[v]) + from;
+        source.push_back(lift && lift->lifted[v] ? ~at : at);
         sch.n_ent += to - from;
         if (sch.clustered) sch.n_ent += sch.n_ent % 2;
         return beg;
@@ -1589,6 +1637,8 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
         std::sort(rest.begin(), rest.end(), [&](i32 a, i32 b) {
             return level[a] != level[b] ? level[a] < level[b] : rank[a] < rank[b];
         });
+    else if (lift)  // (lifting has changed levels)
+        std::stable_sort(rest.begin(), rest.end(), [&](i32 a, i32 b) { return level[a] < level[b]; });
     for (i32 v : rest) add_row_item(v);
     sch.ent.reset(new Entry[(size_t)std::max<i64>(sch.n_ent, 1)]);
     const i32 n_items = (i32)desc.size();
@@ -1598,7 +1648,10 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
     for (i32 i = 0; i < n_items; ++i) {
         const i32 len = (desc[i].info >> ITEM_LEN_SHIFT) & 0xff;
         Entry* e = sch.ent.get() + desc[i].beg;
-        for (i32 k = 0; k < len; ++k) e[k] = Entry{label(delta_col[source[i] + k]), delta_val[source[i] + k]};
+        const bool own = source[i] >= 0;
+        const i32* col = own ? st.col + source[i] : lift->col.data() + ~source[i];
+        const float* val = own ? st.val + source[i] : lift->val.data() + ~source[i];
+        for (i32 k = 0; k < len; ++k) e[k] = Entry{label(col[k]), val[k]};
         if (sch.clustered && len % 2) e[len] = Entry{0, 0.0f};
     }
     if (sch.clustered) make_chunks(sch, n_prefix);
@@ -1607,10 +1660,50 @@ int build_schedule(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
     sch.n_partial = n_partial;
     sch.depth = depth;
     sch.n_root_children = n_root_children;
-    sch.n_labels = csr_cols > 0 ? csr_cols : n_labels;
+    sch.n_labels = st.n_labels;
     return validate_schedule(sch, own_end - own_begin);
 }
 
+// The structure's own schedule, and the one with rows lifted out of the tree where that pays.
+int build_schedules(const Structure& st, const Rules& rules, Schedule& tree, Schedule& lifted) {
+    cbm::Lifted lift;
+    std::vector<i32> rank;
+    if (!st.csr) cbm::lift_rows(st.n, st.rows, st.parent, st.level, st.crow, st.col, st.val, lift);
+    cluster_order(st, rules, rank);
+    if (lift.n_lifted == 0) return build_schedule(st, nullptr, rank, rules, tree);
+    // side by side where they take milliseconds
+    int rc = CBM_B200_OK;
+    std::string what;
+    std::exception_ptr thrown;
+    auto other = [&] {
+        try {
+            rc = build_schedule(st, &lift, rank, rules, lifted);
+            if (rc) what = cbm::last_error_slot();
+        } catch (...) {
+            thrown = std::current_exception();
+        }
+    };
+    std::thread beside;
+    if (lift.n_entries > 1000000) {
+        try {
+            beside = std::thread(other);
+        } catch (const std::system_error&) {  // no thread to be had
+        }
+    }
+    int own = CBM_B200_OK;
+    std::exception_ptr own_thrown;
+    try {
+        own = build_schedule(st, nullptr, rank, rules, tree);
+    } catch (...) {
+        own_thrown = std::current_exception();
+    }
+    if (beside.joinable()) beside.join();
+    else if (own == CBM_B200_OK && !own_thrown) other();
+    if (own_thrown) std::rethrow_exception(own_thrown);
+    if (own) return own;
+    if (thrown) std::rethrow_exception(thrown);
+    return rc ? cbm::fail(rc, what) : CBM_B200_OK;
+}
 
 }  // namespace
 
@@ -1636,7 +1729,10 @@ extern "C" int cbm_b200_schedule_info(int32_t n, const int32_t* mst_row, const i
                                       int32_t* n_partial, int32_t* n_rows) {
     Schedule sch;
     const int rc = guarded("schedule_info", [&] {
-        return build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm, n_labels, own_begin, own_end, sch);
+        Structure st;
+        const int bad = read_structure(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm, n_labels, own_begin,
+                                       own_end, 0, st);
+        return bad ? bad : build_schedule(st, nullptr, {}, Rules(), sch);
     });
     if (rc) return rc;
     if (n_items) *n_items = (i32)sch.desc.size();
@@ -1670,8 +1766,13 @@ extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, c
         if (labels[v] < 0 || labels[v] >= n) return cbm::fail(CBM_B200_ERR_ARG, "schedule_as_planned: label out of range");
     Schedule sch;
     const int rc = guarded("schedule_as_planned", [&] {
-        return build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, sch, 0,
-                              Rules{true, -1, labels});
+        Structure st;
+        const int bad = read_structure(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, 0, st);
+        if (bad) return bad;
+        const Rules rules{true, -1, labels};
+        std::vector<i32> rank;
+        cluster_order(st, rules, rank);
+        return build_schedule(st, nullptr, rank, rules, sch);
     });
     if (rc) return rc;
     if (n_items) *n_items = (i32)sch.desc.size();
@@ -1683,9 +1784,50 @@ extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, c
     return CBM_B200_OK;
 }
 
+extern "C" int cbm_b200_schedule_lifted(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,
+                                        const int32_t* delta_col, const float* delta_val, const float* multiplier,
+                                        const int32_t* labels, int32_t* n_lifted, int32_t* parent, int64_t* crow,
+                                        int64_t capacity, int32_t* col, float* val) {
+    for (i32 v = 0; labels && v < n; ++v)
+        if (labels[v] < 0 || labels[v] >= n) return cbm::fail(CBM_B200_ERR_ARG, "schedule_lifted: label out of range");
+    if (capacity > 0 && (!crow || !col || !val)) return cbm::fail(CBM_B200_ERR_ARG, "schedule_lifted: NULL array");
+    return guarded("schedule_lifted", [&] {
+        Structure st;
+        Schedule tree, lifted;
+        int rc = read_structure(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, 0, st);
+        if (rc == CBM_B200_OK) rc = build_schedules(st, Rules{true, -1, labels}, tree, lifted);
+        if (rc) return rc;
+        // read back from the items, as a product walks over them
+        const Schedule& sch = lifted.desc.empty() ? tree : lifted;
+        std::vector<const RowDesc*> item((size_t)n, nullptr);
+        for (size_t i = (size_t)sch.n_partial; i < sch.desc.size(); ++i) item[sch.desc[i].out_row] = &sch.desc[i];
+        const auto len_of = [](const RowDesc& d) { return (d.info >> ITEM_LEN_SHIFT) & 0xff; };
+        i64 at = 0;
+        i32 differ = 0;
+        for (i32 v = 0; v < n; ++v) {
+            const RowDesc& d = *item[v];
+            const i32 parts = (i32)((unsigned)d.info >> ITEM_NPART_SHIFT);
+            if (parent) parent[v] = d.parent_row < 0 ? n : d.parent_row;
+            differ += (d.parent_row < 0 ? n : d.parent_row) != st.parent[v];
+            if (crow) crow[v] = at;
+            for (i32 k = 0; k <= parts; ++k) {
+                const RowDesc& q = k < parts ? sch.desc[d.first_part + k] : d;
+                for (i32 e = 0; e < len_of(q); ++e, ++at)
+                    if (at < capacity) {
+                        col[at] = sch.ent[(size_t)q.beg + e].col;
+                        val[at] = sch.ent[(size_t)q.beg + e].val;
+                    }
+            }
+        }
+        if (crow) crow[n] = at;
+        if (n_lifted) *n_lifted = differ;
+        return (int)CBM_B200_OK;
+    });
+}
+
 namespace {
-int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized, int32_t device,
-                       cbm_b200_plan** out);
+int plan_from_schedules(Schedule& tree, Schedule& lifted, int32_t n, int32_t n_out, bool normalized, int32_t device,
+                        cbm_b200_plan** out);
 }
 
 extern "C" int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
@@ -1695,13 +1837,15 @@ extern "C" int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int
                                     int32_t own_end, int32_t device, cbm_b200_plan** out) {
     if (!out) return cbm::fail(CBM_B200_ERR_ARG, "plan_create: out is NULL");
     *out = nullptr;
-    Schedule sch;
+    Schedule tree, lifted;
     const int rc0 = guarded("plan_create", [&] {
-        return build_schedule(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm, n_labels, own_begin, own_end,
-                              sch, 0, Rules{true, device, nullptr});
+        Structure st;
+        const int bad = read_structure(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, perm, n_labels, own_begin,
+                                       own_end, 0, st);
+        return bad ? bad : build_schedules(st, Rules{true, device, nullptr}, tree, lifted);
     });
     if (rc0) return rc0;
-    return plan_from_schedule(sch, n, own_end - own_begin, multiplier != nullptr, device, out);
+    return plan_from_schedules(tree, lifted, n, own_end - own_begin, multiplier != nullptr, device, out);
 }
 
 extern "C" int cbm_b200_csr_plan_create(int32_t n_rows, int32_t n_cols, const int32_t* crow,
@@ -1710,23 +1854,34 @@ extern "C" int cbm_b200_csr_plan_create(int32_t n_rows, int32_t n_cols, const in
     if (!out) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: out is NULL");
     *out = nullptr;
     if (n_cols <= 0) return cbm::fail(CBM_B200_ERR_ARG, "csr_plan_create: n_cols must be positive");
-    Schedule sch;
+    Schedule rows, none;
     const int rc0 = guarded("csr_plan_create", [&] {
-        return build_schedule(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, sch, n_cols,
-                              Rules{true, device, nullptr});
+        Structure st;
+        const int bad = read_structure(n_rows, nullptr, nullptr, crow, col, val, nullptr, nullptr, 0, 0, 0, n_cols, st);
+        return bad ? bad : build_schedules(st, Rules{true, device, nullptr}, rows, none);
     });
     if (rc0) return rc0;
-    return plan_from_schedule(sch, n_rows, n_rows, false, device, out);
+    return plan_from_schedules(rows, none, n_rows, n_rows, false, device, out);
 }
 
 namespace {
-int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized, int32_t device,
-                       cbm_b200_plan** out) {
-    const int32_t n_labels = sch.n_labels;
-    std::vector<RowDesc>& desc = sch.desc;
-    const i32 n_rows_owned = sch.n_rows_owned, n_prefix = sch.n_prefix, n_partial = sch.n_partial;
-    const i32 depth = sch.depth, n_root_children = sch.n_root_children;
+int upload_schedule(Schedule& sch, DeviceSchedule& d, i64& bytes) {
+    d.n_items = (i32)sch.desc.size();
+    d.n_prefix = sch.n_prefix;
+    d.n_partial = sch.n_partial;
+    d.segment = sch.segment;
+    d.part_ends.swap(sch.part_ends);
+    d.n_partial_coarse = sch.n_partial_coarse;
+    d.n_entries = sch.n_delta;
+    d.n_chunks = (i32)sch.chunks.size();
+    int rc = upload(&d.d_desc, sch.desc.data(), sch.desc.size(), bytes);
+    if (rc == CBM_B200_OK) rc = upload(&d.d_ent, sch.ent.get(), (size_t)sch.n_ent, bytes);
+    if (rc == CBM_B200_OK && sch.clustered) rc = upload(&d.d_chunks, sch.chunks.data(), sch.chunks.size(), bytes);
+    return rc;
+}
 
+int plan_from_schedules(Schedule& tree, Schedule& lifted, int32_t n, int32_t n_out, bool normalized, int32_t device,
+                        cbm_b200_plan** out) {
     int n_dev = 0;
     CBM_CUDA(cudaGetDeviceCount(&n_dev));
     if (device < 0 || device >= n_dev)
@@ -1738,25 +1893,17 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
     if (!p) return cbm::fail(CBM_B200_ERR_ALLOC, "plan_create: out of host memory");
     p->device = device;
     p->n = n;
-    p->n_labels = n_labels;
+    p->n_labels = tree.n_labels;
     p->n_out = n_out;
-    p->n_rows = n_rows_owned;
-    p->n_items = (i32)desc.size();
-    p->n_prefix = n_prefix;
-    p->n_partial = n_partial;
-    p->segment = sch.segment;
-    p->part_ends.swap(sch.part_ends);
-    p->n_partial_coarse = sch.n_partial_coarse;
-    p->n_delta = sch.n_delta;
-    p->n_chunks = (i32)sch.chunks.size();
-    p->n_root_children = n_root_children;
-    p->depth = depth;
+    p->n_rows = tree.n_rows_owned;
+    p->n_delta = tree.n_delta;
+    p->n_root_children = tree.n_root_children;
+    p->depth = tree.depth;
     p->normalized = normalized;
     int sms = 0;  // (the one attribute: all properties together take milliseconds)
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) p->sm_count = sms;
-    int rc = upload(&p->d_desc, desc.data(), desc.size(), p->device_bytes);
-    if (rc == CBM_B200_OK) rc = upload(&p->d_ent, sch.ent.get(), (size_t)sch.n_ent, p->device_bytes);
-    if (rc == CBM_B200_OK && sch.clustered) rc = upload(&p->d_chunks, sch.chunks.data(), sch.chunks.size(), p->device_bytes);
+    int rc = upload_schedule(tree, p->tree, p->device_bytes);
+    if (rc == CBM_B200_OK && !lifted.desc.empty()) rc = upload_schedule(lifted, p->lifted, p->device_bytes);
     if (rc == CBM_B200_OK) {
         cudaError_t e = cudaMalloc((void**)&p->d_counter, 2 * sizeof(u64));
         if (e == cudaSuccess) e = cudaMemset(p->d_counter, 0, 2 * sizeof(u64));
@@ -1772,8 +1919,8 @@ int plan_from_schedule(Schedule& sch, int32_t n, int32_t n_out, bool normalized,
         p->in_pool = rc == CBM_B200_OK;
     }
     // ready flags for operands of up to 512 columns and parked sums for one slab: most products then allocate nothing
-    if (rc == CBM_B200_OK) rc = grow(p, p->d_flags, p->flags_cap, 4 * (i64)p->n_items, true, p->own_stream);
-    if (rc == CBM_B200_OK) rc = grow(p, p->d_scratch, p->scratch_cap, (i64)p->n_partial * DEFAULT_SLAB, false, p->own_stream);
+    if (rc == CBM_B200_OK) rc = grow(p, p->d_flags, p->flags_cap, 4 * (i64)std::max(p->tree.n_items, p->lifted.n_items), true, p->own_stream);
+    if (rc == CBM_B200_OK) rc = grow(p, p->d_scratch, p->scratch_cap, (i64)std::max(p->tree.n_partial, p->lifted.n_partial) * DEFAULT_SLAB, false, p->own_stream);
     if (rc != CBM_B200_OK) {
         const std::string keep = cbm::last_error_slot();
         cbm_b200_plan_destroy(p);
@@ -1800,17 +1947,18 @@ extern "C" int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64
 extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
                                       int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
     if (!p) return cbm::fail(CBM_B200_ERR_ARG, "plan_schedule: NULL plan");
-    if (n_items) *n_items = p->n_items;
-    if (n_prefix) *n_prefix = p->n_prefix;
-    if (n_partial) *n_partial = p->n_partial;
-    if (n_chunks) *n_chunks = p->n_chunks;
-    if (segment) *segment = p->segment;
+    const DeviceSchedule& d = p->tree;
+    if (n_items) *n_items = d.n_items;
+    if (n_prefix) *n_prefix = d.n_prefix;
+    if (n_partial) *n_partial = d.n_partial;
+    if (n_chunks) *n_chunks = d.n_chunks;
+    if (segment) *segment = d.segment;
     if (fingerprint) {
         DeviceGuard g(p->device);
-        std::unique_ptr<RowDesc[]> desc(new (std::nothrow) RowDesc[(size_t)p->n_items]);
+        std::unique_ptr<RowDesc[]> desc(new (std::nothrow) RowDesc[(size_t)d.n_items]);
         if (!desc) return cbm::fail(CBM_B200_ERR_ALLOC, "plan_schedule: out of host memory");
-        if (p->n_items) CBM_CUDA(cudaMemcpy(desc.get(), p->d_desc, (size_t)p->n_items * sizeof(RowDesc), cudaMemcpyDeviceToHost));
-        *fingerprint = fingerprint_of(desc.get(), (size_t)p->n_items);
+        if (d.n_items) CBM_CUDA(cudaMemcpy(desc.get(), d.d_desc, (size_t)d.n_items * sizeof(RowDesc), cudaMemcpyDeviceToHost));
+        *fingerprint = fingerprint_of(desc.get(), (size_t)d.n_items);
     }
     return CBM_B200_OK;
 }
@@ -1870,7 +2018,7 @@ struct LaunchCfg {
     i32 left_out = 0;          // PARTIAL items, the last ones, that the finishing items do themselves
 };
 
-int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
+int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
              i32 f, int mode, bool may_pack, bool in_turn, LaunchCfg& c) {
     const bool y_vec = ldy % 4 == 0 && aligned16(y);
     const bool x_vec = ldx % 4 == 0 && aligned16(x) && ldx < (i64)1 << 30;
@@ -1878,20 +2026,20 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
     // the rate (4.4 TB/s).  Copying it to aligned rows first costs a launch and one pass over it, about 5 us on a small
     // operand, so it pays when every operand row is fetched several times and the 4-byte fetches would take
     // some 15 us (16 M multiply-adds).
-    c.pack = may_pack && mode != MODE_UPDATE_ONLY && !x_vec && f > 4 && p->n_delta >= 4 * (i64)p->n_labels &&
-             p->n_delta * f >= (i64)1 << 24;
+    c.pack = may_pack && mode != MODE_UPDATE_ONLY && !x_vec && f > 4 && d.n_entries >= 4 * (i64)p->n_labels &&
+             d.n_entries * f >= (i64)1 << 24;
     c.in_turn = in_turn;
     const bool can_v4 = !in_turn && (mode == MODE_UPDATE_ONLY ? y_vec : x_vec || c.pack);
     c.ragged = can_v4 && (!y_vec || f % 4 != 0);
     int tma = p->form;
-    if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY || p->n_chunks > 0) tma = 0;
+    if (!can_v4 || c.ragged || c.pack || mode == MODE_UPDATE_ONLY || d.n_chunks > 0) tma = 0;
     c.tma = tma;
     // Slabs of up to 64 columns gain nothing from the clustered order on large graphs (235 868 rows of 11 entries, 64
     // columns: 106 us against 97): several entries share a fetch there, and what a row costs is its instructions.
     // On smaller graphs the saved round trips per row still win, the more rows wait: 64 columns, few waiting rows, 17 000
     // rows 22 us against 32, 45 000 34 against 34, 60 000 41 against 39; three quarters waiting, 17 000 39 against 45,
     // 50 000 60 against 68.
-    c.chunked = p->n_chunks > 0 && can_v4 && mode != MODE_UPDATE_ONLY && (f > 64 || p->n_rows <= 65536) &&
+    c.chunked = d.n_chunks > 0 && can_v4 && mode != MODE_UPDATE_ONLY && (f > 64 || p->n_rows <= 65536) &&
                 (p->slab_width == 0 || p->slab_width >= 128);
     if (c.chunked) {
         c.sh.v4 = true;
@@ -1901,7 +2049,7 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
         // One chunk to a claim.  Four of them, up to the last quarter, kept waiting rows from being handed out and small
         // products from using all blocks: 17 000 rows, three quarters of them waiting, 256 columns 70 us against 47 (54
         // by the items kernel in breadth-first order), 30 000 with few waiting 54 against 41, the same from 60 000 on.
-        c.claims_per_slab = p->n_chunks;
+        c.claims_per_slab = d.n_chunks;
     } else if (tma) {
         const i32 slab = 256;  // 1 KB row pieces: the copy engine is bound by copies, not bytes
         c.sh.v4 = true;
@@ -1917,15 +2065,15 @@ int plan_cfg(const cbm_b200_plan* p, const char* who, const float* x, i64 ldx, c
         // 47 columns 275 -> 269 us; 50 000 rows in order of length 46 -> 65).
         // A small product keeps single claims: with fewer claims than resident warps, grouping
         // only idles warps.
-        c.group = ((i64)p->n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && p->n_chunks > 0 ? 8 : 4) : 1;
+        c.group = ((i64)d.n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && d.n_chunks > 0 ? 8 : 4) : 1;
     }
     if (!c.chunked) {
-        c.n_pclaims = (p->n_prefix + c.group - 1) / c.group;
-        c.claims_per_slab = c.n_pclaims + (p->n_items - p->n_prefix);
+        c.n_pclaims = (d.n_prefix + c.group - 1) / c.group;
+        c.claims_per_slab = c.n_pclaims + (d.n_items - d.n_prefix);
     }
     c.n_claims = (i64)c.claims_per_slab * c.sh.n_slabs;
-    c.need_flags = (i64)c.sh.n_slabs * p->n_items;
-    c.need_scratch = (i64)c.sh.n_slabs * p->n_partial * c.sh.slab_w;
+    c.need_flags = (i64)c.sh.n_slabs * d.n_items;
+    c.need_scratch = (i64)c.sh.n_slabs * d.n_partial * c.sh.slab_w;
     if (c.need_flags >= (i64)1 << 31)
         return cbm::fail(CBM_B200_ERR_ARG, std::string(who) + ": rows x column slabs exceeds 2^31 work items");
     return CBM_B200_OK;
@@ -2028,6 +2176,7 @@ int launch_frugal(KParams& kp, i32 out, i32 segment, int sm_count, cudaStream_t 
 int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
                 int mode, bool use_scale, u64* counter, i32* flags, float* scratch, i32 epoch,
                 cudaStream_t s, const Bcast* bc = nullptr) {
+    const DeviceSchedule& d = p->schedule_for(mode);
     KParams kp{};
     kp.y_vec = ldy % 4 == 0 && aligned16(y);
     kp.in_turn = c.in_turn;
@@ -2037,9 +2186,9 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
         kp.bcast_relu = bc->relu;
         for (int k = 0; k < bc->n; ++k) kp.bcast[k] = bc->dst[k];
     }
-    kp.desc = p->d_desc;
-    kp.ent = p->d_ent;
-    kp.chunks = p->d_chunks;
+    kp.desc = d.d_desc;
+    kp.ent = d.d_ent;
+    kp.chunks = d.d_chunks;
     kp.ldx_bytes = (unsigned)(4 * ldx);
     kp.x = x;
     kp.y = y;
@@ -2047,14 +2196,14 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.ldy = ldy;
     kp.f = f;
     kp.slab_w = c.sh.slab_w;
-    kp.n_items = p->n_items - c.left_out;
-    kp.n_prefix = p->n_prefix - c.left_out;
+    kp.n_items = d.n_items - c.left_out;
+    kp.n_prefix = d.n_prefix - c.left_out;
     kp.group = c.group;
     kp.n_pclaims = c.n_pclaims;
     kp.claims_per_slab = c.claims_per_slab;
     kp.n_claims = c.n_claims;
     kp.scratch = scratch;
-    kp.n_partial = p->n_partial - c.left_out;
+    kp.n_partial = d.n_partial - c.left_out;
     kp.counter = counter;
     kp.flags = flags;
     kp.epoch = epoch;
@@ -2063,7 +2212,7 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     kp.use_scale = use_scale ? 1 : 0;
     kp.wait_ns = 2000000000ULL;
     if (c.left_out > 0) {
-        const i32 out = c.left_out, seg = p->segment;
+        const i32 out = c.left_out, seg = d.segment;
         if (c.sh.v4) {
             if (c.sh.nv == 1) return launch_frugal<1, true>(kp, out, seg, p->sm_count, s);
             if (c.sh.nv == 2) return launch_frugal<2, true>(kp, out, seg, p->sm_count, s);
@@ -2107,7 +2256,7 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (p->n_rows == 0) return CBM_B200_OK;
     DeviceGuard g(p->device);
     LaunchCfg c;
-    rc = plan_cfg(p, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
+    rc = plan_cfg(p, p->schedule_for(mode), who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
     if (rc) return rc;
 
     if ((rc = grow(p, p->d_flags, p->flags_cap, c.need_flags, true, s))) return rc;
@@ -2522,27 +2671,31 @@ i64 static_need(i64 n_flags, i64 n_scratch) { return 256 + round_up_256(n_flags 
 // sums of as many of its longest rows as there is room for.  50 000 rows of the second benchmark configuration's kind,
 // 500 columns: 10.1 MiB with 5 076 sums, 4.2 MiB with the 1 719 of coarser cuts; 238 us here with the sums that there is
 // room for, 215 with all of them on the ordinary path, 244 with the coarser cuts.
+bool takes_static(const cbm_b200_plan* p, const float* x, i64 ldx, const float* y, i64 ldy, i32 f) {
+    const bool all_vec = f % 4 == 0 && ldx % 4 == 0 && aligned16(x) && ldy % 4 == 0 && aligned16(y);
+    const Shape coarse = pick_shape(f, p->form && all_vec ? 256 : p->slab_width, all_vec);
+    const i64 sums = p->tree.n_partial_coarse;
+    return static_need(coarse.n_slabs * (p->n_rows + sums), (i64)coarse.n_slabs * sums * coarse.slab_w) <=
+           (i64)CBM_B200_STATIC_SCRATCH_BYTES;
+}
+
 bool fit_static(const cbm_b200_plan* p, const float* x, i64 ldx, const float* y, i64 ldy, i32 f, LaunchCfg& c) {
     const bool x_vec = ldx % 4 == 0 && aligned16(x), all_vec = f % 4 == 0 && x_vec && ldy % 4 == 0 && aligned16(y);
-    const i32 want = p->form && all_vec ? 256 : p->slab_width;
-    const Shape coarse = pick_shape(f, want, all_vec);
-    const i64 rows = (i64)p->n_items - p->n_partial;
-    if (static_need(coarse.n_slabs * (rows + p->n_partial_coarse), (i64)coarse.n_slabs * p->n_partial_coarse * coarse.slab_w) >
-        (i64)CBM_B200_STATIC_SCRATCH_BYTES)
-        return false;
+    const i64 rows = p->n_rows;
     c = LaunchCfg{};
-    c.sh = pick_shape(f, want, x_vec && ldx < (i64)1 << 30);
+    c.sh = pick_shape(f, p->form && all_vec ? 256 : p->slab_width, x_vec && ldx < (i64)1 << 30);
     c.ragged = c.sh.v4 && !all_vec;
     const i64 per_sum = (i64)c.sh.n_slabs * (c.sh.slab_w + 1) * (i64)sizeof(i32);
     const i64 room = (i64)CBM_B200_STATIC_SCRATCH_BYTES - static_need(c.sh.n_slabs * rows, 0) - 256;
-    const auto& ends = p->part_ends;
+    const DeviceSchedule& d = p->schedule_for(MODE_FUSED);
+    const auto& ends = d.part_ends;
     const auto past = std::upper_bound(ends.begin(), ends.end(), std::max<i64>(0, room / per_sum));
     const i32 kept = past == ends.begin() ? 0 : past[-1];
-    c.left_out = p->n_partial - kept;
-    const i32 n_prefix = p->n_prefix - c.left_out;
+    c.left_out = d.n_partial - kept;
+    const i32 n_prefix = d.n_prefix - c.left_out;
     c.group = (i64)n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256 ? 4 : 1;
     c.n_pclaims = (n_prefix + c.group - 1) / c.group;
-    c.claims_per_slab = c.n_pclaims + (p->n_items - p->n_prefix);
+    c.claims_per_slab = c.n_pclaims + (d.n_items - d.n_prefix);
     c.n_claims = (i64)c.claims_per_slab * c.sh.n_slabs;
     c.need_flags = (i64)c.sh.n_slabs * (rows + kept);
     c.need_scratch = (i64)c.sh.n_slabs * kept * c.sh.slab_w;
@@ -2564,10 +2717,15 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     if (p->n_rows == 0) return CBM_B200_OK;
 
     LaunchCfg c;
-    rc = plan_cfg(p, who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
+    rc = plan_cfg(p, p->tree, who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
     if (rc) return rc;
     const i64 need = static_need(c.need_flags, c.need_scratch);
-    if (need > (i64)CBM_B200_STATIC_SCRATCH_BYTES && !fit_static(p, x, ldx, y, ldy, f, c))
+    const bool taken = need <= (i64)CBM_B200_STATIC_SCRATCH_BYTES || takes_static(p, x, ldx, y, ldy, f);
+    if (taken) {  // (by its tree; with rows lifted out of it there may be more sums to park)
+        rc = plan_cfg(p, p->schedule_for(MODE_FUSED), who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
+        if (rc) return rc;
+    }
+    if (!taken || (static_need(c.need_flags, c.need_scratch) > (i64)CBM_B200_STATIC_SCRATCH_BYTES && !fit_static(p, x, ldx, y, ldy, f, c)))
         return cbm::fail(CBM_B200_ERR_ARG,
                          std::string(who) + ": this product needs " + std::to_string(need) +
                              " bytes of scratch, the fixed array holds " +

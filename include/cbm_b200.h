@@ -139,6 +139,16 @@ int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, const int32_
                                  int32_t* n_items, int32_t* n_prefix, int32_t* n_partial, int32_t* n_chunks,
                                  int32_t* segment, uint64_t* fingerprint);
 
+/* The rows as the product in one pass computes them: those whose parent saves them few entries are lifted out of the tree
+ * and hang under the virtual root (n) with all their entries.  By the rules of a plan, for a whole matrix in its own
+ * order, with or without communities (labels, may be NULL); needs no GPU.  n_lifted: how many rows that are; parent (n
+ * entries), crow (n + 1), col and val (`capacity` entries of those that crow[n] counts are written): the rows as they
+ * are read back from the schedule.  Any out-pointer may be NULL. */
+int cbm_b200_schedule_lifted(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,
+                             const int32_t* delta_col, const float* delta_val, const float* multiplier,
+                             const int32_t* labels, int32_t* n_lifted, int32_t* parent, int64_t* crow, int64_t capacity,
+                             int32_t* col, float* val);
+
 /* Figures used by the byte model: rows computed by this plan, delta entries of those rows, rows
  * whose parent is the virtual root, tree depth, and device bytes held by the plan. */
 int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64_t* n_delta,

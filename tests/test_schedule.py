@@ -165,3 +165,66 @@ print(L.cbm_b200_{entry}(n, p(row), p(col), p(crow), p(col), p(val), None, *rest
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                           env=dict(os.environ, OMP_NUM_THREADS="2"))
     assert done.returncode == 0 and "memory" in done.stdout, (done.returncode, done.stdout, done.stderr[-300:])
+
+
+def _lifted(c, labels=None):
+    n = c.num_rows
+    p = lambda a: None if a is None else ctypes.c_void_p(a.ctypes.data)
+    mult = None if c.col_multiplier is None else c.col_multiplier.numpy()
+    labels = None if labels is None else np.ascontiguousarray(labels, dtype=np.int32)
+    lifted, parent, crow = ctypes.c_int32(), np.empty(n, np.int32), np.empty(n + 1, np.int64)
+    call = lambda cap, col, val: _lib.lib().cbm_b200_schedule_lifted(
+        n, p(c.mst_row.numpy()), p(c.mst_col.numpy()), p(c._crow), p(c._dcol), p(c._dval), p(mult), p(labels), ctypes.byref(lifted),
+        p(parent), p(crow), cap, p(col), p(val))
+    assert call(0, None, None) == 0, _lib.lib().cbm_b200_last_error()
+    col, val = np.empty(crow[n], np.int32), np.empty(crow[n], np.float32)
+    assert call(len(col), col, val) == 0
+    return lifted.value, parent, crow, col, val
+
+
+def _nested(n):
+    return np.stack([np.repeat(np.arange(n), np.arange(1, n + 1)), np.concatenate([np.arange(i + 1) for i in range(n)])])
+
+
+@pytest.mark.parametrize("ei,alpha,normalized,some_stay", [
+    (with_self_loops(graphs.copy_model(1500, 0.9, 8, 11)), 2, True, False),     # split rows, some levels
+    (graphs.copy_model(3000, 0.8, 3, 5), 0, False, False),                      # a dozen levels that save next to nothing
+    (with_self_loops(graphs.copy_model(3000, 0.97, 60, 3)), 4, True, None),     # savings of all sizes
+    (_nested(400), 0, False, True), (_nested(400), 0, True, True),              # a chain: whole rows would be 100 times the entries
+])
+@pytest.mark.parametrize("communities", [None, 7])
+def test_lifted_rows_are_whole_rows(ei, alpha, normalized, some_stay, communities):
+    c = _cbm(ei, alpha, normalized=normalized)
+    n = c.num_rows
+    labels = None if communities is None else np.random.default_rng(1).integers(0, communities, n)
+    lifted, parent, crow, col, val = _lifted(c, labels)
+    moved = parent != c._parent
+    assert lifted == moved.sum() and np.all(parent[moved] == n)
+    assert some_stay is None or (parent != n).any() == some_stay
+    assert lifted > 0 or some_stay
+    mult = np.ones(n, np.float32) if not normalized else c.col_multiplier.numpy()
+    key = np.unique(ei[0].astype(np.int64) * n + ei[1])
+    whole = np.split(key % n, np.searchsorted(key // n, np.arange(1, n)))
+    for v in range(n):
+        a, b = slice(crow[v], crow[v + 1]), slice(c._crow[v], c._crow[v + 1])
+        if moved[v]:
+            assert np.array_equal(col[a], whole[v]) and np.array_equal(val[a], mult[whole[v]])
+        else:
+            assert np.array_equal(col[a], c._dcol[b]) and np.array_equal(val[a], c._dval[b])
+
+
+@pytest.mark.parametrize("spoil", ["value", "order"])
+def test_a_structure_that_is_no_signed_pattern_is_not_lifted(spoil):
+    """Values that do not cancel, and columns out of order, are taken as they are: no row is computed from other entries."""
+    c = _cbm(graphs.copy_model(3000, 0.8, 3, 5), 0)
+    assert _lifted(c)[0] > 0
+    c._dval, c._dcol = c._dval.copy(), c._dcol.copy()
+    minus = next(v for v in range(c.num_rows) if (c._dval[c._crow[v]:c._crow[v + 1]] < 0).any() and c._crow[v + 1] - c._crow[v] > 1)
+    at = slice(c._crow[minus], c._crow[minus + 1])
+    if spoil == "value":
+        c._dval[at] *= 1.5
+    else:
+        c._dcol[at], c._dval[at] = c._dcol[at][::-1].copy(), c._dval[at][::-1].copy()
+    lifted, parent, crow, col, val = _lifted(c)
+    assert lifted == 0 and np.array_equal(parent, c._parent)
+    assert np.array_equal(col, c._dcol) and np.array_equal(val, c._dval)
