@@ -193,23 +193,12 @@ struct Candidates {
 // exactly.
 // device >= 0 runs the search on that GPU (cbm_candidates.cu) and falls back to the host when the
 // GPU cannot be used; the result is the same set of edges either way.  *used_gpu reports which ran.
-Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int device = -1, bool* used_gpu = nullptr) {
+Candidates make_candidates(const Pattern& a, i32 alpha, int device = -1, bool* used_gpu = nullptr) {
     const i32 n = a.n;
     if (used_gpu) *used_gpu = false;
     struct Tri {
         i32 src, dst, w;
     };
-    // rank of every column in the rare-to-frequent order (ties by id)
-    std::vector<i32> by_freq((size_t)n);
-    {
-        i32 most = 0;
-        for (i32 c = 0; c < n; ++c) most = std::max(most, at.len(c));
-        std::vector<i64> at_freq;
-        bucket_sort(n, most + 1, [&](i64 c) { return at.len((i32)c); }, [](i64 c) { return (i32)c; }, at_freq, by_freq.data());
-    }
-    std::vector<i32> rank((size_t)n);
-    for (i32 i = 0; i < n; ++i) rank[by_freq[i]] = i;
-
     const i32 block = 64;
     const i32 n_blocks = (n + block - 1) / block;
     std::vector<std::vector<Tri>> found((size_t)n_blocks);
@@ -218,26 +207,13 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
     if (device >= 0 && n > 0) {
         const bool trace = std::getenv("CBM_B200_BUILD_TRACE") != nullptr;
         const double t_a = now_s();
-        // rows with their columns replaced by ranks, rarest first: a prefix of such a row is the
-        // set of its rarest columns
-        Raw<i32> row_rank;
-        row_rank.alloc(a.idx.size());
-#pragma omp parallel for schedule(dynamic, 256) if ((i64)a.idx.size() > SHARED_WORK)
-        for (i32 r = 0; r < n; ++r) {
-            i32* b = row_rank.data() + a.ptr[r];
-            for (i64 k = a.ptr[r]; k < a.ptr[r + 1]; ++k) row_rank[(size_t)k] = rank[a.idx[(size_t)k]];
-            std::sort(b, b + a.len(r));
-        }
         std::vector<cbm::CandTriple> triples;
         std::vector<i32> left;
         std::string err;
-        const double t_b = now_s();
-        if (trace) std::fprintf(stderr, "[cbm build] rank rows %.3f s\n", t_b - t_a);
-        if (cbm::gpu_candidates(device, n, alpha, a.ptr.data(), row_rank.data(), by_freq.data(), at.ptr.data(),
-                                at.idx.data(), triples, left, err) == 0) {
+        if (cbm::gpu_candidates(device, n, alpha, a.ptr.data(), a.idx.data(), triples, left, err) == 0) {
             if (used_gpu) *used_gpu = true;
             if (trace) std::fprintf(stderr, "[cbm build] gpu search %.3f s, %zu edges, %zu parents left to the host\n",
-                                    now_s() - t_b, triples.size(), left.size());
+                                    now_s() - t_a, triples.size(), left.size());
             on_host.assign((size_t)n, 0);
             for (i32 u : left) on_host[u] = 1;
             // in the order the host search emits: by parent block, inside a block by (parent, child)
@@ -248,12 +224,22 @@ Candidates make_candidates(const Pattern& a, const Pattern& at, i32 alpha, int d
                           [](const Tri& x, const Tri& y) { return x.src != y.src ? x.src < y.src : x.dst < y.dst; });
         }
     }
-    std::vector<i32>().swap(by_freq);
     const bool host_all = on_host.empty();
     bool any_host = host_all;
     for (char h : on_host) any_host = any_host || h;
 
     if (any_host) {
+    const Pattern at = transpose(a);
+    // rank of every column in the rare-to-frequent order (ties by id)
+    std::vector<i32> rank((size_t)n);
+    {
+        i32 most = 0;
+        for (i32 c = 0; c < n; ++c) most = std::max(most, at.len(c));
+        std::vector<i64> at_freq;
+        std::vector<i32> by_freq((size_t)n);
+        bucket_sort(n, most + 1, [&](i64 c) { return at.len((i32)c); }, [](i64 c) { return (i32)c; }, at_freq, by_freq.data());
+        for (i32 i = 0; i < n; ++i) rank[by_freq[i]] = i;
+    }
 #pragma omp parallel
     {
         std::vector<uint64_t> in_u(((size_t)n + 63) / 64, 0);  // bit per column: is it in row u?
@@ -656,11 +642,9 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
         b->seconds[3] = now_s() - t0;
         Arborescence arb;
         {
-            Pattern at = transpose(a);
             bool on_gpu = false;
-            Candidates g = make_candidates(a, at, alpha, device, &on_gpu);
+            Candidates g = make_candidates(a, alpha, device, &on_gpu);
             b->candidates_on_gpu = on_gpu ? 1 : 0;
-            at.idx.alloc(0);
             b->n_candidates = g.total;
             const double t1 = now_s();
             b->seconds[0] = t1 - t0;
@@ -778,7 +762,7 @@ int build_impl(const int32_t* row, const int32_t* col, int64_t nnz, int32_t n, i
             for (; pv < ev; ++pv) emit(*pv, true);
         }
         if (std::getenv("CBM_B200_BUILD_TRACE"))
-            std::fprintf(stderr, "[cbm build] csr %.4f, transpose + candidates %.4f, arborescence %.4f, tree + deltas %.4f s\n", b->seconds[3],
+            std::fprintf(stderr, "[cbm build] csr %.4f, candidates %.4f, arborescence %.4f, tree + deltas %.4f s\n", b->seconds[3],
                          b->seconds[0] - b->seconds[3], b->seconds[1], now_s() - t2);
         b->seconds[2] = now_s() - t2;
         b->seconds[3] = now_s() - t0;

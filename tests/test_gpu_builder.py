@@ -66,3 +66,18 @@ def test_config4_full_size_on_the_gpu():
     ei = with_self_loops(graphs.make_graph("c4"))
     host, gpu = _both(ei, 4, normalized=True)
     assert gpu.build_info["seconds_candidates"] < 30.0
+
+
+@pytest.mark.parametrize("lengths", [(1, 2, 31, 32, 33, 64, 255, 256, 257), (511, 512, 513, 4095, 4096, 4097, 5000, 9000)])
+def test_rows_at_the_edges_of_the_sorts(lengths):
+    """Rows as long as a warp's registers, a warp's and a block's shared memory hold, one more and one less, each with a near
+    copy that can be its child."""
+    n = 9000
+    rng = np.random.default_rng(sum(lengths))
+    pattern = [rng.integers(0, n, 3) for _ in range(n)]
+    for i, length in enumerate(lengths):
+        pattern[2 * i] = rng.choice(n, length, replace=False)
+        pattern[2 * i + 1] = np.concatenate([pattern[2 * i][: max(1, length - 2)], rng.integers(0, n, 2)])
+    key = np.unique(np.concatenate([v * n + p for v, p in enumerate(pattern)] + [np.array([n * n - 1])]))
+    host, _ = _both(np.stack([key // n, key % n]), 0)
+    assert host.build_info["depth"] > 1
