@@ -121,13 +121,16 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, MINB) cbm_chunks_kernel(
                 // stages that were filled last are waited for (bounded) before leaving.
                 for (unsigned q = seq - STAGES; q < seq; ++q)
                     mbar_wait(bars + 8 * (q % STAGES), (q / STAGES) & 1, p.status, p.wait_ns);
-                break;
+                if (last) draw_last(p, t);
+                else drain(p, 0);
+                return;
             }
             s_info[st] = make_int4(slab, c.first, c.count, c.e0);
             s_ticket[st] = 0;
             if (last) {  // tells the consumers to leave; they have waited for every copy before this
                 mbar_arrive(bars + 8 * st);
-                break;
+                draw_last(p, t);
+                return;
             }
             unsigned char* at = smem + st * STAGE_BYTES;
             const unsigned n_desc = (unsigned)c.count * (unsigned)sizeof(RowDesc);
@@ -136,8 +139,6 @@ __global__ void __launch_bounds__((CONSUMERS + 1) * 32, MINB) cbm_chunks_kernel(
             bulk_copy_g2s(smem_addr(at), p.desc + c.first, n_desc, bars + 8 * st);
             if (n_ent) bulk_copy_g2s(smem_addr(at + DESC_BYTES), p.ent + c.e0, n_ent, bars + 8 * st);
         }
-        leave(p, 0);
-        return;
     }
 
     unsigned st = 0, parity = 0;

@@ -123,7 +123,7 @@ struct KParams {
     i64 n_claims;    // claims_per_slab * n_slabs
     float* scratch;  // n_slabs * n_partial * slab_w floats: partial sums of long rows
     i32 n_partial;   // PARTIAL items (positions [0, n_partial))
-    u64* counter;    // [0] next claim, [1] warps that have left; both 0 between launches
+    u64* counter;    // next claim; 0 between launches
     u64 n_warps;     // claimers in this launch: warps, or the blocks of a clustered plan's kernel
     i32* flags;      // n_slabs * n_items ready flags holding the epoch of the launch that set them
     i32 epoch;
@@ -426,32 +426,62 @@ __device__ __forceinline__ int lanes_log2(i32 wcols) {
     return lanes <= 1 ? 0 : 32 - __clz(lanes - 1);
 }
 
-// A warp signs off; the last one out rewinds both counters for the next launch.  This holds on
-// the drain path after a failed wait too, so a plan stays usable after a timeout.
-__device__ __forceinline__ void leave(const KParams& p, int lane) {
-    if (lane == 0) {
-        if (atomicAdd(p.counter + 1, 1ULL) == p.n_warps - 1) {
-            p.counter[0] = 0;
-            p.counter[1] = 0;
-            __threadfence();
-        }
-    }
+// Claims are drawn from one counter, and every claimer draws until it gets one past the last: together they draw
+// n_claims + n_warps, and whoever draws the last of these rewinds the counter for the next launch.
+__device__ __forceinline__ void draw_last(const KParams& p, u64 t) {
+    if (t == (u64)p.n_claims + p.n_warps - 1) *p.counter = 0;
 }
 
-// Maps a claim number to (slab, first item, item count): inside a slab the prefix is handed out
+// A claimer that gives up draws what is left without working on it, so that the counter is rewound after a failed wait
+// too and a plan stays usable after a timeout.  (Whoever waits for such an item sees the status word.)
+__device__ __forceinline__ void drain(const KParams& p, int lane) {
+    if (lane != 0) return;
+    u64 t;
+    do t = atomicAdd(p.counter, 1ULL);
+    while (t < (u64)p.n_claims);
+    draw_last(p, t);
+}
+
+// The first claims of a block's 8 warps, drawn as one: the draws of all warps at the start of a launch meet at one address,
+// one after the other, and 7 104 of them take 4 us.  In one round (see LaunchCfg) there are no others.  (The shuffle tells
+// the compiler that the number is the same in all lanes: it is kept out of the 40 registers then.)
+template <bool ONE_ROUND>
+__device__ __forceinline__ u64 first_claim(const KParams& p) {
+    __shared__ u64 s_first;
+    if (threadIdx.x == 0) {
+        s_first = atomicAdd(p.counter, 8ULL);
+        if (ONE_ROUND && s_first + 8 == p.n_warps) *p.counter = 0;
+    }
+    __syncthreads();
+    return __shfl_sync(0xffffffffu, s_first + (threadIdx.x >> 5), 0);
+}
+
+__device__ __forceinline__ u64 draw_claim(const KParams& p, int lane) {
+    u64 t = 0;
+    if (lane == 0) t = atomicAdd(p.counter, 1ULL);
+    return __shfl_sync(0xffffffffu, t, 0);
+}
+
+// Maps a claim number to (slab, first item, end of its items): inside a slab the prefix is handed out
 // `group` items at a time, the rest one item at a time.  Only items that never wait are grouped:
 // a warp that sits on an item waiting for a neighbour would starve the items behind it in its
 // group, which others in turn wait for (measured: 16x slower with 4 mixed items per claim).
-__device__ __forceinline__ void decode_claim(const KParams& p, u64 t, i32& slab, i32& first, i32& count) {
+// In one round a claim's items of the prefix lie n_pclaims apart: they stand in order of length, and every warp is to have
+// as much to do as the others.
+template <bool ONE_ROUND = false>
+__device__ __forceinline__ void decode_claim(const KParams& p, u64 t, i32& slab, i32& first, i32& end) {
     const unsigned u = (unsigned)t;  // the host refuses launches of 2^31 claims or more
     slab = (i32)(u / (unsigned)p.claims_per_slab);
     const i32 r = (i32)(u - (unsigned)slab * (unsigned)p.claims_per_slab);
-    if (r < p.n_pclaims) {
-        first = r * p.group;
-        count = min(p.group, p.n_prefix - first);
-    } else {
+    if (r >= p.n_pclaims) {
         first = p.n_prefix + (r - p.n_pclaims);
-        count = 1;
+        end = first + 1;
+    } else if (ONE_ROUND) {
+        first = r;
+        end = p.n_prefix;
+    } else {
+        first = r * p.group;
+        end = min(first + p.group, p.n_prefix);
     }
 }
 
@@ -638,22 +668,19 @@ __device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 firs
 // UNROLL = row fetches in flight per lane, MINB = thread blocks the register budget must allow
 // per SM.
 // NARROW: every slab is at most 64 columns wide.
-template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false, bool NARROW = false>
-__global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
+template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false, bool NARROW = false, bool ONE_ROUND = false>
+__global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const __grid_constant__ KParams p) {
     using V = Vec<V4>;
     using T = typename V::T;
     constexpr int STEP = 32 * V::E;
     const int lane = threadIdx.x & 31;
-    for (;;) {
-        u64 t = 0;
-        if (lane == 0) t = atomicAdd(p.counter, 1ULL);
-        t = __shfl_sync(0xffffffffu, t, 0);
+    for (u64 t = first_claim<ONE_ROUND>(p);; t = draw_claim(p, lane)) {
         if (t >= (u64)p.n_claims) {
-            leave(p, lane);
+            if (!ONE_ROUND && lane == 0) draw_last(p, t);
             return;
         }
-        i32 slab, first, count;
-        decode_claim(p, t, slab, first, count);
+        i32 slab, first, end;
+        decode_claim<ONE_ROUND>(p, t, slab, first, end);
         const i32 c0 = slab * p.slab_w;
         const i32 wcols = min(p.slab_w, p.f - c0);
         bool ok[NV];
@@ -661,13 +688,13 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
         for (int v = 0; v < NV; ++v) ok[v] = (lane * V::E + v * STEP) < wcols;
         if constexpr (NARROW) {
             const int lg = lanes_log2<V::E>(wcols);
-            if (lg >= 3 && count > 1 && first >= p.n_partial && first + count <= p.n_prefix && p.n_bcast == 0) {
-                if (lg == 4) rows_narrow<V4, RAGGED, 4>(p, slab, first, first + count, c0, wcols, lane);
-                else rows_narrow<V4, RAGGED, 3>(p, slab, first, first + count, c0, wcols, lane);
+            if (!ONE_ROUND && lg >= 3 && end - first > 1 && first >= p.n_partial && end <= p.n_prefix && p.n_bcast == 0) {
+                if (lg == 4) rows_narrow<V4, RAGGED, 4>(p, slab, first, end, c0, wcols, lane);
+                else rows_narrow<V4, RAGGED, 3>(p, slab, first, end, c0, wcols, lane);
                 continue;
             }
         }
-        for (i32 pos = first; pos < first + count; ++pos) {
+        for (i32 pos = first; pos < end; pos += ONE_ROUND ? p.n_pclaims : 1) {
             const int4 da = __ldg((const int4*)(p.desc + pos));
             const int4 db = __ldg((const int4*)(p.desc + pos) + 1);
             const i32 info = da.w;
@@ -701,10 +728,11 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const KParams p) {
             }
             if (!finish_item<NV, V4, RAGGED>(p, slab, pos, da.x, da.y, da.z, info, db.y, __int_as_float(db.z),
                                              __int_as_float(db.w), acc, ok, c0, lane)) {
-                leave(p, lane);
+                if (!ONE_ROUND) drain(p, lane);
                 return;
             }
         }
+        if (ONE_ROUND) return;
     }
 }
 
@@ -719,16 +747,13 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 2) cbm_items_frugal_kernel(
     constexpr int STEP = 32 * V::E, UNROLL = 4;
     const int lane = threadIdx.x & 31;
     const i32 kept = p.n_partial;
-    for (;;) {
-        u64 t = 0;
-        if (lane == 0) t = atomicAdd(p.counter, 1ULL);
-        t = __shfl_sync(0xffffffffu, t, 0);
+    for (u64 t = first_claim<false>(p);; t = draw_claim(p, lane)) {
         if (t >= (u64)p.n_claims) {
-            leave(p, lane);
+            if (lane == 0) draw_last(p, t);
             return;
         }
-        i32 slab, first, count;
-        decode_claim(p, t, slab, first, count);
+        i32 slab, first, end;
+        decode_claim(p, t, slab, first, end);
         const i32 c0 = slab * p.slab_w;
         const i32 wcols = min(p.slab_w, p.f - c0);
         bool ok[NV];
@@ -743,7 +768,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 2) cbm_items_frugal_kernel(
             else
                 gather_row<NV, V4, UNROLL>(PairEntries{p.ent}, beg, beg + len, p.x + c0 + lane * V::E, p.ldx, ok, acc, lane);
         };
-        for (i32 pos = first; pos < first + count; ++pos) {
+        for (i32 pos = first; pos < end; ++pos) {
             const i32 item = pos < kept ? pos : pos + out;
             const int4 da = __ldg((const int4*)(p.desc + item));
             const int4 db = __ldg((const int4*)(p.desc + item) + 1);
@@ -763,7 +788,7 @@ __global__ void __launch_bounds__(256, NV == 1 ? 4 : 2) cbm_items_frugal_kernel(
             }
             if (!finish_item<NV, V4, V4>(p, slab, pos, da.x, da.y, da.z - out, info, db.y, __int_as_float(db.z),
                                          __int_as_float(db.w), acc, ok, c0, lane)) {
-                leave(p, lane);
+                drain(p, lane);
                 return;
             }
         }
@@ -875,15 +900,14 @@ __global__ void __launch_bounds__(WARPS * 32, 1) cbm_items_tma_kernel(const KPar
     unsigned parity = 0;  // bit s = phase the next wait on stage s looks for
 
     for (;;) {
-        u64 t = 0;
-        if (lane == 0) t = atomicAdd(p.counter, 1ULL);
-        t = __shfl_sync(0xffffffffu, t, 0);
+        const u64 t = draw_claim(p, lane);
         if (t >= (u64)p.n_claims) {
-            leave(p, lane);
+            if (lane == 0) draw_last(p, t);
             return;
         }
-        i32 slab, first, count;
-        decode_claim(p, t, slab, first, count);
+        i32 slab, first, end;
+        decode_claim(p, t, slab, first, end);
+        const i32 count = end - first;
         const i32 c0 = slab * SLABW;
         const i32 wcols = min(SLABW, p.f - c0);
         const unsigned piece = (unsigned)wcols * 4u;
@@ -994,7 +1018,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) cbm_items_tma_kernel(const KPar
                 mbar_wait(bar0 + 8 * s2, (parity >> s2) & 1u, p.status);
                 parity ^= 1u << s2;
             }
-            leave(p, lane);
+            drain(p, lane);
             return;
         }
         while (cur < count && alive) {  // the last item, and any empty items behind it
@@ -1002,7 +1026,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) cbm_items_tma_kernel(const KPar
             ++cur;
         }
         if (!alive) {
-            leave(p, lane);
+            drain(p, lane);
             return;
         }
     }
@@ -2007,6 +2031,7 @@ struct LaunchCfg {
     Shape sh{};
     int tma = 0;       // 0: register form; otherwise the bulk-copy form (variant number)
     i32 group = 1;     // prefix items per claim
+    bool one_round = false;  // every warp draws once, and does everything there is for it to do
     i32 n_pclaims = 0, claims_per_slab = 0;
     i64 n_claims = 0;
     bool chunked = false;      // the clustered plan's kernel
@@ -2017,6 +2042,13 @@ struct LaunchCfg {
     bool ragged = false;       // 16-byte fetches, but rows of y are not aligned or end inside a vector
     i32 left_out = 0;          // PARTIAL items, the last ones, that the finishing items do themselves
 };
+
+// Blocks of 256 threads that an SM holds of the kernel a product runs, see launch_regs and launch_narrow.
+constexpr int resident_regs(int nv, bool v4, bool ragged) { return nv == 1 ? (v4 ? (ragged ? 5 : 6) : 4) : (nv == 2 ? 3 : 2); }
+constexpr int NARROW_RESIDENT = 6;
+int resident_blocks(const Shape& sh, i32 f, bool ragged, int mode) {
+    return sh.v4 && sh.nv == 1 && f <= 64 && mode != MODE_UPDATE_ONLY ? NARROW_RESIDENT : resident_regs(sh.nv, sh.v4, ragged);
+}
 
 int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
              i32 f, int mode, bool may_pack, bool in_turn, LaunchCfg& c) {
@@ -2066,6 +2098,18 @@ int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, c
         // A small product keeps single claims: with fewer claims than resident warps, grouping
         // only idles warps.
         c.group = ((i64)d.n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && d.n_chunks > 0 ? 8 : 4) : 1;
+        // A product that the resident warps can do in one round draws no second claim: every warp takes its share of the
+        // prefix, and as long as few items wait (a quarter of the warps) one of those or none.  1 000 rows, 16 columns 8.2 ->
+        // 6.2 us, 4 096 rows, 500 columns (two or three items a warp) 32.0 -> 22.0.
+        if (c.group == 1) {
+            const i64 warps = (i64)p->sm_count * resident_blocks(c.sh, f, c.ragged, mode) * 8;
+            const i64 waiting = (i64)(d.n_items - d.n_prefix) * c.sh.n_slabs;
+            if (p->n_blocks == 0 && waiting < warps / 4) {
+                c.one_round = true;
+                c.group = (i32)std::max<i64>(1, ((i64)d.n_prefix * c.sh.n_slabs + (warps - waiting) - 1) / (warps - waiting));
+                while ((i64)((d.n_prefix + c.group - 1) / c.group) * c.sh.n_slabs > warps - waiting) ++c.group;
+            }
+        }
     }
     if (!c.chunked) {
         c.n_pclaims = (d.n_prefix + c.group - 1) / c.group;
@@ -2099,18 +2143,19 @@ int launch_tma(KParams& kp, int sm_count, cudaStream_t s) {
 }
 
 template <int NV, bool V4, bool RAGGED = false>
-int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
+int launch_regs(KParams& kp, bool one_round, int want_blocks, int sm_count, cudaStream_t s) {
     // Unroll depth and resident blocks per SM were chosen by measurement on B200.  For the default
     // form (one float4 per lane, 128-column slabs) 4 gathers in flight per warp at 48 resident
     // warps per SM (40 registers) beat 8 in flight at 32 warps (64 registers) by 3 % on wide
     // operands and tie on narrow ones; forms that spill registers lose more than extra resident
     // warps gain.
     constexpr int kUnroll = NV == 1 ? (V4 ? 4 : 8) : 4;
-    constexpr int kResident = NV == 1 ? (V4 ? (RAGGED ? 5 : 6) : 4) : (NV == 2 ? 3 : 2);
+    constexpr int kResident = resident_regs(NV, V4, RAGGED);
     int blocks = want_blocks > 0 ? want_blocks : sm_count * (NV == 1 && V4 ? kResident : 8);
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
-    cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED><<<blocks, 256, 0, s>>>(kp);
+    if (one_round) cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED, false, true><<<blocks, 256, 0, s>>>(kp);
+    else cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED><<<blocks, 256, 0, s>>>(kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;
 }
@@ -2119,12 +2164,13 @@ int launch_regs(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
 // rows of y are not aligned.  Fetches in flight x resident blocks, 235 868 rows of 11 entries, 64 columns / 400 000 of
 // 22, 47 columns: 4 x 6 97 / 279 us, 6 x 5 100 / 288, 8 x 5 104 / 298, 8 x 4 110 / 310.
 template <bool RAGGED>
-int launch_narrow(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
-    constexpr int kResident = 6;
+int launch_narrow(KParams& kp, bool one_round, int want_blocks, int sm_count, cudaStream_t s) {
+    constexpr int kResident = NARROW_RESIDENT;
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
-    cbm_items_kernel<1, true, 4, kResident, RAGGED, true><<<blocks, 256, 0, s>>>(kp);
+    if (one_round) cbm_items_kernel<1, true, 4, kResident, RAGGED, true, true><<<blocks, 256, 0, s>>>(kp);
+    else cbm_items_kernel<1, true, 4, kResident, RAGGED, true><<<blocks, 256, 0, s>>>(kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;
 }
@@ -2227,20 +2273,20 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
         return c.ragged ? launch_chunks<true>(kp, p->n_blocks, p->sm_count, s)
                         : launch_chunks<false>(kp, p->n_blocks, p->sm_count, s);
     if (c.sh.v4 && c.sh.nv == 1 && f <= 64 && mode != MODE_UPDATE_ONLY)
-        return c.ragged ? launch_narrow<true>(kp, p->n_blocks, p->sm_count, s) : launch_narrow<false>(kp, p->n_blocks, p->sm_count, s);
+        return c.ragged ? launch_narrow<true>(kp, c.one_round, p->n_blocks, p->sm_count, s) : launch_narrow<false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
     if (c.ragged) {
-        if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, p->n_blocks, p->sm_count, s);
-        if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, p->n_blocks, p->sm_count, s);
-        return launch_regs<4, true, true>(kp, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        return launch_regs<4, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
     }
     if (c.sh.v4) {
-        if (c.sh.nv == 1) return launch_regs<1, true>(kp, p->n_blocks, p->sm_count, s);
-        if (c.sh.nv == 2) return launch_regs<2, true>(kp, p->n_blocks, p->sm_count, s);
-        return launch_regs<4, true>(kp, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 1) return launch_regs<1, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 2) return launch_regs<2, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        return launch_regs<4, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
     }
-    if (c.sh.nv == 1) return launch_regs<1, false>(kp, p->n_blocks, p->sm_count, s);
-    if (c.sh.nv == 2) return launch_regs<2, false>(kp, p->n_blocks, p->sm_count, s);
-    return launch_regs<4, false>(kp, p->n_blocks, p->sm_count, s);
+    if (c.sh.nv == 1) return launch_regs<1, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+    if (c.sh.nv == 2) return launch_regs<2, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+    return launch_regs<4, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
 }
 
 int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
