@@ -15,8 +15,10 @@
 //   * Y leaves (and the mask arrives) in whole 128-byte lines, 32 x 32 sums turned round through 4 KB of shared memory
 //     per warp.
 // Every 16-deep step has an accumulator of its own (see cbm_map.cuh), so the sums are added up every 16 columns; with
-// accumulators of 64 columns 128 -> 256 took 96 us.  235 868 rows, against three-term GEMMs that split both operands
-// for every 128 x 128 x 16 tile: 128 -> 256 128 us (201), 256 -> 64 93 (101), 100 000 rows 256 -> 256 100 (153).
+// accumulators of 64 columns 128 -> 256 took 96 us.  The warps that add up and store are what a map waits for: 52 % of their
+// time went into adding, 34 - 49 % into storing.  So the next 8 columns leave tensor memory while 8 are added, and a
+// block of 32 x 32 sums that is all there is stored without a question about single values.  235 868 rows: 128 -> 256 126
+// -> 110 us, 256 -> 64 90 -> 85, 64 -> 256 masked 154 -> 137; 400 000 rows 256 -> 256 342 -> 314, 100 -> 256 194 -> 176.
 #include "cbm_map.cuh"
 
 #include <mutex>
@@ -70,11 +72,11 @@ int check_timeout(const char* who) {
 namespace {
 
 // Two warps of each kind per scheduler: a warp alone on one issues an instruction every 4 - 5 cycles, and with 4
-// epilogue warps (or 4 producers) their work, not memory or the MMAs, was the bound.
+// epilogue warps (or 4 producers, also beside 16 epilogue warps) their work, not memory or the MMAs, was the bound.
 constexpr int PRODUCER_WARPS = 8, EPILOGUE_WARPS = 8;
 constexpr int MMA_WARP = PRODUCER_WARPS + EPILOGUE_WARPS;
 constexpr int THREADS = 20 * 32;  // five warpgroups (of the last only one warp works), 96 registers a thread at launch ...
-constexpr int LAUNCH_REGS = 96, PRODUCER_REGS = 104, EPILOGUE_REGS = 112, MMA_REGS = 40;  // ... and after the split
+constexpr int LAUNCH_REGS = 96, PRODUCER_REGS = 104, EPILOGUE_REGS = 120, MMA_REGS = 24;  // ... and after the split
 static_assert(PRODUCER_REGS > LAUNCH_REGS && EPILOGUE_REGS > LAUNCH_REGS && MMA_REGS < LAUNCH_REGS &&
                   256 * PRODUCER_REGS + 256 * EPILOGUE_REGS + 128 * MMA_REGS <= THREADS * LAUNCH_REGS,
               "setmaxnreg.inc and .dec only go up and down, within the registers of the launch");
@@ -95,6 +97,12 @@ struct MapParams {
     int relu_in, relu_out, add; // max(a, 0) first; max(d, 0) last; d += instead of d =
     int* timeout;
 };
+
+__device__ __forceinline__ void ld8(float (&r)[8], u32 at) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7])
+                 : "r"(at));
+}
 
 // EXTRA: 0 plain, 1 with a mask, 2 with any of a mask and earlier passes' results to add to.
 template <bool B_TRANS, int EXTRA>
@@ -128,18 +136,34 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
         s_gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    // the weights, split, into shared memory
-    const int k8s = 2 * p.steps;
-    for (int i = threadIdx.x; i < p.bn * k8s; i += THREADS) {
-        const int n = B_TRANS ? i % p.bn : i / k8s;
-        const int k8 = B_TRANS ? i / p.bn : i % k8s;
-        float x[8];
+    // The weights, split, into shared memory: two pieces of 8 values a thread at a time, so that their fetches overlap.
+    const int k8s = 2 * p.steps, pieces = p.bn * k8s;
+    const bool b_vec = !B_TRANS && p.ldb % 4 == 0 && (reinterpret_cast<u64>(p.b) & 15) == 0;
+    for (int i0 = threadIdx.x; i0 < pieces; i0 += 2 * THREADS) {
+        float x[2][8];
+        int at_n[2], at_k[2];
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const int k = k8 * 8 + j;
-            x[j] = n0 + n < p.n && k < p.k ? __ldg(B_TRANS ? p.b + (int64_t)k * p.ldb + n0 + n : p.b + (int64_t)(n0 + n) * p.ldb + k) : 0.f;
+        for (int h = 0; h < 2; ++h) {
+            const int i = i0 + h * THREADS;
+            const bool on = i < pieces;
+            const int n = B_TRANS ? i % p.bn : i / k8s, k8 = B_TRANS ? i / p.bn : i % k8s;
+            at_n[h] = n;
+            at_k[h] = k8;
+            const float* from = B_TRANS ? p.b + (int64_t)(k8 * 8) * p.ldb + n0 + n : p.b + (int64_t)(n0 + n) * p.ldb + k8 * 8;
+            if (b_vec && k8 * 8 + 8 <= p.k) {
+                const float4 lo = fetch4(from, on && n0 + n < p.n), hi = fetch4(from + 4, on && n0 + n < p.n);
+                x[h][0] = lo.x, x[h][1] = lo.y, x[h][2] = lo.z, x[h][3] = lo.w;
+                x[h][4] = hi.x, x[h][5] = hi.y, x[h][6] = hi.z, x[h][7] = hi.w;
+            } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                    x[h][j] = fetch1(from + (B_TRANS ? j * p.ldb : j), on && n0 + n < p.n && k8 * 8 + j < p.k);
+            }
         }
-        store_split8(smem + (u32)(k8 >> 3) * block + swizzled((u32)n, (u32)(k8 & 7)), term, x);
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+            if (i0 + h * THREADS < pieces)
+                store_split8(smem + (u32)(at_k[h] >> 3) * block + swizzled((u32)at_n[h], (u32)(at_k[h] & 7)), term, x[h]);
     }
     fence_async();
     fence_before();
@@ -316,26 +340,22 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                 const u32 ds = it & 1, use = it >> 1;
                 if (!warp_wait(d_full + 8 * ds, use & 1, gave_up, p.timeout)) return false;
                 const u32 at = tmem + ds * D_COLS + c_lo + ((u32)(quarter * 32) << 16);
+float r[2][8];
+                ld8(r[0], at);
 #pragma unroll
-                for (int q = 0; q < 4; ++q) {
-                    float r[16];
-                    if (16 * q < width)
-                        asm volatile(
-                            "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-                            "%14, %15}, [%16];"
-                            : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]),
-                              "=f"(r[8]), "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
-                            : "r"(at + 16 * q));
+                for (int q = 0; q < 8; ++q) {  // the next 8 columns are on their way while these are added
                     wait_ld();
 #pragma unroll
-                    for (int i = 0; i < 16; i += 2) {
-                        asm volatile("" : "+f"(r[i]), "+f"(r[i + 1]));  // not before the wait
-                        float &s = acc[q >> 1][16 * (q & 1) + i], &t = acc[q >> 1][16 * (q & 1) + i + 1];
+                    for (int i = 0; i < 8; ++i) asm volatile("" : "+f"(r[q & 1][i]));  // not before the wait
+                    if (q < 7 && 8 * (q + 1) < width) ld8(r[(q + 1) & 1], at + 8 * (q + 1));
+#pragma unroll
+                    for (int i = 0; i < 8; i += 2) {
+                        float &s = acc[q >> 2][8 * (q & 3) + i], &t = acc[q >> 2][8 * (q & 3) + i + 1];
                         if constexpr (decltype(first)::value) {
-                            s = r[i];
-                            t = r[i + 1];
+                            s = r[q & 1][i];
+                            t = r[q & 1][i + 1];
                         } else {
-                            add2(s, t, r[i], r[i + 1]);
+                            add2(s, t, r[q & 1][i], r[q & 1][i + 1]);
                         }
                     }
                 }
@@ -357,6 +377,24 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                 __syncwarp();
                 const int col = 32 * b + col_in, left = col < c_lo + width ? p.n - n0 - col : 0;
                 float* d0 = p.d + (int64_t)row0 * p.ldd + n0 + col;
+                // A block that is all there and goes out in whole lines: nothing is asked about single values.
+                if (EXTRA < 2 && p.d_vec && tile * 128 + 128 <= p.m && 32 * b + 32 <= width && n0 + c_lo + 32 * b + 32 <= p.n) {
+                    const float4* from = mine + (lane >> 3) * 8 + ((lane & 7) ^ (lane >> 3));
+                    const float4* odd = mine + (lane >> 3) * 8 + ((lane & 7) ^ (lane >> 3) ^ 4);
+                    const int64_t step = 4 * p.ldd;
+#pragma unroll
+                    for (int i = 0; i < 8; ++i, d0 += step) {
+                        float4 y = (i & 1 ? odd : from)[32 * i];
+                        if constexpr (EXTRA) {
+                            const u32 bits = keep[b] >> (4 * i);
+                            y = make_float4(bits & 1 ? y.x : 0.f, bits & 2 ? y.y : 0.f, bits & 4 ? y.z : 0.f, bits & 8 ? y.w : 0.f);
+                        }
+                        if (p.relu_out) y = relu(y);
+                        *reinterpret_cast<float4*>(d0) = y;
+                    }
+                    __syncwarp();
+                    continue;
+                }
 #pragma unroll
                 for (int i = 0; i < 8; ++i) {
                     const int r = (lane >> 3) + 4 * i;
