@@ -5,22 +5,28 @@
 // rows.  Both operands are needed with the rows as the contraction, that is transposed: a lane owns one column
 // (or two) and reads it down 32 (8) rows, a warp's reads being 128-byte lines (two), splits, and has neighbours of the
 // contraction in its own registers - written to tensor memory for the first operand, as 16-byte pieces of swizzled
-// K-major rows to shared memory for the second.  8 + 3 warps do that, the next chunk's loads in flight, one warp
+// K-major rows to shared memory for the second.  8 + 7 warps do that, the next chunk's loads in flight, one warp
 // issues the MMAs, 8 warps add the accumulators of every 64 rows to sums in registers.  The ranges' partial results
 // are added in a fixed order by a second kernel, which also turns the tile round where the operands' roles were
 // exchanged.
 //
 // A chunk's way through a block (load, split, store) is a chain that the memory's latency bounds, not its rate, so
-// each task of the second operand asks for its next chunk as soon as its registers are free, and rows without gaps
-// are brought to L2 AHEAD chunks early.  235 868 rows: 64 x 256 125 -> 102 us, 256 x 128 153 -> 129 us.
+// each warp of the second operand asks for its next task's rows before it works on this one's, and rows without gaps
+// are brought to L2 AHEAD chunks early.  With three warps for the second operand they were what everyone waited for (the
+// MMA warp 62 % of its time); seven that take its tasks in turn leave the chain of the first operand.  235 868 rows:
+// 64 x 256 101 -> 92 us, 256 x 128 129 -> 110, 256 x 256 249 -> 202.
 #include "cbm_map.cuh"
 
 namespace cbm_map {
 namespace {
 
-constexpr int A_WARPS = 8, B_WARPS = 3, SUM_WARPS = 8;
+constexpr int A_WARPS = 8, B_WARPS = 7, SUM_WARPS = 8;
 constexpr int MMA_WARP = A_WARPS + B_WARPS, FIRST_SUM_WARP = MMA_WARP + 1;
-constexpr int GRAD_THREADS = (FIRST_SUM_WARP + SUM_WARPS) * 32;  // 20 warps: 96 registers each
+constexpr int GRAD_THREADS = (FIRST_SUM_WARP + SUM_WARPS) * 32;  // 24 warps, 80 registers a thread at launch ...
+constexpr int LAUNCH_REGS = 80, A_REGS = 96, B_REGS = 64, SUM_REGS = 80;  // ... and after the split (the MMA warp has B's share)
+static_assert(A_REGS > LAUNCH_REGS && SUM_REGS == LAUNCH_REGS && B_REGS < LAUNCH_REGS &&
+                  32 * (A_WARPS * A_REGS + (B_WARPS + 1) * B_REGS + SUM_WARPS * SUM_REGS) <= GRAD_THREADS * LAUNCH_REGS,
+              "setmaxnreg.inc and .dec only go up and down, within the registers of the launch");
 // Chunks between a prefetch to L2 and the loads: 3 and 4 measure alike, 8 costs 5 % and 12 13 % (L2 evicts early).
 constexpr int AHEAD = 4;
 constexpr int MAX_PARTS = CBM_B200_DENSE_MAX_CHUNKS;
@@ -71,7 +77,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
     if (warp == MMA_WARP) tmem_alloc(smem_u32(&s_tmem));
     if (threadIdx.x == 0) {
         for (int s = 0; s < A_SLOTS; ++s) {
-            bar_init(full + 8 * s, 4 + B_WARPS);
+            bar_init(full + 8 * s, 4 + p.bn / 64 * 4);  // four A warps, and every task of B
             bar_init(empty + 8 * s, 1);
         }
         for (int s = 0; s < 2; ++s) {
@@ -89,6 +95,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
     volatile int* gave_up = &s_gave_up;
 
     if (warp < A_WARPS) {
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(A_REGS));
         // lane = column; two groups of four warps, alternate chunks.  Lanes past the last column read it again: their
         // rows of the tile are not stored.
         const int quarter = warp & 3, group = warp >> 2;
@@ -148,85 +155,86 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
             __syncwarp();
             if (lane == 0) bar_arrive(full + 8 * slot);
         }
-    } else if (warp < A_WARPS + B_WARPS) {
-        // Task i of this warp: 64 columns by 8 rows, number (warp's own) + 3 i of the (bn / 64) x 4 of a chunk.  A lane has
+    } else if (warp < FIRST_SUM_WARP) {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(B_REGS));
+        if (warp == MMA_WARP) {
+            const u32 idesc = idesc_of((u32)p.bn), b0 = smem_u32(smem);
+            bool ok = true;
+            for (int kb = 0; kb < kblocks; ++kb) {
+                const u32 ds = kb & 1, use = kb >> 1;
+                if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
+                const u32 d = tmem + ds * D_COLS;
+                const int here = min(2, chunks - 2 * kb);
+                for (int c = 0; c < here && ok; ++c) {
+                    const u32 r = 2 * kb + c, slot = r % A_SLOTS;
+                    if (!(ok = warp_wait(full + 8 * slot, (r / A_SLOTS) & 1, gave_up, p.timeout))) break;
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        mma_small(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, b0 + (slot >> 1) * stage + (slot & 1) * 64 + 32 * s, term,
+                                  idesc, c + s > 0);
+                }
+                if (!ok) break;
+                for (int c = 0; c < here; ++c) {
+                    const u32 slot = (2 * kb + c) % A_SLOTS;
+#pragma unroll
+                    for (int s = 0; s < 2; ++s)
+                        mma(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, desc_of(b0 + (slot >> 1) * stage + (slot & 1) * 64 + 32 * s), idesc, true);
+                    commit(empty + 8 * slot);
+                }
+                commit(d_full + 8 * ds);
+            }
+            if (!ok) {  // the MMAs under way end before the block frees its tensor memory
+                commit(drained);
+                for (u32 spins = 0; spins < (1u << 20) && !bar_poll(drained, 0); ++spins) {
+                }
+                __syncwarp();
+            }
+            goto done;
+        }
+        // Task i of a chunk: 64 columns by 8 rows, of the (bn / 64) x 4 of them.  The warps take the tasks of all chunks in
+        // turn, the next one's loads under way.  A lane has
         // columns 2 lane and 2 lane + 1 of the 64 and puts them into rows lane and lane + 32 of the operand tile, so
         // that its 16-byte stores fall into different banks; the sums' columns are put straight on the way out.
-        constexpr int TASKS = (D_COLS / 64 * 4 + B_WARPS - 1) / B_WARPS;
-        const int w = warp - A_WARPS, tasks = p.bn / 64 * 4;
-        float2 v[TASKS][8];
-        auto load = [&](int c, int i) {
-            const int task = w + B_WARPS * i;
-            if (task >= tasks) return;
-            const int col = n0 + (task >> 2) * 64 + 2 * lane, r0 = (first + c) * CHUNK_K + (task & 3) * 8;
+        const int lg = p.bn == 64 ? 2 : 3, tasks = chunks << lg;
+        float2 v[2][8];
+        auto load = [&](int buf, int t) {
+            const int task = t & ((1 << lg) - 1);
+            const int col = n0 + (task >> 2) * 64 + 2 * lane, r0 = (first + (t >> lg)) * CHUNK_K + (task & 3) * 8;
             const int c0 = min(col, (p.n - 1) & ~1), step = c0 + 1 < p.n ? 1 : 0;
             const float* at = p.b + (int64_t)r0 * p.ldb + c0;
             if (r0 + 8 <= p.rows && p.b_vec) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j, at += p.ldb) v[i][j] = fetch_pair(at);
+                for (int j = 0; j < 8; ++j, at += p.ldb) v[buf][j] = fetch_pair(at);
             } else {
 #pragma unroll
                 for (int j = 0; j < 8; ++j, at += p.ldb)
-                    v[i][j] = make_float2(fetch1(at, r0 + j < p.rows), fetch1(at + step, r0 + j < p.rows));
+                    v[buf][j] = make_float2(fetch1(at, r0 + j < p.rows), fetch1(at + step, r0 + j < p.rows));
             }
         };
-        if (chunks > 0) {
+        int t = warp - A_WARPS;
+        if (t < tasks) load(0, t);
+        while (t < tasks) {
 #pragma unroll
-            for (int i = 0; i < TASKS; ++i) load(0, i);
-        }
-        for (int c = 0; c < chunks; ++c) {
-            const u32 slot = (u32)c % A_SLOTS;
-            if (c >= A_SLOTS && !warp_wait(empty + 8 * slot, ((u32)c / A_SLOTS + 1) & 1, gave_up, p.timeout)) goto done;
-            unsigned char* at = smem + (slot >> 1) * stage;
-#pragma unroll
-            for (int i = 0; i < TASKS; ++i) {
-                const int task = w + B_WARPS * i;
-                if (task >= tasks) break;
+            for (int buf = 0; buf < 2; ++buf) {
+                if (t >= tasks) break;
+                if (t + B_WARPS < tasks) load(buf ^ 1, t + B_WARPS);
+                const int c = t >> lg, task = t & ((1 << lg) - 1);
+                const u32 slot = (u32)c % A_SLOTS;
+                if (c >= A_SLOTS && !warp_wait(empty + 8 * slot, ((u32)c / A_SLOTS + 1) & 1, gave_up, p.timeout)) goto done;
+                unsigned char* at = smem + (slot >> 1) * stage;
                 const u32 row = (u32)((task >> 2) * 64 + lane), k8 = (slot & 1) * 4 + (u32)(task & 3);
                 float x[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? relu(v[i][j].x) : v[i][j].x;
+                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? relu(v[buf][j].x) : v[buf][j].x;
                 store_split8(at + swizzled(row, k8), term, x);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? relu(v[i][j].y) : v[i][j].y;
+                for (int j = 0; j < 8; ++j) x[j] = p.relu_b ? relu(v[buf][j].y) : v[buf][j].y;
                 store_split8(at + swizzled(row + 32, k8), term, x);
-                if (c + 1 < chunks) load(c + 1, i);  // as soon as its registers are free, ahead of the other tasks
+                fence_async();
+                __syncwarp();
+                if (lane == 0) bar_arrive(full + 8 * slot);
+                t += B_WARPS;
             }
-            fence_async();
-            __syncwarp();
-            if (lane == 0) bar_arrive(full + 8 * slot);
-        }
-    } else if (warp == MMA_WARP) {
-        const u32 idesc = idesc_of((u32)p.bn), b0 = smem_u32(smem);
-        bool ok = true;
-        for (int kb = 0; kb < kblocks; ++kb) {
-            const u32 ds = kb & 1, use = kb >> 1;
-            if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
-            const u32 d = tmem + ds * D_COLS;
-            const int here = min(2, chunks - 2 * kb);
-            for (int c = 0; c < here && ok; ++c) {
-                const u32 r = 2 * kb + c, slot = r % A_SLOTS;
-                if (!(ok = warp_wait(full + 8 * slot, (r / A_SLOTS) & 1, gave_up, p.timeout))) break;
-#pragma unroll
-                for (int s = 0; s < 2; ++s)
-                    mma_small(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, b0 + (slot >> 1) * stage + (slot & 1) * 64 + 32 * s, term,
-                              idesc, c + s > 0);
-            }
-            if (!ok) break;
-            for (int c = 0; c < here; ++c) {
-                const u32 slot = (2 * kb + c) % A_SLOTS;
-#pragma unroll
-                for (int s = 0; s < 2; ++s)
-                    mma(d, tmem + A_COL + slot * A_SLOT_COLS + 8 * s, desc_of(b0 + (slot >> 1) * stage + (slot & 1) * 64 + 32 * s), idesc, true);
-                commit(empty + 8 * slot);
-            }
-            commit(d_full + 8 * ds);
-        }
-        if (!ok) {  // the MMAs under way end before the block frees its tensor memory
-            commit(drained);
-            for (u32 spins = 0; spins < (1u << 20) && !bar_poll(drained, 0); ++spins) {
-            }
-            __syncwarp();
         }
     } else {
         // lane = row of the tile; accumulator column 32 j + i of this warp's 64 is column 2 i + j of the result
