@@ -8,6 +8,7 @@
 //   2. waits (bounded) until its parent's finished row is published, reads it from L2,
 //   3. applies the row scale, stores the finished row once, and publishes it.
 // Step 1 does not depend on the parent, so the wait in step 2 is normally already satisfied.
+// Rows whose parent saves them little are gathered whole and wait for nobody (cbm_lift.cpp).
 // The dense operand is processed in column slabs so that one slab of X stays resident in the
 // 126 MB L2 while every row gathers from it.
 //
@@ -601,8 +602,8 @@ __device__ __forceinline__ bool finish_item(const KParams& p, i32 slab, i32 pos,
 // lanes for each: for slabs of at most 16 vectors, where a row's fixed costs - descriptor, entries, store, each a trip to
 // memory - outweigh its fetches.  Neighbours in the prefix are of about equal length.  A row's entries are summed as
 // gather_row_narrow sums them, in 32 >> lg interleaved shares: which of the two a row gets depends on where its claim
-// falls, its bits do not.  Four entries of each row are on their way at a time, without conditions as long as all rows have them (two,
-// each with its own: 50 000 rows of 31 entries, 64 columns 44.2 us, 43.2 now).
+// falls, its bits do not.  Four entries of each row are on their way at a time, without conditions as long as all rows have
+// them (two, each with its own: 50 000 rows of 31 entries, 64 columns 44.2 us, 43.0 now).
 template <bool V4, bool RAGGED, int LG>
 __device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 first, i32 end, i32 c0, i32 wcols, int lane) {
     using V = Vec<V4>;
@@ -670,17 +671,98 @@ __device__ __forceinline__ void rows_narrow(const KParams& p, i32 slab, i32 firs
     }
 }
 
+// The same for claims of 8 rows, community order: all descriptors are fetched at once, and then all entries, which follow one another,
+// into the warp's piece of shared memory (400 000 rows of 22 entries, 47 columns 247 us without, 232 with it).
+// Works on as many rows as have room for their entries, and returns the first one after them.
+constexpr int NARROW_ROWS = 8, NARROW_ENTRIES = 256;  // of a claim, that a warp's shared memory takes
+struct NarrowClaim {
+    int4 desc[2 * NARROW_ROWS];
+    int2 ent[NARROW_ENTRIES];
+};
+
+template <bool V4, bool RAGGED, int LG>
+__device__ __forceinline__ i32 rows_narrow_staged(const KParams& p, NarrowClaim& my, i32 slab, i32 first, i32 end, i32 c0, i32 wcols, int lane) {
+    using V = Vec<V4>;
+    using T = typename V::T;
+    constexpr int width = 1 << LG, SHARES = 32 >> LG, UNROLL = 4;
+    const int li = lane & (width - 1);
+    const bool has = li * V::E < wcols;
+    const float* xs = p.x + c0 + li * V::E;
+    i32 e0;
+    {
+        int4 q = make_int4(0, 0, 0, 0);
+        if (lane < 2 * (end - first)) q = __ldg((const int4*)(p.desc + first) + lane);
+        e0 = __shfl_sync(0xffffffffu, q.x, 1);
+        // row r's entries end, counted from the first row's, at what lane 2 r holds
+        const i32 upto = __shfl_down_sync(0xffffffffu, q.x, 1) + ((q.w >> ITEM_LEN_SHIFT) & 0xff) - e0;
+        const i32 rows = __popc(__ballot_sync(0xffffffffu, lane % 2 == 0 && lane < 2 * (end - first) && upto <= NARROW_ENTRIES));
+        if (rows < end - first) end = first + rows / SHARES * SHARES;
+        if (end == first) return first;
+        const i32 n_ent = __shfl_sync(0xffffffffu, upto, 2 * (end - first - 1));
+        __syncwarp();  // (all lanes are done with the claim before)
+        if (lane < 2 * NARROW_ROWS) my.desc[lane] = q;
+        for (i32 i = lane; i < n_ent; i += 32) my.ent[i] = __ldg(reinterpret_cast<const int2*>(p.ent) + e0 + i);
+        __syncwarp();
+    }
+    for (i32 base = first; base < end; base += SHARES) {
+        const i32 pos = base + (lane >> LG);
+        const bool on = pos < end;
+        const int at = 2 * (min(pos, end - 1) - first);
+        const i32 len = on ? (my.desc[at].w >> ITEM_LEN_SHIFT) & 0xff : 0;
+        const i32 most = (i32)__reduce_max_sync(0xffffffffu, (unsigned)len), least = (i32)__reduce_min_sync(0xffffffffu, (unsigned)len);
+        T acc[SHARES];
+#pragma unroll
+        for (int s = 0; s < SHARES; ++s) acc[s] = V::zero();
+        const int2* e = my.ent + (my.desc[at + 1].x - e0);
+        i32 j = 0;
+        for (; j + UNROLL <= least; j += UNROLL) {  // all rows have these entries
+            T t[UNROLL];
+#pragma unroll
+            for (int k = 0; k < UNROLL; ++k) t[k] = V::ld_ro_if(xs + (i64)e[j + k].x * p.ldx, has);
+#pragma unroll
+            for (int k = 0; k < UNROLL; ++k) acc[k % SHARES] = V::fma(__int_as_float(e[j + k].y), t[k], acc[k % SHARES]);
+        }
+        for (; j < most; j += UNROLL) {
+            T t[UNROLL];
+#pragma unroll
+            for (int k = 0; k < UNROLL; ++k) t[k] = V::ld_ro_if(xs + (i64)(j + k < len ? e[j + k].x : 0) * p.ldx, has && j + k < len);
+#pragma unroll
+            for (int k = 0; k < UNROLL; ++k)
+                acc[k % SHARES] = V::fma(j + k < len ? __int_as_float(e[j + k].y) : 0.f, t[k], acc[k % SHARES]);
+        }
+#pragma unroll
+        for (int d = 1; d < SHARES; d <<= 1)
+#pragma unroll
+            for (int s = 0; s < SHARES; s += 2 * d) acc[s] = V::fma(1.0f, acc[s + d], acc[s]);
+        const int4 da = my.desc[at];
+        if (p.use_scale && p.mode != MODE_DELTA_ONLY) acc[0] = V::mul(__int_as_float(my.desc[at + 1].z), acc[0]);
+        if (on && has) {
+            const i32 col = c0 + li * V::E, some = p.f - col;
+            float* y = p.y + (i64)da.x * p.ldy + col;
+            if (RAGGED && !(p.y_vec && some >= V::E)) V::st_some(y, acc[0], some);
+            else if (da.w & ITEM_PUBLISH) V::st(y, acc[0]);
+            else V::st_stream(y, acc[0]);
+        }
+        if (p.mode != MODE_DELTA_ONLY) {
+            __syncwarp();
+            if (on && li == 0 && (da.w & ITEM_PUBLISH)) st_release(p.flags + (i64)slab * p.n_items + pos, p.epoch);
+        }
+    }
+    return end;
+}
+
 // Product kernel, register form: one warp per (item, column slab), the gather held in registers.
 // Serves operands the bulk-copy form cannot take (width not a multiple of 4 floats, unaligned
 // pointers) and the update-only mode, which gathers nothing; it is also the default form.
 // UNROLL = row fetches in flight per lane, MINB = thread blocks the register budget must allow
 // per SM.
-// NARROW: every slab is at most 64 columns wide.
-template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false, bool NARROW = false, bool ONE_ROUND = false>
+// NARROW: every slab is at most 64 columns wide; STAGED: and claims are of up to 8 rows in community order.
+template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false, bool NARROW = false, bool ONE_ROUND = false, bool STAGED = false>
 __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const __grid_constant__ KParams p) {
     using V = Vec<V4>;
     using T = typename V::T;
     constexpr int STEP = 32 * V::E;
+    __shared__ NarrowClaim s_narrow[STAGED ? 8 : 1];
     const int lane = threadIdx.x & 31;
     for (u64 t = first_claim<ONE_ROUND>(p);; t = draw_claim(p, lane)) {
         if (t >= (u64)p.n_claims) {
@@ -696,10 +778,19 @@ __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const __grid_const
         for (int v = 0; v < NV; ++v) ok[v] = (lane * V::E + v * STEP) < wcols;
         if constexpr (NARROW) {
             const int lg = lanes_log2<V::E>(wcols);
-            if (!ONE_ROUND && lg >= 3 && end - first > 1 && first >= p.n_partial && end <= p.n_prefix && p.n_bcast == 0) {
-                if (lg == 4) rows_narrow<V4, RAGGED, 4>(p, slab, first, end, c0, wcols, lane);
-                else rows_narrow<V4, RAGGED, 3>(p, slab, first, end, c0, wcols, lane);
-                continue;
+            if (!ONE_ROUND && lg >= 3 && end - first > 1 && end - first <= NARROW_ROWS && first >= p.n_partial && end <= p.n_prefix && p.n_bcast == 0) {
+                if constexpr (STAGED) {
+                    NarrowClaim& my = s_narrow[threadIdx.x >> 5];
+                    for (i32 from = -1; from != first && first < end;) {
+                        from = first;
+                        first = lg == 4 ? rows_narrow_staged<V4, RAGGED, 4>(p, my, slab, first, end, c0, wcols, lane)
+                                        : rows_narrow_staged<V4, RAGGED, 3>(p, my, slab, first, end, c0, wcols, lane);
+                    }
+                } else {
+                    if (lg == 4) rows_narrow<V4, RAGGED, 4>(p, slab, first, end, c0, wcols, lane);
+                    else rows_narrow<V4, RAGGED, 3>(p, slab, first, end, c0, wcols, lane);
+                    continue;
+                }
             }
         }
         for (i32 pos = first; pos < end; pos += ONE_ROUND ? p.n_pclaims : 1) {
@@ -2178,6 +2269,7 @@ int launch_narrow(KParams& kp, bool one_round, int want_blocks, int sm_count, cu
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
     if (one_round) cbm_items_kernel<1, true, 4, kResident, RAGGED, true, true><<<blocks, 256, 0, s>>>(kp);
+    else if (kp.group == NARROW_ROWS) cbm_items_kernel<1, true, 4, kResident, RAGGED, true, false, true><<<blocks, 256, 0, s>>>(kp);
     else cbm_items_kernel<1, true, 4, kResident, RAGGED, true><<<blocks, 256, 0, s>>>(kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;

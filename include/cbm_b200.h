@@ -111,6 +111,11 @@ void cbm_b200_built_free(cbm_b200_built* b);
  * rows), and the output pointer addresses the shard: output row (label - own_begin); padding rows
  * of the output are never written.  own_begin = 0, own_end = n_labels computes everything.
  * `device` is the CUDA device ordinal that owns the plan.
+ *
+ * The halves of a product (cbm_b200_delta_spmm, cbm_b200_update) go by the tree as it is given.  The product in one pass
+ * may compute a row from all of its entries instead of from its parent's row, where the parent saves it few (see
+ * cbm_b200_schedule_lifted): the same sums in another order.  An infinity or NaN in a column that only the parent names then
+ * stays out of the row, as in A x; taken away again from the parent's row it leaves NaN there.
  * ------------------------------------------------------------------------------------------ */
 int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
                          const int32_t* delta_crow, const int32_t* delta_col,
