@@ -50,11 +50,150 @@ struct SearchParams {
     i64 out_cap;
     i32* skipped;         // parents left to the host (prefix too long for 16-bit counters)
     i32* n_skipped;
+    i32* large;           // parents whose prefix lists more rows than a warp's table takes
+    i32* n_large;
+    i32 n_blocks_of;      // parents in `large`, for the block's search
 };
 
 constexpr int kThreads = 512;
 constexpr int kMaxPrefix = 65000;
 
+// Shared columns that an edge u -> v needs, and the prefix of u's columns that guarantees `hits` of them.  More hits make
+// a longer prefix to count and leave fewer rows to intersect, the candidates are the same: 100 000 copy-model rows of 31
+// entries list 978 rows each with at least 8 hits and 640 with 4, and 0.4 and 2 of them pass; from 64 shared columns
+// on an eighth of them measured best.
+struct Need {
+    i32 need, hits, prefix;
+    bool none;  // no row can have that many
+};
+__device__ __forceinline__ Need need_of(i32 nu, i32 alpha) {
+    const i64 sum = (i64)nu + alpha;
+    const i64 half_floor = sum >= 0 ? sum / 2 : -((-sum + 1) / 2);
+    const i64 need64 = max(half_floor + 1, (i64)1);
+    Need r;
+    r.none = need64 > nu;
+    r.need = (i32)min(need64, (i64)INT32_MAX);
+    r.hits = min(r.need, max(4, min(32, r.need / 8)));
+    r.prefix = nu - r.need + r.hits;
+    return r;
+}
+
+// The search for a parent whose prefix lists few rows, by one warp: the rows are counted in a table in shared memory.  A
+// block to a parent spends its time between barriers there: 100 000 rows of 31 entries 2.5 ms, 1.1 for the nine tenths of them
+// that go here and 0.6 for the others, which are put on a list.
+constexpr int TABLE_BITS = 10, TABLE = 1 << TABLE_BITS, TABLE_TAKES = 704, TABLE_WARPS = 8;
+constexpr int TABLE_BYTES = TABLE * 4 + TABLE * 2;  // a row and a 16-bit count each
+
+__global__ void __launch_bounds__(TABLE_WARPS * 32) candidate_warp_kernel(const SearchParams p) {
+    constexpr int EACH = 4;
+    extern __shared__ i32 s_table[];
+    const int lane = threadIdx.x & 31;
+    i32* key = s_table + (threadIdx.x >> 5) * (TABLE_BYTES / 4);  // -1: free
+    u32* count = reinterpret_cast<u32*>(key + TABLE);             // two to a word
+    for (int i = lane; i < TABLE; i += 32) key[i] = -1;
+    for (int i = lane; i < TABLE / 2; i += 32) count[i] = 0;
+    __syncwarp();
+    for (;;) {
+        i32 u = 0;
+        if (lane == 0) u = (i32)min((u64)p.n, atomicAdd(p.out_count + 1, 1ULL));
+        u = __shfl_sync(0xffffffffu, u, 0);
+        if (u >= p.n) return;
+        const i64 ub = p.row_ptr[u];
+        const i32 nu = (i32)(p.row_ptr[u + 1] - ub);
+        const Need want = need_of(nu, p.alpha);
+        if (want.none) continue;
+        i64 listed = 0;
+        for (i32 i = lane; i < want.prefix && listed <= TABLE_TAKES; i += 32) {
+            const i32 c = p.row_rank[ub + i];
+            listed += p.col_ptr[c + 1] - p.col_ptr[c];
+        }
+        for (int d = 16; d; d >>= 1) listed += __shfl_xor_sync(0xffffffffu, listed, d);
+        if (listed > TABLE_TAKES) {
+            if (lane == 0) p.large[atomicAdd(p.n_large, 1)] = u;
+            continue;
+        }
+        // 32 lists at a time, end to end: lane k holds where the k-th begins and how much lies before it
+        for (i32 i0 = 0; i0 < want.prefix; i0 += 32) {
+            i64 qb = 0;
+            i32 len = 0;
+            if (i0 + lane < want.prefix) {
+                const i32 c = p.row_rank[ub + i0 + lane];
+                qb = p.col_ptr[c];
+                len = (i32)(p.col_ptr[c + 1] - qb);
+            }
+            i32 upto = len;
+            for (int d = 1; d < 32; d <<= 1) {
+                const i32 up = __shfl_up_sync(0xffffffffu, upto, d);
+                if (lane >= d) upto += up;
+            }
+            const i32 total = __shfl_sync(0xffffffffu, upto, 31);
+            for (i32 t0 = 0; t0 < total; t0 += 32 * EACH) {
+                i32 v[EACH];
+#pragma unroll
+                for (int e = 0; e < EACH; ++e) {  // all fetches before the first count
+                    const i32 t = t0 + 32 * e + lane;
+                    int k = 0;  // lists that end at or before t
+#pragma unroll
+                    for (int d = 16; d; d >>= 1)
+                        if (__shfl_sync(0xffffffffu, upto, k + d - 1) <= t) k += d;
+                    const i64 b = __shfl_sync(0xffffffffu, qb, k);
+                    const i32 before = __shfl_sync(0xffffffffu, upto - len, k);
+                    v[e] = t < total ? __ldg(p.col_rows + b + (t - before)) : -1;
+                }
+#pragma unroll
+                for (int e = 0; e < EACH; ++e) {
+                    if (v[e] < 0) continue;
+                    unsigned h = ((unsigned)v[e] * 2654435761u) >> (32 - TABLE_BITS);
+                    for (;;) {  // (there are free places)
+                        const i32 was = atomicCAS(key + h, -1, v[e]);
+                        if (was == -1 || was == v[e]) break;
+                        h = (h + 1) & (TABLE - 1);
+                    }
+                    atomicAdd(count + (h >> 1), (h & 1) ? 0x10000u : 1u);
+                }
+            }
+        }
+        __syncwarp();
+        const bool has_tail = want.prefix < nu;
+        for (int i = lane; i < TABLE; i += 32) {
+            const i32 mine = key[i], hits = (i32)((count[i >> 1] >> (16 * (i & 1))) & 0xffffu);
+            __syncwarp();  // (two lanes share a word of counts)
+            key[i] = -1;
+            if ((i & 1) == 0) count[i >> 1] = 0;
+            bool pass = mine >= 0 && mine != u && hits >= want.hits;
+            pass = pass && p.row_ptr[mine + 1] - p.row_ptr[mine] >= want.need;
+            for (unsigned m = __ballot_sync(0xffffffffu, pass); m; m &= m - 1) {
+                const int from = __ffs(m) - 1;
+                const i32 v = __shfl_sync(0xffffffffu, mine, from);
+                i32 both = __shfl_sync(0xffffffffu, hits, from);
+                const i64 vb = p.row_ptr[v];
+                const i32 nv = (i32)(p.row_ptr[v + 1] - vb);
+                if (has_tail) {  // the whole intersection: each of v's columns is looked for among u's
+                    i32 found = 0;
+                    for (i32 k = lane; k < nv; k += 32) {
+                        const i32 r = p.row_rank[vb + k];
+                        i32 lo = 0, hi = nu;
+                        while (lo < hi) {
+                            const i32 mid = (lo + hi) >> 1;
+                            if (p.row_rank[ub + mid] < r) lo = mid + 1;
+                            else hi = mid;
+                        }
+                        found += lo < nu && p.row_rank[ub + lo] == r;
+                    }
+                    both = (i32)__reduce_add_sync(0xffffffffu, (unsigned)found);
+                }
+                const i32 h = nu + nv - 2 * both;
+                if (h < nv - p.alpha && lane == 0) {  // cbm/cbm_extensions.cpp:93-101
+                    const u64 pos = atomicAdd(p.out_count, 1ULL);
+                    if ((i64)pos < p.out_cap) p.out[pos] = cbm::CandTriple{u, v, h};
+                }
+            }
+        }
+        __syncwarp();
+    }
+}
+
+// The search for the parents on the list, a block to each.
 __global__ void __launch_bounds__(kThreads) candidate_kernel(const SearchParams p) {
     __shared__ i32 s_u, s_touched, s_passed;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, n_warps = kThreads / 32;
@@ -63,22 +202,18 @@ __global__ void __launch_bounds__(kThreads) candidate_kernel(const SearchParams 
     u32* bitmap = p.bitmap + (i64)blockIdx.x * p.bitmap_stride;
     for (;;) {
         if (tid == 0) {
-            s_u = (i32)atomicAdd(p.out_count + 1, 1ULL);
+            const u64 t = atomicAdd(p.out_count + 1, 1ULL);
+            s_u = t < (u64)p.n_blocks_of ? p.large[t] : -1;
             s_touched = s_passed = 0;
         }
         __syncthreads();
         const i32 u = s_u;
-        if (u >= p.n) return;
+        if (u < 0) return;
         const i64 ub = p.row_ptr[u];
         const i32 nu = (i32)(p.row_ptr[u + 1] - ub);
-        // shared columns an edge u -> v needs, and the prefix that guarantees j_hits of them
-        const i64 sum = (i64)nu + p.alpha;
-        const i64 half_floor = sum >= 0 ? sum / 2 : -((-sum + 1) / 2);
-        const i64 need64 = max(half_floor + 1, (i64)1);
-        bool skip = need64 > nu;
-        const i32 need = (i32)min(need64, (i64)INT32_MAX);
-        const i32 j_hits = min(need, max(8, min(32, need / 8)));
-        const i32 plen = nu - need + j_hits;
+        const Need want = need_of(nu, p.alpha);
+        const i32 need = want.need, j_hits = want.hits, plen = want.prefix;
+        bool skip = want.none;
         if (!skip && plen > kMaxPrefix) {
             if (tid == 0) p.skipped[atomicAdd(p.n_skipped, 1)] = u;
             skip = true;
@@ -337,7 +472,8 @@ __global__ void __launch_bounds__(512) sort_rows_block_kernel(i32 n, const i64* 
     }
 }
 
-// Pieces of one allocation: a cudaMalloc and cudaFree for each array took longer than the search of a small graph.
+// Pieces of one allocation: a cudaMalloc and cudaFree take 0.3 ms each, whatever their size up to some 100 MB, and for each
+// array took longer than the search of a small graph.
 struct Arena {
     unsigned char* base = nullptr;
     size_t used = 0;
@@ -385,19 +521,21 @@ int gpu_candidates(int device, int32_t n, int32_t alpha, const int64_t* row_ptr,
     // rows of 265 entries, 16 a row were too few: 4.7 s instead of 1.9).
     p.out_cap = std::max<int64_t>({1ll << 20, 16ll * n, nnz / 2});
     Arena mem;
+    CandTriple* longer = nullptr;  // the list, where the first one was too short
     const size_t o_row_ptr = mem.plan<i64>((size_t)n + 1), o_col_ptr = mem.plan<i64>((size_t)n + 1);
     const size_t o_row_rank = mem.plan<i32>((size_t)nnz), o_rank = mem.plan<i32>((size_t)n), o_count_of_rank = mem.plan<i32>((size_t)n);
     const size_t tiles = ((size_t)n + 1 + SCAN_TILE - 1) / SCAN_TILE, o_totals = mem.plan<i64>(tiles), o_first = mem.plan<i64>((size_t)n + 2);
     const size_t o_col_rows = mem.plan<i32>((size_t)nnz), o_skipped = mem.plan<i32>((size_t)n);
-    const size_t o_touched = mem.plan<i32>((size_t)blocks * p.touched_stride);
-    const size_t o_zero = mem.used;  // cleared together: counters, hits, bitmaps
-    const size_t o_count = mem.plan<u64>(2), o_n_skipped = mem.plan<i32>(1);
+    const size_t o_large = mem.plan<i32>((size_t)n), o_out = mem.plan<CandTriple>((size_t)p.out_cap);
+    const size_t o_touched = mem.plan<i32>((size_t)blocks * p.touched_stride), o_hits = mem.plan<u32>((size_t)blocks * p.hits_stride);
+    const size_t o_zero = mem.used;  // cleared together: counters, counts, bitmaps
+    const size_t o_count = mem.plan<u64>(2), o_n_skipped = mem.plan<i32>(1), o_n_large = mem.plan<i32>(1);
     const size_t o_columns = mem.plan<i32>((size_t)n), o_often = mem.plan<i32>((size_t)n + 1);
     const size_t o_taken = mem.plan<i32>((size_t)n + 1), o_listed = mem.plan<i32>((size_t)n);
-    const size_t o_hits = mem.plan<u32>((size_t)blocks * p.hits_stride), o_bitmap = mem.plan<u32>((size_t)blocks * p.bitmap_stride);
+    const size_t o_bitmap = mem.plan<u32>((size_t)blocks * p.bitmap_stride);
     const size_t zero_bytes = mem.used - o_zero;
     auto cleanup = [&]() {
-        cudaFree(p.out);
+        cudaFree(longer);
         if (prev >= 0) cudaSetDevice(prev);
     };
     auto fail = [&](const char* what, cudaError_t ce) {
@@ -439,6 +577,9 @@ int gpu_candidates(int device, int32_t n, int32_t alpha, const int64_t* row_ptr,
     i32 *d_n_skipped = mem.at<i32>(o_n_skipped), *d_skipped = mem.at<i32>(o_skipped);
     p.hits = mem.at<u32>(o_hits);
     p.touched = mem.at<i32>(o_touched);
+    p.out = mem.at<CandTriple>(o_out);
+    p.large = mem.at<i32>(o_large);
+    p.n_large = mem.at<i32>(o_n_large);
     p.bitmap = mem.at<u32>(o_bitmap);
     p.row_ptr = mem.at<i64>(o_row_ptr);
     p.row_rank = mem.at<i32>(o_row_rank);
@@ -448,9 +589,13 @@ int gpu_candidates(int device, int32_t n, int32_t alpha, const int64_t* row_ptr,
     p.skipped = d_skipped;
     p.n_skipped = d_n_skipped;
     for (int attempt = 0; attempt < 2; ++attempt) {  // a second pass only if the output list was too small
-        if ((e = cudaMalloc((void**)&p.out, (size_t)p.out_cap * sizeof(CandTriple))) != cudaSuccess) return fail("out", e);
+        if (attempt > 0) {
+            if ((e = cudaMalloc((void**)&longer, (size_t)p.out_cap * sizeof(CandTriple))) != cudaSuccess) return fail("out", e);
+            p.out = longer;
+        }
         cudaMemset(d_count, 0, 2 * sizeof(u64));
         cudaMemset(d_n_skipped, 0, sizeof(i32));
+        cudaMemset(p.n_large, 0, sizeof(i32));
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         const bool trace = std::getenv("CBM_B200_BUILD_TRACE") != nullptr;
         if (trace) {
@@ -458,8 +603,18 @@ int gpu_candidates(int device, int32_t n, int32_t alpha, const int64_t* row_ptr,
             cudaEventCreate(&e1);
             cudaEventRecord(e0);
         }
-        candidate_kernel<<<blocks, kThreads>>>(p);
+        const int table_bytes = TABLE_WARPS * TABLE_BYTES;
+        if ((e = cudaFuncSetAttribute(candidate_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, table_bytes)) != cudaSuccess)
+            return fail("shared memory", e);
+        candidate_warp_kernel<<<std::min<int64_t>((int64_t)sms * 4, ((int64_t)n + TABLE_WARPS - 1) / TABLE_WARPS), TABLE_WARPS * 32, table_bytes>>>(p);
         if ((e = cudaGetLastError()) != cudaSuccess) return fail("launch", e);
+        if ((e = cudaMemcpy(&p.n_blocks_of, p.n_large, sizeof(i32), cudaMemcpyDeviceToHost)) != cudaSuccess) return fail("kernel", e);
+        if (p.n_blocks_of > 0) {
+            if ((e = cudaMemsetAsync(p.hits, 0, (size_t)blocks * p.hits_stride * sizeof(u32))) != cudaSuccess) return fail("device memory", e);
+            cudaMemsetAsync(d_count + 1, 0, sizeof(u64));
+            candidate_kernel<<<blocks, kThreads>>>(p);
+            if ((e = cudaGetLastError()) != cudaSuccess) return fail("launch", e);
+        }
         if (trace) cudaEventRecord(e1);
         if ((e = cudaDeviceSynchronize()) != cudaSuccess) return fail("kernel", e);
         if (trace) {
@@ -482,8 +637,6 @@ int gpu_candidates(int device, int32_t n, int32_t alpha, const int64_t* row_ptr,
             cleanup();
             return 0;
         }
-        cudaFree(p.out);
-        p.out = nullptr;
         p.out_cap = (int64_t)h_count[0] + 1024;  // the kernel counted every survivor: now it fits
     }
     err = "gpu_candidates: output list overflowed twice";

@@ -81,3 +81,18 @@ def test_rows_at_the_edges_of_the_sorts(lengths):
     key = np.unique(np.concatenate([v * n + p for v, p in enumerate(pattern)] + [np.array([n * n - 1])]))
     host, _ = _both(np.stack([key // n, key % n]), 0)
     assert host.build_info["depth"] > 1
+
+
+@pytest.mark.parametrize("group", [18, 29, 30, 31, 32, 33, 60])
+def test_parents_at_the_edge_of_a_warps_table(group):
+    """Groups of like rows whose prefixes list just as many rows as a warp counts in shared memory (704), some fewer and
+    some more (23 columns of 29 - 33 rows each); with 60 rows to a group all go to the blocks."""
+    rng = np.random.default_rng(group)
+    rows = []
+    for g in range(40):
+        common = np.arange(40) + 40 * g
+        rows += [np.delete(common, rng.integers(0, 40, rng.integers(0, 3))) for _ in range(group + g % 2)]
+    n = max(len(rows), 1600)  # (40 groups of 40 columns)
+    key = np.unique(np.concatenate([v * n + r for v, r in enumerate(rows)]))
+    host, _ = _both(np.stack([key // n, key % n]), 0)
+    assert host.build_info["depth"] > 2
