@@ -18,7 +18,8 @@
 // accumulators of 64 columns 128 -> 256 took 96 us.  The warps that add up and store are what a map waits for: 52 % of their
 // time went into adding, 34 - 49 % into storing.  So the next 8 columns leave tensor memory while 8 are added, and a
 // block of 32 x 32 sums that is all there is stored without a question about single values.  235 868 rows: 128 -> 256 126
-// -> 110 us, 256 -> 64 90 -> 85, 64 -> 256 masked 154 -> 137; 400 000 rows 256 -> 256 342 -> 314, 100 -> 256 194 -> 176.
+// -> 110 us, 256 -> 64 90 -> 85, 64 -> 256 masked 154 -> 137 (115 with the mask brought to L2 ahead); 400 000 rows 256 ->
+// 256 342 -> 314, 100 -> 256 194 -> 176.
 #include "cbm_map.cuh"
 
 #include <mutex>
@@ -320,6 +321,14 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                             x[b][i].w = fetch1(s + 3, in && left > 3);
                         }
                     }
+                }
+                // The next tile's mask is brought to L2 meanwhile, a row of this warp's columns by each lane: these fetches,
+                // which nothing is ahead of, took a trip to memory per tile (64 -> 256 masked 139 us, 115 with it).
+                {
+                    const int64_t row = (int64_t)(tile + (int)gridDim.y) * 128 + quarter * 32 + lane;
+                    const float* at = p.aux + row * p.ldaux + n0 + c_lo;
+                    if (row < p.m && n0 + c_lo < p.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+                    if (row < p.m && n0 + c_lo + 32 < p.n) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 32));
                 }
 #pragma unroll
                 for (int b = 0; b < 2; ++b) {
