@@ -19,8 +19,12 @@
 // time went into adding, 34 - 49 % into storing.  So the next 8 columns leave tensor memory while 8 are added, and a
 // block of 32 x 32 sums that is all there is stored without a question about single values.  235 868 rows: 128 -> 256 126
 // -> 110 us, 256 -> 64 90 -> 85, 64 -> 256 masked 154 -> 137 (115 with the mask brought to L2 ahead); 400 000 rows 256 ->
-// 256 342 -> 314, 100 -> 256 194 -> 176.
+// 256 342 -> 314, 100 -> 256 194 -> 176.  Where nothing masks the result, such a block leaves by one asynchronous copy of the
+// TMA unit, and the warp goes on to the next: 110 -> 102, 85 -> 81; 314 -> 310, 176 -> 155, 256 -> 47 151 -> 129 (of which
+// a step's MMAs issued as one 7).
 #include "cbm_map.cuh"
+
+#include <cuda.h>
 
 #include <mutex>
 #include <type_traits>
@@ -83,8 +87,10 @@ static_assert(PRODUCER_REGS > LAUNCH_REGS && EPILOGUE_REGS > LAUNCH_REGS && MMA_
               "setmaxnreg.inc and .dec only go up and down, within the registers of the launch");
 constexpr int SMEM_MAX = 192 * 1024;     // for the split weights
 constexpr int TURN_BYTES = 32 * 32 * 4;  // per epilogue warp
+constexpr int SMEM_ALL = SMEM_MAX + EPILOGUE_WARPS * TURN_BYTES + 1024;
 
 struct MapParams {
+    CUtensorMap store;  // d, in boxes of 32 x 32, 128-byte swizzled; used where `boxes` is set
     const float* a;    // [m, k]
     const float* b;    // [n, k], or [k, n] when B_TRANS
     float* d;          // [m, n]
@@ -96,8 +102,27 @@ struct MapParams {
     int steps;         // ceil(k / 16)
     int a_vec, d_vec, aux_vec;  // rows are 16-byte aligned
     int relu_in, relu_out, add; // max(a, 0) first; max(d, 0) last; d += instead of d =
+    int boxes, places;  // 32 x 32 places of shared memory for each warp: 1 or 2
     int* timeout;
 };
+
+// One 16-deep step, issued as one: the five small products, smallest first, the large one, and the arrival at `bar` once
+// they are done.  `b_term`: distance of B's terms, as descriptors count it.
+__device__ __forceinline__ void mma_step(u32 d, u32 a, u64 b, u64 b_term, u32 idesc, u32 bar) {
+    asm volatile(
+        "{\n\t.reg .pred e, no, yes;\n\t.reg .b64 b1, b2;\n\t.reg .b32 a1, a2;\n\t"
+        "elect.sync _|e, 0xffffffff;\n\tsetp.ne.u32 no, 0, 0;\n\tsetp.eq.u32 yes, 0, 0;\n\t"
+        "add.s64 b1, %2, %3;\n\tadd.s64 b2, b1, %3;\n\tadd.u32 a1, %1, 16;\n\tadd.u32 a2, %1, 32;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a2], %2, %4, no;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], b1, %4, yes;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b2, %4, yes;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], %2, %4, yes;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b1, %4, yes;\n\t"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, yes;\n\t"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t}" ::"r"(d),
+        "r"(a), "l"(b), "l"(b_term), "r"(idesc), "r"(bar)
+        : "memory");
+}
 
 __device__ __forceinline__ void ld8(float (&r)[8], u32 at) {
     asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -275,9 +300,7 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                     if (2 * c + s >= p.steps) break;
                     const u32 ds = it & 1, use = it >> 1, d = tmem + ds * D_COLS;
                     if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
-                    mma_small(d, a + 8 * s, b + 32 * s, term, idesc, false);
-                    mma(d, a + 8 * s, desc_of(b + 32 * s), idesc, true);
-                    commit(d_full + 8 * ds);
+                    mma_step(d, a + 8 * s, desc_of(b + 32 * s), (u64)(term >> 4), idesc, d_full + 8 * ds);
                     ++it;
                 }
                 if (ok) commit(a_empty + 8 * slot);
@@ -296,8 +319,9 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
         const int first_width = min(p.bn, (p.bn + 63) / 64 * 32);
         const int c_lo = half * first_width, width = half ? p.bn - first_width : first_width;
         const int row_in = quarter * 32 + (lane >> 3), col_in = c_lo + 4 * (lane & 7);
-        float4* mine = reinterpret_cast<float4*>(turn + (warp - PRODUCER_WARPS) * TURN_BYTES);
-        u32 it = 0;
+        float4* const mine0 = reinterpret_cast<float4*>(turn + (warp - PRODUCER_WARPS) * p.places * TURN_BYTES);
+        float4* mine = mine0;
+        u32 it = 0, boxed = 0;
         for (int tile = blockIdx.y; tile < p.row_tiles; tile += gridDim.y) {
             const int row0 = tile * 128 + row_in;
             // Of the mask only one bit per value is kept, fetched while the products of this tile are under way.
@@ -380,6 +404,39 @@ float r[2][8];
 #pragma unroll
             for (int b = 0; b < 2; ++b) {
                 if (32 * b >= width) break;
+                if (EXTRA == 0 && p.boxes) {
+                    // A box that holds these columns only, or ends past the last one, goes out by one asynchronous copy.  What
+                    // lay in its place before may still be on its way out: the place is free once that has been read.
+                    const bool box = 32 * b + 32 <= width || n0 + c_lo + width >= p.n;
+                    if (box && p.places == 2) {
+                        mine = mine0 + (boxed & 1) * (TURN_BYTES / 16);
+                        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    } else {
+                        mine = mine0;
+                        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+                    }
+                    __syncwarp();
+                    if (box) {
+                        ++boxed;
+#pragma unroll
+                        for (int j = 0; j < 8; ++j) {
+                            float4 y = make_float4(acc[b][4 * j], acc[b][4 * j + 1], acc[b][4 * j + 2], acc[b][4 * j + 3]);
+                            if (p.relu_out) y = relu(y);
+                            mine[lane * 8 + (j ^ (lane & 7))] = y;
+                        }
+                        fence_async();
+                        __syncwarp();
+                        const int row = tile * 128 + quarter * 32;
+                        if (lane == 0) {
+                            if (row < p.m)
+                                asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];" ::"l"(&p.store),
+                                             "r"(n0 + c_lo + 32 * b), "r"(row), "r"(smem_u32(mine))
+                                             : "memory");
+                            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+                        }
+                        continue;
+                    }
+                }
 #pragma unroll
                 for (int j = 0; j < 8; ++j)
                     mine[lane * 8 + (j ^ (lane & 7))] = make_float4(acc[b][4 * j], acc[b][4 * j + 1], acc[b][4 * j + 2], acc[b][4 * j + 3]);
@@ -435,10 +492,32 @@ float r[2][8];
         }
     }
 done:
+    if (EXTRA == 0 && p.boxes) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // before the memory they read is given up
     __syncwarp();
     fence_before();
     __syncthreads();
     if (warp == MMA_WARP) tmem_free(tmem);
+}
+
+// The map of d for asynchronous stores; false where the driver has none to offer.
+bool make_boxes(CUtensorMap* map, float* d, int64_t ldd, int m, int n) {
+    using Encode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
+                                const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+    static const Encode encode = [] {
+        void* fn = nullptr;
+        cudaDriverEntryPointQueryResult got;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &fn, cudaEnableDefault, &got) != cudaSuccess || got != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            fn = nullptr;
+        }
+        return reinterpret_cast<Encode>(fn);
+    }();
+    if (!encode || ldd * 4 >= (int64_t)1 << 40) return false;
+    const cuuint64_t size[2] = {(cuuint64_t)n, (cuuint64_t)m}, pitch[1] = {(cuuint64_t)ldd * 4};
+    const cuuint32_t box[2] = {32, 32}, step[2] = {1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 2, d, size, pitch, box, step, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
 bool aligned_rows(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && ld % 4 == 0; }
@@ -447,12 +526,12 @@ int round_up(int v, int to) { return (v + to - 1) / to * to; }
 
 template <bool B_TRANS, int EXTRA>
 int launch(const char* who, const MapParams& p, int sms, cudaStream_t stream) {
-    if (!allow_smem<map_kernel<B_TRANS, EXTRA>>(SMEM_MAX + EPILOGUE_WARPS * TURN_BYTES + 1024))
+    if (!allow_smem<map_kernel<B_TRANS, EXTRA>>(SMEM_ALL))
         return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": shared memory size refused");
     const int n_tiles = (p.n + p.bn - 1) / p.bn;
     const dim3 grid(n_tiles, std::max(1, std::min(p.row_tiles, sms / n_tiles)));
     // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
-    const int smem = std::max(3 * ((p.steps + 3) / 4) * p.bn * 128 + EPILOGUE_WARPS * TURN_BYTES + 1024, 120 * 1024);
+    const int smem = std::max(3 * ((p.steps + 3) / 4) * p.bn * 128 + p.places * EPILOGUE_WARPS * TURN_BYTES + 1024, 120 * 1024);
     map_kernel<B_TRANS, EXTRA><<<grid, THREADS, smem, stream>>>(p);
     if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
     return CBM_B200_OK;
@@ -498,6 +577,8 @@ int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_
         p.relu_in = relu_in;
         p.relu_out = relu_out && last;
         p.add = k0 > 0;
+        p.places = 3 * ((p.steps + 3) / 4) * bn * 128 + 2 * EPILOGUE_WARPS * TURN_BYTES + 1024 <= SMEM_ALL ? 2 : 1;
+        p.boxes = p.d_vec && passes == 1 && !aux && make_boxes(&p.store, d, ldd, m, n);
         if (aux) {
             p.aux = aux;
             p.ldaux = ldaux;
