@@ -1787,45 +1787,56 @@ int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vect
     return validate_schedule(sch, own_end - own_begin);
 }
 
+// Runs both, side by side if `wide` and a thread can be had, and lets the first one's exception out before the other's.
+template <class F, class G>
+void run_both(bool wide, F first, G second) {
+    std::exception_ptr first_thrown, second_thrown;
+    const auto guarded_second = [&] {
+        try {
+            second();
+        } catch (...) {
+            second_thrown = std::current_exception();
+        }
+    };
+    std::thread beside;
+    if (wide) {
+        try {
+            beside = std::thread(guarded_second);
+        } catch (const std::system_error&) {  // no thread to be had
+        }
+    }
+    try {
+        first();
+    } catch (...) {
+        first_thrown = std::current_exception();
+    }
+    if (beside.joinable()) beside.join();
+    else if (!first_thrown) guarded_second();
+    if (first_thrown) std::rethrow_exception(first_thrown);
+    if (second_thrown) std::rethrow_exception(second_thrown);
+}
+
 // The structure's own schedule, and the one with rows lifted out of the tree where that pays.
 int build_schedules(const Structure& st, const Rules& rules, Schedule& tree, Schedule& lifted) {
     cbm::Lifted lift;
     std::vector<i32> rank;
-    if (!st.csr) cbm::lift_rows(st.n, st.rows, st.parent, st.level, st.crow, st.col, st.val, lift);
-    cluster_order(st, rules, rank);
+    const bool wide = st.crow[st.n] > 1000000;  // steps of milliseconds
+    run_both(
+        wide, [&] { cluster_order(st, rules, rank); },
+        [&] {
+            if (!st.csr) cbm::lift_rows(st.n, st.rows, st.parent, st.level, st.crow, st.col, st.val, lift);
+        });
     if (lift.n_lifted == 0) return build_schedule(st, nullptr, rank, rules, tree);
-    // side by side where they take milliseconds
-    int rc = CBM_B200_OK;
-    std::string what;
-    std::exception_ptr thrown;
-    auto other = [&] {
-        try {
-            rc = build_schedule(st, &lift, rank, rules, lifted);
-            if (rc) what = cbm::last_error_slot();
-        } catch (...) {
-            thrown = std::current_exception();
-        }
-    };
-    std::thread beside;
-    if (lift.n_entries > 1000000) {
-        try {
-            beside = std::thread(other);
-        } catch (const std::system_error&) {  // no thread to be had
-        }
-    }
-    int own = CBM_B200_OK;
-    std::exception_ptr own_thrown;
-    try {
-        own = build_schedule(st, nullptr, rank, rules, tree);
-    } catch (...) {
-        own_thrown = std::current_exception();
-    }
-    if (beside.joinable()) beside.join();
-    else if (own == CBM_B200_OK && !own_thrown) other();
-    if (own_thrown) std::rethrow_exception(own_thrown);
-    if (own) return own;
-    if (thrown) std::rethrow_exception(thrown);
-    return rc ? cbm::fail(rc, what) : CBM_B200_OK;
+    int rc = CBM_B200_OK, rc_lifted = CBM_B200_OK;
+    std::string what;  // (the message of an error belongs to its thread)
+    run_both(
+        wide, [&] { rc = build_schedule(st, nullptr, rank, rules, tree); },
+        [&] {
+            rc_lifted = build_schedule(st, &lift, rank, rules, lifted);
+            if (rc_lifted) what = cbm::last_error_slot();
+        });
+    if (rc) return rc;
+    return rc_lifted ? cbm::fail(rc_lifted, what) : CBM_B200_OK;
 }
 
 }  // namespace

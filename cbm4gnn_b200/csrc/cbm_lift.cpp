@@ -78,11 +78,11 @@ void lift_rows(i32 n, const std::vector<i32>& order, const std::vector<i32>& par
     i64 least = 0, limit = NEVER;
     std::vector<i32> lev((size_t)n + 1, 0), needed((size_t)n, -1);
     i32 round = 0;
+    for (i32 k = 0; k < first; ++k) lev[order[k]] = 1;
     for (const i64 s : {NEVER, (i64)0, (i64)4, (i64)8, (i64)16, (i64)32, (i64)64, (i64)128, ALL}) {
         i64 extra = 0, waits = 0, buffer = 0;
         i32 depth = 1;
         ++round;
-        for (i32 k = 0; k < first; ++k) lev[order[k]] = 1;
         for (i32 k = first; k < rows; ++k) {
             const i32 v = order[k];
             if (lifts(v, s)) {
@@ -125,19 +125,27 @@ void lift_rows(i32 n, const std::vector<i32>& order, const std::vector<i32>& par
         }
     out.col.resize((size_t)room);
     out.val.resize((size_t)room);
-    for (i32 k = first; k < rows; ++k) {
-        const i32 v = order[k], u = parent[v];
-        if (place[v] < 0) continue;
-        const bool top = parent[u] == n;
-        const i32* pc = top ? col + crow[u] : out.col.data() + place[u];
-        const float* pv = top ? val + crow[u] : out.val.data() + place[u];
-        bool ascending = true;
-        for (i64 e = 1; top && e < whole[u]; ++e) ascending = ascending && pc[e - 1] < pc[e];
-        if (!ascending || !merge(pc, pv, whole[u], col + crow[v], val + crow[v], crow[v + 1] - crow[v], out.col.data() + place[v],
-                                 out.val.data() + place[v], whole[v])) {
-            out = Lifted();
-            return;
+    // level by level: a level's rows need only those above them
+    bool whole_rows = true;
+    for (i32 k0 = first, k1; k0 < rows && whole_rows; k0 = k1) {
+        for (k1 = k0; k1 < rows && level[order[k1]] == level[order[k0]];) ++k1;
+#pragma omp parallel for schedule(dynamic, 256) reduction(&& : whole_rows) if (k1 - k0 > 4096)
+        for (i32 k = k0; k < k1; ++k) {
+            const i32 v = order[k], u = parent[v];
+            if (place[v] < 0) continue;
+            const bool top = parent[u] == n;
+            const i32* pc = top ? col + crow[u] : out.col.data() + place[u];
+            const float* pv = top ? val + crow[u] : out.val.data() + place[u];
+            bool ascending = true;
+            for (i64 e = 1; top && e < whole[u]; ++e) ascending = ascending && pc[e - 1] < pc[e];
+            whole_rows = whole_rows && ascending &&
+                         merge(pc, pv, whole[u], col + crow[v], val + crow[v], crow[v + 1] - crow[v], out.col.data() + place[v],
+                               out.val.data() + place[v], whole[v]);
         }
+    }
+    if (!whole_rows) {
+        out = Lifted();
+        return;
     }
     out.parent = parent;
     out.level = level;
