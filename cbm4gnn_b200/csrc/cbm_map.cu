@@ -21,7 +21,7 @@
 // -> 110 us, 256 -> 64 90 -> 85, 64 -> 256 masked 154 -> 137 (115 with the mask brought to L2 ahead); 400 000 rows 256 ->
 // 256 342 -> 314, 100 -> 256 194 -> 176.  Where nothing masks the result, such a block leaves by one asynchronous copy of the
 // TMA unit, and the warp goes on to the next: 110 -> 102, 85 -> 81; 314 -> 310, 176 -> 155, 256 -> 47 151 -> 129 (of which
-// a step's MMAs issued as one 7).
+// a step's MMAs issued as one 7).  Narrow tiles: see PAIR.
 #include "cbm_map.cuh"
 
 #include <cuda.h>
@@ -106,8 +106,9 @@ struct MapParams {
     int* timeout;
 };
 
-// One 16-deep step, issued as one: the five small products, smallest first, the large one, and the arrival at `bar` once
-// they are done.  `b_term`: distance of B's terms, as descriptors count it.
+// One 16-deep step, issued as one: the five small products, smallest first, and the large one; then the arrival at `bar`
+// once they are done.  `b_term`: distance of B's terms, as descriptors count it.
+template <bool ARRIVE>
 __device__ __forceinline__ void mma_step(u32 d, u32 a, u64 b, u64 b_term, u32 idesc, u32 bar) {
     asm volatile(
         "{\n\t.reg .pred e, no, yes;\n\t.reg .b64 b1, b2;\n\t.reg .b32 a1, a2;\n\t"
@@ -119,9 +120,10 @@ __device__ __forceinline__ void mma_step(u32 d, u32 a, u64 b, u64 b_term, u32 id
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [a1], %2, %4, yes;\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], b1, %4, yes;\n\t"
         "@e tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %4, yes;\n\t"
-        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%5];\n\t}" ::"r"(d),
-        "r"(a), "l"(b), "l"(b_term), "r"(idesc), "r"(bar)
+        "}" ::"r"(d),
+        "r"(a), "l"(b), "l"(b_term), "r"(idesc)
         : "memory");
+    if (ARRIVE) commit(bar);
 }
 
 __device__ __forceinline__ void ld8(float (&r)[8], u32 at) {
@@ -130,8 +132,11 @@ __device__ __forceinline__ void ld8(float (&r)[8], u32 at) {
                  : "r"(at));
 }
 
+// PAIR, for tiles of up to 64 columns: an accumulator's place holds two, those of a chunk's two steps, which go from the MMA
+// warp to the sum warps and back together.  What bounds a narrow tile is that way, whatever is left out of the rest (256 ->
+// 47: 130 us without the fetches, without the stores or with one product of six): 129 -> 115 us, 256 -> 64 82 -> 74.
 // EXTRA: 0 plain, 1 with a mask, 2 with any of a mask and earlier passes' results to add to.
-template <bool B_TRANS, int EXTRA>
+template <bool B_TRANS, int EXTRA, bool PAIR>
 __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__ MapParams p) {
     extern __shared__ unsigned char smem_raw[];
     __shared__ u64 s_bar[2 * A_SLOTS + 5];  // A full x4, A empty x4, accumulator full x2, accumulator empty x2, drained
@@ -295,12 +300,22 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
                 const u32 slot = run % A_SLOTS, a = tmem + A_COL + slot * A_SLOT_COLS;
                 const u32 b = b0 + (u32)(c >> 1) * block + 64 * (c & 1);
                 if (!(ok = warp_wait(a_full + 8 * slot, (run / A_SLOTS) & 1, gave_up, p.timeout))) break;
+                if constexpr (PAIR) {
+                    const u32 ds = it & 1, use = it >> 1, d = tmem + ds * D_COLS;
+                    if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
+                    mma_step<false>(d, a, desc_of(b), (u64)(term >> 4), idesc, 0);
+                    if (2 * c + 1 < p.steps) mma_step<false>(d + D_COLS / 2, a + 8, desc_of(b + 32), (u64)(term >> 4), idesc, 0);
+                    commit(d_full + 8 * ds);
+                    commit(a_empty + 8 * slot);
+                    ++it;
+                    continue;
+                }
 #pragma unroll
                 for (int s = 0; s < 2; ++s) {
                     if (2 * c + s >= p.steps) break;
                     const u32 ds = it & 1, use = it >> 1, d = tmem + ds * D_COLS;
                     if (use > 0 && !(ok = warp_wait(d_empty + 8 * ds, (use + 1) & 1, gave_up, p.timeout))) break;
-                    mma_step(d, a + 8 * s, desc_of(b + 32 * s), (u64)(term >> 4), idesc, d_full + 8 * ds);
+                    mma_step<true>(d, a + 8 * s, desc_of(b + 32 * s), (u64)(term >> 4), idesc, d_full + 8 * ds);
                     ++it;
                 }
                 if (ok) commit(a_empty + 8 * slot);
@@ -368,8 +383,9 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
             }
             // The first step sets the sums, the others add to them (told apart at compile time: the sums must not
             // be live while the mask is fetched).
-            float acc[2][32];
-            auto collect = [&](auto first) -> bool {
+            constexpr int BLOCKS = PAIR ? 1 : 2;  // of 32 columns
+            float acc[BLOCKS][32];
+            auto collect = [&](auto first, bool second) -> bool {
                 const u32 ds = it & 1, use = it >> 1;
                 if (!warp_wait(d_full + 8 * ds, use & 1, gave_up, p.timeout)) return false;
                 const u32 at = tmem + ds * D_COLS + c_lo + ((u32)(quarter * 32) << 16);
@@ -377,14 +393,16 @@ float r[2][8];
                 ld8(r[0], at);
 #pragma unroll
                 for (int q = 0; q < 8; ++q) {  // the next 8 columns are on their way while these are added
+                    const bool more = PAIR ? (q != 3 || second) : 8 * (q + 1) < width;
+                    if (PAIR && q == 4 && !second) break;
                     wait_ld();
 #pragma unroll
                     for (int i = 0; i < 8; ++i) asm volatile("" : "+f"(r[q & 1][i]));  // not before the wait
-                    if (q < 7 && 8 * (q + 1) < width) ld8(r[(q + 1) & 1], at + 8 * (q + 1));
+                    if (q < 7 && more) ld8(r[(q + 1) & 1], PAIR && q >= 3 ? at + D_COLS / 2 + 8 * (q - 3) : at + 8 * (q + 1));
 #pragma unroll
                     for (int i = 0; i < 8; i += 2) {
-                        float &s = acc[q >> 2][8 * (q & 3) + i], &t = acc[q >> 2][8 * (q & 3) + i + 1];
-                        if constexpr (decltype(first)::value) {
+                        float &s = acc[PAIR ? 0 : q >> 2][8 * (q & 3) + i], &t = acc[PAIR ? 0 : q >> 2][8 * (q & 3) + i + 1];
+                        if (decltype(first)::value && !(PAIR && q >= 4)) {
                             s = r[q & 1][i];
                             t = r[q & 1][i + 1];
                         } else {
@@ -398,16 +416,24 @@ float r[2][8];
                 ++it;
                 return true;
             };
-            if (!collect(std::true_type{})) goto done;
-            for (int s = 1; s < p.steps; ++s)
-                if (!collect(std::false_type{})) goto done;
+            if constexpr (PAIR) {
+                if (!collect(std::true_type{}, p.steps > 1)) goto done;
+                for (int s = 2; s < p.steps; s += 2)
+                    if (!collect(std::false_type{}, s + 1 < p.steps)) goto done;
+            } else {
+                if (!collect(std::true_type{}, false)) goto done;
+                for (int s = 1; s < p.steps; ++s)
+                    if (!collect(std::false_type{}, false)) goto done;
+            }
 #pragma unroll
-            for (int b = 0; b < 2; ++b) {
+            for (int b = 0; b < BLOCKS; ++b) {
                 if (32 * b >= width) break;
                 if (EXTRA == 0 && p.boxes) {
-                    // A box that holds these columns only, or ends past the last one, goes out by one asynchronous copy.  What
-                    // lay in its place before may still be on its way out: the place is free once that has been read.
-                    const bool box = 32 * b + 32 <= width || n0 + c_lo + width >= p.n;
+                    // A box that holds these columns only, or that the last column cuts off, goes out by one asynchronous copy.
+                    // (What is cut off is cut at 16 bytes: a width that ends elsewhere leaves its last block value by value.)
+                    // What lay in its place before may still be on its way out: the place is free once that has been read.
+                    const bool whole = 32 * b + 32 <= width && n0 + c_lo + 32 * b + 32 <= p.n;
+                    const bool box = whole || (p.n % 4 == 0 && n0 + c_lo + width >= p.n);
                     if (box && p.places == 2) {
                         mine = mine0 + (boxed & 1) * (TURN_BYTES / 16);
                         if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
@@ -524,17 +550,22 @@ bool aligned_rows(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_
 
 int round_up(int v, int to) { return (v + to - 1) / to * to; }
 
-template <bool B_TRANS, int EXTRA>
-int launch(const char* who, const MapParams& p, int sms, cudaStream_t stream) {
-    if (!allow_smem<map_kernel<B_TRANS, EXTRA>>(SMEM_ALL))
+template <bool B_TRANS, int EXTRA, bool PAIR>
+int launch_form(const char* who, const MapParams& p, int sms, cudaStream_t stream) {
+    if (!allow_smem<map_kernel<B_TRANS, EXTRA, PAIR>>(SMEM_ALL))
         return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": shared memory size refused");
     const int n_tiles = (p.n + p.bn - 1) / p.bn;
     const dim3 grid(n_tiles, std::max(1, std::min(p.row_tiles, sms / n_tiles)));
     // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
     const int smem = std::max(3 * ((p.steps + 3) / 4) * p.bn * 128 + p.places * EPILOGUE_WARPS * TURN_BYTES + 1024, 120 * 1024);
-    map_kernel<B_TRANS, EXTRA><<<grid, THREADS, smem, stream>>>(p);
+    map_kernel<B_TRANS, EXTRA, PAIR><<<grid, THREADS, smem, stream>>>(p);
     if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
     return CBM_B200_OK;
+}
+
+template <bool B_TRANS, int EXTRA>
+int launch(const char* who, const MapParams& p, int sms, cudaStream_t stream) {
+    return p.bn <= 64 ? launch_form<B_TRANS, EXTRA, true>(who, p, sms, stream) : launch_form<B_TRANS, EXTRA, false>(who, p, sms, stream);
 }
 
 // d [m, n] = a [m, k] b^T, b [n, k] (b_trans: [k, n]).
@@ -578,7 +609,8 @@ int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_
         p.relu_out = relu_out && last;
         p.add = k0 > 0;
         p.places = 3 * ((p.steps + 3) / 4) * bn * 128 + 2 * EPILOGUE_WARPS * TURN_BYTES + 1024 <= SMEM_ALL ? 2 : 1;
-        p.boxes = p.d_vec && passes == 1 && !aux && make_boxes(&p.store, d, ldd, m, n);
+        // (a map of the result takes the host 2 us, and a block that has one tile has nothing to go on to)
+        p.boxes = p.d_vec && passes == 1 && !aux && row_tiles >= sms && make_boxes(&p.store, d, ldd, m, n);
         if (aux) {
             p.aux = aux;
             p.ldaux = ldaux;

@@ -2,7 +2,7 @@
 import pytest
 import torch
 
-from cbm4gnn_b200 import dense, stack
+from cbm4gnn_b200 import _lib, dense, stack
 from cbm4gnn_b200.gcn import GCNModel
 
 pytestmark = pytest.mark.gpu
@@ -212,3 +212,22 @@ def test_narrow_products_are_contiguous(width, listed_bytes, monkeypatch):
     want, = torch.autograd.grad(h @ model.layers[1].lin.weight.double().t(), x, torch.ones(50, 5, device="cuda").double())
     torch.testing.assert_close(gx, want, atol=1e-5, rtol=1e-5)
     assert model.layers[0].cached_a_t.matmul(x).is_contiguous()
+
+
+@pytest.mark.parametrize("n,n_in,n_out", [(18944, 16, 4), (18945, 17, 33), (18975, 40, 47), (19000, 64, 48), (20001, 33, 64), (19071, 100, 100),
+                                          (19072, 16, 112), (19073, 64, 200), (18816, 31, 256), (38000, 70, 96)])
+@pytest.mark.parametrize("relu", [False, True])
+def test_results_go_out_in_boxes_and_value_by_value_alike(n, n_in, n_out, relu):
+    """From a tile for every SM on (148 x 128 rows) rows that are 16-byte aligned leave in boxes of 32 x 32 (cut off at the
+    last row and column), others value by value: the same bits, and nothing beside the columns is written."""
+    x, w = _operand(n, n_in, 0, 1), _operand(n_out, n_in, 0, 2)
+    fn = _lib.lib().cbm_b200_dense_forward_relu if relu else _lib.lib().cbm_b200_dense_forward
+    got = []
+    for pitch in (-(-n_out // 4) * 4 + 4, -(-n_out // 4) * 4 + 1):
+        room = torch.full((n + 1, pitch), 7.0, device="cuda")
+        _lib.check(fn(x.data_ptr(), n_in, w.data_ptr(), n_in, room.data_ptr(), pitch, n, n_in, n_out,
+                      torch.cuda.current_stream().cuda_stream))
+        assert torch.all(room[:n, n_out:] == 7.0) and torch.all(room[n] == 7.0)
+        got.append(room[:n, :n_out])
+    assert torch.equal(*got)
+    _close(got[0], x, w.t()) if not relu else None
