@@ -35,6 +35,7 @@ HEADERS = [
     os.path.join(_PKG_DIR, "csrc", "cbm_candidates.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_chunks.cuh"),
     os.path.join(_PKG_DIR, "csrc", "cbm_cluster.h"),
+    os.path.join(_PKG_DIR, "csrc", "cbm_launch.cuh"),
     os.path.join(_PKG_DIR, "csrc", "cbm_lift.h"),
     os.path.join(_PKG_DIR, "csrc", "cbm_map.cuh"),
 ]

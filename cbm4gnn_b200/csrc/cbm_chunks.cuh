@@ -89,6 +89,7 @@ constexpr int STAGE_BYTES = DESC_BYTES + CHUNK_ENTRIES * (int)sizeof(Entry);
 
 template <bool RAGGED, int UNROLL, int MINB>
 __global__ void __launch_bounds__((CONSUMERS + 1) * 32, MINB) cbm_chunks_kernel(const __grid_constant__ KParams p) {
+    cbm::wait_before();
     using V = Vec<true>;
     __shared__ __align__(128) unsigned char smem[STAGES * STAGE_BYTES];  // descriptors, entries of each stage
     __shared__ u64 s_bar[2 * STAGES];                                    // full, then empty

@@ -38,6 +38,7 @@
 #include "cbm_b200.h"
 #include "cbm_cluster.h"
 #include "cbm_common.h"
+#include "cbm_launch.cuh"
 #include "cbm_lift.h"
 
 namespace cbm {
@@ -186,15 +187,15 @@ struct Vec<true> {
     using T = float4;
     static constexpr int E = 4;
     static __device__ __forceinline__ T zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-    // Read-only fetch that is skipped (giving zeros) when `on` is false.  Written as volatile asm
-    // so that a batch of fetches stays a batch: the compiler may not sink one below its use.
+    // Fetch of the operand that is skipped (giving zeros) when `on` is false.  Written as volatile asm
+    // so that a batch of fetches stays a batch: the compiler may not sink one below its use.  (Not ld.global.nc: see cbm_launch.cuh.)
     static __device__ __forceinline__ T ld_ro_if(const float* p, bool on) {
         T v;
         asm volatile(
             "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
             "mov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
             "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t"
-            "@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+            "@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
             : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
             : "l"(p), "r"((int)on));
         return v;
@@ -202,7 +203,7 @@ struct Vec<true> {
     // The same fetch without the predicate, for slabs in which every lane has columns.
     static __device__ __forceinline__ T ld_ro(const float* p) {
         T v;
-        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
                      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                      : "l"(p));
         return v;
@@ -278,14 +279,14 @@ struct Vec<false> {
         T v;
         asm volatile(
             "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t"
-            "@q ld.global.nc.f32 %0, [%1];\n\t}"
+            "@q ld.global.f32 %0, [%1];\n\t}"
             : "=f"(v)
             : "l"(p), "r"((int)on));
         return v;
     }
     static __device__ __forceinline__ T ld_ro(const float* p) {
         T v;
-        asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+        asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
         return v;
     }
     static __device__ __forceinline__ T ld_l2(const float* p) { return __ldcg(p); }
@@ -759,6 +760,7 @@ __device__ __forceinline__ i32 rows_narrow_staged(const KParams& p, NarrowClaim&
 // NARROW: every slab is at most 64 columns wide; STAGED: and claims are of up to 8 rows in community order.
 template <int NV, bool V4, int UNROLL, int MINB, bool RAGGED = false, bool NARROW = false, bool ONE_ROUND = false, bool STAGED = false>
 __global__ void __launch_bounds__(256, MINB) cbm_items_kernel(const __grid_constant__ KParams p) {
+    cbm::wait_before();
     using V = Vec<V4>;
     using T = typename V::T;
     constexpr int STEP = 32 * V::E;
@@ -2264,8 +2266,8 @@ int launch_regs(KParams& kp, bool one_round, int want_blocks, int sm_count, cuda
     int blocks = want_blocks > 0 ? want_blocks : sm_count * (NV == 1 && V4 ? kResident : 8);
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
-    if (one_round) cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED, false, true><<<blocks, 256, 0, s>>>(kp);
-    else cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED><<<blocks, 256, 0, s>>>(kp);
+    if (one_round) cbm::launch_next(cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED, false, true>, blocks, 256, 0, s, kp);
+    else cbm::launch_next(cbm_items_kernel<NV, V4, kUnroll, kResident, RAGGED>, blocks, 256, 0, s, kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;
 }
@@ -2279,9 +2281,9 @@ int launch_narrow(KParams& kp, bool one_round, int want_blocks, int sm_count, cu
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
     kp.n_warps = (u64)blocks * 8;
-    if (one_round) cbm_items_kernel<1, true, 4, kResident, RAGGED, true, true><<<blocks, 256, 0, s>>>(kp);
-    else if (kp.group == NARROW_ROWS) cbm_items_kernel<1, true, 4, kResident, RAGGED, true, false, true><<<blocks, 256, 0, s>>>(kp);
-    else cbm_items_kernel<1, true, 4, kResident, RAGGED, true><<<blocks, 256, 0, s>>>(kp);
+    if (one_round) cbm::launch_next(cbm_items_kernel<1, true, 4, kResident, RAGGED, true, true>, blocks, 256, 0, s, kp);
+    else if (kp.group == NARROW_ROWS) cbm::launch_next(cbm_items_kernel<1, true, 4, kResident, RAGGED, true, false, true>, blocks, 256, 0, s, kp);
+    else cbm::launch_next(cbm_items_kernel<1, true, 4, kResident, RAGGED, true>, blocks, 256, 0, s, kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;
 }
@@ -2292,25 +2294,25 @@ int launch_chunks(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, kp.n_claims));
     kp.n_warps = (u64)blocks;  // one claimer per block
-    cbm_chunks_kernel<RAGGED, 4, kResident><<<blocks, (CONSUMERS + 1) * 32, 0, s>>>(kp);
+    cbm::launch_next(cbm_chunks_kernel<RAGGED, 4, kResident>, blocks, (CONSUMERS + 1) * 32, 0, s, kp);
     CBM_CUDA(cudaGetLastError());
     return CBM_B200_OK;
 }
 
 // Rows of `f` floats copied to rows of 4 * vecs floats, zero-filled: one thread per vector of the result, the
 // source read 4 bytes at a time (its rows are not aligned).  Bound by HBM.
-__global__ void __launch_bounds__(256) pack_rows_kernel(const float* __restrict__ x, i64 ldx, float* __restrict__ out,
-                                                        i32 f, i32 vecs, i64 n_vec) {
+__global__ void __launch_bounds__(256) pack_rows_kernel(const float* x, i64 ldx, float* out, i32 f, i32 vecs, i64 n_vec) {
+    cbm::wait_before();
     const i64 i = (i64)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_vec) return;
     const i64 row = i / vecs;
     const i32 c = (i32)(i - row * vecs) * 4;
     const float* r = x + row * ldx + c;
     float4 v;
-    v.x = __ldg(r);
-    v.y = c + 1 < f ? __ldg(r + 1) : 0.f;
-    v.z = c + 2 < f ? __ldg(r + 2) : 0.f;
-    v.w = c + 3 < f ? __ldg(r + 3) : 0.f;
+    v.x = r[0];
+    v.y = c + 1 < f ? r[1] : 0.f;
+    v.z = c + 2 < f ? r[2] : 0.f;
+    v.w = c + 3 < f ? r[3] : 0.f;
     reinterpret_cast<float4*>(out)[i] = v;
 }
 
@@ -2426,7 +2428,7 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
         const i32 vecs = (f + 3) / 4;
         const i64 n_vec = (i64)p->n_labels * vecs;
         if ((rc = grow(p, p->d_pack, p->pack_cap, 4 * n_vec, false, s))) return rc;
-        pack_rows_kernel<<<(unsigned)((n_vec + 255) / 256), 256, 0, s>>>(x, ldx, p->d_pack, f, vecs, n_vec);
+        cbm::launch_next(pack_rows_kernel, (unsigned)((n_vec + 255) / 256), 256, 0, s, x, ldx, p->d_pack, f, vecs, n_vec);
         CBM_CUDA(cudaGetLastError());
         x = p->d_pack;
         ldx = 4 * (i64)vecs;

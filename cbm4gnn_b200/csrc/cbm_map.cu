@@ -22,6 +22,7 @@
 // 256 342 -> 314, 100 -> 256 194 -> 176.  Where nothing masks the result, such a block leaves by one asynchronous copy of the
 // TMA unit, and the warp goes on to the next: 110 -> 102, 85 -> 81; 314 -> 310, 176 -> 155, 256 -> 47 151 -> 129 (of which
 // a step's MMAs issued as one 7).  Narrow tiles: see PAIR.
+#include "cbm_launch.cuh"
 #include "cbm_map.cuh"
 
 #include <cuda.h>
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(THREADS, 1) map_kernel(const __grid_constant__
         s_gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    cbm::wait_before();
     // The weights, split, into shared memory: two pieces of 8 values a thread at a time, so that their fetches overlap.
     const int k8s = 2 * p.steps, pieces = p.bn * k8s;
     const bool b_vec = !B_TRANS && p.ldb % 4 == 0 && (reinterpret_cast<u64>(p.b) & 15) == 0;
@@ -558,7 +560,7 @@ int launch_form(const char* who, const MapParams& p, int sms, cudaStream_t strea
     const dim3 grid(n_tiles, std::max(1, std::min(p.row_tiles, sms / n_tiles)));
     // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
     const int smem = std::max(3 * ((p.steps + 3) / 4) * p.bn * 128 + p.places * EPILOGUE_WARPS * TURN_BYTES + 1024, 120 * 1024);
-    map_kernel<B_TRANS, EXTRA, PAIR><<<grid, THREADS, smem, stream>>>(p);
+    cbm::launch_next(map_kernel<B_TRANS, EXTRA, PAIR>, grid, THREADS, smem, stream, p);
     if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
     return CBM_B200_OK;
 }

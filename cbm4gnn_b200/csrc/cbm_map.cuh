@@ -165,12 +165,13 @@ __device__ __forceinline__ void mma_small(u32 d, u32 a, u32 b, u32 b_term, u32 i
 }
 
 // ---- operands -----------------------------------------------------------------------------------
-// Read-only fetches, zero where `on` is false.  Written as volatile asm so that a batch of fetches stays a batch,
-// ahead of the work it is meant to hide behind: the compiler may not sink one to its use.
+// Fetches, zero where `on` is false.  Written as volatile asm so that a batch of fetches stays a batch,
+// ahead of the work it is meant to hide behind: the compiler may not sink one to its use.  (Not
+// ld.global.nc: see cbm_launch.cuh.)
 __device__ __forceinline__ float fetch1(const float* p, bool on) {
     float v;
     asm volatile(
-        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.nc.f32 %0, [%1];\n\t}"
+        "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\tmov.f32 %0, 0f00000000;\n\t@q ld.global.f32 %0, [%1];\n\t}"
         : "=f"(v)
         : "l"(p), "r"((int)on));
     return v;
@@ -179,7 +180,7 @@ __device__ __forceinline__ float4 fetch4(const float* p, bool on) {
     float4 v;
     asm volatile(
         "{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\tmov.f32 %0, 0f00000000;\n\tmov.f32 %1, 0f00000000;\n\t"
-        "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@q ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
+        "mov.f32 %2, 0f00000000;\n\tmov.f32 %3, 0f00000000;\n\t@q ld.global.v4.f32 {%0, %1, %2, %3}, [%4];\n\t}"
         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
         : "l"(p), "r"((int)on));
     return v;

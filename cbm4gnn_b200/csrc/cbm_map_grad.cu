@@ -15,6 +15,7 @@
 // are brought to L2 AHEAD chunks early.  With three warps for the second operand they were what everyone waited for (the
 // MMA warp 62 % of its time); seven that take its tasks in turn leave the chain of the first operand.  235 868 rows:
 // 64 x 256 101 -> 92 us, 256 x 128 129 -> 110, 256 x 256 249 -> 202.
+#include "cbm_launch.cuh"
 #include "cbm_map.cuh"
 
 namespace cbm_map {
@@ -49,12 +50,12 @@ struct GradParams {
 // Fetches without a condition, volatile for the same reason as fetch1.
 __device__ __forceinline__ float fetch(const float* p) {
     float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float2 fetch_pair(const float* p) {
     float2 v;
-    asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
     return v;
 }
 
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(GRAD_THREADS, 1) grad_kernel(const __grid_cons
         s_gave_up = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    cbm::wait_before();
     fence_before();
     __syncthreads();
     fence_after();
@@ -298,8 +300,8 @@ done:
 
 // out = sum of `parts` partial results [m, n], in a fixed order: 8 threads of a block add every eighth part of an
 // element, the 8 sums are added in turn.  `turn`: out is [n, m].
-__global__ void __launch_bounds__(256) reduce_parts_kernel(const float* __restrict__ part, int parts, int m, int n,
-                                                           float* __restrict__ out, int64_t ldo, int turn) {
+__global__ void __launch_bounds__(256) reduce_parts_kernel(const float* part, int parts, int m, int n, float* out, int64_t ldo, int turn) {
+    cbm::wait_before();
     __shared__ float s[8][32];
     const int64_t size = (int64_t)m * n, i = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
     const int g = threadIdx.x >> 5;
@@ -399,9 +401,9 @@ int run_grad(const float* dy, int64_t lddy, const float* x, int64_t ldx, float* 
     static_assert(2 * 3 * D_COLS * 128 + 1024 <= 120 * 1024, "two stages of B");
     if (!allow_smem<grad_kernel>(smem))
         return cbm::fail(CBM_B200_ERR_CUDA, "dense_grad_weight: shared memory size refused");
-    grad_kernel<<<dim3(t.m_tiles * t.n_tiles, t.ranges), GRAD_THREADS, smem, s>>>(p);
+    cbm::launch_next(grad_kernel, dim3(t.m_tiles * t.n_tiles, t.ranges), GRAD_THREADS, smem, s, p);
     const int64_t size = (int64_t)n_in * n_out;
-    reduce_parts_kernel<<<(unsigned)((size + 31) / 32), 256, 0, s>>>(p.part, t.ranges, p.m, p.n, dw, lddw, t.turn ? 1 : 0);
+    cbm::launch_next(reduce_parts_kernel, (unsigned)((size + 31) / 32), 256, 0, s, p.part, t.ranges, p.m, p.n, dw, lddw, t.turn ? 1 : 0);
     if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, "dense_grad_weight: launch failed");
     return CBM_B200_OK;
 }

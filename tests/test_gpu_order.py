@@ -1,0 +1,84 @@
+"""Kernels whose blocks are set up while the one before them on the stream is ending (cbm_launch.cuh) see all of what it
+wrote: a chain of calls issued in one go gives the bits of the same calls waited for one by one."""
+import numpy as np
+import pytest
+import torch
+
+from cbm4gnn_b200 import dense, graphs
+from cbm4gnn_b200.cbm import cbm_matrix
+from helpers import with_self_loops
+
+pytestmark = pytest.mark.gpu
+
+
+def _chain(c, f, after):
+    """Products there and back between the same two buffers, whose rows share cache lines where `f` is odd, the operand
+    changed by torch's kernels too; maps, their gradients and the sum of its parts behind them."""
+    gen = torch.Generator(device="cuda").manual_seed(f)
+    x, y = torch.randn((2, c.num_rows, f), generator=gen, device="cuda")
+    w = torch.randn((f, f), generator=gen, device="cuda") / f ** 0.5
+    seen = []
+    for _ in range(4):
+        c.omp_mkl_csr_fused_spmm_update(x, y)
+        after()
+        c.omp_mkl_csr_fused_spmm_update(y, x)
+        after()
+        h = dense.dense_forward(x, w)
+        after()
+        g = dense.dense_grad_weight(h, y)
+        after()
+        gx = dense.dense_grad_input(h, g / g.norm(), relu_output=x)
+        after()
+        x.copy_(gx).div_(gx.norm())
+        after()
+        w = w + g / g.norm()
+        after()
+        seen += [h, g, gx, y.clone()]
+    return seen
+
+
+@pytest.fixture(scope="module", params=["waiting rows", "communities"])
+def matrix(request):
+    ei = with_self_loops(graphs.copy_model(3000, 0.9, 8, 11) if request.param == "waiting rows" else graphs.make_graph("c3", scale=0.05))
+    return cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
+
+
+# widths: row groups of a few lanes, two odd pitches (the operand is copied to aligned rows first), whole slabs, several
+@pytest.mark.parametrize("f", [8, 33, 47, 64, 128, 260])
+def test_calls_in_one_go_give_the_bits_of_calls_one_by_one(matrix, f):
+    want = _chain(matrix, f, torch.cuda.synchronize)
+    got = _chain(matrix, f, lambda: None)
+    matrix.plan(0).status()
+    assert len(got) == len(want) and all(torch.equal(a, b) for a, b in zip(got, want))
+    assert all(bool(torch.isfinite(a).all()) for a in got)
+
+
+def test_captured_branches_that_join(matrix):
+    """A product and a map on two branches of a captured graph, and a map of both behind the join."""
+    x, y = torch.randn((2, matrix.num_rows, 64), device="cuda")
+    w = torch.randn((64, 64), device="cuda")
+    side = torch.cuda.Stream()
+
+    def work():
+        here = torch.cuda.current_stream()
+        matrix.omp_mkl_csr_fused_spmm_update(x, y)
+        side.wait_stream(here)
+        with torch.cuda.stream(side):
+            a = dense.dense_forward(x, w)
+        b = dense.dense_forward(y, w)
+        here.wait_stream(side)
+        return dense.dense_grad_weight(a, b)
+
+    first = torch.cuda.Stream()
+    with torch.cuda.stream(first):  # workspaces grow outside the capture
+        want = work().clone()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        got = work()
+    x.mul_(2)
+    graph.replay()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert np.isfinite(float(want.norm()))
+    assert torch.equal(got, want * 4)  # (of powers of two, nothing is rounded)
