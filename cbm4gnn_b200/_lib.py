@@ -58,6 +58,7 @@ EXPORTED = [
     "cbm_b200_plan_destroy",
     "cbm_b200_schedule_info",
     "cbm_b200_schedule_as_planned",
+    "cbm_b200_csr_schedule_as_planned",
     "cbm_b200_schedule_lifted",
     "cbm_b200_plan_schedule",
     "cbm_b200_plan_info",
@@ -185,6 +186,8 @@ def lib() -> ctypes.CDLL:
         c_void_p, c_void_p, c_int32, c_int32, c_int32, i32p, i32p, i32p, i32p)
     sig("cbm_b200_schedule_as_planned", c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
         c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
+    sig("cbm_b200_csr_schedule_as_planned", c_int32, c_int32, c_int32, *[c_void_p] * 4, i32p, i32p, i32p, i32p, i32p,
+        POINTER(c_uint64))
     sig("cbm_b200_schedule_lifted", c_int32, c_int32, *[c_void_p] * 7, i32p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p)
     sig("cbm_b200_plan_schedule", c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
     sig("cbm_b200_plan_info", c_int32, c_void_p, i32p, POINTER(c_int64), i32p, i32p,

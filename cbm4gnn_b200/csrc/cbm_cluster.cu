@@ -50,8 +50,8 @@ __global__ void __launch_bounds__(256) propagate_kernel(int32_t n, const int32_t
     const int32_t have = min(31, len);
     int32_t u = -1;
     if (lane < have) u = col[beg + (len <= 31 ? lane : (int32_t)((int64_t)lane * len / 31))];
-    else if (lane == 31 && par < n) u = par;
-    const int32_t l = u >= 0 && u != v ? __ldg(label + u) : -1 - lane;  // lanes without a column match nobody
+    else if (lane == 31) u = par;
+    const int32_t l = u >= 0 && u < n && u != v ? __ldg(label + u) : -1 - lane;  // lanes without a row match nobody
     const unsigned same = __match_any_sync(0xffffffffu, l);
     // most frequent label; the row's own wins ties, then an arbitrary but fixed order of the labels
     const unsigned score =
@@ -97,6 +97,7 @@ bool cbm::cluster_rows(int32_t n, const int32_t* crow, const int32_t* col, const
             }
             ok = cudaGetLastError() == cudaSuccess &&
                  cudaMemcpy(label, b.label, rows, cudaMemcpyDeviceToHost) == cudaSuccess;
+            for (int32_t v = 0; ok && v < n; ++v) ok = label[v] >= 0 && label[v] < n;  // the caller counts by them
         }
         if (!ok) cudaGetLastError();
     }

@@ -1504,8 +1504,10 @@ struct Rules {
 // fetched from L2 anyway and a launch is bound by latency), and where about 1 000 consecutive entries of
 // the sorted rows still name mostly different columns.  On B200, width 128: rows of 22 entries in
 // communities of 55 (ratio 0.4) gain 40 %, rows of 11 in communities of 118 (0.5) gain 15 %; copy-model graphs
-// (0.75 - 0.95), whose common columns are few hubs, gain nothing.
+// (0.75 - 0.95), whose common columns are few hubs, gain nothing.  Only for square matrices: the search takes a column for the
+// row of that number.
 bool cluster_order(const Structure& st, const Rules& rules, std::vector<i32>& rank) {
+    if (!st.square) return false;
     const i32 n = st.n;
     const i32 *crow = st.crow, *col = st.col;
     std::vector<i32> label;
@@ -1892,18 +1894,18 @@ uint64_t fingerprint_of(const RowDesc* desc, size_t n) {
 }
 }  // namespace
 
-extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
-                                            const int32_t* delta_crow, const int32_t* delta_col,
-                                            const float* delta_val, const float* multiplier,
-                                            const int32_t* labels, int32_t* n_items, int32_t* n_prefix,
-                                            int32_t* n_partial, int32_t* n_chunks, int32_t* segment,
-                                            uint64_t* fingerprint) {
+namespace {
+// The schedule of a whole matrix in its own order by the rules of a plan; csr_cols as for read_structure.
+int schedule_as_planned(const char* who, int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* crow,
+                        const int32_t* col, const float* val, const float* multiplier, int32_t csr_cols, const int32_t* labels,
+                        int32_t* n_items, int32_t* n_prefix, int32_t* n_partial, int32_t* n_chunks, int32_t* segment,
+                        uint64_t* fingerprint) {
     for (i32 v = 0; labels && v < n; ++v)
-        if (labels[v] < 0 || labels[v] >= n) return cbm::fail(CBM_B200_ERR_ARG, "schedule_as_planned: label out of range");
+        if (labels[v] < 0 || labels[v] >= n) return cbm::fail(CBM_B200_ERR_ARG, std::string(who) + ": label out of range");
     Schedule sch;
-    const int rc = guarded("schedule_as_planned", [&] {
+    const int rc = guarded(who, [&] {
         Structure st;
-        const int bad = read_structure(n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, nullptr, 0, 0, n, 0, st);
+        const int bad = read_structure(n, mst_row, mst_col, crow, col, val, multiplier, nullptr, 0, 0, n, csr_cols, st);
         if (bad) return bad;
         const Rules rules{true, -1, labels};
         std::vector<i32> rank;
@@ -1918,6 +1920,26 @@ extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, c
     if (segment) *segment = sch.segment;
     if (fingerprint) *fingerprint = fingerprint_of(sch.desc.data(), sch.desc.size());
     return CBM_B200_OK;
+}
+}  // namespace
+
+extern "C" int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
+                                            const int32_t* delta_crow, const int32_t* delta_col,
+                                            const float* delta_val, const float* multiplier,
+                                            const int32_t* labels, int32_t* n_items, int32_t* n_prefix,
+                                            int32_t* n_partial, int32_t* n_chunks, int32_t* segment,
+                                            uint64_t* fingerprint) {
+    return schedule_as_planned("schedule_as_planned", n, mst_row, mst_col, delta_crow, delta_col, delta_val, multiplier, 0, labels,
+                               n_items, n_prefix, n_partial, n_chunks, segment, fingerprint);
+}
+
+extern "C" int cbm_b200_csr_schedule_as_planned(int32_t n_rows, int32_t n_cols, const int32_t* crow, const int32_t* col,
+                                                const float* val, const int32_t* labels, int32_t* n_items,
+                                                int32_t* n_prefix, int32_t* n_partial, int32_t* n_chunks,
+                                                int32_t* segment, uint64_t* fingerprint) {
+    if (n_cols <= 0) return cbm::fail(CBM_B200_ERR_ARG, "csr_schedule_as_planned: n_cols must be positive");
+    return schedule_as_planned("csr_schedule_as_planned", n_rows, nullptr, nullptr, crow, col, val, nullptr, n_cols, labels, n_items,
+                               n_prefix, n_partial, n_chunks, segment, fingerprint);
 }
 
 extern "C" int cbm_b200_schedule_lifted(int32_t n, const int32_t* mst_row, const int32_t* mst_col, const int32_t* delta_crow,

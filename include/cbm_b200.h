@@ -144,6 +144,12 @@ int cbm_b200_schedule_as_planned(int32_t n, const int32_t* mst_row, const int32_
                                  int32_t* n_items, int32_t* n_prefix, int32_t* n_partial, int32_t* n_chunks,
                                  int32_t* segment, uint64_t* fingerprint);
 
+/* The same for a matrix given as CSR, by the rules of cbm_b200_csr_plan_create.  Communities are those of the rows' own
+ * numbers: a matrix with more or fewer columns than rows keeps its order, whatever `labels` says. */
+int cbm_b200_csr_schedule_as_planned(int32_t n_rows, int32_t n_cols, const int32_t* crow, const int32_t* col,
+                                     const float* val, const int32_t* labels, int32_t* n_items, int32_t* n_prefix,
+                                     int32_t* n_partial, int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
+
 /* The rows as the product in one pass computes them: those whose parent saves them few entries are lifted out of the tree
  * and hang under the virtual root (n) with all their entries.  By the rules of a plan, for a whole matrix in its own
  * order, with or without communities (labels, may be NULL); needs no GPU.  n_lifted: how many rows that are; parent (n

@@ -496,3 +496,24 @@ def test_host_operands_with_ragged_width(c1):
 def test_l2_probe_reports_a_plausible_rate():
     r = _lib.lib().cbm_b200_probe_l2_read_gbps(torch.cuda.current_device())
     assert 2000.0 < r < 60000.0
+
+
+@pytest.mark.parametrize("n_rows,n_cols", [(20_000, 60_000), (60_000, 20_000)])
+def test_csr_plan_of_many_rows_and_other_columns(n_rows, n_cols):
+    """Rectangular matrices with as many rows, and entries a row, as those whose communities are looked for: rows in blocks of
+    40 that name the same 60 columns and would be such communities."""
+    import scipy.sparse as sp
+    from cbm4gnn_b200.cbm import csr_matrix_plan
+    rng = np.random.default_rng(n_rows)
+    col = (np.arange(n_rows)[:, None] // 40 * 60 + rng.integers(0, 60, (n_rows, 8))) % n_cols
+    a = sp.csr_matrix((rng.standard_normal(8 * n_rows).astype(np.float32), (np.repeat(np.arange(n_rows), 8), col.ravel())),
+                      shape=(n_rows, n_cols))
+    a.sum_duplicates()
+    a.sort_indices()
+    assert len(a.data) > 4 * n_rows
+    plan = csr_matrix_plan(a.indptr, a.indices, a.data, n_cols)
+    for f in (128, 47):
+        x = rng.standard_normal((n_cols, f)).astype(np.float32)
+        y = plan.matmul(_dev(x))
+        plan.status()
+        np.testing.assert_allclose(y.cpu().numpy(), a.astype(np.float64) @ x.astype(np.float64), **TOL)

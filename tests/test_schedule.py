@@ -228,3 +228,25 @@ def test_a_structure_that_is_no_signed_pattern_is_not_lifted(spoil):
     lifted, parent, crow, col, val = _lifted(c)
     assert lifted == 0 and np.array_equal(parent, c._parent)
     assert np.array_equal(col, c._dcol) and np.array_equal(val, c._dval)
+
+
+def _csr_as_planned(n_rows, n_cols, labels, seed=0):
+    rng = np.random.default_rng(seed)
+    crow = np.arange(0, 8 * n_rows + 1, 8, dtype=np.int32)
+    col = np.sort(rng.integers(0, n_cols, (n_rows, 8)), axis=1).astype(np.int32)
+    val, labels = np.ones(8 * n_rows, np.float32), np.ascontiguousarray(labels, dtype=np.int32)
+    p = lambda a: ctypes.c_void_p(a.ctypes.data)
+    out, mark = [ctypes.c_int32() for _ in range(5)], ctypes.c_uint64()
+    rc = _lib.lib().cbm_b200_csr_schedule_as_planned(n_rows, n_cols, p(crow), p(col), p(val), p(labels),
+                                                     *[ctypes.byref(o) for o in out], ctypes.byref(mark))
+    assert rc == 0, _lib.lib().cbm_b200_last_error()
+    return [o.value for o in out]
+
+
+@pytest.mark.parametrize("n_rows,n_cols", [(300, 299), (300, 300), (300, 301), (200, 1000), (1000, 200), (1, 5)])
+def test_only_square_matrices_are_ordered_by_community(n_rows, n_cols):
+    """A column number is a row's number only where there are as many of them: nobody looks for communities, whose search
+    follows columns to rows, in other matrices."""
+    n_items, n_prefix, n_partial, n_chunks, _ = _csr_as_planned(n_rows, n_cols, np.arange(n_rows) % 3 % n_rows)
+    assert n_items == n_prefix == n_rows and n_partial == 0
+    assert (n_chunks > 0) == (n_rows == n_cols)
