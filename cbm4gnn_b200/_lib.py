@@ -62,6 +62,7 @@ EXPORTED = [
     "cbm_b200_schedule_lifted",
     "cbm_b200_plan_schedule",
     "cbm_b200_plan_info",
+    "cbm_b200_one_round_group",
     "cbm_b200_plan_tune",
     "cbm_b200_plan_status",
     "cbm_b200_spmm_update",
@@ -192,6 +193,7 @@ def lib() -> ctypes.CDLL:
     sig("cbm_b200_plan_schedule", c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
     sig("cbm_b200_plan_info", c_int32, c_void_p, i32p, POINTER(c_int64), i32p, i32p,
         POINTER(c_int64))
+    sig("cbm_b200_one_round_group", c_int32, c_int32, c_int32, c_int32, c_int32)
     sig("cbm_b200_plan_tune", c_int32, c_void_p, c_int32, c_int32, c_int32, c_int32)
     sig("cbm_b200_plan_status", c_int32, c_void_p, c_void_p)
     for name in ("cbm_b200_spmm_update", "cbm_b200_fused_spmm_update", "cbm_b200_delta_spmm"):

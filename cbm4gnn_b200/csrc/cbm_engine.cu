@@ -2184,6 +2184,18 @@ int resident_blocks(const Shape& sh, i32 f, bool ragged, int mode) {
     return sh.v4 && sh.nv == 1 && f <= 64 && mode != MODE_UPDATE_ONLY ? NARROW_RESIDENT : resident_regs(sh.nv, sh.v4, ragged);
 }
 
+// A product that the resident warps can do in one round draws no second claim: every warp takes its share of the
+// prefix, and as long as few items wait (a quarter of the warps) one of those or none.  1 000 rows, 16 columns 8.2 ->
+// 6.2 us, 4 096 rows, 500 columns (two or three items a warp) 32.0 -> 22.0.
+// Returns the items of the prefix that a warp takes, 0 where one round does not do: an operand so wide that there are more
+// slabs than warps has some left over even with all of a slab's prefix to one warp.
+i32 one_round_group(i32 n_prefix, i32 n_waiting, i64 n_slabs, i64 warps) {
+    const i64 waiting = n_waiting * n_slabs;
+    if (waiting >= warps / 4) return 0;
+    const i64 per_slab = (warps - waiting) / n_slabs;  // warps for a slab's prefix
+    return per_slab == 0 ? 0 : (i32)((n_prefix + per_slab - 1) / per_slab);
+}
+
 int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
              i32 f, int mode, bool may_pack, bool in_turn, LaunchCfg& c) {
     const bool y_vec = ldy % 4 == 0 && aligned16(y);
@@ -2232,17 +2244,11 @@ int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, c
         // A small product keeps single claims: with fewer claims than resident warps, grouping
         // only idles warps.
         c.group = ((i64)d.n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && d.n_chunks > 0 ? 8 : 4) : 1;
-        // A product that the resident warps can do in one round draws no second claim: every warp takes its share of the
-        // prefix, and as long as few items wait (a quarter of the warps) one of those or none.  1 000 rows, 16 columns 8.2 ->
-        // 6.2 us, 4 096 rows, 500 columns (two or three items a warp) 32.0 -> 22.0.
-        if (c.group == 1) {
+        if (c.group == 1 && p->n_blocks == 0) {
             const i64 warps = (i64)p->sm_count * resident_blocks(c.sh, f, c.ragged, mode) * 8;
-            const i64 waiting = (i64)(d.n_items - d.n_prefix) * c.sh.n_slabs;
-            if (p->n_blocks == 0 && waiting < warps / 4) {
-                c.one_round = true;
-                c.group = (i32)std::max<i64>(1, ((i64)d.n_prefix * c.sh.n_slabs + (warps - waiting) - 1) / (warps - waiting));
-                while ((i64)((d.n_prefix + c.group - 1) / c.group) * c.sh.n_slabs > warps - waiting) ++c.group;
-            }
+            const i32 group = one_round_group(d.n_prefix, d.n_items - d.n_prefix, c.sh.n_slabs, warps);
+            c.one_round = group > 0;
+            if (c.one_round) c.group = group;
         }
     }
     if (!c.chunked) {
@@ -2460,6 +2466,10 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
 }
 
 }  // namespace
+
+extern "C" int32_t cbm_b200_one_round_group(int32_t n_prefix, int32_t n_waiting, int32_t n_slabs, int32_t warps) {
+    return n_prefix < 0 || n_waiting < 0 || n_slabs < 1 || warps < 1 ? 0 : one_round_group(n_prefix, n_waiting, n_slabs, warps);
+}
 
 extern "C" int cbm_b200_spmm_update(cbm_b200_plan* p, const float* x, int64_t ldx, float* y,
                                     int64_t ldy, int32_t f, void* stream) {

@@ -171,6 +171,11 @@ int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64_t* n_delta
 int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
                            int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
 
+/* The rule by which a product draws its claims in one round, each warp once: how many of the n_prefix items that never wait
+ * a warp takes of each of n_slabs column slabs, of which each has n_waiting further items for a warp of their own, when
+ * `warps` warps are resident.  0: more than one round.  Needs no GPU. */
+int32_t cbm_b200_one_round_group(int32_t n_prefix, int32_t n_waiting, int32_t n_slabs, int32_t warps);
+
 /* Tuning knobs (0 keeps the default): column-slab width in floats, thread blocks per launch, the
  * column-chunk width (a multiple of 4) of the host-buffer pipeline below, and the kernel form
  * (0 = gather held in registers, the default; 1 = operand rows staged in shared memory by bulk

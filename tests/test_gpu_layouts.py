@@ -133,3 +133,20 @@ def test_plans_of_one_graph_are_the_same(n, mu, deg_in):
     for _ in range(4):
         c._plans.clear()
         assert c.plan(0).schedule() == first
+
+
+@pytest.mark.parametrize("rows,f,aligned,slab", [(4, 1_000_000, True, 0), (4, 909_312, True, 0), (4, 909_440, True, 0), (6, 300_000, False, 0),
+                                                 (3, 227_328, False, 0), (3, 227_392, False, 0), (5, 230_000, True, 32)])
+def test_more_slabs_than_warps(rows, f, aligned, slab):
+    """Few rows by so many columns that there are more column slabs than resident warps (7 104 of 128 columns on 148 SMs,
+    3 552 of 64 where rows are not aligned), and just as many."""
+    ei = np.stack([np.repeat(np.arange(rows), rows), np.tile(np.arange(rows), rows)])
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=100, normalized=True)
+    if slab:
+        c.plan(0).tune(slab_width=slab)
+    x = np.random.default_rng(f).standard_normal((rows, f)).astype(np.float32)
+    xd, yd = _buffer(rows, f, f if aligned else f + 1), _buffer(rows, f, f if aligned else f + 1)
+    xd.copy_(torch.from_numpy(x))
+    c.omp_mkl_csr_fused_spmm_update(xd, yd)
+    c.plan(0).status()
+    np.testing.assert_allclose(yd.cpu().numpy(), sparse_product(ei, x, True), **TOL)

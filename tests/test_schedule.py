@@ -250,3 +250,19 @@ def test_only_square_matrices_are_ordered_by_community(n_rows, n_cols):
     n_items, n_prefix, n_partial, n_chunks, _ = _csr_as_planned(n_rows, n_cols, np.arange(n_rows) % 3 % n_rows)
     assert n_items == n_prefix == n_rows and n_partial == 0
     assert (n_chunks > 0) == (n_rows == n_cols)
+
+
+@pytest.mark.parametrize("warps", [2368, 3552, 7104])
+def test_one_round_has_a_warp_for_every_claim(warps):
+    """From no slab to a warp up to several times as many slabs as there are warps, where there can be no such round."""
+    group_of = _lib.lib().cbm_b200_one_round_group
+    for n_slabs in [1, 2, 3, 4, 7, 111, warps // 4, warps // 2 - 1, warps // 2, warps // 2 + 1, warps - 1, warps, warps + 1, 7813, 40_000]:
+        for n_prefix in [1, 2, 3, 4, 5, 8, 63, 1000]:
+            for n_waiting in [0, 1, 5, 500]:
+                group = group_of(n_prefix, n_waiting, n_slabs, warps)
+                waiting = n_waiting * n_slabs
+                fits = lambda g: -(-n_prefix // g) * n_slabs + waiting <= warps
+                if waiting >= warps // 4 or n_slabs + waiting > warps:  # (all of a slab's prefix to one warp)
+                    assert group == 0
+                else:
+                    assert 1 <= group <= n_prefix and fits(group) and (group == 1 or not fits(group - 1))
