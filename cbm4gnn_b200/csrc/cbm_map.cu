@@ -89,6 +89,12 @@ static_assert(PRODUCER_REGS > LAUNCH_REGS && EPILOGUE_REGS > LAUNCH_REGS && MMA_
 constexpr int SMEM_MAX = 192 * 1024;     // for the split weights
 constexpr int TURN_BYTES = 32 * 32 * 4;  // per epilogue warp
 constexpr int SMEM_ALL = SMEM_MAX + EPILOGUE_WARPS * TURN_BYTES + 1024;
+// An SM gives shared memory out in steps, and L1 the rest: 60 KB beside 196 KB (of which each block has 1 KB, and some bytes of
+// its own), 28 KB beside more.  Rows that are no whole 128-byte lines need that room, as two chunks have a line
+// in common.  A second place for results that takes it away costs more than it gives: 235 868 rows, 300 -> 80 156 us with it,
+// 102 without; 300 -> 300 491 and 395; 180 000 rows, 200 -> 96 79 and 61.  Where it leaves it, it is worth having: 64 -> 128 29 us,
+// 31 without.
+constexpr int SMEM_BESIDE_L1 = 194 * 1024;
 
 struct MapParams {
     CUtensorMap store;  // d, in boxes of 32 x 32, 128-byte swizzled; used where `boxes` is set
@@ -552,6 +558,10 @@ bool aligned_rows(const void* p, int64_t ld) { return (reinterpret_cast<uintptr_
 
 int round_up(int v, int to) { return (v + to - 1) / to * to; }
 
+int smem_of(int steps, int bn, int places) {
+    return 3 * ((steps + 3) / 4) * bn * 128 + places * EPILOGUE_WARPS * TURN_BYTES + 1024;
+}
+
 template <bool B_TRANS, int EXTRA, bool PAIR>
 int launch_form(const char* who, const MapParams& p, int sms, cudaStream_t stream) {
     if (!allow_smem<map_kernel<B_TRANS, EXTRA, PAIR>>(SMEM_ALL))
@@ -559,7 +569,7 @@ int launch_form(const char* who, const MapParams& p, int sms, cudaStream_t strea
     const int n_tiles = (p.n + p.bn - 1) / p.bn;
     const dim3 grid(n_tiles, std::max(1, std::min(p.row_tiles, sms / n_tiles)));
     // at least half of an SM's shared memory, so that two blocks, which both want all tensor memory, never share one
-    const int smem = std::max(3 * ((p.steps + 3) / 4) * p.bn * 128 + p.places * EPILOGUE_WARPS * TURN_BYTES + 1024, 120 * 1024);
+    const int smem = std::max(smem_of(p.steps, p.bn, p.places), 120 * 1024);
     cbm::launch_next(map_kernel<B_TRANS, EXTRA, PAIR>, grid, THREADS, smem, stream, p);
     if (cudaGetLastError() != cudaSuccess) return cbm::fail(CBM_B200_ERR_CUDA, std::string(who) + ": launch failed");
     return CBM_B200_OK;
@@ -610,9 +620,9 @@ int run_map(const char* who, const float* a, int64_t lda, const float* b, int64_
         p.relu_in = relu_in;
         p.relu_out = relu_out && last;
         p.add = k0 > 0;
-        p.places = 3 * ((p.steps + 3) / 4) * bn * 128 + 2 * EPILOGUE_WARPS * TURN_BYTES + 1024 <= SMEM_ALL ? 2 : 1;
         // (a map of the result takes the host 2 us, and a block that has one tile has nothing to go on to)
         p.boxes = p.d_vec && passes == 1 && !aux && row_tiles >= sms && make_boxes(&p.store, d, ldd, m, n);
+        p.places = p.boxes && smem_of(p.steps, bn, 2) <= SMEM_BESIDE_L1 ? 2 : 1;
         if (aux) {
             p.aux = aux;
             p.ldaux = ldaux;
