@@ -1395,6 +1395,7 @@ struct Schedule {
     std::vector<RowDesc> desc;
     std::unique_ptr<Entry[]> ent;  // not cleared first: the threads that fill it touch its pages
     i64 n_ent = 0;
+    std::vector<i64> source;    // per item: its first entry in the delta arrays, or ~ its first in those of the lifted rows
     std::vector<Chunk> chunks;  // clustered plans
     bool clustered = false;
     i32 segment = 0;  // delta entries of a PARTIAL item
@@ -1653,9 +1654,9 @@ int read_structure(int32_t n, const int32_t* mst_row, const int32_t* mst_col, co
     return CBM_B200_OK;
 }
 
-// The schedule (layout described at RowDesc) of the structure's rows, or with `lift` of the tree with some of them
-// lifted; `rank`: their order by community, empty where the graph has none.
-int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vector<i32>& rank, const Rules& rules, Schedule& sch) {
+// The schedule (layout described at RowDesc), its entries aside, of the structure's rows, or with `lift` of the tree with some
+// of them lifted; `rank`: their order by community, empty where the graph has none.
+int lay_out(const Structure& st, const cbm::Lifted* lift, const std::vector<i32>& rank, const Rules& rules, Schedule& sch) {
     const i32 n = st.n, own_begin = st.own_begin, own_end = st.own_end;
     const std::vector<i32>&parent = lift ? lift->parent : st.parent, &level = lift ? lift->level : st.level;
     const std::vector<i32>& owned_rows = st.rows;
@@ -1675,13 +1676,12 @@ int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vect
     std::vector<RowDesc>& desc = sch.desc;
     sch.clustered = !rank.empty();
     sch.segment = SEG;
-    // items get their entry ranges now; the entries are filled in at the end, on several threads
-    std::vector<i64> source;  // per item: its first entry in the delta arrays, or ~ its first in those of the lifted rows
-    source.reserve((size_t)n);
+    // items get their entry ranges only: the entries are filled in afterwards
+    sch.source.reserve((size_t)n);
     auto append_entries = [&](i32 v, i32 from, i32 to) {  // entries [from, to) of row v
         const i32 beg = (i32)sch.n_ent;
         const i64 at = (lift ? lift->at[v] : st.crow[v]) + from;
-        source.push_back(lift && lift->lifted[v] ? ~at : at);
+        sch.source.push_back(lift && lift->lifted[v] ? ~at : at);
         sch.n_ent += to - from;
         if (sch.clustered) sch.n_ent += sch.n_ent % 2;
         return beg;
@@ -1767,20 +1767,6 @@ int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vect
     else if (lift)  // (lifting has changed levels)
         std::stable_sort(rest.begin(), rest.end(), [&](i32 a, i32 b) { return level[a] < level[b]; });
     for (i32 v : rest) add_row_item(v);
-    sch.ent.reset(new Entry[(size_t)std::max<i64>(sch.n_ent, 1)]);
-    const i32 n_items = (i32)desc.size();
-    // (half of the threads: those that have finished spin for a while, beside the caller's first product)
-    const int threads = (int)std::max<i64>(1, std::min<i64>(omp_get_max_threads() / 2, sch.n_ent / 100000));
-#pragma omp parallel for schedule(static) num_threads(threads)
-    for (i32 i = 0; i < n_items; ++i) {
-        const i32 len = (desc[i].info >> ITEM_LEN_SHIFT) & 0xff;
-        Entry* e = sch.ent.get() + desc[i].beg;
-        const bool own = source[i] >= 0;
-        const i32* col = own ? st.col + source[i] : lift->col.data() + ~source[i];
-        const float* val = own ? st.val + source[i] : lift->val.data() + ~source[i];
-        for (i32 k = 0; k < len; ++k) e[k] = Entry{label(col[k]), val[k]};
-        if (sch.clustered && len % 2) e[len] = Entry{0, 0.0f};
-    }
     if (sch.clustered) make_chunks(sch, n_prefix);
     sch.n_rows_owned = (i32)owned_rows.size();
     sch.n_prefix = n_prefix;
@@ -1791,7 +1777,33 @@ int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vect
     return validate_schedule(sch, own_end - own_begin);
 }
 
+// The entries of a schedule, on several threads.
+void fill_entries(const Structure& st, const cbm::Lifted* lift, Schedule& sch) {
+    sch.ent.reset(new Entry[(size_t)std::max<i64>(sch.n_ent, 1)]);
+    const i32 n_items = (i32)sch.desc.size();
+    // (half of the threads: those that have finished spin for a while, beside the caller's first product)
+    const int threads = (int)std::max<i64>(1, std::min<i64>(omp_get_max_threads() / 2, sch.n_ent / 100000));
+#pragma omp parallel for schedule(static) num_threads(threads)
+    for (i32 i = 0; i < n_items; ++i) {
+        const i32 len = (sch.desc[i].info >> ITEM_LEN_SHIFT) & 0xff;
+        Entry* e = sch.ent.get() + sch.desc[i].beg;
+        const bool own = sch.source[i] >= 0;
+        const i32* col = own ? st.col + sch.source[i] : lift->col.data() + ~sch.source[i];
+        const float* val = own ? st.val + sch.source[i] : lift->val.data() + ~sch.source[i];
+        for (i32 k = 0; k < len; ++k) e[k] = Entry{st.label(col[k]), val[k]};
+        if (sch.clustered && len % 2) e[len] = Entry{0, 0.0f};
+    }
+    std::vector<i64>().swap(sch.source);
+}
+
+int build_schedule(const Structure& st, const cbm::Lifted* lift, const std::vector<i32>& rank, const Rules& rules, Schedule& sch) {
+    const int rc = lay_out(st, lift, rank, rules, sch);
+    if (rc == CBM_B200_OK) fill_entries(st, lift, sch);
+    return rc;
+}
+
 // Runs both, side by side if `wide` and a thread can be had, and lets the first one's exception out before the other's.
+// The second one opens no team of threads: OpenMP would keep another for it, and ends the process where it cannot.
 template <class F, class G>
 void run_both(bool wide, F first, G second) {
     std::exception_ptr first_thrown, second_thrown;
@@ -1820,27 +1832,40 @@ void run_both(bool wide, F first, G second) {
     if (second_thrown) std::rethrow_exception(second_thrown);
 }
 
-// The structure's own schedule, and the one with rows lifted out of the tree where that pays.
-int build_schedules(const Structure& st, const Rules& rules, Schedule& tree, Schedule& lifted) {
+int build_both(const Structure& st, const Rules& rules, Schedule& tree, Schedule& lifted) {
     cbm::Lifted lift;
     std::vector<i32> rank;
     const bool wide = st.crow[st.n] > 1000000;  // steps of milliseconds
     run_both(
-        wide, [&] { cluster_order(st, rules, rank); },
+        wide,
         [&] {
             if (!st.csr) cbm::lift_rows(st.n, st.rows, st.parent, st.level, st.crow, st.col, st.val, lift);
-        });
+        },
+        [&] { cluster_order(st, rules, rank); });
     if (lift.n_lifted == 0) return build_schedule(st, nullptr, rank, rules, tree);
     int rc = CBM_B200_OK, rc_lifted = CBM_B200_OK;
-    std::string what;  // (the message of an error belongs to its thread)
     run_both(
         wide, [&] { rc = build_schedule(st, nullptr, rank, rules, tree); },
-        [&] {
-            rc_lifted = build_schedule(st, &lift, rank, rules, lifted);
-            if (rc_lifted) what = cbm::last_error_slot();
-        });
+        [&] { rc_lifted = lay_out(st, &lift, rank, rules, lifted); });
     if (rc) return rc;
-    return rc_lifted ? cbm::fail(rc_lifted, what) : CBM_B200_OK;
+    if (rc_lifted) lifted = Schedule();
+    else fill_entries(st, &lift, lifted);
+    return CBM_B200_OK;
+}
+
+// The structure's own schedule, and the one with rows lifted out of the tree where that pays, can be made and has memory:
+// the product can do without it.
+int build_schedules(const Structure& st, const Rules& rules, Schedule& tree, Schedule& lifted) {
+    try {
+        return build_both(st, rules, tree, lifted);
+    } catch (const std::bad_alloc&) {
+    } catch (const std::length_error&) {
+    }
+    tree = Schedule();
+    lifted = Schedule();
+    std::vector<i32> rank;
+    cluster_order(st, rules, rank);
+    return build_schedule(st, nullptr, rank, rules, tree);
 }
 
 }  // namespace

@@ -266,3 +266,79 @@ def test_one_round_has_a_warp_for_every_claim(warps):
                     assert group == 0
                 else:
                     assert 1 <= group <= n_prefix and fits(group) and (group == 1 or not fits(group - 1))
+
+
+def _run_on_pairs(pairs, more, body):
+    """``body`` in a process of its own, on a structure of ``pairs`` rows of 4 entries and as many children with ``more``
+    entries beside their parent's: all children are lifted."""
+    import os
+    import subprocess
+    import sys
+    code = f"""
+import ctypes, os, resource, threading
+import numpy as np
+L = ctypes.CDLL({_lib.LIB_PATH!r})
+L.cbm_b200_last_error.restype = ctypes.c_char_p
+pairs, more = {pairs}, {more}
+n = 2 * pairs
+row = np.full(n + 2, pairs, np.int32)
+row[0], row[n + 1] = 0, n
+row[1:pairs + 1] = np.arange(1, pairs + 1)  # row i has the child pairs + i
+col = np.concatenate([np.arange(pairs, n), np.arange(pairs)]).astype(np.int32)
+length = np.concatenate([np.full(pairs, 4), np.full(pairs, more)])
+crow = np.concatenate([[0], np.cumsum(length)]).astype(np.int32)
+dcol = np.concatenate([np.tile(np.arange(4), pairs), np.tile(np.arange(4, 4 + more), pairs)]).astype(np.int32)
+val = np.ones(len(dcol), np.float32)
+p = lambda a: ctypes.c_void_p(a.ctypes.data)
+def lifted():
+    count = ctypes.c_int32(-1)
+    rc = L.cbm_b200_schedule_lifted(n, p(row), p(col), p(crow), p(dcol), p(val), None, None, ctypes.byref(count), None, None,
+                                    ctypes.c_int64(0), None, None)
+    return rc, count.value
+{body}
+"""
+    _lib.lib()  # (built)
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                          env=dict(os.environ, OMP_NUM_THREADS="4", MALLOC_MMAP_THRESHOLD_="65536", MALLOC_ARENA_MAX="1"))
+    assert done.returncode == 0, (done.returncode, done.stdout, done.stderr[-300:])
+    return done.stdout
+
+
+def test_one_team_of_threads_makes_both_schedules():
+    """Beside the calling thread's team (4 with it) there is one thread more, not a second team."""
+    said = _run_on_pairs(12_000, 100, """
+base, most, done = threading.active_count(), 0, False
+def watch():
+    global most
+    while not done:
+        most = max(most, len(os.listdir("/proc/self/task")))
+before = len(os.listdir("/proc/self/task"))
+watcher = threading.Thread(target=watch)
+watcher.start()
+for _ in range(20):
+    assert lifted() == (0, pairs)
+done = True
+watcher.join()
+print(most - before - 1)
+""")
+    assert 1 <= int(said) <= 3 + 1
+
+
+def test_a_plan_without_memory_for_lifted_rows_goes_by_its_tree():
+    """With less and less memory: both schedules, then the tree's alone, then an error."""
+    said = _run_on_pairs(200_000, 10, """
+assert lifted() == (0, pairs)
+used = int(next(s for s in open("/proc/self/status") if s.startswith("VmSize")).split()[1]) * 1024
+hard = resource.getrlimit(resource.RLIMIT_AS)[1]
+seen = []
+for room in range(600, 0, -8):  # bytes a row
+    resource.setrlimit(resource.RLIMIT_AS, (used + room * n, hard))
+    rc, count = lifted()
+    resource.setrlimit(resource.RLIMIT_AS, (hard, hard))
+    assert rc == 0 or b"memory" in L.cbm_b200_last_error()
+    seen.append((rc, count if rc == 0 else 0))
+    if rc:
+        break
+print(sorted(set(seen)) == [(0, 0), (0, pairs), (seen[-1][0], 0)], sorted(set(seen)))
+""")
+    assert said.startswith("True"), said
