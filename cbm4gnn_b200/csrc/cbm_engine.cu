@@ -2223,6 +2223,7 @@ i32 one_round_group(i32 n_prefix, i32 n_waiting, i64 n_slabs, i64 warps) {
 
 int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, const float* x, i64 ldx, const float* y, i64 ldy,
              i32 f, int mode, bool may_pack, bool in_turn, LaunchCfg& c) {
+    c = LaunchCfg{};  // (it may hold what was found for another schedule)
     const bool y_vec = ldy % 4 == 0 && aligned16(y);
     const bool x_vec = ldx % 4 == 0 && aligned16(x) && ldx < (i64)1 << 30;
     // An operand whose rows are not 16-byte aligned can only be fetched 4 bytes a lane, at less than half

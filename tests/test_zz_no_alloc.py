@@ -115,3 +115,27 @@ def test_what_is_refused_does_not_depend_on_how_finely_rows_are_cut(make, alpha)
         # an unaligned operand of this size is copied to aligned rows by the ordinary entry point, and its sums are added
         # in another order where the last slab is narrow: within fp32 rounding of the longest row
         torch.testing.assert_close(got, want, atol=0 if not unaligned else 1e-5, rtol=0 if not unaligned else 1e-5)
+
+
+@pytest.mark.parametrize("f", [16, 64, 128])
+def test_more_claims_by_the_lifted_rows_than_by_the_tree(f):
+    """37 000 rows and 1 500 children that are lifted: by the tree one round of claims does (fewer than 256 rows for each of
+    148 SMs wait for nobody), as the product goes there are more."""
+    L = _lib.lib()
+    roots, children = 37_000, 1_500
+    n = roots + children
+    mst_row = np.full(n + 2, children, np.int32)
+    mst_row[:children + 1] = np.arange(children + 1)
+    mst_row[n + 1] = n
+    mst_col = np.concatenate([np.arange(roots, n), np.arange(roots)]).astype(np.int32)
+    crow = np.concatenate([[0], np.cumsum(np.where(np.arange(n) < roots, 3, 2))]).astype(np.int32)
+    col = np.concatenate([(np.arange(roots)[:, None] + [0, 1, 2]).ravel(), (np.arange(children)[:, None] + [3, 4]).ravel()])
+    c = cbm_matrix.from_arrays(mst_row, mst_col, crow, col.astype(np.int32), np.ones(len(col), np.float32))
+    x = torch.randn((n, f), generator=torch.Generator(device="cuda").manual_seed(f), device="cuda")
+    y = torch.full((n, f), float("nan"), device="cuda")
+    want = x.double()[:roots] + x.double()[1:roots + 1] + x.double()[2:roots + 2]
+    want = torch.cat([want, want[:children] + x.double()[3:children + 3] + x.double()[4:children + 4]])
+    for _ in range(2):
+        _call(L.cbm_b200_spmm_update_static, c.plan(0), x, y.fill_(float("nan")), f, 0)
+        c.plan(0).status()
+        torch.testing.assert_close(y.double(), want, atol=1e-5, rtol=1e-5)  # (sums of five)
