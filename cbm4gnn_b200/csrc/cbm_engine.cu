@@ -1231,6 +1231,12 @@ struct DeviceSchedule {
     Chunk* d_chunks = nullptr;
 };
 
+void free_schedule(const DeviceSchedule& d) {
+    cudaFree(d.d_desc);
+    cudaFree(d.d_ent);
+    cudaFree(d.d_chunks);
+}
+
 struct cbm_b200_plan {
     int device = 0;
     i32 n = 0;
@@ -1371,11 +1377,8 @@ extern "C" void cbm_b200_plan_destroy(cbm_b200_plan* p) {
         cudaStreamSynchronize(p->own_stream);
         pool_leave(p->device);
     }
-    for (const DeviceSchedule* d : {&p->tree, &p->lifted}) {
-        cudaFree(d->d_desc);
-        cudaFree(d->d_ent);
-        cudaFree(d->d_chunks);
-    }
+    free_schedule(p->tree);
+    free_schedule(p->lifted);
     cudaFree(p->d_counter);
     cudaFree(p->d_status);
     cudaFreeHost(p->bounce);
@@ -2086,7 +2089,14 @@ int plan_from_schedules(Schedule& tree, Schedule& lifted, int32_t n, int32_t n_o
     int sms = 0;  // (the one attribute: all properties together take milliseconds)
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) == cudaSuccess) p->sm_count = sms;
     int rc = upload_schedule(tree, p->tree, p->device_bytes);
-    if (rc == CBM_B200_OK && !lifted.desc.empty()) rc = upload_schedule(lifted, p->lifted, p->device_bytes);
+    const i64 tree_bytes = p->device_bytes;
+    const auto without_lifted = [&] {  // the plan does without that schedule where the device has no room for it
+        free_schedule(p->lifted);
+        cudaGetLastError();
+        p->lifted = DeviceSchedule();
+        p->device_bytes = tree_bytes;
+    };
+    if (rc == CBM_B200_OK && !lifted.desc.empty() && upload_schedule(lifted, p->lifted, p->device_bytes) != CBM_B200_OK) without_lifted();
     if (rc == CBM_B200_OK) {
         cudaError_t e = cudaMalloc((void**)&p->d_counter, 2 * sizeof(u64));
         if (e == cudaSuccess) e = cudaMemset(p->d_counter, 0, 2 * sizeof(u64));
@@ -2102,8 +2112,17 @@ int plan_from_schedules(Schedule& tree, Schedule& lifted, int32_t n, int32_t n_o
         p->in_pool = rc == CBM_B200_OK;
     }
     // ready flags for operands of up to 512 columns and parked sums for one slab: most products then allocate nothing
-    if (rc == CBM_B200_OK) rc = grow(p, p->d_flags, p->flags_cap, 4 * (i64)std::max(p->tree.n_items, p->lifted.n_items), true, p->own_stream);
-    if (rc == CBM_B200_OK) rc = grow(p, p->d_scratch, p->scratch_cap, (i64)std::max(p->tree.n_partial, p->lifted.n_partial) * DEFAULT_SLAB, false, p->own_stream);
+    const auto first_room = [&] {
+        const int bad = grow(p, p->d_flags, p->flags_cap, 4 * (i64)std::max(p->tree.n_items, p->lifted.n_items), true, p->own_stream);
+        return bad ? bad : grow(p, p->d_scratch, p->scratch_cap, (i64)std::max(p->tree.n_partial, p->lifted.n_partial) * DEFAULT_SLAB, false, p->own_stream);
+    };
+    if (rc == CBM_B200_OK) rc = first_room();
+    if (rc != CBM_B200_OK && p->in_pool && p->lifted.n_items > 0) {
+        const i64 beside = p->flags_cap * (i64)sizeof(i32) + p->scratch_cap * (i64)sizeof(float) + 16;
+        without_lifted();
+        p->device_bytes += beside;
+        rc = first_room();
+    }
     if (rc != CBM_B200_OK) {
         const std::string keep = cbm::last_error_slot();
         cbm_b200_plan_destroy(p);
@@ -2196,6 +2215,7 @@ struct LaunchCfg {
     bool chunked = false;      // the clustered plan's kernel
     i64 need_flags = 0;        // int32 words
     i64 need_scratch = 0;      // floats
+    i64 need_pack = 0;         // floats
     bool in_turn = false;      // see KParams
     bool pack = false;         // the operand is first copied to 16-byte aligned rows
     bool ragged = false;       // 16-byte fetches, but rows of y are not aligned or end inside a vector
@@ -2284,6 +2304,7 @@ int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, c
     c.n_claims = (i64)c.claims_per_slab * c.sh.n_slabs;
     c.need_flags = (i64)c.sh.n_slabs * d.n_items;
     c.need_scratch = (i64)c.sh.n_slabs * d.n_partial * c.sh.slab_w;
+    c.need_pack = c.pack ? (i64)p->n_labels * ((f + 3) / 4 * 4) : 0;
     if (c.need_flags >= (i64)1 << 31)
         return cbm::fail(CBM_B200_ERR_ARG, std::string(who) + ": rows x column slabs exceeds 2^31 work items");
     return CBM_B200_OK;
@@ -2386,10 +2407,9 @@ int launch_frugal(KParams& kp, i32 out, i32 segment, int sm_count, cudaStream_t 
     return CBM_B200_OK;
 }
 
-int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
+int launch_plan(cbm_b200_plan* p, const DeviceSchedule& d, const LaunchCfg& c, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
                 int mode, bool use_scale, u64* counter, i32* flags, float* scratch, i32 epoch,
                 cudaStream_t s, const Bcast* bc = nullptr) {
-    const DeviceSchedule& d = p->schedule_for(mode);
     KParams kp{};
     kp.y_vec = ldy % 4 == 0 && aligned16(y);
     kp.in_turn = c.in_turn;
@@ -2456,6 +2476,21 @@ int launch_plan(cbm_b200_plan* p, const LaunchCfg& c, const float* x, i64 ldx, f
     return launch_regs<4, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
 }
 
+bool has_room(const cbm_b200_plan* p, const LaunchCfg& c) {
+    return c.need_flags <= p->flags_cap && c.need_scratch <= p->scratch_cap && c.need_pack <= p->pack_cap;
+}
+
+int make_room(cbm_b200_plan* p, const LaunchCfg& c, cudaStream_t s) {
+    int rc = grow(p, p->d_flags, p->flags_cap, c.need_flags, true, s);
+    if (rc == CBM_B200_OK) rc = grow(p, p->d_scratch, p->scratch_cap, c.need_scratch, false, s);
+    return rc ? rc : grow(p, p->d_pack, p->pack_cap, c.need_pack, false, s);
+}
+
+bool is_captured(cudaStream_t s) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
+}
+
 int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
              int mode, bool use_scale, cudaStream_t s, const Bcast* bc = nullptr, bool in_turn = false) {
     if (!p) return cbm::fail(CBM_B200_ERR_ARG, std::string(who) + ": NULL plan");
@@ -2469,11 +2504,15 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (p->n_rows == 0) return CBM_B200_OK;
     DeviceGuard g(p->device);
     LaunchCfg c;
-    rc = plan_cfg(p, p->schedule_for(mode), who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
-    if (rc) return rc;
-
-    if ((rc = grow(p, p->d_flags, p->flags_cap, c.need_flags, true, s))) return rc;
-    if ((rc = grow(p, p->d_scratch, p->scratch_cap, c.need_scratch, false, s))) return rc;
+    const DeviceSchedule* d = &p->schedule_for(mode);
+    rc = plan_cfg(p, *d, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
+    // With rows lifted out of the tree a product may have more sums to park: where they find no room, it goes by the tree.
+    if (d != &p->tree && (rc || (!has_room(p, c) && (is_captured(s) || make_room(p, c, s))))) {
+        (void)cudaGetLastError();
+        d = &p->tree;
+        rc = plan_cfg(p, *d, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
+    }
+    if (rc || (rc = make_room(p, c, s))) return rc;
     if (p->epoch == INT32_MAX) {  // epochs exhausted: start over on clean flags
         CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)p->flags_cap * sizeof(i32), s));
         p->epoch = 0;
@@ -2481,13 +2520,12 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (c.pack) {
         const i32 vecs = (f + 3) / 4;
         const i64 n_vec = (i64)p->n_labels * vecs;
-        if ((rc = grow(p, p->d_pack, p->pack_cap, 4 * n_vec, false, s))) return rc;
         cbm::launch_next(pack_rows_kernel, (unsigned)((n_vec + 255) / 256), 256, 0, s, x, ldx, p->d_pack, f, vecs, n_vec);
         CBM_CUDA(cudaGetLastError());
         x = p->d_pack;
         ldx = 4 * (i64)vecs;
     }
-    return launch_plan(p, c, x, ldx, y, ldy, f, mode, use_scale, p->d_counter, p->d_flags, p->d_scratch,
+    return launch_plan(p, *d, c, x, ldx, y, ldy, f, mode, use_scale, p->d_counter, p->d_flags, p->d_scratch,
                        ++p->epoch, s, bc);
 }
 
@@ -2959,7 +2997,7 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     // counters and flags must start at zero; the partial sums are written before they are read
     CBM_CUDA(cudaMemsetAsync(base, 0, (size_t)(off_flags + c.need_flags * (i64)sizeof(i32)), s));
     // flags were just cleared, so any non-zero mark will do as this launch's epoch
-    return launch_plan(p, c, x, ldx, y, ldy, f, MODE_FUSED, normalized != 0,
+    return launch_plan(p, p->schedule_for(MODE_FUSED), c, x, ldx, y, ldy, f, MODE_FUSED, normalized != 0,
                        reinterpret_cast<u64*>(base), reinterpret_cast<i32*>(base + off_flags),
                        reinterpret_cast<float*>(base + off_slots), 1, s);
 }

@@ -82,3 +82,29 @@ def test_captured_branches_that_join(matrix):
     torch.cuda.synchronize()
     assert np.isfinite(float(want.norm()))
     assert torch.equal(got, want * 4)  # (of powers of two, nothing is rounded)
+
+
+def test_first_product_of_a_plan_may_be_a_captured_one():
+    """Two column slabs of rows that park no sums by the tree: 100 roots of 60 entries, children with 50 more, 1 000 short
+    rows.  Lifted, the children are cut in two and would need more workspace than a plan begins with."""
+    roots, short = 100, 1000
+    n = 2 * roots + short
+    mst_row = np.full(n + 2, roots, np.int32)
+    mst_row[:roots + 1] = np.arange(roots + 1)
+    mst_row[n + 1] = n
+    mst_col = np.concatenate([np.arange(roots, 2 * roots), np.arange(roots), np.arange(2 * roots, n)]).astype(np.int32)
+    rows = [np.arange(60) + i for i in range(roots)] + [np.arange(60, 110) + i for i in range(roots)] + [np.arange(3) + i for i in range(short)]
+    crow = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int32)
+    col = np.concatenate(rows).astype(np.int32)
+    c = cbm_matrix.from_arrays(mst_row, mst_col, crow, col, np.ones(len(col), np.float32))
+    x = torch.randn((n, 256), generator=torch.Generator(device="cuda").manual_seed(1), device="cuda")
+    y = torch.empty_like(x)
+    c.plan(0)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        c.omp_mkl_csr_spmm_update(x, y)
+    graph.replay()
+    c.plan(0).status()
+    want = torch.stack([x.double()[torch.from_numpy(r).cuda()].sum(0) for r in rows])
+    want[roots:2 * roots] += want[:roots]
+    torch.testing.assert_close(y.double(), want, atol=1e-4, rtol=1e-4)
