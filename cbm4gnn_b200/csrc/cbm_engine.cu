@@ -2517,6 +2517,9 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
         CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)p->flags_cap * sizeof(i32), s));
         p->epoch = 0;
     }
+    // A graph launches this very epoch each time: its flags are cleared as part of it, lest a row takes its parent's row or
+    // parked sums of the launch before for this one's.
+    if (d->n_items > d->n_prefix && is_captured(s)) CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)c.need_flags * sizeof(i32), s));
     if (c.pack) {
         const i32 vecs = (f + 3) / 4;
         const i64 n_vec = (i64)p->n_labels * vecs;

@@ -108,3 +108,37 @@ def test_first_product_of_a_plan_may_be_a_captured_one():
     want = torch.stack([x.double()[torch.from_numpy(r).cuda()].sum(0) for r in rows])
     want[roots:2 * roots] += want[:roots]
     torch.testing.assert_close(y.double(), want, atol=1e-4, rtol=1e-4)
+
+
+@pytest.mark.parametrize("f", [16, 64, 256])
+@pytest.mark.parametrize("entry", ["spmm_update", "update"])
+def test_a_captured_product_waits_in_every_replay(entry, f):
+    """A chain of rows, each of which waits for the one before: replays see their own launch's rows, not those that the
+    replay before left."""
+    n = 1500
+    ei = np.stack([np.repeat(np.arange(n), np.arange(1, n + 1)), np.concatenate([np.arange(i + 1) for i in range(n)])])
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=0)
+    x = torch.randn((n, f), generator=torch.Generator(device="cuda").manual_seed(f), device="cuda")
+    y = torch.empty_like(x)
+
+    def work():
+        if entry == "update":
+            c.seq_mkl_csr_spmm(x, y)
+            c.omp_mkl_csr_update(y)
+        else:
+            c.omp_mkl_csr_spmm_update(x, y)
+
+    work()  # workspaces grow outside the capture
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        work()
+    for scale in (1.0, -2.0, 0.5):
+        x.mul_(scale)
+        for _ in range(2):
+            y.fill_(float("nan"))
+            graph.replay()
+            got = y.clone()
+            work()
+            c.plan(0).status()
+            assert torch.equal(got, y)
+        torch.testing.assert_close(got.double(), x.double().cumsum(0), atol=1e-3, rtol=1e-4)  # (sums of up to 1 500)
