@@ -61,6 +61,7 @@ EXPORTED = [
     "cbm_b200_csr_schedule_as_planned",
     "cbm_b200_schedule_lifted",
     "cbm_b200_plan_schedule",
+    "cbm_b200_plan_product_schedule",
     "cbm_b200_plan_info",
     "cbm_b200_one_round_group",
     "cbm_b200_plan_tune",
@@ -190,7 +191,8 @@ def lib() -> ctypes.CDLL:
     sig("cbm_b200_csr_schedule_as_planned", c_int32, c_int32, c_int32, *[c_void_p] * 4, i32p, i32p, i32p, i32p, i32p,
         POINTER(c_uint64))
     sig("cbm_b200_schedule_lifted", c_int32, c_int32, *[c_void_p] * 7, i32p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p)
-    sig("cbm_b200_plan_schedule", c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
+    for name in ("cbm_b200_plan_schedule", "cbm_b200_plan_product_schedule"):
+        sig(name, c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
     sig("cbm_b200_plan_info", c_int32, c_void_p, i32p, POINTER(c_int64), i32p, i32p,
         POINTER(c_int64))
     sig("cbm_b200_one_round_group", c_int32, c_int32, c_int32, c_int32, c_int32)

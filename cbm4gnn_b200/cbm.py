@@ -85,10 +85,13 @@ class _Plan:
     def tune(self, slab_width=0, n_blocks=0, host_chunk=0, form=0):
         _lib.check(_lib.lib().cbm_b200_plan_tune(self.handle, slab_width, n_blocks, host_chunk, form))
 
-    def schedule(self) -> dict:
-        """The schedule's sizes and fingerprint (include/cbm_b200.h, cbm_b200_plan_schedule)."""
+    def schedule(self, in_one_pass: bool = False) -> dict:
+        """Sizes and fingerprint of the tree's schedule or of the one that the product in one pass goes by
+        (include/cbm_b200.h, cbm_b200_plan_schedule and cbm_b200_plan_product_schedule)."""
         sizes, mark = [ctypes.c_int32() for _ in range(5)], ctypes.c_uint64()
-        _lib.check(_lib.lib().cbm_b200_plan_schedule(self.handle, *map(ctypes.byref, sizes), ctypes.byref(mark)))
+        L = _lib.lib()
+        of = L.cbm_b200_plan_product_schedule if in_one_pass else L.cbm_b200_plan_schedule
+        _lib.check(of(self.handle, *map(ctypes.byref, sizes), ctypes.byref(mark)))
         names = "n_items", "n_prefix", "n_partial", "n_chunks", "segment"
         return dict(zip(names, (v.value for v in sizes)), fingerprint=mark.value)
 

@@ -2146,10 +2146,9 @@ extern "C" int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64
     return CBM_B200_OK;
 }
 
-extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
-                                      int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
-    if (!p) return cbm::fail(CBM_B200_ERR_ARG, "plan_schedule: NULL plan");
-    const DeviceSchedule& d = p->tree;
+namespace {
+int schedule_of(const cbm_b200_plan* p, const DeviceSchedule& d, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+                int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
     if (n_items) *n_items = d.n_items;
     if (n_prefix) *n_prefix = d.n_prefix;
     if (n_partial) *n_partial = d.n_partial;
@@ -2163,6 +2162,19 @@ extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, 
         *fingerprint = fingerprint_of(desc.get(), (size_t)d.n_items);
     }
     return CBM_B200_OK;
+}
+}  // namespace
+
+extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+                                      int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
+    if (!p) return cbm::fail(CBM_B200_ERR_ARG, "plan_schedule: NULL plan");
+    return schedule_of(p, p->tree, n_items, n_prefix, n_partial, n_chunks, segment, fingerprint);
+}
+
+extern "C" int cbm_b200_plan_product_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+                                              int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
+    if (!p) return cbm::fail(CBM_B200_ERR_ARG, "plan_product_schedule: NULL plan");
+    return schedule_of(p, p->schedule_for(MODE_FUSED), n_items, n_prefix, n_partial, n_chunks, segment, fingerprint);
 }
 
 extern "C" int cbm_b200_plan_tune(cbm_b200_plan* p, int32_t slab_width, int32_t n_blocks,

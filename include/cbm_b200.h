@@ -171,6 +171,11 @@ int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64_t* n_delta
 int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
                            int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
 
+/* The same of the schedule that the product in one pass goes by: with rows lifted out of the tree where the plan has such a
+ * one, otherwise the tree's. */
+int cbm_b200_plan_product_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+                                   int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
+
 /* The rule by which a product draws its claims in one round, each warp once: how many of the n_prefix items that never wait
  * a warp takes of each of n_slabs column slabs, of which each has n_waiting further items for a warp of their own, when
  * `warps` warps are resident.  0: more than one round.  Needs no GPU. */

@@ -8,17 +8,25 @@ import torch
 
 from cbm4gnn_b200 import _lib, graphs
 from cbm4gnn_b200.cbm import cbm_matrix
-from helpers import sparse_product, with_self_loops
+from helpers import chains, near_cliques, sparse_product, waiting_rows, with_self_loops
 
 pytestmark = pytest.mark.gpu
 TOL = dict(atol=1e-4, rtol=1e-4)
 
 
-@pytest.fixture(scope="module")
-def copy_graph():
-    ei = with_self_loops(graphs.copy_model(3000, 0.9, 8, 11))
+@pytest.fixture(scope="module", params=["split rows", "waiting rows"])
+def copy_graph(request):
+    """Split rows, and rows that wait in the tree but not in the product in one pass, which has them lifted; or a split row and
+    a chain of rows that wait there too."""
+    if request.param == "split rows":
+        ei = with_self_loops(graphs.copy_model(3000, 0.9, 8, 11))
+    else:
+        rest = np.arange(500, 1100)
+        ei = np.concatenate([chains(500, 1), np.stack([rest, rest]), np.stack([np.full(400, 500), np.arange(600, 1000)])], axis=1)
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
     assert (np.diff(c._crow) > 192).any() and c.build_info["depth"] > 2  # split rows and waiting rows
+    made = c.plan(0).schedule(in_one_pass=True)
+    assert made["n_partial"] > 0 and (waiting_rows(c) > 300) == (request.param == "waiting rows")
     return ei, c
 
 
@@ -49,12 +57,16 @@ def test_widths_and_pitches(copy_graph, f, aligned_x, aligned_y):
     torch.testing.assert_close(c.seq_torch_csr_fused_matmul(xd), yd, atol=0, rtol=1e-6)
 
 
-@pytest.fixture(scope="module", params=[2, 40])
+@pytest.fixture(scope="module", params=[2, 40, "near cliques"])
 def community_graph(request):
     """Enough rows with common columns that the plan works on them community by community (16 384 and more); with 40
-    expected links per node rows also share a parent, so that some of them wait."""
+    expected links per node rows also share a parent, so that some of them wait in the tree; near cliques' rows wait in the
+    product in one pass too."""
     n = 16384 + 5
-    ei = with_self_loops(graphs.stochastic_block_model(n, 400, 3.5, 0.8, 8.0 if request.param == 2 else 40.0, 1.0, 5))
+    if request.param == "near cliques":
+        ei = near_cliques(n, 80, 0.1, 5)
+    else:
+        ei = with_self_loops(graphs.stochastic_block_model(n, 400, 3.5, 0.8, 8.0 if request.param == 2 else 40.0, 1.0, 5))
     ei = np.concatenate([ei, [[7] * 700, list(range(1000, 1700))]], axis=1)  # one row that is split
     key = np.unique(ei[0] * n + ei[1])
     ei = np.stack([key // n, key % n])
@@ -62,6 +74,8 @@ def community_graph(request):
     made = c.plan(0).schedule()
     assert made["n_chunks"] > 0 and made["n_partial"] > 0 and made["n_items"] > made["n_prefix"]
     assert request.param == 2 or c.build_info["depth"] > 1
+    in_one_pass = c.plan(0).schedule(in_one_pass=True)
+    assert in_one_pass["n_chunks"] > 0 and (waiting_rows(c) > 8000) == (request.param == "near cliques")
     return ei, c
 
 
@@ -128,11 +142,12 @@ def test_rows_side_by_side(many_rows, f, pad):
 def test_plans_of_one_graph_are_the_same(n, mu, deg_in):
     ei = with_self_loops(graphs.stochastic_block_model(n, n // 50, mu, 0.8, deg_in, 3.0, 5))
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True, build_device=0)
-    first = c.plan(0).schedule()
+    first, in_one_pass = c.plan(0).schedule(), c.plan(0).schedule(in_one_pass=True)
     assert first["n_chunks"] > 0  # rows in the order of communities found on the GPU
+    assert in_one_pass["n_chunks"] > 0 and in_one_pass["fingerprint"] != first["fingerprint"]  # (with rows lifted)
     for _ in range(4):
         c._plans.clear()
-        assert c.plan(0).schedule() == first
+        assert c.plan(0).schedule() == first and c.plan(0).schedule(in_one_pass=True) == in_one_pass
 
 
 @pytest.mark.parametrize("rows,f,aligned,slab", [(4, 1_000_000, True, 0), (4, 909_312, True, 0), (4, 909_440, True, 0), (6, 300_000, False, 0),

@@ -6,7 +6,7 @@ import torch
 
 from cbm4gnn_b200 import dense, graphs
 from cbm4gnn_b200.cbm import cbm_matrix
-from helpers import with_self_loops
+from helpers import chains, near_cliques, waiting_rows, with_self_loops
 
 pytestmark = pytest.mark.gpu
 
@@ -37,10 +37,25 @@ def _chain(c, f, after):
     return seen
 
 
-@pytest.fixture(scope="module", params=["waiting rows", "communities"])
+# kind of graph: rows, whether rows wait for a parent in the product in one pass, whether the plan is in community order
+KINDS = {"split rows": (3000, False, False), "few communities": (11793, False, False), "chains": (2800, True, False),
+         "communities": (70_000, False, True), "near cliques": (17_000, True, True)}
+
+
+@pytest.fixture(scope="module", params=KINDS)
 def matrix(request):
-    ei = with_self_loops(graphs.copy_model(3000, 0.9, 8, 11) if request.param == "waiting rows" else graphs.make_graph("c3", scale=0.05))
-    return cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
+    ei = {"split rows": lambda: graphs.copy_model(3000, 0.9, 8, 11), "few communities": lambda: graphs.make_graph("c3", scale=0.05),
+          "chains": lambda: chains(400, 7), "communities": lambda: graphs.stochastic_block_model(70_000, 1400, 3.5, 0.8, 12.0, 3.0, 5),
+          "near cliques": lambda: near_cliques(17_000, 80, 0.1, 5)}[request.param]()
+    ei = ei if KINDS[request.param][1] else with_self_loops(ei)
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True, build_device=0)
+    made, (rows, waits, clustered) = c.plan(0).schedule(in_one_pass=True), KINDS[request.param]
+    assert c.num_rows == rows and (made["n_chunks"] > 0) == clustered
+    # Rows that wait: the normalized wait; in community order, on up to 65 536 rows or from 65 columns on: the chunk kernel's.
+    assert (waiting_rows(c) > 1000) == waits
+    # Up to 64 columns, more than 65 536 rows and 256 for each of 148 SMs that never wait: the staged narrow kernel.
+    assert request.param != "communities" or rows > 65_536 and made["n_prefix"] - made["n_partial"] >= 37_888
+    return c
 
 
 # widths: row groups of a few lanes, two odd pitches (the operand is copied to aligned rows first), whole slabs, several
