@@ -165,3 +165,35 @@ def test_more_slabs_than_warps(rows, f, aligned, slab):
     c.omp_mkl_csr_fused_spmm_update(xd, yd)
     c.plan(0).status()
     np.testing.assert_allclose(yd.cpu().numpy(), sparse_product(ei, x, True), **TOL)
+
+
+@pytest.fixture(scope="module")
+def waiting_chains():
+    """So many waiting rows (a quarter of the resident warps and more) that claims are drawn in more than one round, and one
+    row that is split."""
+    ei = chains(400, 7)
+    rest = np.arange(2800, 3400)
+    ei = np.concatenate([ei, np.stack([rest, rest]), np.stack([np.full(400, 2800), np.arange(2900, 3300)])], axis=1)
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
+    assert waiting_rows(c) > 1776 and c.plan(0).schedule(in_one_pass=True)["n_partial"] > 0
+    return ei, c
+
+
+@pytest.mark.parametrize("slab,form", [(0, 0), (64, 0), (256, 0), (512, 0), (0, 1)])
+@pytest.mark.parametrize("f,pad", [(512, 0), (512, 1), (515, 0), (40, 0)])
+def test_every_form_waits(waiting_chains, slab, form, f, pad):
+    """One, two and four vectors or values a lane, aligned and not, bulk copies, and the allocation-free product."""
+    ei, c = waiting_chains
+    x = np.random.default_rng(f).standard_normal((c.num_rows, f)).astype(np.float32)
+    xd, yd, static = (_buffer(c.num_rows, f, f + pad) for _ in range(3))
+    xd.copy_(torch.from_numpy(x))
+    c.plan(0).tune(slab_width=slab, form=form)
+    try:
+        c.omp_mkl_csr_fused_spmm_update(xd, yd)
+        _lib.check(_lib.lib().cbm_b200_spmm_update_static(c.plan(0).handle, xd.data_ptr(), f + pad, static.data_ptr(), f + pad, f, 1,
+                                                          torch.cuda.current_stream().cuda_stream))
+        c.plan(0).status()
+    finally:
+        c.plan(0).tune()
+    np.testing.assert_allclose(yd.cpu().numpy(), sparse_product(ei, x, True), **TOL)
+    torch.testing.assert_close(static, yd, **TOL)
