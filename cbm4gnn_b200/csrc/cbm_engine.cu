@@ -2098,8 +2098,8 @@ int plan_from_schedules(Schedule& tree, Schedule& lifted, int32_t n, int32_t n_o
     };
     if (rc == CBM_B200_OK && !lifted.desc.empty() && upload_schedule(lifted, p->lifted, p->device_bytes) != CBM_B200_OK) without_lifted();
     if (rc == CBM_B200_OK) {
-        cudaError_t e = cudaMalloc((void**)&p->d_counter, 2 * sizeof(u64));
-        if (e == cudaSuccess) e = cudaMemset(p->d_counter, 0, 2 * sizeof(u64));
+        cudaError_t e = cudaMalloc((void**)&p->d_counter, sizeof(u64));
+        if (e == cudaSuccess) e = cudaMemset(p->d_counter, 0, sizeof(u64));
         if (e == cudaSuccess) e = cudaMalloc((void**)&p->d_status, sizeof(i32));
         if (e == cudaSuccess) e = cudaMemset(p->d_status, 0, sizeof(i32));
         if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&p->own_stream, cudaStreamNonBlocking);
