@@ -191,8 +191,8 @@ def lib() -> ctypes.CDLL:
     sig("cbm_b200_csr_schedule_as_planned", c_int32, c_int32, c_int32, *[c_void_p] * 4, i32p, i32p, i32p, i32p, i32p,
         POINTER(c_uint64))
     sig("cbm_b200_schedule_lifted", c_int32, c_int32, *[c_void_p] * 7, i32p, c_void_p, c_void_p, c_int64, c_void_p, c_void_p)
-    for name in ("cbm_b200_plan_schedule", "cbm_b200_plan_product_schedule"):
-        sig(name, c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
+    sig("cbm_b200_plan_schedule", c_int32, c_void_p, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
+    sig("cbm_b200_plan_product_schedule", c_int32, c_void_p, c_int32, i32p, i32p, i32p, i32p, i32p, POINTER(c_uint64))
     sig("cbm_b200_plan_info", c_int32, c_void_p, i32p, POINTER(c_int64), i32p, i32p,
         POINTER(c_int64))
     sig("cbm_b200_one_round_group", c_int32, c_int32, c_int32, c_int32, c_int32)

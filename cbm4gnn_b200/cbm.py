@@ -85,13 +85,14 @@ class _Plan:
     def tune(self, slab_width=0, n_blocks=0, host_chunk=0, form=0):
         _lib.check(_lib.lib().cbm_b200_plan_tune(self.handle, slab_width, n_blocks, host_chunk, form))
 
-    def schedule(self, in_one_pass: bool = False) -> dict:
-        """Sizes and fingerprint of the tree's schedule or of the one that the product in one pass goes by
+    def schedule(self, columns: int | None = None) -> dict:
+        """Sizes and fingerprint of the tree's schedule or of the one that the product in one pass of so many columns goes by
         (include/cbm_b200.h, cbm_b200_plan_schedule and cbm_b200_plan_product_schedule)."""
         sizes, mark = [ctypes.c_int32() for _ in range(5)], ctypes.c_uint64()
         L = _lib.lib()
-        of = L.cbm_b200_plan_product_schedule if in_one_pass else L.cbm_b200_plan_schedule
-        _lib.check(of(self.handle, *map(ctypes.byref, sizes), ctypes.byref(mark)))
+        out = *map(ctypes.byref, sizes), ctypes.byref(mark)
+        _lib.check(L.cbm_b200_plan_schedule(self.handle, *out) if columns is None
+                   else L.cbm_b200_plan_product_schedule(self.handle, columns, *out))
         names = "n_items", "n_prefix", "n_partial", "n_chunks", "segment"
         return dict(zip(names, (v.value for v in sizes)), fingerprint=mark.value)
 

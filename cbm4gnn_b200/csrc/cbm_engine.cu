@@ -1223,6 +1223,8 @@ struct DeviceSchedule {
     i32 n_partial = 0; // PARTIAL items = scratch slots per slab
     i32 segment = 0;   // entries of a PARTIAL item
     i32 n_chunks = 0;  // 0: not clustered
+    i32 n_waits = 0;   // rows with a parent
+    i32 depth = 0;
     i64 n_entries = 0;
     std::vector<i32> part_ends;  // see Schedule
     i32 n_partial_coarse = 0;
@@ -1244,9 +1246,28 @@ struct cbm_b200_plan {
     i32 n_out = 0;     // rows of the output shard (owned label range)
     i32 n_rows = 0;    // rows actually computed
     // The structure's own schedule, and the one with rows lifted out of the tree (cbm_lift.cpp), which the product in
-    // one pass goes by where there is one.  The halves of the product (delta product, update) need the tree itself.
+    // one pass goes by where there is one that pays at `f` columns.  The halves of the product (delta product, update) need
+    // the tree itself.
     DeviceSchedule tree, lifted;
-    const DeviceSchedule& schedule_for(i32 mode) const { return mode == MODE_FUSED && lifted.n_items > 0 ? lifted : tree; }
+    const DeviceSchedule& schedule_for(i32 mode, i32 f) const {
+        return mode == MODE_FUSED && lifted.n_items > 0 && !tree_pays(f) ? lifted : tree;
+    }
+    // Rows are lifted by what entries, waits and levels cost at 128 columns (cbm_lift.cpp).  The more columns, the more the
+    // entries count, and a level as much as before: 5 000 rows of 156 entries, of which the tree saves a quarter, 128 columns
+    // lifted 30 us, by the tree 37, 256 columns 60 and 51, 1 024 columns 198 and 152; 20 000 rows of 74, a sixth saved, 128
+    // columns 56 and 52, 256 113 and 91.  Where rows are short, they have too little to gather while they wait (8 000 rows of 65 in
+    // communities, 40 by the tree, 1 024 columns 126 and 187; 5 000 of 37, 13 by the tree, 57 and 82; 100 000 of 40, 36 by the
+    // tree, 256 columns 238 and 255), and in community order lifted rows are faster at all widths (17 000 rows of 59, 32
+    // by the tree, 1 024 columns 198 and 295).
+    bool long_rows() const { return tree.n_entries >= 48 * (i64)n_rows; }
+    bool tree_pays(i32 f) const {
+        if (lifted.n_chunks > 0 || !long_rows()) return false;
+        const i64 slabs = (f + 127) / 128;
+        const auto cost = [&](const DeviceSchedule& d) {
+            return (d.n_entries + 4 * (i64)d.n_waits) * slabs + (d.depth > 1 ? 25000 * (i64)d.depth : 0);
+        };
+        return cost(tree) < cost(lifted);
+    }
     float* d_scratch = nullptr;
     i64 scratch_cap = 0;
     i64 n_delta = 0;
@@ -2059,6 +2080,8 @@ int upload_schedule(Schedule& sch, DeviceSchedule& d, i64& bytes) {
     d.part_ends.swap(sch.part_ends);
     d.n_partial_coarse = sch.n_partial_coarse;
     d.n_entries = sch.n_delta;
+    d.n_waits = sch.n_rows_owned - sch.n_root_children;
+    d.depth = sch.depth;
     d.n_chunks = (i32)sch.chunks.size();
     int rc = upload(&d.d_desc, sch.desc.data(), sch.desc.size(), bytes);
     if (rc == CBM_B200_OK) rc = upload(&d.d_ent, sch.ent.get(), (size_t)sch.n_ent, bytes);
@@ -2171,10 +2194,11 @@ extern "C" int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, 
     return schedule_of(p, p->tree, n_items, n_prefix, n_partial, n_chunks, segment, fingerprint);
 }
 
-extern "C" int cbm_b200_plan_product_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
-                                              int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
+extern "C" int cbm_b200_plan_product_schedule(const cbm_b200_plan* p, int32_t f, int32_t* n_items, int32_t* n_prefix,
+                                              int32_t* n_partial, int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint) {
     if (!p) return cbm::fail(CBM_B200_ERR_ARG, "plan_product_schedule: NULL plan");
-    return schedule_of(p, p->schedule_for(MODE_FUSED), n_items, n_prefix, n_partial, n_chunks, segment, fingerprint);
+    if (f <= 0) return cbm::fail(CBM_B200_ERR_ARG, "plan_product_schedule: f must be positive");
+    return schedule_of(p, p->schedule_for(MODE_FUSED, f), n_items, n_prefix, n_partial, n_chunks, segment, fingerprint);
 }
 
 extern "C" int cbm_b200_plan_tune(cbm_b200_plan* p, int32_t slab_width, int32_t n_blocks,
@@ -2516,7 +2540,7 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     if (p->n_rows == 0) return CBM_B200_OK;
     DeviceGuard g(p->device);
     LaunchCfg c;
-    const DeviceSchedule* d = &p->schedule_for(mode);
+    const DeviceSchedule* d = &p->schedule_for(mode, f);
     rc = plan_cfg(p, *d, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
     // With rows lifted out of the tree a product may have more sums to park: where they find no room, it goes by the tree.
     if (d != &p->tree && (rc || (!has_room(p, c) && (is_captured(s) || make_room(p, c, s))))) {
@@ -2957,7 +2981,7 @@ bool fit_static(const cbm_b200_plan* p, const float* x, i64 ldx, const float* y,
     c.ragged = c.sh.v4 && !all_vec;
     const i64 per_sum = (i64)c.sh.n_slabs * (c.sh.slab_w + 1) * (i64)sizeof(i32);
     const i64 room = (i64)CBM_B200_STATIC_SCRATCH_BYTES - static_need(c.sh.n_slabs * rows, 0) - 256;
-    const DeviceSchedule& d = p->schedule_for(MODE_FUSED);
+    const DeviceSchedule& d = p->schedule_for(MODE_FUSED, f);
     const auto& ends = d.part_ends;
     const auto past = std::upper_bound(ends.begin(), ends.end(), std::max<i64>(0, room / per_sum));
     const i32 kept = past == ends.begin() ? 0 : past[-1];
@@ -2992,7 +3016,7 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     const i64 need = static_need(c.need_flags, c.need_scratch);
     const bool taken = need <= (i64)CBM_B200_STATIC_SCRATCH_BYTES || takes_static(p, x, ldx, y, ldy, f);
     if (taken) {  // (by its tree; with rows lifted out of it there may be more sums to park)
-        rc = plan_cfg(p, p->schedule_for(MODE_FUSED), who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
+        rc = plan_cfg(p, p->schedule_for(MODE_FUSED, f), who, x, ldx, y, ldy, f, MODE_FUSED, false, false, c);
         if (rc) return rc;
     }
     if (!taken || (static_need(c.need_flags, c.need_scratch) > (i64)CBM_B200_STATIC_SCRATCH_BYTES && !fit_static(p, x, ldx, y, ldy, f, c)))
@@ -3012,7 +3036,7 @@ extern "C" int cbm_b200_spmm_update_static(cbm_b200_plan* p, const float* x, int
     // counters and flags must start at zero; the partial sums are written before they are read
     CBM_CUDA(cudaMemsetAsync(base, 0, (size_t)(off_flags + c.need_flags * (i64)sizeof(i32)), s));
     // flags were just cleared, so any non-zero mark will do as this launch's epoch
-    return launch_plan(p, p->schedule_for(MODE_FUSED), c, x, ldx, y, ldy, f, MODE_FUSED, normalized != 0,
+    return launch_plan(p, p->schedule_for(MODE_FUSED, f), c, x, ldx, y, ldy, f, MODE_FUSED, normalized != 0,
                        reinterpret_cast<u64*>(base), reinterpret_cast<i32*>(base + off_flags),
                        reinterpret_cast<float*>(base + off_slots), 1, s);
 }

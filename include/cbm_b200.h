@@ -114,7 +114,7 @@ void cbm_b200_built_free(cbm_b200_built* b);
  *
  * The halves of a product (cbm_b200_delta_spmm, cbm_b200_update) go by the tree as it is given.  The product in one pass
  * may compute a row from all of its entries instead of from its parent's row, where the parent saves it few (see
- * cbm_b200_schedule_lifted): the same sums in another order.  An infinity or NaN in a column that only the parent names then
+ * cbm_b200_schedule_lifted; for operands wider than 128 columns more saved entries are worth a wait): the same sums in another order.  An infinity or NaN in a column that only the parent names then
  * stays out of the row, as in A x; taken away again from the parent's row it leaves NaN there.
  * ------------------------------------------------------------------------------------------ */
 int cbm_b200_plan_create(int32_t n, const int32_t* mst_row, const int32_t* mst_col,
@@ -171,9 +171,9 @@ int cbm_b200_plan_info(const cbm_b200_plan* p, int32_t* n_rows, int64_t* n_delta
 int cbm_b200_plan_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
                            int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
 
-/* The same of the schedule that the product in one pass goes by: with rows lifted out of the tree where the plan has such a
- * one, otherwise the tree's. */
-int cbm_b200_plan_product_schedule(const cbm_b200_plan* p, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
+/* The same of the schedule that the product in one pass of f columns goes by: with rows lifted out of the tree where the plan
+ * has such a one and it pays at that width, otherwise the tree's. */
+int cbm_b200_plan_product_schedule(const cbm_b200_plan* p, int32_t f, int32_t* n_items, int32_t* n_prefix, int32_t* n_partial,
                                    int32_t* n_chunks, int32_t* segment, uint64_t* fingerprint);
 
 /* The rule by which a product draws its claims in one round, each warp once: how many of the n_prefix items that never wait

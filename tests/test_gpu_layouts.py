@@ -25,7 +25,7 @@ def copy_graph(request):
         ei = np.concatenate([chains(500, 1), np.stack([rest, rest]), np.stack([np.full(400, 500), np.arange(600, 1000)])], axis=1)
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
     assert (np.diff(c._crow) > 192).any() and c.build_info["depth"] > 2  # split rows and waiting rows
-    made = c.plan(0).schedule(in_one_pass=True)
+    made = c.plan(0).schedule(columns=64)
     assert made["n_partial"] > 0 and (waiting_rows(c) > 300) == (request.param == "waiting rows")
     return ei, c
 
@@ -74,7 +74,7 @@ def community_graph(request):
     made = c.plan(0).schedule()
     assert made["n_chunks"] > 0 and made["n_partial"] > 0 and made["n_items"] > made["n_prefix"]
     assert request.param == 2 or c.build_info["depth"] > 1
-    in_one_pass = c.plan(0).schedule(in_one_pass=True)
+    in_one_pass = c.plan(0).schedule(columns=64)
     assert in_one_pass["n_chunks"] > 0 and (waiting_rows(c) > 8000) == (request.param == "near cliques")
     return ei, c
 
@@ -142,12 +142,12 @@ def test_rows_side_by_side(many_rows, f, pad):
 def test_plans_of_one_graph_are_the_same(n, mu, deg_in):
     ei = with_self_loops(graphs.stochastic_block_model(n, n // 50, mu, 0.8, deg_in, 3.0, 5))
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True, build_device=0)
-    first, in_one_pass = c.plan(0).schedule(), c.plan(0).schedule(in_one_pass=True)
+    first, in_one_pass = c.plan(0).schedule(), c.plan(0).schedule(columns=64)
     assert first["n_chunks"] > 0  # rows in the order of communities found on the GPU
     assert in_one_pass["n_chunks"] > 0 and in_one_pass["fingerprint"] != first["fingerprint"]  # (with rows lifted)
     for _ in range(4):
         c._plans.clear()
-        assert c.plan(0).schedule() == first and c.plan(0).schedule(in_one_pass=True) == in_one_pass
+        assert c.plan(0).schedule() == first and c.plan(0).schedule(columns=64) == in_one_pass
 
 
 @pytest.mark.parametrize("rows,f,aligned,slab", [(4, 1_000_000, True, 0), (4, 909_312, True, 0), (4, 909_440, True, 0), (6, 300_000, False, 0),
@@ -175,7 +175,7 @@ def waiting_chains():
     rest = np.arange(2800, 3400)
     ei = np.concatenate([ei, np.stack([rest, rest]), np.stack([np.full(400, 2800), np.arange(2900, 3300)])], axis=1)
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True)
-    assert waiting_rows(c) > 1776 and c.plan(0).schedule(in_one_pass=True)["n_partial"] > 0
+    assert waiting_rows(c) > 1776 and c.plan(0).schedule(columns=64)["n_partial"] > 0
     return ei, c
 
 
@@ -197,3 +197,27 @@ def test_every_form_waits(waiting_chains, slab, form, f, pad):
         c.plan(0).tune()
     np.testing.assert_allclose(yd.cpu().numpy(), sparse_product(ei, x, True), **TOL)
     torch.testing.assert_close(static, yd, **TOL)
+
+
+@pytest.mark.parametrize("n,p_copy,links,by_tree_from", [(3000, 0.95, 20, 500), (6000, 0.9, 8, 1024), (4096, 0.8, 3, None)])
+def test_wide_products_go_by_the_tree_where_it_saves_much(n, p_copy, links, by_tree_from):
+    ei = with_self_loops(graphs.copy_model(n, p_copy, links, 3))
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=4, normalized=True, build_device=0)
+    tree, narrow = c.plan(0).schedule(), c.plan(0).schedule(columns=128)
+    assert tree != narrow and waiting_rows(c) < (c._parent != c.num_rows).sum()
+    for f in (128, 500, 1024):
+        goes_by = c.plan(0).schedule(columns=f)
+        assert goes_by == (tree if by_tree_from is not None and f >= by_tree_from else narrow)
+        x = torch.randn((c.num_rows, f), generator=torch.Generator(device="cuda").manual_seed(f), device="cuda")
+        y, own, sent, static = (torch.full_like(x, float("nan")) for _ in range(4))
+        c.omp_mkl_csr_fused_spmm_update(x, y)
+        _deliver(c, x, own, sent)
+        rc = _lib.lib().cbm_b200_spmm_update_static(c.plan(0).handle, x.data_ptr(), f, static.data_ptr(), f, f, 1,
+                                                    torch.cuda.current_stream().cuda_stream)
+        c.plan(0).status()
+        np.testing.assert_allclose(y.cpu().numpy(), sparse_product(ei, x.cpu().numpy(), True), **TOL)
+        assert torch.equal(own, y) and torch.equal(sent, y)
+        if rc == 0:
+            torch.testing.assert_close(static, y, **TOL)
+        else:
+            assert b"bytes of scratch" in _lib.lib().cbm_b200_last_error()

@@ -49,7 +49,7 @@ def matrix(request):
           "near cliques": lambda: near_cliques(17_000, 80, 0.1, 5)}[request.param]()
     ei = ei if KINDS[request.param][1] else with_self_loops(ei)
     c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=2, normalized=True, build_device=0)
-    made, (rows, waits, clustered) = c.plan(0).schedule(in_one_pass=True), KINDS[request.param]
+    made, (rows, waits, clustered) = c.plan(0).schedule(columns=64), KINDS[request.param]
     assert c.num_rows == rows and (made["n_chunks"] > 0) == clustered
     # Rows that wait: the normalized wait; in community order, on up to 65 536 rows or from 65 columns on: the chunk kernel's.
     assert (waiting_rows(c) > 1000) == waits
