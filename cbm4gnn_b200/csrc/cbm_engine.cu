@@ -2325,7 +2325,10 @@ int plan_cfg(const cbm_b200_plan* p, const DeviceSchedule& d, const char* who, c
         // 47 columns 275 -> 269 us; 50 000 rows in order of length 46 -> 65).
         // A small product keeps single claims: with fewer claims than resident warps, grouping
         // only idles warps.
-        c.group = ((i64)d.n_prefix * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && d.n_chunks > 0 ? 8 : 4) : 1;
+        // (Long rows: four to a claim is too coarse for so few claims, and lifted rows do not bring it about sooner: 14 000 rows
+        // of 177 entries, 500 columns 288 us, 246 with single claims.)
+        const i32 n_apart = p->long_rows() ? std::min(d.n_prefix, p->tree.n_prefix) : d.n_prefix;
+        c.group = ((i64)n_apart * c.sh.n_slabs >= (i64)p->sm_count * 256) ? (f <= 64 && d.n_chunks > 0 ? 8 : 4) : 1;
         if (c.group == 1 && p->n_blocks == 0) {
             const i64 warps = (i64)p->sm_count * resident_blocks(c.sh, f, c.ragged, mode) * 8;
             const i32 group = one_round_group(d.n_prefix, d.n_items - d.n_prefix, c.sh.n_slabs, warps);
