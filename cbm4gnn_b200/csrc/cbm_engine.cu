@@ -2369,7 +2369,7 @@ int launch_tma(KParams& kp, int sm_count, cudaStream_t s) {
 }
 
 template <int NV, bool V4, bool RAGGED = false>
-int launch_regs(KParams& kp, bool one_round, int want_blocks, int sm_count, cudaStream_t s) {
+int launch_regs(KParams& kp, bool one_round, int want_blocks, int sm_count, const cbm::Stream& s) {
     // Unroll depth and resident blocks per SM were chosen by measurement on B200.  For the default
     // form (one float4 per lane, 128-column slabs) 4 gathers in flight per warp at 48 resident
     // warps per SM (40 registers) beat 8 in flight at 32 warps (64 registers) by 3 % on wide
@@ -2390,7 +2390,7 @@ int launch_regs(KParams& kp, bool one_round, int want_blocks, int sm_count, cuda
 // rows of y are not aligned.  Fetches in flight x resident blocks, 235 868 rows of 11 entries, 64 columns / 400 000 of
 // 22, 47 columns: 4 x 6 97 / 279 us, 6 x 5 100 / 288, 8 x 5 104 / 298, 8 x 4 110 / 310.
 template <bool RAGGED>
-int launch_narrow(KParams& kp, bool one_round, int want_blocks, int sm_count, cudaStream_t s) {
+int launch_narrow(KParams& kp, bool one_round, int want_blocks, int sm_count, const cbm::Stream& s) {
     constexpr int kResident = NARROW_RESIDENT;
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, (kp.n_claims + 7) / 8));
@@ -2403,7 +2403,7 @@ int launch_narrow(KParams& kp, bool one_round, int want_blocks, int sm_count, cu
 }
 
 template <bool RAGGED>
-int launch_chunks(KParams& kp, int want_blocks, int sm_count, cudaStream_t s) {
+int launch_chunks(KParams& kp, int want_blocks, int sm_count, const cbm::Stream& s) {
     constexpr int kResident = 3;  // 45 consumer warps per SM at 40 registers
     int blocks = want_blocks > 0 ? want_blocks : sm_count * kResident;
     blocks = (int)std::max<i64>(1, std::min<i64>(blocks, kp.n_claims));
@@ -2448,7 +2448,7 @@ int launch_frugal(KParams& kp, i32 out, i32 segment, int sm_count, cudaStream_t 
 
 int launch_plan(cbm_b200_plan* p, const DeviceSchedule& d, const LaunchCfg& c, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
                 int mode, bool use_scale, u64* counter, i32* flags, float* scratch, i32 epoch,
-                cudaStream_t s, const Bcast* bc = nullptr) {
+                const cbm::Stream& on, const Bcast* bc = nullptr) {
     KParams kp{};
     kp.y_vec = ldy % 4 == 0 && aligned16(y);
     kp.in_turn = c.in_turn;
@@ -2486,33 +2486,33 @@ int launch_plan(cbm_b200_plan* p, const DeviceSchedule& d, const LaunchCfg& c, c
     if (c.left_out > 0) {
         const i32 out = c.left_out, seg = d.segment;
         if (c.sh.v4) {
-            if (c.sh.nv == 1) return launch_frugal<1, true>(kp, out, seg, p->sm_count, s);
-            if (c.sh.nv == 2) return launch_frugal<2, true>(kp, out, seg, p->sm_count, s);
-            return launch_frugal<4, true>(kp, out, seg, p->sm_count, s);
+            if (c.sh.nv == 1) return launch_frugal<1, true>(kp, out, seg, p->sm_count, on.s);
+            if (c.sh.nv == 2) return launch_frugal<2, true>(kp, out, seg, p->sm_count, on.s);
+            return launch_frugal<4, true>(kp, out, seg, p->sm_count, on.s);
         }
-        if (c.sh.nv == 1) return launch_frugal<1, false>(kp, out, seg, p->sm_count, s);
-        if (c.sh.nv == 2) return launch_frugal<2, false>(kp, out, seg, p->sm_count, s);
-        return launch_frugal<4, false>(kp, out, seg, p->sm_count, s);
+        if (c.sh.nv == 1) return launch_frugal<1, false>(kp, out, seg, p->sm_count, on.s);
+        if (c.sh.nv == 2) return launch_frugal<2, false>(kp, out, seg, p->sm_count, on.s);
+        return launch_frugal<4, false>(kp, out, seg, p->sm_count, on.s);
     }
-    if (c.tma) return launch_tma<256, 16, 2, 7>(kp, p->sm_count, s);
+    if (c.tma) return launch_tma<256, 16, 2, 7>(kp, p->sm_count, on.s);
     if (c.chunked)
-        return c.ragged ? launch_chunks<true>(kp, p->n_blocks, p->sm_count, s)
-                        : launch_chunks<false>(kp, p->n_blocks, p->sm_count, s);
+        return c.ragged ? launch_chunks<true>(kp, p->n_blocks, p->sm_count, on)
+                        : launch_chunks<false>(kp, p->n_blocks, p->sm_count, on);
     if (c.sh.v4 && c.sh.nv == 1 && f <= 64 && mode != MODE_UPDATE_ONLY)
-        return c.ragged ? launch_narrow<true>(kp, c.one_round, p->n_blocks, p->sm_count, s) : launch_narrow<false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        return c.ragged ? launch_narrow<true>(kp, c.one_round, p->n_blocks, p->sm_count, on) : launch_narrow<false>(kp, c.one_round, p->n_blocks, p->sm_count, on);
     if (c.ragged) {
-        if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
-        if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
-        return launch_regs<4, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 1) return launch_regs<1, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, on);
+        if (c.sh.nv == 2) return launch_regs<2, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, on);
+        return launch_regs<4, true, true>(kp, c.one_round, p->n_blocks, p->sm_count, on);
     }
     if (c.sh.v4) {
-        if (c.sh.nv == 1) return launch_regs<1, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
-        if (c.sh.nv == 2) return launch_regs<2, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
-        return launch_regs<4, true>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+        if (c.sh.nv == 1) return launch_regs<1, true>(kp, c.one_round, p->n_blocks, p->sm_count, on);
+        if (c.sh.nv == 2) return launch_regs<2, true>(kp, c.one_round, p->n_blocks, p->sm_count, on);
+        return launch_regs<4, true>(kp, c.one_round, p->n_blocks, p->sm_count, on);
     }
-    if (c.sh.nv == 1) return launch_regs<1, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
-    if (c.sh.nv == 2) return launch_regs<2, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
-    return launch_regs<4, false>(kp, c.one_round, p->n_blocks, p->sm_count, s);
+    if (c.sh.nv == 1) return launch_regs<1, false>(kp, c.one_round, p->n_blocks, p->sm_count, on);
+    if (c.sh.nv == 2) return launch_regs<2, false>(kp, c.one_round, p->n_blocks, p->sm_count, on);
+    return launch_regs<4, false>(kp, c.one_round, p->n_blocks, p->sm_count, on);
 }
 
 bool has_room(const cbm_b200_plan* p, const LaunchCfg& c) {
@@ -2523,11 +2523,6 @@ int make_room(cbm_b200_plan* p, const LaunchCfg& c, cudaStream_t s) {
     int rc = grow(p, p->d_flags, p->flags_cap, c.need_flags, true, s);
     if (rc == CBM_B200_OK) rc = grow(p, p->d_scratch, p->scratch_cap, c.need_scratch, false, s);
     return rc ? rc : grow(p, p->d_pack, p->pack_cap, c.need_pack, false, s);
-}
-
-bool is_captured(cudaStream_t s) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    return cudaStreamIsCapturing(s, &capture) != cudaSuccess || capture != cudaStreamCaptureStatusNone;
 }
 
 int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* y, i64 ldy, i32 f,
@@ -2542,11 +2537,12 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
                          std::string(who) + ": plan was created without a multiplier");
     if (p->n_rows == 0) return CBM_B200_OK;
     DeviceGuard g(p->device);
+    const cbm::Stream on(s);
     LaunchCfg c;
     const DeviceSchedule* d = &p->schedule_for(mode, f);
     rc = plan_cfg(p, *d, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
     // With rows lifted out of the tree a product may have more sums to park: where they find no room, it goes by the tree.
-    if (d != &p->tree && (rc || (!has_room(p, c) && (is_captured(s) || make_room(p, c, s))))) {
+    if (d != &p->tree && (rc || (!has_room(p, c) && (on.captured || make_room(p, c, s))))) {
         (void)cudaGetLastError();
         d = &p->tree;
         rc = plan_cfg(p, *d, who, x, ldx, y, ldy, f, mode, !in_turn, in_turn, c);
@@ -2558,17 +2554,17 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
     }
     // A graph launches this very epoch each time: its flags are cleared as part of it, lest a row takes its parent's row or
     // parked sums of the launch before for this one's.
-    if (d->n_items > d->n_prefix && is_captured(s)) CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)c.need_flags * sizeof(i32), s));
+    if (on.captured && d->n_items > d->n_prefix) CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)c.need_flags * sizeof(i32), s));
     if (c.pack) {
         const i32 vecs = (f + 3) / 4;
         const i64 n_vec = (i64)p->n_labels * vecs;
-        cbm::launch_next(pack_rows_kernel, (unsigned)((n_vec + 255) / 256), 256, 0, s, x, ldx, p->d_pack, f, vecs, n_vec);
+        cbm::launch_next(pack_rows_kernel, (unsigned)((n_vec + 255) / 256), 256, 0, on, x, ldx, p->d_pack, f, vecs, n_vec);
         CBM_CUDA(cudaGetLastError());
         x = p->d_pack;
         ldx = 4 * (i64)vecs;
     }
     return launch_plan(p, *d, c, x, ldx, y, ldy, f, mode, use_scale, p->d_counter, p->d_flags, p->d_scratch,
-                       ++p->epoch, s, bc);
+                       ++p->epoch, on, bc);
 }
 
 }  // namespace

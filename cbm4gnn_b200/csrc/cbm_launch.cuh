@@ -20,14 +20,22 @@ namespace cbm {
 
 __device__ __forceinline__ void wait_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A stream, and whether what is issued to it is captured into a graph.
+struct Stream {
+    cudaStream_t s;
+    bool captured;
+    Stream(cudaStream_t stream) : s(stream) {
+        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+        const bool asked = cudaStreamIsCapturing(s, &capture) == cudaSuccess;
+        if (!asked) (void)cudaGetLastError();  // (a stream that another one's capture forbids to use: the launch says so)
+        captured = !asked || capture != cudaStreamCaptureStatusNone;
+    }
+};
+
 // Under stream capture the launch is a plain one: what a graph's branches and joins wait for stays whole kernels.
 // Errors are left for cudaGetLastError.
 template <class... P, class... A>
-void launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t s, const A&... args) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const bool asked = cudaStreamIsCapturing(s, &capture) == cudaSuccess;
-    if (!asked) (void)cudaGetLastError();  // (a stream that another one's capture forbids to use: the launch says so)
-    const bool plain = !asked || capture != cudaStreamCaptureStatusNone;
+void launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, const Stream& on, const A&... args) {
     cudaLaunchAttribute early = {};
     early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     early.val.programmaticStreamSerializationAllowed = 1;
@@ -35,9 +43,9 @@ void launch_next(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem,
     config.gridDim = grid;
     config.blockDim = dim3(threads);
     config.dynamicSmemBytes = smem;
-    config.stream = s;
+    config.stream = on.s;
     config.attrs = &early;
-    config.numAttrs = plain ? 0 : 1;
+    config.numAttrs = on.captured ? 0 : 1;
     (void)cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...);
 }
 
