@@ -21,7 +21,8 @@ using i64 = int64_t;
 
 // What a waiting row and a level of the tree cost beside the entries, in entries.  A wait is some trips to L2 (flag, parent
 // row, flag), each as long as a batch of fetches; a level about 1.2 us of the chain, in which the GPU gathers 20 000 to
-// 40 000 row pieces of 512 bytes.
+// 40 000 row pieces of 512 bytes.  For operands of up to 128 columns, that is; wider products choose between the two
+// schedules by their width (cbm_b200_plan::tree_pays).
 constexpr i64 WAIT_COST = 8, LEVEL_COST = 20000;
 constexpr i64 LONGEST = 1 << 20;  // lifted rows stay well below what a schedule can cut into segments
 
