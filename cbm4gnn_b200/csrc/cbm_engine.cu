@@ -1860,12 +1860,19 @@ int build_both(const Structure& st, const Rules& rules, Schedule& tree, Schedule
     cbm::Lifted lift;
     std::vector<i32> rank;
     const bool wide = st.crow[st.n] > 1000000;  // steps of milliseconds
+    // A thread begins on the first device: it goes to the caller's, which it leaves as the current one, so that no other
+    // GPU gets a context.
+    int current = -1;
+    if (rules.device >= 0 && cudaGetDevice(&current) != cudaSuccess) current = -1;
     run_both(
         wide,
         [&] {
             if (!st.csr) cbm::lift_rows(st.n, st.rows, st.parent, st.level, st.crow, st.col, st.val, lift);
         },
-        [&] { cluster_order(st, rules, rank); });
+        [&] {
+            if (current >= 0) cudaSetDevice(current);
+            cluster_order(st, rules, rank);
+        });
     if (lift.n_lifted == 0) return build_schedule(st, nullptr, rank, rules, tree);
     int rc = CBM_B200_OK, rc_lifted = CBM_B200_OK;
     run_both(
