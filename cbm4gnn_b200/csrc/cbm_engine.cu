@@ -1279,6 +1279,8 @@ struct cbm_b200_plan {
     i32* d_flags = nullptr;
     i64 flags_cap = 0;
     bool in_pool = false;  // counted among the plans that share the device's workspace pool
+    bool captured = false;       // a graph may hold the workspaces' addresses:
+    std::vector<void*> retired;  // those that larger ones have replaced since are kept for it
     u64* d_counter = nullptr;
     i32* d_status = nullptr;
     i32 epoch = 0;
@@ -1369,11 +1371,19 @@ void pool_leave(int device) {
 template <class T>
 int grow(cbm_b200_plan* p, T*& at, i64& cap, i64 need, bool zeroed, cudaStream_t s) {
     if (need <= cap) return CBM_B200_OK;
-    if (at) {  // a launch in flight may still read the old one, on whatever stream
-        CBM_CUDA(cudaDeviceSynchronize());
-        CBM_CUDA(cudaFreeAsync(at, s));
+    if (at && p->captured) {
+        try {
+            p->retired.push_back(at);
+        } catch (const std::bad_alloc&) {
+            return cbm::fail(CBM_B200_ERR_ALLOC, "out of host memory");
+        }
+    } else {
+        if (at) {  // a launch in flight may still read the old one, on whatever stream
+            CBM_CUDA(cudaDeviceSynchronize());
+            CBM_CUDA(cudaFreeAsync(at, s));
+        }
+        p->device_bytes -= cap * (i64)sizeof(T);
     }
-    p->device_bytes -= cap * (i64)sizeof(T);
     at = nullptr;
     cap = 0;
     void* fresh = nullptr;
@@ -1395,6 +1405,7 @@ extern "C" void cbm_b200_plan_destroy(cbm_b200_plan* p) {
         cudaDeviceSynchronize();
         for (void* at : {(void*)p->d_pack, (void*)p->d_flags, (void*)p->d_scratch})
             if (at) cudaFreeAsync(at, p->own_stream);
+        for (void* at : p->retired) cudaFreeAsync(at, p->own_stream);
         cudaStreamSynchronize(p->own_stream);
         pool_leave(p->device);
     }
@@ -2559,6 +2570,7 @@ int run_plan(cbm_b200_plan* p, const char* who, const float* x, i64 ldx, float* 
         CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)p->flags_cap * sizeof(i32), s));
         p->epoch = 0;
     }
+    p->captured = p->captured || on.captured;
     // A graph launches this very epoch each time: its flags are cleared as part of it, lest a row takes its parent's row or
     // parked sums of the launch before for this one's.
     if (on.captured && d->n_items > d->n_prefix) CBM_CUDA(cudaMemsetAsync(p->d_flags, 0, (size_t)c.need_flags * sizeof(i32), s));

@@ -157,3 +157,28 @@ def test_a_captured_product_waits_in_every_replay(entry, f):
             c.plan(0).status()
             assert torch.equal(got, y)
         torch.testing.assert_close(got.double(), x.double().cumsum(0), atol=1e-3, rtol=1e-4)  # (sums of up to 1 500)
+
+
+def test_a_captured_product_outlives_the_growth_of_its_workspaces():
+    """Wider products of the plan replace its flags, parked sums and the operand's aligned copy; a graph goes on with those it
+    was captured with."""
+    ei = with_self_loops(graphs.copy_model(3000, 0.95, 20, 77))
+    c = cbm_matrix(torch.from_numpy(ei).to(torch.int32), torch.ones(ei.shape[1]), alpha=4, normalized=True, build_device=0)
+    gen = torch.Generator(device="cuda").manual_seed(2)
+    x, y = torch.randn((2, c.num_rows, 301), generator=gen, device="cuda")  # (copied to aligned rows first)
+    c.omp_mkl_csr_fused_spmm_update(x, y)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        c.omp_mkl_csr_fused_spmm_update(x, y)
+    for f in (1001, 2003):
+        wide, out = torch.randn((2, c.num_rows, f), generator=gen, device="cuda")
+        c.omp_mkl_csr_fused_spmm_update(wide, out)
+        x.mul_(-0.5)
+        y.fill_(float("nan"))
+        graph.replay()
+        again = torch.empty_like(out)
+        c.omp_mkl_csr_fused_spmm_update(wide, again)
+        want = torch.empty_like(y)
+        c.omp_mkl_csr_fused_spmm_update(x, want)
+        c.plan(0).status()
+        assert torch.equal(y, want) and torch.equal(out, again)
